@@ -1,19 +1,25 @@
-// Grammar-mask token sampler on the GPU: one 1024-thread CTA per row.
+// Grammar-mask token sampler on the GPU: a cluster of eight 1024-thread CTAs per row.
 //
 // Same rule as the host oracle (csrc/core/sampler.cc): allow-mask -> temperature -> min_p -> top_k -> top_p ->
 // categorical draw with a SplitMix64 (seed, position) uniform; greedy when T < 1e-5 or top_k == 1 (strict whole-row
 // finiteness, lowest id wins ties).  Nothing is sorted.  The ranked order (scaled logit descending, id ascending) is
-// handled with 8-bit radix selections over an order-preserving integer key:
+// handled with selections, digit by digit, over an order-preserving integer key:
 //   * top-k   : select the k-th largest key by COUNT; ties at that key are admitted lowest id first
 //   * top-p   : select by MASS the key at which the cumulative weight reaches top_p * total
 //   * the draw: select by MASS the key at which the cumulative weight reaches u * nucleus mass, then the tie index
 // Weights exp(scaled - max) are accumulated as 2^-40 fixed point in 64-bit integers, so every sum is independent of
 // the order in which threads add and the result is bit-reproducible.  Without top_k / top_p the draw walks the
-// survivors in token order (per-thread segments and a block scan), as the oracle does.
+// survivors in token order (warps own consecutive tokens), as the oracle does.
 // Parity target in the reference: native/cuda/kernels/v41_sampling_gpu.cu:238,523,921,1046,1701 (K1 prepare,
 // K2 categorical, K3 top-k pivot, K4 membership / rank order, K5 nucleus) and v41_sampling_gpu.h:52-170.
+#include <cooperative_groups.h>
+
+#include <atomic>
+
 #include "ds41_api.h"
 #include "ds41_launch.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace ds41 {
 
@@ -51,95 +57,65 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
   return static_cast<float>(static_cast<uint32_t>(x >> 40)) * (1.0f / 16777216.0f);
 }
 
-// Walk the row with several independent 16-byte loads in flight per thread (one CTA owns a whole row, so the walk is
-// bound by load latency).  Every thread still sees its tokens in ascending order, and every lane of a warp calls
-// f(i, value, valid) together, so f may use warp collectives.
-template <class F>
-__device__ __forceinline__ void for_vocab4(const float* lg, int vocab, F f) {
-  const int lane = threadIdx.x & 31, wbase = threadIdx.x - lane, B = blockDim.x;
-  constexpr int U = 4;
-  if ((reinterpret_cast<uintptr_t>(lg) & 15) == 0) {
-    const int n4 = vocab >> 2;
-    const float4* lg4 = reinterpret_cast<const float4*>(lg);
-    for (int base = wbase; base < n4; base += U * B) {
-      float4 v[U];
-#pragma unroll
-      for (int j = 0; j < U; ++j) {
-        const int q = base + j * B + lane;
-        v[j] = q < n4 ? lg4[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int j = 0; j < U; ++j) {
-        if (base + j * B >= n4) break;
-        const int q = base + j * B + lane;
-        const bool ok = q < n4;
-        f(4 * q, v[j].x, ok);
-        f(4 * q + 1, v[j].y, ok);
-        f(4 * q + 2, v[j].z, ok);
-        f(4 * q + 3, v[j].w, ok);
-      }
-    }
-    if (wbase == 0 && 4 * n4 < vocab) {          // up to three trailing tokens, warp 0
-      const int i = 4 * n4 + lane;
-      f(i, i < vocab ? lg[i] : 0.f, i < vocab);
-    }
-    return;
-  }
-  for (int base = wbase; base < vocab; base += U * B) {
-    float v[U];
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-      const int i = base + j * B + lane;
-      v[j] = i < vocab ? lg[i] : 0.f;
-    }
-#pragma unroll
-    for (int j = 0; j < U; ++j) {
-      const int i = base + j * B + lane;
-      if (base + j * B < vocab) f(i, v[j], i < vocab);
-    }
-  }
-}
+// A row is shared by a cluster of eight CTAs.  One CTA per row walked 517 KB up to fifteen times from L2 with a fraction of one
+// SM's bandwidth: 780 us for sixteen rows of 129280 logits.  Now each CTA reads its eighth once, keeps the order keys of the
+// scaled logits in shared memory, and only histograms, sums and short lists travel, through distributed shared memory: 68 us for
+// the same rows.  Every CTA draws the same conclusions from the same integers, so there is no broadcast step and all control
+// flow is uniform in the cluster.  What is left is a chain of cluster barriers (2000 cycles each) and of passes over the keys
+// (5000 to 7000 cycles); the reads from memory are 2 % of it.
+constexpr int kSampleCluster = 8;
+constexpr int kSampleMaxSlice = 49152;     // keys per CTA that fit its shared memory; longer slices are read again from L2
 
-constexpr int kSampleListCap = 2048;   // survivors of a top-k cut are kept in shared memory up to this many
+struct SamplePart {                        // what one CTA found in its slice
+  float best;
+  int best_i;
+  unsigned int allowed, bad;
+};
+
+constexpr int kSampleList = 512;           // candidates that are gathered and compared one by one instead of histogrammed
+
+struct SampleMember {
+  uint32_t key, count;
+  unsigned long long mass;                 // by count: the count
+};
 
 struct SampleShared {
-  float list_val[kSampleListCap];       // raw logits of the tokens above the top-k cut key (any order)
-  int list_id[kSampleListCap];
-  int list_n;
-  unsigned int cnt[256];
-  unsigned long long mass[256];
-  unsigned long long scan[kSampleThreads];
-  unsigned long long total;
+  // histograms of the even and odd passes: the other one may still be read by peers.  A weight is counted in pieces of
+  // 14 bits, whose sums over a slice of up to 2^18 tokens fit 32 bits (64-bit additions in shared memory are compare-and-swap
+  // loops: 22 us a pass); longer slices take the first 512 words as 64-bit sums.
+  unsigned int cnt[2][256];
+  alignas(8) unsigned int mass[2][3][256];
+  unsigned int tot_cnt[256];
+  unsigned long long tot_mass[256];
+  SamplePart part[kSampleCluster];
+  unsigned long long slot[3][kSampleCluster];      // one exchange each
+  unsigned long long warp[kSampleThreads / 32];
+  SamplePart warp_part[kSampleThreads / 32];
+  unsigned long long total;                        // weight of a selection's candidates
   double remaining;
-  unsigned int digit, tie_count;
-  int flag, token;
-  float fmax;
-  int imax;
+  unsigned int digit, tie_count, best_key, n_above;
+  int token;
+  unsigned int own_n, far_n[kSampleCluster];
+  uint2 own_list[kSampleList];                     // {key, token} of this CTA's members
+  int n_list;                                      // members of the last selection that were gathered; -1: too many
+  int list_id[kSampleList + 1];
+  SampleMember list[kSampleList + 1];
 };
+constexpr int kSampleMostPieces = 1 << 18;         // 2^18 x 2^14 = 2^32
 
-// What a selection walks: the whole row, or (n_list >= 0) the compact list of the tokens above the top-k cut key.
-struct RowView {
-  const float* lg;
-  int vocab;
+// This CTA's part of the row: tokens [id0, id0 + n), as order keys; 0 = the token is not allowed (no finite value has key 0).
+struct SampleSlice {
+  const uint32_t* keys;      // in shared memory, or null: made again from the logits
+  const float* logits;
   const uint32_t* mask;
-  const float* list_val;
-  const int* list_id;
-  int n_list;
+  int id0, n;
+  float inv_t;
+  bool wide;                 // weights are summed in 64 bits: some slice of the row is longer than kSampleMostPieces
+  __device__ __forceinline__ uint32_t operator[](int i) const {
+    if (keys != nullptr) return keys[i];
+    return mask_allows(mask, id0 + i) ? order_key(__fmul_rn(logits[i], inv_t)) : 0u;
+  }
 };
-
-template <class F>
-__device__ __forceinline__ void for_view(const RowView& v, F f) {
-  if (v.n_list < 0) {
-    for_vocab4(v.lg, v.vocab, [&](int i, float x, bool valid) { f(i, x, valid && mask_allows(v.mask, i)); });
-    return;
-  }
-  const int lane = threadIdx.x & 31, wbase = threadIdx.x - lane;
-  for (int base = wbase; base < v.n_list; base += blockDim.x) {
-    const int j = base + lane;
-    const bool valid = j < v.n_list;
-    f(valid ? v.list_id[j] : 0, valid ? v.list_val[j] : 0.f, valid);
-  }
-}
 
 // The candidate set of a selection: allowed tokens with key > excl, plus `tie_mult` tokens of key `tie_key`
 // (the admitted part of a tie group cut by an earlier selection; tie_key <= excl whenever tie_mult > 0).
@@ -149,92 +125,248 @@ struct CandSet {
   unsigned long long tie_mult;
 };
 
-// Radix selection, high keys first.  by_mass: find the key at which the running weight reaches `target`; else the key
-// at which the running count reaches it.  On return sh.remaining is what the ties at the returned key must still
-// supply and sh.tie_count how many candidates carry that key.
-__device__ uint32_t radix_select(SampleShared& sh, const RowView& view, float inv_t, float max_scaled, CandSet set,
-                                 bool by_mass, double target) {
-  uint32_t prefix = 0, prefix_mask = 0;
-  if (threadIdx.x == 0) sh.remaining = target;
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int d = threadIdx.x; d < 256; d += blockDim.x) {
-      sh.cnt[d] = 0;
-      sh.mass[d] = 0;
-    }
-    __syncthreads();
-    // lanes of a warp that hit the same digit add once: logits of one row share their top key bytes, so unaggregated
-    // shared-memory atomics would serialise on a handful of counters.  Integer sums: the result does not depend on
-    // the grouping.
-    for_view(view, [&](int i, float v, bool valid) {
-      const float s = __fmul_rn(v, inv_t);
-      const uint32_t k = order_key(s);
-      const bool act = valid && k > set.excl && (k & prefix_mask) == prefix;
-      const uint32_t d = (k >> shift) & 255u;
-      const unsigned peers = __match_any_sync(0xffffffffu, act ? d : 256u);
-      if (act) {
-        const int leader = __ffs(peers) - 1;
-        const int lane = threadIdx.x & 31;
-        unsigned long long wsum = 0;
-        if (by_mass) {
-          const unsigned long long w = weight_fx(s, max_scaled);           // <= 2^40: two 20/21-bit halves
-          const unsigned lo = __reduce_add_sync(peers, static_cast<unsigned>(w & 0xFFFFFu));
-          const unsigned hi = __reduce_add_sync(peers, static_cast<unsigned>(w >> 20));
-          wsum = (static_cast<unsigned long long>(hi) << 20) + lo;
-        }
-        if (lane == leader) {
-          atomicAdd(&sh.cnt[d], static_cast<unsigned>(__popc(peers)));
-          if (by_mass) atomicAdd(&sh.mass[d], wsum);
-        }
-      }
-    });
-    if (threadIdx.x == 0 && set.tie_mult > 0 && (set.tie_key & prefix_mask) == prefix) {
-      const uint32_t d = (set.tie_key >> shift) & 255u;
-      atomicAdd(&sh.cnt[d], static_cast<unsigned int>(set.tie_mult));
-      if (by_mass) atomicAdd(&sh.mass[d], set.tie_mult * weight_fx(key_value(set.tie_key), max_scaled));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double acc = 0.0;
-      int pick = -1, lowest = -1;
-      for (int d = 255; d >= 0; --d) {
-        if (sh.cnt[d] == 0) continue;
-        lowest = d;
-        const double v = by_mass ? static_cast<double>(sh.mass[d]) : static_cast<double>(sh.cnt[d]);
-        if (acc + v >= sh.remaining) { pick = d; break; }
-        acc += v;
-      }
-      if (pick < 0) {           // rounding left the target just above the total: end on the lowest key present
-        pick = lowest < 0 ? 0 : lowest;
-        acc -= by_mass ? static_cast<double>(sh.mass[pick]) : static_cast<double>(sh.cnt[pick]);
-        if (acc < 0.0) acc = 0.0;
-      }
-      sh.remaining -= acc;
-      sh.digit = static_cast<unsigned int>(pick);
-      sh.tie_count = sh.cnt[pick];
-    }
-    __syncthreads();
-    prefix |= sh.digit << shift;
-    prefix_mask |= 255u << shift;
-    __syncthreads();
+// Sum over the cluster; `slot` is used once per launch, so no second barrier protects it.
+__device__ unsigned long long cluster_sum(SampleShared& sh, cg::cluster_group& cl, int slot, unsigned long long v) {
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  if ((threadIdx.x & 31) == 0) sh.warp[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    unsigned long long mine = sh.warp[threadIdx.x];
+    for (int off = 16; off > 0; off >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, off);
+    if (threadIdx.x < kSampleCluster) *cl.map_shared_rank(&sh.slot[slot][cl.block_rank()], threadIdx.x) = mine;
   }
-  return prefix;
+  cl.sync();
+  unsigned long long all = 0;
+  for (int c = 0; c < kSampleCluster; ++c) all += sh.slot[slot][c];
+  return all;
 }
 
-// Block-wide exclusive scan of one value per thread (Hillis-Steele in shared memory); returns the exclusive prefix and
-// leaves the grand total in sh.total.
-__device__ unsigned long long block_scan(SampleShared& sh, unsigned long long v) {
-  sh.scan[threadIdx.x] = v;
-  __syncthreads();
-  for (int off = 1; off < kSampleThreads; off <<= 1) {
-    const unsigned long long add = threadIdx.x >= off ? sh.scan[threadIdx.x - off] : 0ull;
-    __syncthreads();
-    sh.scan[threadIdx.x] += add;
-    __syncthreads();
+// Eighths below the maximum, highest first, the last bucket open: the first digit of a selection.  It spreads the tokens of a
+// row over the bins, where the top byte of a key (sign and exponent) put a row into half a dozen: the lanes of a warp then met
+// in the same counters and a pass took 40 us.
+__device__ __forceinline__ uint32_t bucket_of(uint32_t key, float max_scaled) {
+  const float d = (max_scaled - key_value(key)) * 8.0f;
+  return 255u - (d >= 255.0f ? 255u : static_cast<uint32_t>(d));
+}
+
+// Every CTA gathers the members of all slices that `is_member` names (fewer than kSampleList) and the tie group, if it takes part.
+template <class F>
+__device__ void gather_members(SampleShared& sh, cg::cluster_group& cl, const SampleSlice& row, float max_scaled,
+                               const CandSet& set, bool by_mass, bool tie, F is_member) {
+  const int tid = threadIdx.x;
+  for (int i = tid; i < row.n; i += kSampleThreads) {
+    const uint32_t k = row[i];
+    if (k > set.excl && is_member(k)) {
+      const unsigned at = atomicAdd(&sh.own_n, 1u);
+      if (at < kSampleList) sh.own_list[at] = make_uint2(k, static_cast<uint32_t>(row.id0 + i));
+    }
   }
-  const unsigned long long incl = sh.scan[threadIdx.x];
-  if (threadIdx.x == kSampleThreads - 1) sh.total = incl;
+  cl.sync();
+  if (tid < kSampleCluster) sh.far_n[tid] = *cl.map_shared_rank(&sh.own_n, tid);
   __syncthreads();
-  return incl - v;
+  constexpr int kPer = kSampleThreads / kSampleCluster;      // threads that read one peer's members
+  const int from = tid / kPer;
+  int before = 0, n = 0;
+#pragma unroll
+  for (int r = 0; r < kSampleCluster; ++r) {
+    before = r == from ? n : before;
+    n += static_cast<int>(sh.far_n[r]);
+  }
+  n = min(n, kSampleList);
+  for (int i = tid % kPer; i < static_cast<int>(sh.far_n[from]) && before + i < kSampleList; i += kPer) {
+    const uint2 m = *cl.map_shared_rank(&sh.own_list[i], from);
+    sh.list[before + i] = {m.x, 1u, by_mass ? weight_fx(key_value(m.x), max_scaled) : 1ull};
+    sh.list_id[before + i] = static_cast<int>(m.y);
+  }
+  if (tid == 0) {
+    if (tie)
+      sh.list[n] = {set.tie_key, static_cast<uint32_t>(set.tie_mult),
+                    set.tie_mult * (by_mass ? weight_fx(key_value(set.tie_key), max_scaled) : 1ull)};
+    sh.n_list = n;
+  }
+  __syncthreads();
+}
+
+// The highest key whose members and the ones above weigh at least the target (`frac` >= 0: that share of the list's weight),
+// each thread summing what lies above its own member.
+__device__ uint32_t solve_list(SampleShared& sh, bool tie, double target, double frac) {
+  const int tid = threadIdx.x, total = sh.n_list + (tie ? 1 : 0);
+  uint32_t key = 0, equal = 0, higher = 0, low = 0xFFFFFFFFu;
+  unsigned long long above = 0, same = 0, all = 0;
+  if (tid == 0) sh.best_key = 0;
+  __syncthreads();
+  if (tid < total) {
+    key = sh.list[tid].key;
+#pragma unroll 4
+    for (int j = 0; j < total; ++j) {
+      const SampleMember m = sh.list[j];
+      all += m.mass;
+      above += m.key > key ? m.mass : 0ull;
+      same += m.key == key ? m.mass : 0ull;
+      higher += m.key > key ? m.count : 0u;
+      equal += m.key == key ? m.count : 0u;
+      low = min(low, m.key);
+    }
+    if (frac >= 0.0) target = frac * static_cast<double>(all);
+    // rounding can leave the target just above the total: then the lowest key present is the one
+    if (static_cast<double>(above + same) >= target || key == low) atomicMax(&sh.best_key, key);
+  }
+  __syncthreads();
+  const uint32_t best = sh.best_key;
+  if (tid < total && key == best) {              // members of one key write the same
+    sh.remaining = target - static_cast<double>(above);
+    sh.tie_count = equal;
+    sh.n_above = higher;
+    if (frac >= 0.0) sh.total = all;
+  }
+  __syncthreads();
+  return best;
+}
+
+// Selection by five digits (the bucket, then the bytes of the key), high keys first.  by_mass: find the key at which the running weight reaches the target; else the key at
+// which the running count reaches it.  `frac` >= 0: the target is that share of the set's weight, which is left in sh.total.
+// On return sh.remaining is what the ties at the returned key must still supply and sh.tie_count how many candidates carry it.
+// `pass` counts the histograms of the launch.
+__device__ uint32_t radix_select(SampleShared& sh, cg::cluster_group& cl, const SampleSlice& row, float max_scaled, CandSet set,
+                                 bool by_mass, double target, double frac, int& pass) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  uint32_t prefix = 0, prefix_mask = 0, bucket = 0;
+  for (int shift = 32; shift >= 0; shift -= 8, ++pass) {
+    unsigned int* cnt = sh.cnt[pass & 1];
+    unsigned int(*mass)[256] = sh.mass[pass & 1];
+    const bool first = shift == 32;
+    if (tid < 256) cnt[tid] = mass[0][tid] = mass[1][tid] = mass[2][tid] = 0;
+    auto add_mass = [&](uint32_t d, unsigned long long w) {
+      if (row.wide) {
+        atomicAdd(reinterpret_cast<unsigned long long*>(mass[0]) + d, w);
+        return;
+      }
+      constexpr unsigned kPiece = (1u << 14) - 1;
+      const unsigned a = static_cast<unsigned>(w) & kPiece, b = static_cast<unsigned>(w >> 14) & kPiece;
+      const unsigned c = static_cast<unsigned>(w >> 28);
+      if (a != 0) atomicAdd(&mass[0][d], a);
+      if (b != 0) atomicAdd(&mass[1][d], b);
+      if (c != 0) atomicAdd(&mass[2][d], c);
+    };
+    __syncthreads();
+    auto member = [&](uint32_t k) { return first || (bucket_of(k, max_scaled) == bucket && (k & prefix_mask) == prefix); };
+    auto digit = [&](uint32_t k) { return first ? bucket_of(k, max_scaled) : (k >> shift) & 255u; };
+    // Integer sums: the result does not depend on the order or the grouping of the additions.  After the first digit lanes of
+    // a warp that hit the same one add once, since the tokens that are left share their top bytes.
+    for (int base = 0; base < row.n; base += kSampleThreads) {
+      const uint32_t k = base + tid < row.n ? row[base + tid] : 0u;
+      const bool act = k > set.excl && member(k);
+      if (!__any_sync(0xffffffffu, act)) continue;
+      if (first) {
+        if (act) {
+          const uint32_t d = digit(k);
+          atomicAdd(&cnt[d], 1u);
+          if (by_mass) add_mass(d, weight_fx(key_value(k), max_scaled));
+        }
+        continue;
+      }
+      const uint32_t d = digit(k);
+      const unsigned peers = __match_any_sync(0xffffffffu, act ? d : 256u);
+      if (act) {
+        if (by_mass) add_mass(d, weight_fx(key_value(k), max_scaled));
+        if (lane == __ffs(peers) - 1) atomicAdd(&cnt[d], static_cast<unsigned>(__popc(peers)));
+      }
+    }
+    if (cl.block_rank() == 0 && tid == 0 && set.tie_mult > 0 && member(set.tie_key)) {
+      const uint32_t d = digit(set.tie_key);
+      atomicAdd(&cnt[d], static_cast<unsigned int>(set.tie_mult));
+    }
+    cl.sync();
+    if (tid < 256) {
+      unsigned int c = 0;
+      unsigned long long m = 0;
+#pragma unroll
+      for (int r = 0; r < kSampleCluster; ++r) {
+        c += *cl.map_shared_rank(&cnt[tid], r);
+        if (by_mass && row.wide)
+          m += *cl.map_shared_rank(reinterpret_cast<unsigned long long*>(mass[0]) + tid, r);
+        else if (by_mass)
+          m += *cl.map_shared_rank(&mass[0][tid], r) + (static_cast<unsigned long long>(*cl.map_shared_rank(&mass[1][tid], r)) << 14) +
+               (static_cast<unsigned long long>(*cl.map_shared_rank(&mass[2][tid], r)) << 28);
+      }
+      if (by_mass && set.tie_mult > 0 && member(set.tie_key) && digit(set.tie_key) == static_cast<uint32_t>(tid))
+        m += set.tie_mult * weight_fx(key_value(set.tie_key), max_scaled);
+      sh.tot_cnt[tid] = c;
+      sh.tot_mass[tid] = by_mass ? m : c;
+    }
+    if (tid == 0) {
+      sh.own_n = 0;
+      sh.n_list = -1;
+    }
+    __syncthreads();
+    if (tid < 32) {
+      // eight bins per lane from the highest down: the first bin in use whose running sum reaches the target
+      unsigned long long sum = 0;
+      unsigned members = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        sum += sh.tot_mass[255 - 8 * lane - j];
+        members += sh.tot_cnt[255 - 8 * lane - j];
+      }
+      const bool used = members != 0;
+      unsigned long long incl = sum;
+      unsigned higher = members;
+      for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, off);
+        const unsigned more = __shfl_up_sync(0xffffffffu, higher, off);
+        if (lane >= off) {
+          incl += up;
+          higher += more;
+        }
+      }
+      higher -= members;
+      const unsigned long long all = __shfl_sync(0xffffffffu, incl, 31);
+      if (first && frac >= 0.0) target = frac * static_cast<double>(all);
+      const unsigned reach = __ballot_sync(0xffffffffu, used && static_cast<double>(incl) >= target);
+      const unsigned any = __ballot_sync(0xffffffffu, used);
+      // rounding can leave the target just above the total: then the selection ends on the lowest key present
+      const int owner = reach != 0 ? __ffs(reach) - 1 : (any != 0 ? 31 - __clz(any) : 0);
+      if (lane == owner) {
+        unsigned long long acc = incl - sum, at = acc;
+        int pick = -1;
+        for (int j = 0; j < 8; ++j) {
+          const int d = 255 - 8 * lane - j;
+          if (sh.tot_cnt[d] == 0) continue;
+          if (pick >= 0) higher += sh.tot_cnt[pick];
+          pick = d;
+          at = acc;
+          acc += sh.tot_mass[d];
+          if (reach != 0 && static_cast<double>(acc) >= target) break;
+        }
+        if (pick < 0) pick = 0;
+        sh.remaining = target - static_cast<double>(at);
+        sh.digit = static_cast<unsigned int>(pick);
+        sh.tie_count = sh.tot_cnt[pick];
+        sh.n_above = first ? higher : sh.n_above + higher;
+        if (first) sh.total = all;
+      }
+    }
+    __syncthreads();
+    target = sh.remaining;
+    if (first) {
+      bucket = sh.digit;
+      if (sh.tie_count < kSampleList) {
+        ++pass;
+        const bool tie = set.tie_mult > 0 && member(set.tie_key) && bucket_of(set.tie_key, max_scaled) == bucket;
+        const unsigned above = sh.n_above;
+        gather_members(sh, cl, row, max_scaled, set, by_mass, tie,
+                       [&](uint32_t k) { return bucket_of(k, max_scaled) == bucket; });
+        const uint32_t key = solve_list(sh, tie, target, -1.0);
+        if (tid == 0) sh.n_above += above;
+        __syncthreads();
+        return key;
+      }
+    } else {
+      prefix |= sh.digit << shift;
+      prefix_mask |= 255u << shift;
+    }
+  }
+  return prefix;
 }
 
 __global__ void __launch_bounds__(kSampleThreads)
@@ -242,76 +374,108 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
                    int mask_words, const ds41_sample_row* __restrict__ rows, int* __restrict__ tokens,
                    int* __restrict__ status) {
   __shared__ SampleShared sh;
+  extern __shared__ uint32_t key_store[];
   pdl_launch_dependents();
   pdl_wait();
-  const int row = blockIdx.x;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = static_cast<int>(cl.block_rank()), row = blockIdx.x / kSampleCluster;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const ds41_sample_row p = rows[row];
-  const float* lg = logits + 1ll * row * ld;
   const uint32_t* mask = (masks != nullptr && p.mask_row >= 0) ? masks + 1ll * p.mask_row * mask_words : nullptr;
-  const int tid = threadIdx.x;
+  // every return below is taken by the whole cluster at once, and after the last look into a peer's memory
   auto finish = [&](int st, int tok) {
-    if (tid == 0) {
+    cl.sync();
+    if (rank == 0 && tid == 0) {
       status[row] = st;
       if (st == kSampleOk) tokens[row] = tok;
     }
   };
   if (!(p.temperature >= 0.0f) || isinf(p.temperature)) return finish(kSampleBadTemperature, 0);
   if (!(p.top_p > 0.0f) || !(p.min_p >= 0.0f) || p.min_p > 1.0f) return finish(kSampleBadParameter, 0);
-  if (tid == 0) { sh.flag = 0; sh.fmax = -INFINITY; sh.imax = -1; }
-  __syncthreads();
   const bool greedy = p.temperature < 1e-5f || p.top_k == 1;
   const float inv_t = greedy ? 1.0f : 1.0f / p.temperature;
 
-  // ---- prepare: finiteness, allowed count, maximum (greedy: arg max with the lowest id on ties)
-  float best = -INFINITY;
-  int best_i = -1, n_allowed = 0, bad = 0;
-  for_vocab4(lg, vocab, [&](int i, float v, bool valid) {
-    if (!valid) return;
-    const bool ok = mask_allows(mask, i);
-    if (greedy) {
-      if (!isfinite(v)) bad = 1;
-    } else if (ok && (isnan(v) || v == INFINITY)) {
-      bad = 1;
-    }
-    if (!ok) return;
-    ++n_allowed;
+  // ---- the slice: order keys, finiteness, allowed count, maximum (greedy: arg max with the lowest id on ties)
+  const int slice = ((vocab + kSampleCluster - 1) / kSampleCluster + 31) & ~31;
+  SampleSlice own;
+  own.id0 = min(vocab, rank * slice);
+  own.n = min(vocab, own.id0 + slice) - own.id0;
+  own.logits = logits + 1ll * row * ld + own.id0;
+  own.mask = mask;
+  own.inv_t = inv_t;
+  own.keys = slice <= kSampleMaxSlice ? key_store : nullptr;
+  own.wide = slice > kSampleMostPieces;
+  SamplePart mine{-INFINITY, -1, 0u, 0u};
+  auto take = [&](int i, float v) {
+    const bool ok = mask_allows(mask, own.id0 + i);
+    if (greedy ? !isfinite(v) : ok && (isnan(v) || v == INFINITY)) mine.bad = 1u;
     const float s = __fmul_rn(v, inv_t);
-    if (best_i < 0 || s > best) { best = s; best_i = i; }      // ascending i per thread: first maximum kept
-  });
-  for (int off = 16; off > 0; off >>= 1) {
-    const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-    const int oi = __shfl_xor_sync(0xffffffffu, best_i, off);
-    n_allowed += __shfl_xor_sync(0xffffffffu, n_allowed, off);
-    bad |= __shfl_xor_sync(0xffffffffu, bad, off);
-    if (oi >= 0 && (best_i < 0 || ob > best || (ob == best && oi < best_i))) { best = ob; best_i = oi; }
-  }
-  if ((tid & 31) == 0) {
-    sh.scan[tid >> 5] = (static_cast<unsigned long long>(__float_as_uint(best)) << 32) | static_cast<uint32_t>(best_i);
-    sh.cnt[tid >> 5] = static_cast<unsigned int>(n_allowed);
-    if (bad) atomicOr(&sh.flag, 1);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    float b = -INFINITY;
-    int bi = -1;
-    unsigned int n = 0;
-    for (int w = 0; w < kSampleThreads / 32; ++w) {
-      const float ob = __uint_as_float(static_cast<uint32_t>(sh.scan[w] >> 32));
-      const int oi = static_cast<int>(static_cast<uint32_t>(sh.scan[w]));
-      n += sh.cnt[w];
-      if (oi >= 0 && (bi < 0 || ob > b || (ob == b && oi < bi))) { b = ob; bi = oi; }
+    if (ok) {
+      ++mine.allowed;
+      if (mine.best_i < 0 || s > mine.best) { mine.best = s; mine.best_i = own.id0 + i; }    // ascending: first maximum kept
     }
-    sh.fmax = b;
-    sh.imax = bi;
-    sh.tie_count = n;
+    if (own.keys != nullptr) key_store[i] = ok ? order_key(s) : 0u;
+  };
+  int done = 0;
+  if ((reinterpret_cast<uintptr_t>(own.logits) & 15) == 0) {
+    const int n4 = own.n >> 2;
+    const float4* src = reinterpret_cast<const float4*>(own.logits);
+    for (int base = 0; base < n4; base += 4 * kSampleThreads) {
+      float4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int q = base + j * kSampleThreads + tid;
+        if (q < n4) v[j] = src[q];
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int q = base + j * kSampleThreads + tid;
+        if (q < n4) {
+          take(4 * q, v[j].x);
+          take(4 * q + 1, v[j].y);
+          take(4 * q + 2, v[j].z);
+          take(4 * q + 3, v[j].w);
+        }
+      }
+    }
+    done = 4 * n4;
   }
+  for (int i = done + tid; i < own.n; i += kSampleThreads) take(i, own.logits[i]);
+  auto merge = [](SamplePart& a, const SamplePart& b) {
+    a.allowed += b.allowed;
+    a.bad |= b.bad;
+    if (b.best_i >= 0 && (a.best_i < 0 || b.best > a.best || (b.best == a.best && b.best_i < a.best_i))) {
+      a.best = b.best;
+      a.best_i = b.best_i;
+    }
+  };
+  auto merge_warp = [&](SamplePart& a) {
+    for (int off = 16; off > 0; off >>= 1) {
+      SamplePart o;
+      o.best = __shfl_xor_sync(0xffffffffu, a.best, off);
+      o.best_i = __shfl_xor_sync(0xffffffffu, a.best_i, off);
+      o.allowed = __shfl_xor_sync(0xffffffffu, a.allowed, off);
+      o.bad = __shfl_xor_sync(0xffffffffu, a.bad, off);
+      merge(a, o);
+    }
+  };
+  static_assert(kSampleThreads == 1024, "one warp merges the warps");
+  merge_warp(mine);
+  if (lane == 0) sh.warp_part[warp] = mine;
   __syncthreads();
-  if (sh.flag) return finish(kSampleNonFinite, 0);
-  if (sh.imax < 0 || sh.tie_count == 0) return finish(kSampleEmpty, 0);
-  if (greedy) return finish(kSampleOk, sh.imax);
-  const float max_scaled = sh.fmax;
+  if (warp == 0) {
+    mine = sh.warp_part[lane];
+    merge_warp(mine);
+    if (lane < kSampleCluster) *cl.map_shared_rank(&sh.part[rank], lane) = mine;
+  }
+  cl.sync();
+  SamplePart all = sh.part[0];
+  for (int c = 1; c < kSampleCluster; ++c) merge(all, sh.part[c]);
+  if (all.bad != 0u) return finish(kSampleNonFinite, 0);
+  if (all.best_i < 0 || all.allowed == 0) return finish(kSampleEmpty, 0);
+  if (greedy) return finish(kSampleOk, all.best_i);
+  const float max_scaled = all.best;
   if (!isfinite(max_scaled)) return finish(kSampleEmpty, 0);
-  __syncthreads();
 
   const float u = fminf(fmaxf(uniform01(p.seed, p.position), 0.0f), 0.99999994f);
   const float min_scaled = p.min_p > 0.0f ? max_scaled + logf(p.min_p) : -INFINITY;
@@ -320,160 +484,158 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   const bool filtered = p.top_k > 0 || p.top_p < 1.0f;
 
   if (!filtered) {
-    // ---- categorical over the survivors in token order
-    const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
-    const int i0 = min(vocab, tid * seg), i1 = min(vocab, i0 + seg);
-    unsigned long long mine = 0;
-    for (int i = i0; i < i1; ++i) {
-      if (!mask_allows(mask, i)) continue;
-      const float s = __fmul_rn(lg[i], inv_t);
-      if (order_key(s) > excl0) mine += weight_fx(s, max_scaled);
-    }
-    const unsigned long long before = block_scan(sh, mine);
-    const double target = static_cast<double>(u) * static_cast<double>(sh.total);
+    // ---- categorical over the survivors in token order: a warp owns consecutive tokens, 32 at a time
+    const int per_warp = ((own.n + kSampleThreads / 32 - 1) / (kSampleThreads / 32) + 31) & ~31;
+    const int w0 = min(own.n, warp * per_warp), w1 = min(own.n, w0 + per_warp);
+    auto weight = [&](int i) -> unsigned long long {
+      const uint32_t k = i < w1 ? own[i] : 0u;
+      return k > excl0 ? weight_fx(key_value(k), max_scaled) : 0ull;
+    };
+    unsigned long long sum = 0;
+    for (int i = w0 + lane; i < w1; i += 32) sum += weight(i);
+    const unsigned long long total = cluster_sum(sh, cl, 0, sum);
+    const double target = static_cast<double>(u) * static_cast<double>(total);
+    unsigned long long before = 0;
+    for (int c = 0; c < rank; ++c) before += sh.slot[0][c];
+    for (int w = 0; w < warp; ++w) before += sh.warp[w];
+    const unsigned long long in_warp = sh.warp[warp];
     if (tid == 0) sh.token = -1;
     __syncthreads();
-    // the first thread whose inclusive sum reaches the target owns the draw
-    if (mine > 0 && static_cast<double>(before + mine) >= target &&
-        (static_cast<double>(before) < target || before == 0)) {
-      unsigned long long run = before;
-      for (int i = i0; i < i1; ++i) {
-        if (!mask_allows(mask, i)) continue;
-        const float s = __fmul_rn(lg[i], inv_t);
-        if (order_key(s) <= excl0) continue;
-        run += weight_fx(s, max_scaled);
-        if (static_cast<double>(run) >= target && run > 0) { atomicCAS(&sh.token, -1, i); break; }
+    // the first warp whose running sum reaches the target owns the draw
+    if (in_warp > 0 && static_cast<double>(before + in_warp) >= target && (static_cast<double>(before) < target || before == 0)) {
+      for (int i0 = w0; i0 < w1; i0 += 32) {
+        unsigned long long incl = weight(i0 + lane);
+        for (int off = 1; off < 32; off <<= 1) {
+          const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, off);
+          if (lane >= off) incl += up;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, before + incl > 0 && static_cast<double>(before + incl) >= target);
+        if (hit != 0) {
+          if (lane == 0) sh.token = own.id0 + i0 + __ffs(hit) - 1;
+          break;
+        }
+        before += __shfl_sync(0xffffffffu, incl, 31);
       }
     }
     __syncthreads();
-    if (sh.token < 0) {
-      // rounding: nothing reached the target - the last survivor wins
-      int last = -1;
-      for (int i = i1 - 1; i >= i0; --i) {
-        if (mask_allows(mask, i) && order_key(__fmul_rn(lg[i], inv_t)) > excl0) { last = i; break; }
-      }
-      if (last >= 0) atomicMax(&sh.token, last);
-      __syncthreads();
-    }
-    return finish(sh.token >= 0 ? kSampleOk : kSampleEmpty, sh.token);
+    // at most one CTA drew; where rounding left the target above every sum, the last survivor wins
+    int last = sh.token;
+    const int drawn = static_cast<int>(cluster_sum(sh, cl, 1, tid == 0 && last >= 0 ? 1ull + last : 0ull)) - 1;
+    if (drawn >= 0) return finish(kSampleOk, drawn);
+    last = -1;
+    for (int i = tid; i < own.n; i += kSampleThreads)
+      if (own[i] > excl0) last = max(last, i);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) atomicMax(&sh.token, last);
+    __syncthreads();
+    if (tid < kSampleCluster)
+      *cl.map_shared_rank(&sh.slot[2][rank], tid) = sh.token >= 0 ? 1ull + own.id0 + sh.token : 0ull;
+    cl.sync();
+    unsigned long long top = 0;
+    for (int c = 0; c < kSampleCluster; ++c) top = max(top, sh.slot[2][c]);
+    return finish(top > 0 ? kSampleOk : kSampleEmpty, static_cast<int>(top) - 1);
   }
 
   // ---- ranked path
   CandSet set{excl0, 0u, 0ull};
-  RowView view{lg, vocab, mask, sh.list_val, sh.list_id, -1};
-  // survivor count
-  int mine_n = 0;
-  for_view(view, [&](int i, float v, bool valid) {
-    if (valid && order_key(__fmul_rn(v, inv_t)) > excl0) ++mine_n;
-  });
-  block_scan(sh, static_cast<unsigned long long>(mine_n));
-  const unsigned long long survivors = sh.total;
-  __syncthreads();
-  if (survivors == 0) return finish(kSampleEmpty, 0);
-  uint32_t list_key = 0xFFFFFFFFu;      // keys above this one live in the compact list (when view.n_list >= 0)
-  if (p.top_k > 0 && static_cast<unsigned long long>(p.top_k) < survivors) {
-    const uint32_t pk = radix_select(sh, view, inv_t, max_scaled, set, false, static_cast<double>(p.top_k));
-    const double need = sh.remaining;
-    const unsigned long long ties = sh.tie_count;
+  int pass = 0;
+  // Once few candidates are left they are gathered, and what is still to be selected among them takes no more passes.
+  bool gathered = false;
+  auto gather_all = [&]() {
+    const unsigned left = sh.n_above;              // candidates above the key just selected, without the tie group
     __syncthreads();
+    if (left >= kSampleList) return;
+    cl.sync();                                     // peers are done with this CTA's former members
+    if (tid == 0) sh.own_n = 0;
+    __syncthreads();
+    gather_members(sh, cl, own, max_scaled, set, true, true, [](uint32_t) { return true; });
+    gathered = true;
+  };
+  auto select = [&](double target, double frac) {
+    return gathered ? solve_list(sh, true, target, frac) : radix_select(sh, cl, own, max_scaled, set, true, target, frac, pass);
+  };
+  unsigned long long survivors = all.allowed;
+  if (p.min_p > 0.0f) {
+    unsigned long long n = 0;
+    for (int i = tid; i < own.n; i += kSampleThreads) n += own[i] > excl0 ? 1 : 0;
+    survivors = cluster_sum(sh, cl, 0, n);
+  }
+  if (survivors == 0) return finish(kSampleEmpty, 0);
+  if (p.top_k > 0 && static_cast<unsigned long long>(p.top_k) < survivors) {
+    const uint32_t pk = radix_select(sh, cl, own, max_scaled, set, false, static_cast<double>(p.top_k), -1.0, pass);
     set.excl = pk;
     set.tie_key = pk;
-    set.tie_mult = static_cast<unsigned long long>(fmin(fmax(need, 1.0), static_cast<double>(ties)));
-    if (p.top_k <= kSampleListCap) {
-      // fewer than top_k tokens lie above the cut key: gather them once; every later selection walks this list
-      // instead of the row (the admitted ties of the cut key stay described by set.tie_key / set.tie_mult)
-      if (tid == 0) sh.list_n = 0;
-      __syncthreads();
-      for_view(view, [&](int i, float v, bool valid) {
-        const bool keep = valid && order_key(__fmul_rn(v, inv_t)) > pk;
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (m == 0) return;
-        const int lane = threadIdx.x & 31;
-        int at = 0;
-        if (lane == __ffs(m) - 1) at = atomicAdd(&sh.list_n, __popc(m));
-        at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
-        if (keep && at < kSampleListCap) {
-          sh.list_val[at] = v;
-          sh.list_id[at] = i;
-        }
-      });
-      __syncthreads();
-      if (sh.list_n <= kSampleListCap) {
-        view.n_list = sh.list_n;
-        list_key = pk;
-      }
-    }
+    set.tie_mult = static_cast<unsigned long long>(fmin(fmax(sh.remaining, 1.0), static_cast<double>(sh.tie_count)));
+    gather_all();
   }
-  // total weight of the kept set
-  unsigned long long mine_w = 0;
-  for_view(view, [&](int i, float v, bool valid) {
-    if (!valid) return;
-    const float s = __fmul_rn(v, inv_t);
-    if (order_key(s) > set.excl) mine_w += weight_fx(s, max_scaled);
-  });
-  block_scan(sh, mine_w);
-  unsigned long long total = sh.total + set.tie_mult * (set.tie_mult ? weight_fx(key_value(set.tie_key), max_scaled) : 0ull);
-  __syncthreads();
-  double mass = static_cast<double>(total);
+  double draw_of = -1.0, draw_frac = static_cast<double>(u);
   if (p.top_p < 1.0f) {
-    const double target = static_cast<double>(p.top_p) * mass;
-    const uint32_t pp = radix_select(sh, view, inv_t, max_scaled, set, true, target);
+    const uint32_t pp = select(0.0, static_cast<double>(p.top_p));
+    const double target = static_cast<double>(p.top_p) * static_cast<double>(sh.total);
     const double need = sh.remaining;
     const unsigned long long ties = sh.tie_count;
-    __syncthreads();
     const double w = static_cast<double>(weight_fx(key_value(pp), max_scaled));
     unsigned long long take = w > 0.0 ? static_cast<unsigned long long>(ceil(need / w)) : ties;
     if (take < 1) take = 1;
     if (take > ties) take = ties;
-    mass = (target - need) + static_cast<double>(take) * w;
+    draw_of = static_cast<double>(u) * ((target - need) + static_cast<double>(take) * w);
+    draw_frac = -1.0;
     set.excl = pp;
     set.tie_key = pp;
     set.tie_mult = take;
+    gather_all();
   }
   // ---- the draw
-  const double target = static_cast<double>(u) * mass;
-  const uint32_t dk = radix_select(sh, view, inv_t, max_scaled, set, true, target);
+  const uint32_t dk = select(draw_of, draw_frac);
   const double need = sh.remaining;
   const unsigned long long ties = sh.tie_count;
-  __syncthreads();
   const double w = static_cast<double>(weight_fx(key_value(dk), max_scaled));
   long long tie_index = w > 0.0 ? static_cast<long long>(ceil(need / w)) - 1 : 0;
   if (tie_index < 0) tie_index = 0;
   if (tie_index > static_cast<long long>(ties) - 1) tie_index = static_cast<long long>(ties) - 1;
-  // the tie_index-th allowed token with key == dk in id order
-  if (view.n_list >= 0 && dk > list_key) {
-    // all tokens of that key are in the list: the one with exactly tie_index smaller ids among them
-    if (tid == 0) sh.token = -1;
-    __syncthreads();
-    for (int j = tid; j < view.n_list; j += blockDim.x) {
-      if (order_key(__fmul_rn(sh.list_val[j], inv_t)) != dk) continue;
-      long long rank = 0;
-      for (int q = 0; q < view.n_list; ++q)
-        if (sh.list_id[q] < sh.list_id[j] && order_key(__fmul_rn(sh.list_val[q], inv_t)) == dk) ++rank;
-      if (rank == tie_index) sh.token = sh.list_id[j];
-    }
-    __syncthreads();
-    return finish(sh.token >= 0 ? kSampleOk : kSampleInternal, sh.token);
-  }
-  const int seg = (vocab + kSampleThreads - 1) / kSampleThreads;
-  const int i0 = min(vocab, tid * seg), i1 = min(vocab, i0 + seg);
-  unsigned long long eq = 0;
-  for (int i = i0; i < i1; ++i)
-    if (mask_allows(mask, i) && order_key(__fmul_rn(lg[i], inv_t)) == dk) ++eq;
-  const unsigned long long before = block_scan(sh, eq);
-  if (tid == 0) sh.token = -1;
-  __syncthreads();
-  if (eq > 0 && static_cast<long long>(before) <= tie_index && tie_index < static_cast<long long>(before + eq)) {
-    long long seen = static_cast<long long>(before);
-    for (int i = i0; i < i1; ++i) {
-      if (mask_allows(mask, i) && order_key(__fmul_rn(lg[i], inv_t)) == dk) {
-        if (seen == tie_index) { sh.token = i; break; }
-        ++seen;
+  if (sh.n_list >= 0 && !(set.tie_mult > 0 && dk == set.tie_key)) {
+    // every token of that key is in the list: the one with exactly tie_index smaller ids among them
+    if (tid < sh.n_list && sh.list[tid].key == dk) {
+      int before = 0;
+      for (int j = 0; j < sh.n_list; ++j) before += sh.list[j].key == dk && sh.list_id[j] < sh.list_id[tid] ? 1 : 0;
+      if (before == tie_index && rank == 0) {
+        status[row] = kSampleOk;
+        tokens[row] = sh.list_id[tid];
       }
     }
+    cl.sync();                                     // peers may still gather from this CTA
+    return;
   }
-  __syncthreads();
-  finish(sh.token >= 0 ? kSampleOk : kSampleInternal, sh.token);
+  // the tie_index-th allowed token with key == dk in id order: the CTA that holds it, then its first warp, 32 tokens at a time
+  unsigned long long eq = 0;
+  for (int i = tid; i < own.n; i += kSampleThreads) eq += own[i] == dk ? 1 : 0;
+  cluster_sum(sh, cl, 1, eq);
+  long long before = 0;
+  int holder = -1;
+  for (int c = 0; c < kSampleCluster; ++c) {
+    const long long here = static_cast<long long>(sh.slot[1][c]);
+    if (holder < 0 && tie_index < before + here) holder = c;
+    if (holder < 0) before += here;
+  }
+  if (holder < 0) return finish(kSampleInternal, 0);
+  if (rank == holder && warp == 0) {
+    int rest = static_cast<int>(tie_index - before);
+    for (int i0 = 0; i0 < own.n; i0 += 32) {
+      unsigned hit = __ballot_sync(0xffffffffu, i0 + lane < own.n && own[i0 + lane] == dk);
+      const int n = __popc(hit);
+      if (rest >= n) {
+        rest -= n;
+        continue;
+      }
+      for (; rest > 0; --rest) hit &= hit - 1;
+      if (lane == 0) {
+        status[row] = kSampleOk;
+        tokens[row] = own.id0 + i0 + __ffs(hit) - 1;
+      }
+      break;
+    }
+  }
+  cl.sync();
 }
 
 }  // namespace ds41
@@ -485,6 +647,16 @@ extern "C" int ds41_sample_rows(const float* logits, long long ld, int rows, int
   if (logits == nullptr || params == nullptr || tokens == nullptr || status == nullptr || rows <= 0 || vocab <= 0)
     return cudaErrorInvalidValue;
   if (masks != nullptr && mask_words != (vocab + 31) / 32) return cudaErrorInvalidValue;
-  return launch_pdl(sample_rows_kernel, dim3(rows), dim3(kSampleThreads), 0, static_cast<cudaStream_t>(stream), logits,
-                    ld, vocab, masks, mask_words, params, tokens, status);
+  const int slice = ((vocab + kSampleCluster - 1) / kSampleCluster + 31) & ~31;
+  const size_t smem = slice <= kSampleMaxSlice ? 4ull * slice : 0;
+  static std::atomic<bool> configured[64];
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !configured[dev].load(std::memory_order_acquire)) {
+    const cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kSampleMaxSlice);
+    if (e != cudaSuccess) return e;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  return launch_pdl_cluster(sample_rows_kernel, dim3(rows * kSampleCluster), dim3(kSampleThreads), kSampleCluster, smem,
+                            static_cast<cudaStream_t>(stream), logits, ld, vocab, masks, mask_words, params, tokens, status);
 }

@@ -137,3 +137,30 @@ def test_sampler_adversarial_rows_match_host_oracle():
         if (st[r] == 0) != (err == 0) or (err == 0 and tok[r] != want):
             bad.append((r, int(st[r]), int(tok[r]), want, err))
     assert not bad, bad[:8]
+
+
+@pytest.mark.parametrize("vocab,offset", [(3, 0), (31, 1), (257, 3), (8 * 32 + 1, 0), (20011, 1), (8 * 49152 + 5, 0),
+                                          ((8 << 18) + 3, 0)])
+def test_sampler_slices_of_a_row(vocab, offset):
+    """Where a row's eight slices are empty, short, unaligned or longer than a CTA's shared memory.  The draw takes integer
+    weights, so only one that lands on a cumulative boundary of the oracle's float sums may differ."""
+    from ds41rt_b200.ops.sampling import RowParams, pack_params, sample_rows
+    rng = np.random.default_rng(vocab)
+    asked = [dict(temperature=0.0), dict(temperature=1.0), dict(temperature=0.7, top_p=0.8), dict(temperature=0.9, top_k=7),
+             dict(temperature=1.1, min_p=0.1), dict(temperature=1.0, top_k=2, top_p=0.9)]
+    flat = rng.normal(0, 2, size=len(asked) * vocab + offset).astype(np.float32)
+    flat[offset + vocab:offset + 2 * vocab] = 0.0            # all equal
+    dev = torch.device("cuda")
+    logits = torch.from_numpy(flat).to(dev)[offset:].view(len(asked), vocab)
+    words = (vocab + 31) // 32
+    masks = rng.integers(0, 2 ** 32, size=(1, words), dtype=np.uint64).astype(np.uint32)
+    masks[0, 0] |= 2
+    wrong = 0
+    for mask_row in (-1, 0):
+        params = [RowParams(seed=5 + i, position=i, mask_row=mask_row, **a) for i, a in enumerate(asked)]
+        tok, st = sample_rows(logits, pack_params(params, dev), torch.from_numpy(masks.view(np.int32)).to(dev))
+        for r, p in enumerate(params):
+            want, err = _oracle(flat[offset + r * vocab:offset + (r + 1) * vocab], masks[0] if mask_row == 0 else None, p)
+            assert (int(st[r]) == 0) == (err == 0)
+            wrong += err == 0 and int(tok[r]) != want
+    assert wrong <= 1, wrong
