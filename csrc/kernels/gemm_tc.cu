@@ -27,6 +27,8 @@ constexpr int kTileKBytes = 128;       // one 128-byte swizzle span of K per sta
 constexpr int kGemmThreads = 256;      // warps: 0 TMA, 1 MMA, 2-5 epilogue, 6-7 all-gather copiers
 constexpr int kStagingBytes = 32768;   // TMA-store staging: 4 epilogue warps x 2 buffers x [32 rows][128 B]
 
+constexpr int kModeF32Staged = 16;
+
 // tensor maps of the TMA-store epilogue (mode 6): m[0] = the output, or with reduce-scatter m[d] = this rank's slot
 // in rank d's buffer
 struct StoreMaps {
@@ -42,6 +44,7 @@ struct GemmParams {
                           // 6 bf16 [m,n] staged in shared memory and written by TMA stores; 7 scatter rows;
                           // 8 indexer scores: rows of M are (query, head) pairs, 32 heads per query; out[query][n] =
                           //   sum_head relu(acc) * row_w[query][head], -inf at n >= col_limit[query]
+                          // kModeF32Staged: 1 staged in shared memory and written by TMA stores (the host chooses it)
   long long ldo;          // leading dimension of the output in elements
   long long out_batch_stride;
   long long out_split_stride;
@@ -620,6 +623,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               ++st_pair;
             }
           }
+        } else if (p.out_mode == kModeF32Staged) {
+          if constexpr (KIND == 0 && Cfg::kStaging > 0) {
+            // 32 columns fill a staging buffer of [32 rows][128 B]: whole lines leave in one TMA store, where a thread's own
+            // stores put 16 bytes into each of 32 rows per instruction
+            uint8_t* buf = staging + quad * 8192 + (st_pair & 1u) * 4096;
+            if (lane == 0) bulk_wait_group_read<1>();       // the store issued from this buffer two chunks ago has read it
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              *reinterpret_cast<uint4*>(buf + lane * 128 + ((q ^ (lane & 7)) << 4)) =
+                  make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            fence_async_smem();
+            __syncwarp();
+            const int row0 = (rot ? (mt + rot) % m_tiles : mt) * kBM + quad * 32;
+            if (lane == 0) {
+              if (n0 < p.N && row0 < p.M) tma_store_3d(&stm.m[0], buf, n0, row0, b);
+              bulk_commit_group();
+            }
+            ++st_pair;
+          }
         } else if (p.out_mode == 8) {
           // One epilogue warp = the 32 heads of one query row.  relu x head weight, then a butterfly that leaves the
           // sum over heads of column l on lane l (31 shuffles for 32 columns), then one coalesced row store.
@@ -704,7 +727,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       acc = (acc + 1 == Cfg::kAccStages) ? 0 : acc + 1;
       if (acc == 0) acc_phase ^= 1;
     }
-    if (p.out_mode == 6 && lane == 0) bulk_wait_group<0>();   // every TMA store of this warp has been performed
+    if ((p.out_mode == 6 || p.out_mode == kModeF32Staged) && lane == 0) bulk_wait_group<0>();   // every TMA store of this warp has been performed
   } else if (warp >= 6) {
     // ------------------------------------------------------------ all-gather copiers (2 warps)
     if (p.ag_world > 1) {
@@ -929,6 +952,12 @@ extern "C" int ds41_gemm_tc(const ds41_gemm_args* a, void* stream) {
   p.ldo = a->ldo; p.out_batch_stride = a->out_batch_stride;
   p.out = k_splits > 1 ? a->split_workspace : a->out;
   if (p.out == nullptr && a->rs_world == 0) return cudaErrorInvalidValue;
+  if (out_mode == 1 && kind == 0 && k_splits == 1 && bn >= 64 && a->rs_world == 0 && a->softcap == 0.f && (a->ldo & 3) == 0 &&
+      (reinterpret_cast<uintptr_t>(a->out) & 15) == 0 && (batch == 1 || (a->out_batch_stride & 3) == 0)) {
+    e = make_tensor_map_3d(&peer.m[0], a->out, TmaDtype::kF32, N, M, batch, a->ldo * 4, a->out_batch_stride * 4, 32, 32, true);
+    if (e != cudaSuccess) return e;
+    p.out_mode = kModeF32Staged;
+  }
   // split planes are laid out [split][batch][rows][ldo]
   const long long plane = (out_mode == 1 ? 1ll * M : 1ll * N) * a->ldo;
   p.out_split_stride = k_splits > 1 ? plane * batch : 0;

@@ -1071,8 +1071,12 @@ class DS41Engine(RowsEngine):
             self._qkv(l, lw, R, inv, sources)
             src = None if self.layer_prefix_plain else cfg.source_of(l)
             nqb = lw.w_qb.shape[0]
-            self._run("gemm_qb", G.gemm_raw, lw.w_qb, self.q_lat, self.qb_out, nqb, R, Q, lda=Q, ldb=Q, ldo=self.nqb, out_mode=2,
-                       status=self.status, static_operand=1)
+            if G.wide(R, nqb) and self.nqb % 8 == 0:
+                self._run("gemm_qb", G.gemm_raw, self.q_lat, lw.w_qb, self.qb_out, R, nqb, Q, lda=Q, ldb=Q, ldo=self.nqb,
+                          out_mode=6, bn=256, status=self.status, static_operand=2)
+            else:
+                self._run("gemm_qb", G.gemm_raw, lw.w_qb, self.q_lat, self.qb_out, nqb, R, Q, lda=Q, ldb=Q, ldo=self.nqb,
+                          out_mode=2, status=self.status, static_operand=1)
             if lw.index_heads_cols and src is not None:
                 ratio = cfg.source_layers[src]
                 # index layers above the candidate layer score and select only inside its candidate blocks
@@ -1135,6 +1139,11 @@ class DS41Engine(RowsEngine):
                           static_operand=1)
                 self._run("reduce_groups", k.ds41_reduce_groups, lib.ptr(self.planes_oa), s_a, self.GL, R, cfg.o_lora,
                           lib.ptr(self.oa), C.c_longlong(self.GL * cfg.o_lora), st())
+            elif G.wide(R, cfg.o_lora, self.GL) and cfg.o_lora % 8 == 0:
+                self._run("gemm_wo_a", G.gemm_raw, self.attn_out, lw.wo_a, self.oa, R, cfg.o_lora, kg, lda=self.HL * D,
+                          ldb=kg, ldo=self.GL * cfg.o_lora, out_mode=6, bn=256, batch=self.GL, a_batch_stride=kg,
+                          b_batch_stride=cfg.o_lora * kg, out_batch_stride=cfg.o_lora, status=self.status,
+                          static_operand=2)
             else:
                 self._run("gemm_wo_a", G.gemm_raw, lw.wo_a, self.attn_out, self.oa, cfg.o_lora, R, kg, lda=kg,
                           ldb=self.HL * D, ldo=self.GL * cfg.o_lora, out_mode=2, batch=self.GL,
@@ -1543,10 +1552,14 @@ class DS41Engine(RowsEngine):
         partial shared expert for all rows plus the complete routed sum of its own slice."""
         cfg, k, st, H = self.cfg, self.k, lib.stream, self.cfg.hidden
         s_s = self._splits(H, self.I_sh, R)
-        self._run("gemm_shared_down", G.linear_planes, self.shared_act[:R], lw.w2_sh,
-                  self.planes_shared.view(-1)[: s_s * R * H].view(s_s, R, H), s_s, status=self.status)
-        self._run("reduce_planes", k.ds41_reduce_planes, lib.ptr(self.planes_shared), s_s, C.c_longlong(R * H),
-                  lib.ptr(self.moe_plane), 0, C.c_longlong(R * H), st())
+        if s_s == 1:                 # nothing to sum: the product goes straight into the plane
+            self._run("gemm_shared_down", G.linear_planes, self.shared_act[:R], lw.w2_sh, self.moe_plane[None, :R], 1,
+                      status=self.status)
+        else:
+            self._run("gemm_shared_down", G.linear_planes, self.shared_act[:R], lw.w2_sh,
+                      self.planes_shared.view(-1)[: s_s * R * H].view(s_s, R, H), s_s, status=self.status)
+            self._run("reduce_planes", k.ds41_reduce_planes, lib.ptr(self.planes_shared), s_s, C.c_longlong(R * H),
+                      lib.ptr(self.moe_plane), 0, C.c_longlong(R * H), st())
         if self._ep is None:
             self._make_ep(lw)
         lo, hi = R * self.rank // self.world, R * (self.rank + 1) // self.world

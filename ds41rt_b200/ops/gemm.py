@@ -88,12 +88,23 @@ def matmul_nt(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = No
     return out
 
 
+def wide(rows: int, n: int, batch: int = 1) -> bool:
+    """Does a long pass take a product with the rows as the 128-row operand and 256 weight rows as the other one?  Each weight
+    and activation byte then serves twice the products of a 128 x 128 tile of the swapped form, and results leave in TMA
+    stores (8192 rows x 33k x 1280: 954 us swapped, 545 us wide; 333 rows: 65 and 47) - once such tiles fill the GPU;
+    below that the swapped form's smaller tiles and its split over K keep more SMs busy."""
+    return rows > 128 and -(-rows // 128) * -(-n // 256) * batch >= 148
+
+
 def linear_planes(x: torch.Tensor, w: torch.Tensor, planes: torch.Tensor, splits: int, *, status=None, signal=None):
     """Swap-AB split-K projection: planes[s, rows, N] (fp32) partial sums of x @ w.T.  `signal`: see gemm_raw."""
     rows, K = x.shape
     N = w.shape[0]
     assert planes.dtype == torch.float32 and planes.is_contiguous()
-    if splits == 1:
+    if splits == 1 and signal is None and wide(rows, N):
+        gemm_raw(x, w, planes, rows, N, K, lda=x.stride(0), ldb=w.stride(0), ldo=N, out_mode=1, bn=256, status=status,
+                 static_operand=2)
+    elif splits == 1:
         gemm_raw(w, x, planes, N, rows, K, lda=w.stride(0), ldb=x.stride(0), ldo=N, out_mode=3, status=status,
                  static_operand=1, signal=signal)
     else:
