@@ -221,19 +221,19 @@ class ExpertParallelMoE:
         self._mark("count+plan")
         lib.check(k.ds41_ep_dispatch(C.byref(a), self.dispatch_blocks, st()), "ep_dispatch")
         self._mark("dispatch")
+        # the rows that exist (groups start on 128-row boundaries: the rest of the buffers is padding)
+        live = lib.ptr(self.tile_row0), lib.ptr(self.tile_end), lib.ptr(self.n_tiles), self.max_tiles
         if self.nv is not None:
             lib.check(k.ds41_ep_wait(C.byref(a), 2, st()), "ep_wait")
-            cap, zero = self.cap, C.c_longlong(0)
-            lib.check(k.ds41_act_quant_nvfp4_rows(lib.ptr(self.recv_x), C.c_longlong(H), lib.ptr(self.xq), C.c_longlong(H),
-                                                  lib.ptr(self.xq_sf), cap, H, C.c_float(self.nv[0]),
-                                                  lib.ptr(self.total_rows), 1, zero, zero, zero, None, st()), "quant")
+            cap = self.cap
+            lib.check(k.ds41_act_quant_nvfp4_tiles(lib.ptr(self.recv_x), C.c_longlong(H), lib.ptr(self.xq), C.c_longlong(H),
+                                                   lib.ptr(self.xq_sf), cap, H, C.c_float(self.nv[0]), *live, st()), "quant")
             self._grouped(self.w13, self.xq, self.act, I, H, lda=H, ldo=I, out_mode=4, up_row_offset=I,
                           sfa=self.w13_sf, sfa_batch_stride=self.w13_sf[0].numel(), sfb=self.xq_sf, alpha=self.nv[0],
                           alpha_batch=self.w13_gs)
             self._mark("wait+quant+fc1")
-            lib.check(k.ds41_act_quant_nvfp4_rows(lib.ptr(self.act), C.c_longlong(I), lib.ptr(self.actq), C.c_longlong(I),
-                                                  lib.ptr(self.actq_sf), cap, I, C.c_float(self.nv[1]),
-                                                  lib.ptr(self.total_rows), 1, zero, zero, zero, None, st()), "quant")
+            lib.check(k.ds41_act_quant_nvfp4_tiles(lib.ptr(self.act), C.c_longlong(I), lib.ptr(self.actq), C.c_longlong(I),
+                                                   lib.ptr(self.actq_sf), cap, I, C.c_float(self.nv[1]), *live, st()), "quant")
             self._grouped(self.w2, self.actq, self.comb, H, I, lda=I, ldo=H, out_mode=7, table=1, sfa=self.w2_sf,
                           sfa_batch_stride=self.w2_sf[0].numel(), sfb=self.actq_sf, alpha=self.nv[1],
                           alpha_batch=self.w2_gs)
@@ -246,14 +246,13 @@ class ExpertParallelMoE:
                               sfa=self.w13_sf, sfa_batch_stride=self.w13_sf[0].numel(), sfb=self.xq_sf, wait_phase=2)
             else:
                 lib.check(k.ds41_ep_wait(C.byref(a), 2, st()), "ep_wait")
-                lib.check(k.ds41_act_quant_mx_rows(lib.ptr(self.recv_x), C.c_longlong(H), lib.ptr(self.xq),
-                                                   C.c_longlong(H), lib.ptr(self.xq_sf), cap, H,
-                                                   lib.ptr(self.total_rows), st()), "act_quant")
+                lib.check(k.ds41_act_quant_mx_tiles(lib.ptr(self.recv_x), C.c_longlong(H), lib.ptr(self.xq),
+                                                    C.c_longlong(H), lib.ptr(self.xq_sf), cap, H, *live, st()), "act_quant")
                 self._grouped(self.w13, self.xq, self.act, I, H, lda=H, ldo=I, out_mode=4, up_row_offset=I,
                               sfa=self.w13_sf, sfa_batch_stride=self.w13_sf[0].numel(), sfb=self.xq_sf)
             self._mark("wait+quant+fc1")
-            lib.check(k.ds41_act_quant_mx_rows(lib.ptr(self.act), C.c_longlong(I), lib.ptr(self.actq), C.c_longlong(I),
-                                               lib.ptr(self.actq_sf), cap, I, lib.ptr(self.total_rows), st()), "act_quant")
+            lib.check(k.ds41_act_quant_mx_tiles(lib.ptr(self.act), C.c_longlong(I), lib.ptr(self.actq), C.c_longlong(I),
+                                                lib.ptr(self.actq_sf), cap, I, *live, st()), "act_quant")
             self._grouped(self.w2, self.actq, self.comb, H, I, lda=I, ldo=H, out_mode=7, table=1, sfa=self.w2_sf,
                           sfa_batch_stride=self.w2_sf[0].numel(), sfb=self.actq_sf)
             self._mark("quant+fc2")

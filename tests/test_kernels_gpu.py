@@ -574,3 +574,47 @@ def test_hc_mixes_on_the_tensor_cores_match_the_dot_product_kernel(rows, H):
     assert float((b[0].cpu() - pre1).abs().max()) < 1e-3
     assert float((b[1].cpu() - post1).abs().max()) < 1e-3
     assert float((b[2].cpu().view(rows, 4, 4) - comb1).abs().max()) < 1e-3
+
+
+@pytest.mark.parametrize("kind,K", [("mx", 128), ("mx", 640), ("mx", 2304), ("nvfp4", 64), ("nvfp4", 768), ("nvfp4", 5120)])
+def test_tile_quantisers_touch_the_rows_of_the_table(kind, K):
+    """Groups on 128-row boundaries with ragged tails: the table's rows are those of the host oracle, bit for bit, and every
+    other byte stays as it was."""
+    from ds41rt_b200.ops import lib, quant_ref as Q
+    from ds41rt_b200.ops.mx import pack_sf_atoms, unpack_sf_atoms
+    k = lib.kernels()
+    torch.manual_seed(K)
+    sizes, bn = [1, 128, 0, 127, 9, 65], 64
+    rows, row0, end = 0, [], []
+    for n in sizes:
+        for r in range(rows, rows + n, bn):
+            row0.append(r)
+            end.append(min(r + bn, rows + n))
+        rows += (n + 127) // 128 * 128
+    live = torch.cat([torch.arange(a, b) for a, b in zip(row0, end)])
+    i32 = dict(dtype=torch.int32, device="cuda")
+    t0, t1, n = torch.tensor(row0 + [0] * 4, **i32), torch.tensor(end + [rows] * 4, **i32), torch.tensor([len(row0)], **i32)
+    x = (torch.randn(rows, K, device="cuda") * torch.exp(torch.randn(rows, 1, device="cuda"))).bfloat16()
+    table = lib.ptr(t0), lib.ptr(t1), lib.ptr(n), len(row0) + 4, lib.stream()
+    per = 128 if kind == "mx" else 64                      # columns of a scale atom
+    q = torch.full((rows, K if kind == "mx" else K // 2), 0xAB, dtype=torch.uint8, device="cuda")
+    sf = torch.full((rows // 128, K // per, 512), 0xAB, dtype=torch.uint8, device="cuda")
+    head = lib.ptr(x), C.c_longlong(K), lib.ptr(q), C.c_longlong(K), lib.ptr(sf), rows, K
+    if kind == "mx":
+        lib.check(k.ds41_act_quant_mx_tiles(*head, *table), "quant")
+        want = torch.zeros(rows, K, dtype=torch.uint8, device="cuda")
+        want_sf = torch.zeros_like(sf)
+        lib.check(k.ds41_act_quant_mx(lib.ptr(x), C.c_longlong(K), C.c_longlong(0), lib.ptr(want), C.c_longlong(K),
+                                      C.c_longlong(0), lib.ptr(want_sf), C.c_longlong(0), rows, K, 1, 128, None, lib.stream()),
+                  "quant")
+    else:
+        gs = float(x.float().abs().amax() / (448 * 6))
+        lib.check(k.ds41_act_quant_nvfp4_tiles(*head, C.c_float(gs), *table), "quant")
+        want, want_s, _ = Q.quant_nvfp4(x.float(), gs)
+        want_sf = pack_sf_atoms(want_s.view(torch.uint8))
+    torch.cuda.synchronize()
+    dead = torch.ones(rows, dtype=torch.bool)
+    dead[live] = False
+    got_s, want_s = unpack_sf_atoms(sf.cpu(), rows), unpack_sf_atoms(want_sf.cpu(), rows)
+    assert torch.equal(q.cpu()[live], want.cpu()[live]) and bool((q.cpu()[dead] == 0xAB).all())
+    assert torch.equal(got_s[live], want_s[live]) and bool((got_s[dead] == 0xAB).all())
