@@ -8,11 +8,15 @@
 //  spec_accept   : accept-prefix rule of speculative verification: draft j is accepted while it equals the
 //                  target's choice after draft j-1; emits accepted count and the tokens to emit
 //                  (rust/crates/ds41rt-core/src/dspark_verify.rs:18-52)
+#include <cooperative_groups.h>
+
 #include "ds41_api.h"
 #include "ds41_launch.cuh"
 #include "ds41_ptx.cuh"
 
 namespace ds41 {
+
+namespace cg = cooperative_groups;
 
 struct ArgmaxParams {
   const float* logits;    // [rows][ld]
@@ -25,11 +29,18 @@ struct ArgmaxParams {
   int* row_status;        // optional [rows]: 1 = non-finite logit seen, 2 = no allowed candidate
 };
 
-__global__ void __launch_bounds__(1024) argmax_rows_kernel(ArgmaxParams p) {
-  __shared__ float wv[32];
-  __shared__ int wi[32];
+// A cluster of eight CTAs shares a row: one CTA keeps too few loads in flight for half a megabyte (129280 columns, 1 row: 17.6 us
+// with one CTA of 1024 threads, 5 with the cluster; 32 rows 18.0 and 8.4).  Every thread has kArgmaxDeep 16-byte loads in flight.
+constexpr int kArgmaxCtas = 8, kArgmaxThreads = 512, kArgmaxDeep = 4;
+__global__ void __launch_bounds__(kArgmaxThreads) argmax_rows_kernel(ArgmaxParams p) {
+  __shared__ float wv[kArgmaxThreads / 32];
+  __shared__ int wi[kArgmaxThreads / 32];
   __shared__ int bad;
-  const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ float cta_v;
+  __shared__ int cta_i;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int r = blockIdx.x / kArgmaxCtas, part = blockIdx.x % kArgmaxCtas;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_launch_dependents();
   pdl_wait();
   if (tid == 0) bad = 0;
@@ -46,39 +57,66 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(ArgmaxParams p) {
     if (mrow != nullptr) ok = (mrow[tok >> 5] >> (tok & 31)) & 1u;
     if (ok && (x > v || (x == v && tok < idx))) { v = x; idx = tok; }
   };
+  const int per = ((p.vocab_local + kArgmaxCtas - 1) / kArgmaxCtas + 3) / 4 * 4;       // whole 16-byte pieces
+  const int i0 = min(p.vocab_local, part * per), i1 = min(p.vocab_local, i0 + per);
+  int i = i0 + tid;
   if ((p.ld & 3) == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15) == 0) {
-    // 16-byte loads, two of them in flight per thread: a row is half a megabyte read by one block
-    const int n4 = p.vocab_local >> 2;
-    for (int g = tid; g < n4; g += 2048) {
-      const float4 a = *reinterpret_cast<const float4*>(row + 4 * g);
-      const bool second = g + 1024 < n4;
-      const float4 b = second ? *reinterpret_cast<const float4*>(row + 4 * (g + 1024)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      take(4 * g, a.x); take(4 * g + 1, a.y); take(4 * g + 2, a.z); take(4 * g + 3, a.w);
-      if (second) {
-        const int h = 4 * (g + 1024);
-        take(h, b.x); take(h + 1, b.y); take(h + 2, b.z); take(h + 3, b.w);
+    const int g1 = i1 >> 2;
+    for (int g0 = (i0 >> 2) + tid; g0 < g1; g0 += kArgmaxThreads * kArgmaxDeep) {
+      float4 a[kArgmaxDeep];
+#pragma unroll
+      for (int u = 0; u < kArgmaxDeep; ++u)
+        if (g0 + u * kArgmaxThreads < g1) a[u] = *reinterpret_cast<const float4*>(row + 4 * (g0 + u * kArgmaxThreads));
+#pragma unroll
+      for (int u = 0; u < kArgmaxDeep; ++u) {
+        const int g = g0 + u * kArgmaxThreads;
+        if (g < g1) { take(4 * g, a[u].x); take(4 * g + 1, a[u].y); take(4 * g + 2, a[u].z); take(4 * g + 3, a[u].w); }
       }
     }
-    for (int i = 4 * n4 + tid; i < p.vocab_local; i += 1024) take(i, row[i]);
-  } else {
-    for (int i = tid; i < p.vocab_local; i += 1024) take(i, row[i]);
+    i = max(i0, 4 * g1) + tid;
   }
+  for (; i < i1; i += kArgmaxThreads) take(i, row[i]);
   if (nonfinite) bad = 1;
+  auto better = [&](float ov, int oi) {
+    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
+  };
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, v, o);
     const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
+    better(ov, oi);
   }
   if (lane == 0) { wv[warp] = v; wi[warp] = idx; }
   __syncthreads();
   if (tid == 0) {
-    for (int w = 1; w < 32; ++w)
-      if (wv[w] > v || (wv[w] == v && wi[w] < idx)) { v = wv[w]; idx = wi[w]; }
-    p.best_val[r] = v;
-    p.best_idx[r] = idx == 0x7fffffff ? -1 : idx;
-    if (p.row_status != nullptr) p.row_status[r] = bad ? 1 : (idx == 0x7fffffff ? 2 : 0);
+    for (int w = 1; w < kArgmaxThreads / 32; ++w) better(wv[w], wi[w]);
+    cta_v = v;
+    cta_i = idx;
   }
+  cluster.sync();
+  if (part == 0 && warp == 0) {
+    int any_bad = 0;
+    v = -INFINITY;
+    idx = 0x7fffffff;
+    if (lane < kArgmaxCtas) {
+      v = *cluster.map_shared_rank(&cta_v, lane);
+      idx = *cluster.map_shared_rank(&cta_i, lane);
+      any_bad = *cluster.map_shared_rank(&bad, lane);
+    }
+    any_bad = __any_sync(0xffffffffu, any_bad);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+      better(ov, oi);
+    }
+    if (lane == 0) {
+      p.best_val[r] = v;
+      p.best_idx[r] = idx == 0x7fffffff ? -1 : idx;
+      if (p.row_status != nullptr) p.row_status[r] = any_bad ? 1 : (idx == 0x7fffffff ? 2 : 0);
+    }
+  }
+  cluster.sync();            // the first CTA may still read the others' shared memory
 }
 
 // candidates from `n_ranks` shards: vals[k][rows], idxs[k][rows] (pointer tables, possibly peer memory)
@@ -181,7 +219,8 @@ extern "C" int ds41_argmax_rows(const float* logits, long long ld, int rows, int
                                 int* row_status, void* stream) {
   if (rows <= 0 || vocab_local <= 0) return cudaErrorInvalidValue;
   ArgmaxParams p{logits, ld, vocab_local, vocab_offset, mask, mask_words, best_val, best_idx, row_status};
-  return launch_pdl(argmax_rows_kernel, dim3(rows), dim3(1024), 0, static_cast<cudaStream_t>(stream), p);
+  return launch_pdl_cluster(argmax_rows_kernel, dim3(rows * kArgmaxCtas), dim3(kArgmaxThreads), kArgmaxCtas, 0,
+                            static_cast<cudaStream_t>(stream), p);
 }
 
 extern "C" int ds41_argmax_merge(const float* const* vals, const int* const* idxs, int n_ranks, int rows, int* out,

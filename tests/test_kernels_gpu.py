@@ -618,3 +618,38 @@ def test_tile_quantisers_touch_the_rows_of_the_table(kind, K):
     got_s, want_s = unpack_sf_atoms(sf.cpu(), rows), unpack_sf_atoms(want_sf.cpu(), rows)
     assert torch.equal(q.cpu()[live], want.cpu()[live]) and bool((q.cpu()[dead] == 0xAB).all())
     assert torch.equal(got_s[live], want_s[live]) and bool((got_s[dead] == 0xAB).all())
+
+
+@pytest.mark.parametrize("vocab,ld,rows", [(3, 3, 1), (31, 32, 2), (4096, 4096, 3), (65537, 65540, 2), (129280, 129280, 5)])
+def test_argmax_rows_over_a_cluster(vocab, ld, rows):
+    """Largest allowed logit, lowest id among equals, at the edges of the eight parts of a row; statuses."""
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    torch.manual_seed(vocab)
+    logits = torch.randn(rows, ld, device="cuda")
+    per = -(-(-(-vocab // 8)) // 4) * 4
+    for i, at in enumerate((vocab - 1, 0, min(per, vocab - 1), min(2 * per - 1, vocab - 1), vocab // 2)[:rows]):
+        logits[i, at] = 50.0
+        logits[i, min(at + per, vocab - 1)] = 50.0                  # the same value in a later part
+    words = (vocab + 31) // 32
+    mask = torch.full((rows, words), -1, dtype=torch.int32, device="cuda")
+    if rows > 1:
+        mask[1] = 0
+    best, idx = torch.zeros(rows, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda")
+    status = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    for m in (None, mask):
+        lib.check(k.ds41_argmax_rows(lib.ptr(logits), C.c_longlong(ld), rows, vocab, 0, lib.ptr(m), words, lib.ptr(best),
+                                     lib.ptr(idx), lib.ptr(status), lib.stream()), "argmax")
+        torch.cuda.synchronize()
+        want = logits[:, :vocab].cpu()
+        for r in range(rows):
+            if m is not None and r == 1:
+                assert int(idx[r]) == -1 and int(status[r]) == 2
+            else:
+                top = want[r].max()
+                assert int(idx[r]) == int((want[r] == top).nonzero()[0]) and float(best[r]) == float(top) and int(status[r]) == 0
+    logits[rows - 1, vocab - 1] = float("nan")
+    lib.check(k.ds41_argmax_rows(lib.ptr(logits), C.c_longlong(ld), rows, vocab, 0, None, words, lib.ptr(best), lib.ptr(idx),
+                                 lib.ptr(status), lib.stream()), "argmax")
+    torch.cuda.synchronize()
+    assert status.tolist() == [0] * (rows - 1) + [1]
