@@ -60,7 +60,7 @@ struct HcStepParams {
   int* status;
 };
 
-__global__ void __launch_bounds__(256) hc_step_kernel(HcStepParams p) {
+__global__ void __launch_bounds__(256, 3) hc_step_kernel(HcStepParams p) {
   __shared__ float xs[kMult][kSlice];
   __shared__ float sqc[kSlice];
   __shared__ float proj[kStride];
@@ -69,6 +69,18 @@ __global__ void __launch_bounds__(256) hc_step_kernel(HcStepParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_slices = gridDim.x;
   pdl_launch_dependents();
+  // The launch is one chain of latencies (H 5120: 17.9 us for 1 row and 22.8 for 16 when each step loaded what it needed, 15.1
+  // and 20.9 now), so what does not depend on the previous kernel is fetched while that one ends: this warp's three rows of the
+  // mixing matrix (2 MB in all, from HBM when much weight has passed since the last layer).
+  constexpr int kMixSteps = kMult * kSlice / 32;
+  float fn[3][kMixSteps];
+#pragma unroll
+  for (int i = 0; i < kMixSteps; ++i) {
+    const int idx = lane + 32 * i;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      fn[j][i] = __ldg(p.fn + 1ll * (warp + 8 * j) * (kMult * H) + 1ll * (idx / kSlice) * H + c0 + idx % kSlice);
+  }
   pdl_wait();
   if (p.wait_flags != nullptr && p.parts.n_ranks > 1) {
     if (tid < p.parts.n_ranks) flag_wait_ge(p.wait_flags[tid], *p.wait_epoch, p.status, 400 + tid);
@@ -131,13 +143,12 @@ __global__ void __launch_bounds__(256) hc_step_kernel(HcStepParams p) {
   {
     float dot[3] = {0.f, 0.f, 0.f};
     float sq = 0.f;
-#pragma unroll 8
-    for (int idx = lane; idx < kMult * kSlice; idx += 32) {
-      const int d = idx / kSlice, c = idx % kSlice;
-      const long long kcol = 1ll * d * H + c0 + c;
-      const float x = xs[d][c];
 #pragma unroll
-      for (int j = 0; j < 3; ++j) dot[j] = fmaf(x, p.fn[1ll * (warp + 8 * j) * (kMult * H) + kcol], dot[j]);
+    for (int i = 0; i < kMixSteps; ++i) {
+      const int idx = lane + 32 * i;
+      const float x = xs[idx / kSlice][idx % kSlice];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) dot[j] = fmaf(x, fn[j][i], dot[j]);
       sq = fmaf(x, x, sq);
     }
 #pragma unroll
@@ -164,11 +175,49 @@ __global__ void __launch_bounds__(256) hc_step_kernel(HcStepParams p) {
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  for (int j = warp; j < kStride; j += 8) {
-    float acc = 0.f;
-    for (int s = lane; s < n_slices; s += 32) acc += __ldcg(p.partial + (1ll * s * p.rows + r) * kStride + j);
-    acc = warp_sum(acc);
-    if (lane == 0) proj[j] = acc;
+  // all that the finish reads is asked for at once: this warp's sums over the slices, the collapsed row, the norm weight
+  const int n_items = H / 8;
+  constexpr int kHeld = 3;                 // pieces of eight columns that a thread holds from here on
+  float4 xa[kHeld], xb[kHeld], wa[kHeld], wb[kHeld];
+  auto fetch = [&](int i, float4& a, float4& b, float4& u, float4& v) {
+    a = b = make_float4(0.f, 0.f, 0.f, 0.f);
+    u = v = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (i < n_items) {
+      a = __ldcg(reinterpret_cast<const float4*>(p.xc + 1ll * r * H + 8 * i));
+      b = __ldcg(reinterpret_cast<const float4*>(p.xc + 1ll * r * H + 8 * i + 4));
+      if (p.norm_w != nullptr) {
+        const float* w = p.norm_w + 8 * i;
+        u = make_float4(w[0], w[1], w[2], w[3]);
+        v = make_float4(w[4], w[5], w[6], w[7]);
+      }
+    }
+  };
+  {
+    constexpr int kSums = (kStride + 7) / 8;
+    float acc[kSums];
+#pragma unroll
+    for (int q = 0; q < kSums; ++q) acc[q] = 0.f;
+    for (int s0 = 0; s0 < n_slices; s0 += 64) {
+      float t[kSums][2];
+#pragma unroll
+      for (int q = 0; q < kSums; ++q)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int s = s0 + 32 * u + lane, j = warp + 8 * q;
+          t[q][u] = s < n_slices && j < kStride ? __ldcg(p.partial + (1ll * s * p.rows + r) * kStride + j) : 0.f;
+        }
+      if (s0 == 0) {
+#pragma unroll
+        for (int n = 0; n < kHeld; ++n) fetch(tid + 256 * n, xa[n], xb[n], wa[n], wb[n]);
+      }
+#pragma unroll
+      for (int q = 0; q < kSums; ++q) acc[q] = (acc[q] + t[q][0]) + t[q][1];
+    }
+#pragma unroll
+    for (int q = 0; q < kSums; ++q) {
+      const float v = warp_sum(acc[q]);
+      if (lane == 0 && warp + 8 * q < kStride) proj[warp + 8 * q] = v;
+    }
   }
   __syncthreads();
   if (warp == 0) {
@@ -202,19 +251,14 @@ __global__ void __launch_bounds__(256) hc_step_kernel(HcStepParams p) {
   }
   // ---------------------------------------------------------------- RMSNorm of the collapsed row (all warps)
   const float inv = rsqrtf(proj[kProj + 1] / H + p.norm_eps);
-  const int n_items = H / 8;
-  for (int i = tid; i < ((n_items + 255) / 256) * 256; i += 256) {
+  auto finish = [&](int i, float4 a, float4 b, float4 wu, float4 wv) {
     const bool live = i < n_items;
     float y[8];
     if (live) {
-      const float4 a = __ldcg(reinterpret_cast<const float4*>(p.xc + 1ll * r * H + 8 * i));
-      const float4 b = __ldcg(reinterpret_cast<const float4*>(p.xc + 1ll * r * H + 8 * i + 4));
       const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      const float w[8] = {wu.x, wu.y, wu.z, wu.w, wv.x, wv.y, wv.z, wv.w};
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float w = p.norm_w != nullptr ? p.norm_w[8 * i + q] : 1.f;
-        y[q] = bf16_round(x[q] * inv * w);
-      }
+      for (int q = 0; q < 8; ++q) y[q] = bf16_round(x[q] * inv * w[q]);
       uint4 o;
       __nv_bfloat162 t0 = __floats2bfloat162_rn(y[0], y[1]), t1 = __floats2bfloat162_rn(y[2], y[3]);
       __nv_bfloat162 t2 = __floats2bfloat162_rn(y[4], y[5]), t3 = __floats2bfloat162_rn(y[6], y[7]);
@@ -253,6 +297,15 @@ __global__ void __launch_bounds__(256) hc_step_kernel(HcStepParams p) {
         }
       }
     }
+  };
+  const int n_all = (n_items + 255) / 256;             // whole warps walk the row together
+#pragma unroll
+  for (int n = 0; n < kHeld; ++n)
+    if (n < n_all) finish(tid + 256 * n, xa[n], xb[n], wa[n], wb[n]);
+  for (int n = kHeld; n < n_all; ++n) {
+    float4 a, b, u, v;
+    fetch(tid + 256 * n, a, b, u, v);
+    finish(tid + 256 * n, a, b, u, v);
   }
 }
 
