@@ -25,6 +25,7 @@
 #include "ds41_api.h"
 #include "ds41_launch.cuh"
 #include "ds41_ptx.cuh"
+#include "ds41_tma.h"
 
 namespace ds41 {
 
@@ -205,6 +206,87 @@ hc_post_mix_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_out, 
   }   // row groups of this block
 }
 
+// Eight columns of the four streams of a row: new streams from the old ones and the sublayer's result (`sub`, unrounded).
+__device__ __forceinline__ void expand_piece(const uint4 (&raw)[kHcMaxMult], const float (&sub)[8], const float (&cm)[16],
+                                             const float (&pw)[4], float (&out)[kHcMaxMult][8], float& sq) {
+  float s_in[kHcMaxMult][8];
+#pragma unroll
+  for (int s = 0; s < kHcMaxMult; ++s) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[s]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 v = __bfloat1622float2(h[q]);
+      s_in[s][2 * q] = v.x;
+      s_in[s][2 * q + 1] = v.y;
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float sb = bf16_round(sub[j]);
+#pragma unroll
+    for (int d = 0; d < kHcMaxMult; ++d) {
+      float acc = 0.f;
+#pragma unroll
+      for (int s = 0; s < kHcMaxMult; ++s) acc = fmaf(cm[s * 4 + d], s_in[s][j], acc);
+      out[d][j] = bf16_round(fmaf(pw[d], sb, acc));
+      sq = fmaf(out[d][j], out[d][j], sq);
+    }
+  }
+}
+
+// The streams as they are.
+__device__ __forceinline__ void keep_piece(const uint4 (&raw)[kHcMaxMult], float (&out)[kHcMaxMult][8], float& sq) {
+#pragma unroll
+  for (int s = 0; s < kHcMaxMult; ++s) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[s]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float2 v = __bfloat1622float2(h[q]);
+      out[s][2 * q] = v.x;
+      out[s][2 * q + 1] = v.y;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sq = fmaf(out[s][j], out[s][j], sq);
+  }
+}
+
+__device__ __forceinline__ void store_piece(__nv_bfloat16* to, long long stride, const float (&out)[kHcMaxMult][8]) {
+#pragma unroll
+  for (int d = 0; d < kHcMaxMult; ++d) {
+    uint4 w;
+    __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&w);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) o2[q] = __floats2bfloat162_rn(out[d][2 * q], out[d][2 * q + 1]);
+    *reinterpret_cast<uint4*>(to + d * stride) = w;
+  }
+}
+
+// Collapse with the incoming weights: the same arithmetic and summation order as hc_finish, so that both give identical rows.
+__device__ __forceinline__ void collapse_piece(const float (&p_in)[kHcMaxMult], const float (&out)[kHcMaxMult][8],
+                                               float (&keep)[8], float& x_sq) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float x = bf16_round(fmaf(p_in[3], out[3][2 * q], fmaf(p_in[2], out[2][2 * q],
+                               fmaf(p_in[1], out[1][2 * q], p_in[0] * out[0][2 * q]))));
+    const float y = bf16_round(fmaf(p_in[3], out[3][2 * q + 1], fmaf(p_in[2], out[2][2 * q + 1],
+                               fmaf(p_in[1], out[1][2 * q + 1], p_in[0] * out[0][2 * q + 1]))));
+    keep[2 * q] = x;
+    keep[2 * q + 1] = y;
+    x_sq = fmaf(x, x, fmaf(y, y, x_sq));
+  }
+}
+
+__device__ __forceinline__ void norm_piece(const float (&keep)[8], float inv, const float* norm_w, __nv_bfloat16* to) {
+  float y[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) y[q] = bf16_round(keep[q] * inv * (norm_w != nullptr ? norm_w[q] : 1.f));
+  uint4 o;
+  __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) o2[q] = __floats2bfloat162_rn(y[2 * q], y[2 * q + 1]);
+  *reinterpret_cast<uint4*>(to) = o;
+}
+
 // Expand alone, for passes whose mixes projection runs as a GEMM afterwards: one block per row walks the row's H
 // columns in groups of eight (16-byte stream loads and stores, two 16-byte loads per partial plane), with the row's
 // 4 + 16 mixing coefficients in registers, and leaves the sum of squares of the new streams in
@@ -257,26 +339,9 @@ hc_expand_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_out, Pa
 #pragma unroll
     for (int s = 0; s < kHcMaxMult; ++s)
       raw[s] = *reinterpret_cast<const uint4*>(streams_in + (1ll * r * kHcMaxMult + s) * H + c);
-    float s_in[kHcMaxMult][8];
-#pragma unroll
-    for (int s = 0; s < kHcMaxMult; ++s) {
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw[s]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 v = __bfloat1622float2(h[q]);
-        s_in[s][2 * q] = v.x;
-        s_in[s][2 * q + 1] = v.y;
-      }
-    }
     float out[kHcMaxMult][8];
     if (!expand) {
-#pragma unroll
-      for (int s = 0; s < kHcMaxMult; ++s)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          out[s][j] = s_in[s][j];
-          sq = fmaf(s_in[s][j], s_in[s][j], sq);
-        }
+      keep_piece(raw, out, sq);
     } else {
     float sub[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     // rank-major, split-minor order; four planes (eight 16-byte loads) in flight before the first add
@@ -299,39 +364,11 @@ hc_expand_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_out, Pa
         sub[4] += v[u][1].x; sub[5] += v[u][1].y; sub[6] += v[u][1].z; sub[7] += v[u][1].w;
       }
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sb = bf16_round(sub[j]);
-#pragma unroll
-      for (int d = 0; d < kHcMaxMult; ++d) {
-        float acc = 0.f;
-#pragma unroll
-        for (int s = 0; s < kHcMaxMult; ++s) acc = fmaf(cm[s * 4 + d], s_in[s][j], acc);
-        out[d][j] = bf16_round(fmaf(pw[d], sb, acc));
-        sq = fmaf(out[d][j], out[d][j], sq);
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < kHcMaxMult; ++d) {
-      uint4 w;
-      __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&w);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) o2[q] = __floats2bfloat162_rn(out[d][2 * q], out[d][2 * q + 1]);
-      *reinterpret_cast<uint4*>(streams_out + (1ll * r * kHcMaxMult + d) * H + c) = w;
-    }
+    expand_piece(raw, sub, cm, pw, out, sq);
+    store_piece(streams_out + 1ll * r * kHcMaxMult * H + c, H, out);
     }   // expand
     if (xn != nullptr) {
-      // same arithmetic and summation order as hc_finish, so that both forms give identical rows
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float x = bf16_round(fmaf(p_in[3], out[3][2 * q], fmaf(p_in[2], out[2][2 * q],
-                                   fmaf(p_in[1], out[1][2 * q], p_in[0] * out[0][2 * q]))));
-        const float y = bf16_round(fmaf(p_in[3], out[3][2 * q + 1], fmaf(p_in[2], out[2][2 * q + 1],
-                                   fmaf(p_in[1], out[1][2 * q + 1], p_in[0] * out[0][2 * q + 1]))));
-        keep[n][2 * q] = x;
-        keep[n][2 * q + 1] = y;
-        x_sq = fmaf(x, x, fmaf(y, y, x_sq));
-      }
+      collapse_piece(p_in, out, keep[n], x_sq);
       if (tap_mean != nullptr) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -360,14 +397,146 @@ hc_expand_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_out, Pa
   for (int n = 0; n < kMaxItems; ++n) {
     const int g = tid + 256 * n;
     if (g >= H / 8) continue;
-    float y[8];
+    norm_piece(keep[n], inv, norm_w != nullptr ? norm_w + 8 * g : nullptr, xn + 1ll * r * H + 8 * g);
+  }
+}
+
+// The same for a long pass on one rank: bound by the bytes (four streams in and out, one plane, the normalised row: 22 H per
+// row).  One block per row reached 3.3 TB/s (8192 rows x 5120: 282 us): a thread's loads wait behind its own arithmetic and the
+// row's two barriers.  Here a producer thread brings whole rows (streams, plane, coefficients) into a ring by bulk copies and
+// two groups of 256 threads take them in turn, one CTA per SM: 179 us, 5.2 TB/s.  A thread's columns and every sum's order are
+// those of hc_expand_kernel, so the results are the same bits.
+constexpr int kStreamRows = 256;       // passes from here on (333 rows: 20.8 us as a block per row, 15.6 so)
+constexpr int kStreamGroups = 2, kStreamThreads = 256 * kStreamGroups + 32;
+struct StreamRing {
+  int plane_off, coef_off, stage_bytes, stages;
+};
+inline StreamRing stream_ring(int H, bool expand) {
+  StreamRing g{};
+  g.plane_off = (kHcMaxMult * H * 2 + 127) / 128 * 128;
+  g.coef_off = g.plane_off + (expand ? (4 * H + 127) / 128 * 128 : 0);
+  g.stage_bytes = g.coef_off + 128;                       // comb 64, post 16, collapse weights 16 bytes
+  g.stages = (220 * 1024) / g.stage_bytes < 4 ? (220 * 1024) / g.stage_bytes : 4;
+  return g;
+}
+
+__global__ void __launch_bounds__(kStreamThreads, 1)
+hc_expand_stream_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_out, const float* plane,
+                        const float* __restrict__ post, const float* __restrict__ comb, float* __restrict__ partial, int rows,
+                        int H, int* status, const float* __restrict__ pre_in, const float* __restrict__ norm_w,
+                        __nv_bfloat16* __restrict__ xn, float* __restrict__ tap_mean, float norm_eps, StreamRing ring) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ uint64_t full[4], empty[4];
+  __shared__ float sums[kStreamGroups][2][2][8];          // [group][row parity][streams, collapsed row][warp]
+  constexpr int kMaxItems = 3;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool expand = plane != nullptr;
+  pdl_launch_dependents();
+  if (tid == 0) {
+    for (int s = 0; s < ring.stages; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 8);
+    }
+    mbar_init_fence();
+  }
+  __syncthreads();
+  pdl_wait();
+  const int mine = (rows - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  if (warp == 8 * kStreamGroups) {
+    if (lane == 0) {
+      const uint32_t row_bytes = kHcMaxMult * H * 2;
+      const uint32_t tx = row_bytes + 16 + (expand ? 4 * H + 64 + 16 : 0);
+      for (int i = 0; i < mine; ++i) {
+        const int s = i % ring.stages;
+        const long long r = blockIdx.x + 1ll * i * gridDim.x;
+        if (!mbar_wait(&empty[s], ((i / ring.stages) & 1) ^ 1, status, 410)) break;
+        uint8_t* to = smem + s * ring.stage_bytes;
+        mbar_expect_tx(&full[s], tx);
+        bulk_load(to, streams_in + r * kHcMaxMult * H, row_bytes, &full[s]);
+        if (expand) {
+          bulk_load(to + ring.plane_off, plane + r * H, 4 * H, &full[s]);
+          bulk_load(to + ring.coef_off, comb + r * 16, 64, &full[s]);
+          bulk_load(to + ring.coef_off + 64, post + r * 4, 16, &full[s]);
+        }
+        bulk_load(to + ring.coef_off + 80, pre_in + r * 4, 16, &full[s]);
+      }
+    }
+  } else {
+    const int group = warp >> 3, t = tid & 255, w8 = warp & 7;
+    int parity = 0;
+    // a wait that gives up leaves its report in `status`; the group stays together, so that no barrier is left alone
+    for (int i = group; i < mine; i += kStreamGroups, parity ^= 1) {
+      const int s = i % ring.stages;
+      const long long r = blockIdx.x + 1ll * i * gridDim.x;
+      mbar_wait(&full[s], (i / ring.stages) & 1, status, 411);
+      const uint8_t* row = smem + s * ring.stage_bytes;
+      const float* coef = reinterpret_cast<const float*>(row + ring.coef_off);
+      float cm[16], pw[4], p_in[kHcMaxMult], keep[kMaxItems][8];
+      float sq = 0.f, x_sq = 0.f;
+      if (expand) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) y[q] = bf16_round(keep[n][q] * inv * (norm_w != nullptr ? norm_w[8 * g + q] : 1.f));
-    uint4 o;
-    __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
+        for (int q = 0; q < 16; ++q) cm[q] = coef[q];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) o2[q] = __floats2bfloat162_rn(y[2 * q], y[2 * q + 1]);
-    *reinterpret_cast<uint4*>(xn + 1ll * r * H + 8 * g) = o;
+        for (int q = 0; q < 4; ++q) pw[q] = coef[16 + q];
+      }
+#pragma unroll
+      for (int q = 0; q < kHcMaxMult; ++q) p_in[q] = coef[20 + q];
+#pragma unroll
+      for (int n = 0; n < kMaxItems; ++n) {
+        const int g = t + 256 * n;
+        if (g >= H / 8) continue;
+        uint4 raw[kHcMaxMult];
+#pragma unroll
+        for (int k = 0; k < kHcMaxMult; ++k) raw[k] = *reinterpret_cast<const uint4*>(row + 2ll * (k * H + 8 * g));
+        float out[kHcMaxMult][8];
+        if (expand) {
+          const float4* pl = reinterpret_cast<const float4*>(row + ring.plane_off) + 2 * g;
+          const float4 a = pl[0], b = pl[1];
+          const float sub[8] = {0.f + a.x, 0.f + a.y, 0.f + a.z, 0.f + a.w, 0.f + b.x, 0.f + b.y, 0.f + b.z, 0.f + b.w};
+          expand_piece(raw, sub, cm, pw, out, sq);
+          store_piece(streams_out + r * kHcMaxMult * H + 8 * g, H, out);
+        } else {
+          keep_piece(raw, out, sq);
+        }
+        collapse_piece(p_in, out, keep[n], x_sq);
+        if (tap_mean != nullptr) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) tap_mean[r * H + 8 * g + j] = 0.25f * (out[0][j] + out[1][j] + out[2][j] + out[3][j]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);               // this warp has read the row
+      sq = warp_sum(sq);
+      x_sq = warp_sum(x_sq);
+      float (*mem)[8] = sums[group][parity];
+      if (lane == 0) {
+        mem[0][w8] = sq;
+        mem[1][w8] = x_sq;
+      }
+      named_barrier(1 + group, 256);                       // the other parity's sums were read before this barrier
+      float u = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) u += mem[1][w];
+      const float inv = rsqrtf(u / H + norm_eps);
+      if (t == 0) {
+        float v = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v += mem[0][w];
+        partial[r * kHcPartialStride + kHcProj] = v;
+      }
+#pragma unroll
+      for (int n = 0; n < kMaxItems; ++n) {
+        const int g = t + 256 * n;
+        if (g < H / 8) norm_piece(keep[n], inv, norm_w != nullptr ? norm_w + 8 * g : nullptr, xn + r * H + 8 * g);
+      }
+    }
+  }
+  __syncthreads();
+  if (status != nullptr && *reinterpret_cast<volatile int*>(status) != kStatusOk) {
+    // a wait gave up: copies that may still be in flight land before the CTA's memory goes away
+    const long long start = clock64();
+    while (clock64() - start < 2000000ll) __nanosleep(1000);
+    __syncthreads();
   }
 }
 
@@ -609,6 +778,28 @@ extern "C" int ds41_hc_post_mix(const void* streams_in, void* streams_out, const
   const int slices = H / kHcSlice;
   int rpb = rows * slices / (2 * 148) / kHcRowsPerBlock * kHcRowsPerBlock;
   rpb = rpb < kHcRowsPerBlock ? kHcRowsPerBlock : (rpb > 64 ? 64 : rpb);
+  // long passes of one rank: rows through a ring in shared memory, where copies of whole rows are possible (16-byte pieces)
+  const bool aligned = ((reinterpret_cast<uintptr_t>(streams_in) | reinterpret_cast<uintptr_t>(post) |
+                         reinterpret_cast<uintptr_t>(comb) | reinterpret_cast<uintptr_t>(pre_in) |
+                         reinterpret_cast<uintptr_t>(n_ranks > 0 ? parts.base[0] : nullptr)) & 15) == 0;
+  if (fn == nullptr && xn != nullptr && n_ranks <= 1 && (n_ranks == 0 || n_splits == 1) && rows >= kStreamRows && aligned) {
+    const StreamRing ring = stream_ring(H, n_ranks > 0);
+    static std::atomic<bool> ready[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!ready[dev].load(std::memory_order_acquire)) {
+      cudaError_t e = cudaFuncSetAttribute(hc_expand_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 222 * 1024);
+      if (e != cudaSuccess) return e;
+      ready[dev].store(true, std::memory_order_release);
+    }
+    const int grid = rows < sm_count() ? rows : sm_count();
+    return launch_pdl(hc_expand_stream_kernel, dim3(grid), dim3(kStreamThreads), static_cast<size_t>(ring.stages) * ring.stage_bytes,
+                      static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(streams_in),
+                      static_cast<__nv_bfloat16*>(streams_out), n_ranks > 0 ? parts.base[0] : static_cast<const float*>(nullptr),
+                      post, comb, partial, rows, H, status, pre_in, norm_w, static_cast<__nv_bfloat16*>(xn), tap_mean,
+                      norm_eps, ring);
+  }
   if (fn == nullptr)      // expand only; the sum of squares of row r lands in partial[r * 25 + 24] (one slice)
     return launch_pdl(hc_expand_kernel, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream),
                       static_cast<const __nv_bfloat16*>(streams_in), static_cast<__nv_bfloat16*>(streams_out), parts,
