@@ -31,7 +31,7 @@ struct RouterParams {
   __nv_bfloat16* shared_act;   // [rows][I_sh]
 };
 
-// one block of 512 threads per row; E <= 512
+// Few rows: one block of 512 threads per row, which hides the latency of the split planes; E <= 512
 __global__ void __launch_bounds__(512) router_select_kernel(RouterParams p) {
   __shared__ float score[512];
   __shared__ float biased[512];
@@ -101,6 +101,94 @@ __global__ void __launch_bounds__(512) router_select_kernel(RouterParams p) {
       p.ids[r * p.topk + k] = chosen[k];
       p.weights[r * p.topk + k] = chosen_score[k] / (sum + 1e-20f) * p.route_scale;
     }
+  }
+}
+
+// A float as an unsigned number of the same order; NaN as low as -inf, so that it is never preferred.
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t u = __float_as_uint(v != v ? -INFINITY : v);
+  return u ^ (static_cast<uint32_t>(static_cast<int32_t>(u) >> 31) | 0x80000000u);
+}
+
+// Many rows: bound by the bytes of the planes.  The first `sel_blocks` blocks choose experts, a warp per row with its scores in
+// registers (no block barriers: a choice is a maximum over a lane's scores and two warp reductions); the others compute the
+// shared expert's activation, four columns per thread.  8192 rows of 384 + 2 x 2304 columns: 189 us as a block per row, 67 so.
+constexpr int kRouterRows = 512;       // passes from here on (64 rows of several planes: 7 us as a block per row, 13 as a warp)
+__global__ void __launch_bounds__(256) router_rows_kernel(RouterParams p, int sel_blocks) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long plane = 1ll * p.rows * p.ntot;
+  if (blockIdx.x >= sel_blocks) {
+    const int per_row = p.I_sh / 4;
+    const long long item = 1ll * (blockIdx.x - sel_blocks) * 256 + threadIdx.x;
+    if (item >= 1ll * p.rows * per_row) return;
+    const int r = static_cast<int>(item / per_row), i = static_cast<int>(item - 1ll * r * per_row) * 4;
+    const float* row0 = p.planes + 1ll * r * p.ntot + p.E + i;
+    float g[4] = {0.f, 0.f, 0.f, 0.f}, u[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int s = 0; s < p.splits; ++s) {
+      const float4 a = *reinterpret_cast<const float4*>(row0 + s * plane);
+      const float4 b = *reinterpret_cast<const float4*>(row0 + s * plane + p.I_sh);
+      g[0] += a.x; g[1] += a.y; g[2] += a.z; g[3] += a.w;
+      u[0] += b.x; u[1] += b.y; u[2] += b.z; u[3] += b.w;
+    }
+    float act[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float gj = fminf(bf16_round(g[j]), p.limit);
+      const float uj = fminf(fmaxf(bf16_round(u[j]), -p.limit), p.limit);
+      act[j] = gj / (1.0f + __expf(-gj)) * uj;
+    }
+    store4(p.shared_act + 1ll * r * p.I_sh + i, make_float4(act[0], act[1], act[2], act[3]));
+    return;
+  }
+  const int r = blockIdx.x * 8 + warp;
+  if (r >= p.rows) return;
+  const float* row0 = p.planes + 1ll * r * p.ntot;
+  constexpr int kPer = 16;                 // scores of a lane: experts lane, lane + 32, ...
+  float score[kPer];
+  uint32_t key[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) score[j] = 0.f;
+  for (int s = 0; s < p.splits; ++s)
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if (lane + 32 * j < p.E) score[j] += row0[s * plane + lane + 32 * j];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const int e = lane + 32 * j;
+    key[j] = order_key(-INFINITY);
+    if (e < p.E) {
+      const float a = score[j];
+      const float sp = a > 20.f ? a : log1pf(__expf(a));
+      score[j] = sqrtf(sp);
+      key[j] = order_key(score[j] + p.bias[e]);
+    }
+  }
+  float sum = 0.f, mine = 0.f;
+  int my_id = 0;
+  for (int k = 0; k < p.topk; ++k) {
+    uint32_t best = key[0];
+    int at = 0;
+    float sc = score[0];
+#pragma unroll
+    for (int j = 1; j < kPer; ++j)
+      if (key[j] > best) { best = key[j]; at = j; sc = score[j]; }
+    const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+    const int e = __reduce_min_sync(0xffffffffu, best == top ? lane + 32 * at : 0x7fffffff);      // ties: the lowest id
+    sc = __shfl_sync(0xffffffffu, sc, e & 31);
+    sum += sc;
+    if (lane == k) { mine = sc; my_id = e; }
+    if (lane == (e & 31)) {
+#pragma unroll
+      for (int j = 0; j < kPer; ++j)
+        if (j == e >> 5) key[j] = order_key(-INFINITY);
+    }
+  }
+  if (lane < p.topk) {
+    p.ids[r * p.topk + lane] = my_id;
+    p.weights[r * p.topk + lane] = mine / (sum + 1e-20f) * p.route_scale;
   }
 }
 
@@ -423,7 +511,15 @@ extern "C" int ds41_router_select(const float* planes, int splits, int rows, int
   if (rows <= 0 || E > 512 || topk > 16 || E + 2 * I_sh > ntot) return cudaErrorInvalidValue;
   RouterParams p{planes, splits, rows, ntot, E, I_sh, topk, bias, route_scale, limit, ids, weights,
                  static_cast<__nv_bfloat16*>(shared_act)};
-  return launch_pdl(router_select_kernel, dim3(rows, I_sh > 0 ? 2 : 1), dim3(512), 0, static_cast<cudaStream_t>(stream), p);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // four columns per thread: every piece of a row starts on 16 bytes
+  if (rows >= kRouterRows && topk >= 1 && splits >= 1 && ((E | I_sh | ntot) & 3) == 0 &&
+      (reinterpret_cast<uintptr_t>(planes) & 15) == 0 && (reinterpret_cast<uintptr_t>(shared_act) & 7) == 0) {
+    const int sel_blocks = (rows + 7) / 8;
+    const long long act_blocks = (1ll * rows * (I_sh / 4) + 255) / 256;
+    return launch_pdl(router_rows_kernel, dim3(static_cast<unsigned>(sel_blocks + act_blocks)), dim3(256), 0, st, p, sel_blocks);
+  }
+  return launch_pdl(router_select_kernel, dim3(rows, I_sh > 0 ? 2 : 1), dim3(512), 0, st, p);
 }
 
 extern "C" int ds41_moe_plan(const int* ids, const float* weights, const int* row_slot, int rows, int topk, int e0,

@@ -653,3 +653,41 @@ def test_argmax_rows_over_a_cluster(vocab, ld, rows):
                                  lib.ptr(status), lib.stream()), "argmax")
     torch.cuda.synchronize()
     assert status.tolist() == [0] * (rows - 1) + [1]
+
+
+@pytest.mark.parametrize("rows,splits,E,I_sh", [(512, 3, 384, 64), (513, 1, 36, 4), (777, 1, 512, 0), (2049, 1, 384, 2304)])
+def test_router_rows(rows, splits, E, I_sh):
+    """A warp per row: experts, order (ties to the lowest id, masked experts last) and weights of the plain statement."""
+    from ds41rt_b200.ops import lib
+    from ds41rt_b200.models import reference as R
+    k = lib.kernels()
+    torch.manual_seed(rows)
+    topk = 6
+    planes = torch.randn(splits, rows, E + 2 * I_sh, device="cuda")
+    planes[:, 1, :E] = 0.25                                          # every score alike
+    bias = torch.zeros(E, device="cuda")
+    bias[E // 2:] = float("-inf")
+    ids = torch.full((rows, topk), -7, dtype=torch.int32, device="cuda")
+    wts = torch.zeros(rows, topk, device="cuda")
+    act = torch.zeros(rows, max(I_sh, 1), device="cuda", dtype=torch.bfloat16)
+    lib.check(k.ds41_router_select(lib.ptr(planes), splits, rows, E + 2 * I_sh, E, I_sh, topk, lib.ptr(bias), C.c_float(1.5),
+                                   C.c_float(10.0), lib.ptr(ids), lib.ptr(wts), lib.ptr(act), lib.stream()), "router")
+    torch.cuda.synchronize()
+    total = planes[0].clone()
+    for s in range(1, splits):
+        total += planes[s]
+    total = total.cpu()
+    score = torch.sqrt(torch.nn.functional.softplus(total[:, :E]))
+    order = torch.sort(score + bias.cpu(), dim=-1, descending=True, stable=True)
+    gap = (order.values[:, :topk] - order.values[:, 1:topk + 1]).min(-1).values
+    clear = gap > 1e-5                                               # log1p / sqrt differ in the last places
+    clear[1] = True
+    assert int(clear.sum()) > rows * 0.9
+    want = order.indices[:, :topk]
+    assert torch.equal(ids.cpu().long()[clear], want[clear])
+    sel = torch.gather(score, 1, want)
+    assert ((wts.cpu() - sel / sel.sum(-1, keepdim=True) * 1.5)[clear]).abs().max() < 1e-5
+    if I_sh:
+        w = R.swiglu_clamped(total[:, E:E + I_sh].bfloat16().float(), total[:, E + I_sh:].bfloat16().float(), 10.0)
+        # one rounding to bf16 (2^-9) and the fast exponential's few units of 2^-23
+        assert ((act.float().cpu() - w).abs() <= w.abs() * 2.0 ** -8 + 1e-6).all()
