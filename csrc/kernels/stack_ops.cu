@@ -25,7 +25,9 @@ struct Moments {
 __device__ __forceinline__ Moments merge(Moments a, Moments b) {
   const float n = a.n + b.n;
   if (n == 0.f) return a;
-  const float d = b.mean - a.mean, f = b.n / n;
+  // halves of equal size in all but a row's last pieces: no division in the chain of merges that every row waits for twice
+  // (1 row of 2048 columns, layer norms: 11.1 us with the divisions, 10.0 without; 8 rows, RMS norms: 6.6 and 5.8)
+  const float d = b.mean - a.mean, f = b.n == a.n ? 0.5f : __fdividef(b.n, n);
   return {a.mean + d * f, a.m2 + b.m2 + d * d * (a.n * f), n};
 }
 __device__ __forceinline__ Moments merge_lanes(Moments v) {          // result in lane 0, then in every lane
@@ -57,7 +59,9 @@ __device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, 
     const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
     q += (live > 0 ? a * a : 0.f) + (live > 1 ? b * b : 0.f) + (live > 2 ? c * c : 0.f) + (live > 3 ? d * d : 0.f);
   }
-  Moments t = merge_lanes({mean, q, cnt});
+  Moments t{mean, q, cnt};
+  if (kind == 0) t = merge_lanes(t);
+  else t.m2 = warp_sum(q);                 // no means to merge
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
   if (lane == 0) {
     slot[warp] = t.mean;
@@ -77,7 +81,8 @@ __device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, 
       t = {far[w], far[32 + w], far[64 + w]};
     }
   }
-  t = merge_lanes(t);
+  if (kind == 0) t = merge_lanes(t);
+  else t.m2 = warp_sum(t.m2);
   return make_float2(t.mean, 1.0f / sqrtf(t.m2 / W + eps));
 }
 
@@ -235,7 +240,7 @@ template <typename T>
 __global__ void __launch_bounds__(512) polynorm_kernel(ds41_proj z, const float* coef, int ff, int ld_out, float eps,
                                                        T* out) {
   extern __shared__ float zrow[];
-  __shared__ float red[33];
+  __shared__ float red[3][32];
   const int r = blockIdx.x;
   pdl_launch_dependents();
   pdl_wait();
@@ -258,9 +263,21 @@ __global__ void __launch_bounds__(512) polynorm_kernel(ds41_proj z, const float*
     add(v.z);
     add(v.w);
   }
-  s2 = block_sum(s2, red);
-  s4 = block_sum(s4, red);
-  s6 = block_sum(s6, red);
+  // the three sums over the block behind one barrier; every warp adds the warps' shares itself (2048 rows of 11008 columns: 34.3
+  // us with one block-wide sum after the other, 32.1 so; 1 row 5.3 and 4.7)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+  s2 = warp_sum(s2);
+  s4 = warp_sum(s4);
+  s6 = warp_sum(s6);
+  if (lane == 0) {
+    red[0][warp] = s2;
+    red[1][warp] = s4;
+    red[2][warp] = s6;
+  }
+  __syncthreads();
+  s2 = warp_sum(lane < n_warps ? red[0][lane] : 0.f);
+  s4 = warp_sum(lane < n_warps ? red[1][lane] : 0.f);
+  s6 = warp_sum(lane < n_warps ? red[2][lane] : 0.f);
   const float a = coef[0] / sqrtf(s2 / ff + eps), b = coef[1] / sqrtf(s4 / ff + eps), c = coef[2] / sqrtf(s6 / ff + eps);
   const float e = coef[3];
   auto act = [&](float v) { return ((c * v + b) * v + a) * v + e; };
