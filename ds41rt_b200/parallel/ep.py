@@ -69,10 +69,9 @@ class ExpertParallelMoE:
         # is what bounds it); NVFP4 carries four times the scale columns and stays at 64
         self.bn = 128 if (not scaled or self.mx) else 64
         self.bn2 = 128 if scaled else 256          # FC2
-        # `tile_tokens` overrides both for the block-scaled FP8 kind (128 or 192).  With hundreds of experts a pass gives
-        # each about 128 rows: 128-token tiles then leave every second expert with a nearly empty second tile that still
-        # streams the expert's weights, while a 192-token tile holds the whole expert and multiplies only the columns
-        # it has
+        # `tile_tokens` overrides both for the block-scaled FP8 kind (128 or 192); without it each pass takes the width that
+        # suits its size (see _tile), unless `capacity` leaves no padding behind the last group for a wide tile's scales
+        self.by_size = tile_tokens is None and capacity is None and self.mx and not self.fp4
         if tile_tokens is not None and self.mx and not self.fp4:
             assert tile_tokens in (128, 192)
             self.bn = self.bn2 = tile_tokens
@@ -138,6 +137,17 @@ class ExpertParallelMoE:
         assert (w13_sf is not None) == (self.mx or self.nv is not None)
         self.w13, self.w2, self.w13_sf, self.w2_sf = w13, w2, w13_sf, w2_sf
         self.w13_gs, self.w2_gs = w13_gs, w2_gs
+
+    def _tile(self, tokens: int) -> None:
+        """Width of this pass's expert tiles in tokens (block-scaled FP8).  Every tile streams its expert's weights, so what
+        counts is how many tiles an expert of the mean size needs: around 128 rows half of the experts need a second, nearly
+        empty 128-token tile, and up to 192 all of them, while one 192-token tile holds the expert and multiplies only the
+        columns it has.  Below, and where both widths need the same number, the narrow tile is cheaper.  FC1 + FC2 of 128
+        experts, 5120 x 2304, us with 128 / 192 tokens: 96 rows each 1005 / 1067, 112 1059 / 1141, 128 1334 / 1226, 150 1774 /
+        1266, 170 1770 / 1359, 192 1763 / 1700, 230 1850 / 2163, 256 2194 / 2212, 320 2549 / 2394, 384 3176 / 3032, 512 4291 /
+        3594."""
+        rows = tokens * self.topk / self.e_local          # every rank sends about this pass's tokens
+        self.bn = self.bn2 = 192 if 124 <= rows <= 192 or rows >= 288 else 128
 
     # ------------------------------------------------------------------ argument blocks
     def _ep_args(self, x, ids, weights, tokens) -> lib.EpArgs:
@@ -215,6 +225,8 @@ class ExpertParallelMoE:
         assert T <= self.max_tokens and x.dtype == torch.bfloat16 and x.is_contiguous()
         assert ids.dtype == torch.int32 and weights.dtype == torch.float32
         k, st, H, I = lib.kernels("any"), lib.stream, self.H, self.I
+        if self.by_size:
+            self._tile(T)
         a = self._ep_args(x, ids, weights, T)
         lib.check(k.ds41_ep_count(C.byref(a), st()), "ep_count")
         lib.check(k.ds41_ep_plan(C.byref(a), st()), "ep_plan")
