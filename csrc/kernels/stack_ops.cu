@@ -42,8 +42,48 @@ __device__ __forceinline__ Moments merge_lanes(Moments v) {          // result i
 // four columns that the threads hold; `n` columns of the row are in this CTA, piece i covers columns 4 (tid + i blockDim).
 // Deviations are taken from each thread's own mean and merged pairwise, over the warp, the CTA and the cluster, in an order
 // that is the same in every thread.  `slot` holds 3 x 32 floats; at most 32 warps (4 per CTA of a cluster of 8).
-template <int CL, int NI>
+// FULL: every thread holds whole pieces and the warps' number is a power of two, so that both halves of every merge count the
+// same and nothing but means and deviations travels.
+template <int CL, int NI, bool FULL>
 __device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, int kind, float eps, float* slot) {
+  if constexpr (FULL) {
+    static_assert(CL == 1, "one CTA per row");
+    float s = 0.f, q = 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    float mean = kind == 0 ? s * (1.0f / (4 * NI)) : 0.f;            // an RMS norm merges with zero means
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
+      q += (a * a + b * b) + (c * c + d * d);
+    }
+    float half = 2.0f * NI;                // half the number of columns that one side of a merge has
+    auto merge_over = [&](int o) {         // both sides compute the same
+      const float m = __shfl_xor_sync(0xffffffffu, mean, o), t = __shfl_xor_sync(0xffffffffu, q, o), d = m - mean;
+      q = (q + t) + d * d * half;
+      mean = 0.5f * (mean + m);
+      half *= 2.0f;
+    };
+    if (kind == 0) {
+#pragma unroll
+      for (int o = 16; o; o >>= 1) merge_over(o);
+    } else {
+      q = warp_sum(q);
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
+    if (lane == 0) {
+      slot[warp] = mean;
+      slot[32 + warp] = q;
+    }
+    __syncthreads();
+    mean = slot[lane & (n_warps - 1)];
+    q = slot[32 + (lane & (n_warps - 1))];
+    for (int o = n_warps >> 1; o; o >>= 1) {
+      if (kind == 0) merge_over(o);
+      else q += __shfl_xor_sync(0xffffffffu, q, o);
+    }
+    return make_float2(mean, 1.0f / sqrtf(q / W + eps));
+  }
   float cnt = 0.f, s = 0.f;              // columns beyond the row hold zeros
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
@@ -102,7 +142,11 @@ __device__ __forceinline__ float4 routed_at4(const ds41_resid_args& p, int r, in
   return s;
 }
 
-template <typename T, int CL, int NI>
+// Many rows: bound by the instructions of a row rather than its bytes (ncu: 45 % of issue slots at 22 % of the memory's rate, more
+// threads or more rows an SM made it slower), so rows that fill the threads' pieces (FULL) drop every test of a column against the
+// row's end: launches of a prompt of 2048 rows x 4096
+// columns with three kept streams 75 -> 57 us on average, without kept streams 49 -> 39, 953 rows 28 -> 22.
+template <typename T, int CL, int NI, bool FULL>
 __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_step_kernel(ds41_resid_args p) {
   __shared__ float slots[2][96];
   const int per = ((p.W + CL - 1) / CL + 3) / 4 * 4;
@@ -116,7 +160,7 @@ __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_s
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
     at[i] = 4 * (threadIdx.x + i * blockDim.x);
-    live[i] = n - at[i];
+    live[i] = FULL ? 4 : n - at[i];
     x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (p.tokens != nullptr) {
@@ -159,6 +203,7 @@ __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_s
   };
   if (kEarly && p.mix != nullptr) add_older();
   auto clip = [&](float4& v, int i) {         // columns beyond the row hold zeros
+    if (FULL) return;
     if (live[i] < 4) v.w = 0.f;
     if (live[i] < 3) v.z = 0.f;
     if (live[i] < 2) v.y = 0.f;
@@ -181,7 +226,7 @@ __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_s
       }
     }
     float2 s = make_float2(0.f, 1.f);
-    if (p.post_w != nullptr) s = row_norm<CL, NI>(y, n, p.W, p.post_rms ? 1 : p.norm_kind, p.eps, slots[0]);
+    if (p.post_w != nullptr) s = row_norm<CL, NI, FULL>(y, n, p.W, p.post_rms ? 1 : p.norm_kind, p.eps, slots[0]);
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (live[i] > 0) {
@@ -217,7 +262,7 @@ __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_s
     }
   }
   if (p.next_w != nullptr) {
-    const float2 s = row_norm<CL, NI>(x, n, p.W, p.norm_kind, p.eps, slots[1]);
+    const float2 s = row_norm<CL, NI, FULL>(x, n, p.W, p.norm_kind, p.eps, slots[1]);
     T* h = static_cast<T*>(p.h) + 1ll * r * p.ldh + c0;
 #pragma unroll
     for (int i = 0; i < NI; ++i)
@@ -412,8 +457,13 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const T* src, int ld, 
 
 template <typename T, int CL, int NI>
 static cudaError_t launch_resid_ni(const ds41_resid_args& a, int threads, cudaStream_t st) {
-  if constexpr (CL == 1) return launch_pdl(resid_step_kernel<T, CL, NI>, dim3(a.rows), dim3(threads), 0, st, a);
-  else return launch_pdl_cluster(resid_step_kernel<T, CL, NI>, dim3(a.rows * CL), dim3(threads), CL, 0, st, a);
+  if constexpr (CL == 1) {
+    if (a.W == 4 * NI * threads && (threads & (threads - 1)) == 0)
+      return launch_pdl(resid_step_kernel<T, CL, NI, true>, dim3(a.rows), dim3(threads), 0, st, a);
+    return launch_pdl(resid_step_kernel<T, CL, NI, false>, dim3(a.rows), dim3(threads), 0, st, a);
+  } else {
+    return launch_pdl_cluster(resid_step_kernel<T, CL, NI, false>, dim3(a.rows * CL), dim3(threads), CL, 0, st, a);
+  }
 }
 
 template <typename T, int CL>

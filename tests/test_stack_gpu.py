@@ -347,6 +347,12 @@ def test_residual_step(rows, W, kind):
     torch.testing.assert_close(hb[:, :W].cpu().double(), norm(d(E[toks]), d(nw), eps), rtol=1e-2, atol=1e-2)
 
 
+@pytest.mark.parametrize("rows,W,kind", [(40, 128, 1), (33, 1024, 0), (40, 1024, 1), (33, 2048, 0), (40, 4096, 1), (33, 16384, 0)])
+def test_residual_step_of_whole_pieces(rows, W, kind):
+    """Rows that fill every thread's pieces: no column is tested against the row's end, moments merge in equal halves."""
+    test_residual_step(rows, W, kind)
+
+
 @pytest.mark.parametrize("ff", [37, 640, 5000])
 def test_polynorm_and_gates(ff):
     lib, S, k = _stack()
