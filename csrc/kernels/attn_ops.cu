@@ -99,19 +99,21 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
   const float* row0 = p.planes + 1ll * r * p.ntot;
   if (blockIdx.y == 0) {
     // ---- q latent (Q <= 2048: up to 8 columns per thread, all split loads issued together)
+    // the planes outside, the columns inside: four planes of all columns in flight (a decode pass waits for little else:
+    // 10.7 -> 9.0 us on average, 8192 rows 78 -> 55)
     float vals[8];
     float sq = 0.f;
 #pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      const int c = tid + 256 * n;
-      float a = 0.f;
-      if (c < p.Q) {
+    for (int n = 0; n < 8; ++n) vals[n] = 0.f;
 #pragma unroll 4
-        for (int s = 0; s < p.splits; ++s) a += row0[s * plane + c];
-        a = bf16_round(a);
-      }
-      vals[n] = a;
-      sq = fmaf(a, a, sq);
+    for (int s = 0; s < p.splits; ++s)
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+        if (tid + 256 * n < p.Q) vals[n] += row0[s * plane + tid + 256 * n];
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      vals[n] = bf16_round(vals[n]);
+      sq = fmaf(vals[n], vals[n], sq);
     }
     const float tot = block_sum_256(sq, scratch);
     const float inv = rsqrtf(tot / p.Q + p.eps);
@@ -122,7 +124,26 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
     }
     return;
   }
+  if (blockIdx.y == 2) {
+    // ---- extras (fp32 pass-through; index weights scaled)
+    for (int c0 = tid; c0 < p.extra_f32; c0 += 256 * 4) {
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+      for (int s = 0; s < p.splits; ++s)
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+          if (c0 + 256 * n < p.extra_f32) a[n] += row0[s * plane + p.Q + p.D + c0 + 256 * n];
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        const int c = c0 + 256 * n;
+        if (c >= p.extra_f32) break;
+        p.extras[1ll * r * p.extra_f32 + c] = c >= p.extra_f32 - p.index_heads ? a[n] * p.index_scale : a[n];
+      }
+    }
+    return;
+  }
   // ---- kv: thread handles adjacent pairs so RoPE stays in-thread (D <= 2048)
+  const int pos = p.row_pos[r], slot = p.row_slot[r];
   float2 kvv[4];
   float sq = 0.f;
 #pragma unroll
@@ -144,8 +165,6 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
   }
   const float tot = block_sum_256(sq, scratch);
   const float inv = rsqrtf(tot / p.D + p.eps);
-  const int pos = p.row_pos[r];
-  const int slot = p.row_slot[r];
   const long long ring_row = 1ll * slot * p.ring + (pos % p.ring);
   __nv_bfloat16* dst = p.win + ring_row * p.D;
   uint8_t* dst8 = reinterpret_cast<uint8_t*>(p.win) + ring_row * p.kv_row_bytes;
@@ -174,13 +193,6 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
     } else if (active && slot >= 0) {
       reinterpret_cast<__nv_bfloat162*>(dst)[i] = __floats2bfloat162_rn(a, b);
     }
-  }
-  // ---- extras (fp32 pass-through; index weights scaled)
-  for (int c = tid; c < p.extra_f32; c += 256) {
-    float a = 0.f;
-    for (int s = 0; s < p.splits; ++s) a += row0[s * plane + p.Q + p.D + c];
-    if (c >= p.extra_f32 - p.index_heads) a *= p.index_scale;
-    p.extras[1ll * r * p.extra_f32 + c] = a;
   }
 }
 
@@ -336,7 +348,7 @@ extern "C" int ds41_qkv_post(const float* planes, int splits, int rows, int ntot
                   kv_norm_w, inv_freq, row_pos, row_slot, static_cast<__nv_bfloat16*>(q_lat),
                   static_cast<__nv_bfloat16*>(win), ring, kv_row_bytes, extras, eps};
   if ((Q + D) & 1) return cudaErrorInvalidValue;   // kv columns are read as aligned float2
-  return launch_pdl(qkv_post_kernel, dim3(rows, 2), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
+  return launch_pdl(qkv_post_kernel, dim3(rows, p.extra_f32 > 0 ? 3 : 2), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
 }
 
 extern "C" int ds41_compress(const float* extras, int extra_stride, int rows, int D, int ID, int rope_dim, int ratio,
