@@ -24,7 +24,7 @@ namespace ds41 {
 
 constexpr int kBM = 128;
 constexpr int kTileKBytes = 128;       // one 128-byte swizzle span of K per stage
-constexpr int kGemmThreads = 256;      // warps: 0 TMA, 1 MMA, 2-5 epilogue, 6-7 all-gather copiers
+constexpr int kGemmThreads = 256;      // warps: 0 TMA, 1 MMA, 2-5 epilogue, 6-7 all-gather copiers, 8-11 second epilogue set
 constexpr int kStagingBytes = 32768;   // TMA-store staging: 4 epilogue warps x 2 buffers x [32 rows][128 B]
 
 constexpr int kModeF32Staged = 16;
@@ -134,6 +134,11 @@ struct GemmCfg {
   static constexpr int kTmemNeeded = kAccStages * kAccCols + kStages * kSfCols;
   static constexpr int kTmemCols = kTmemNeeded <= 32 ? 32 : kTmemNeeded <= 64 ? 64 : kTmemNeeded <= 128 ? 128
                                    : kTmemNeeded <= 256 ? 256 : 512;
+  // The widest block-scaled dual tile has a single accumulator set: the tensor cores wait for its epilogue (about 40
+  // instructions per column and thread), so two sets of four warps share its columns.  FC1 of 384 experts x 128 rows, 5120 x
+  // 2304: 2445 us with one set, 2198 with two.
+  static constexpr int kEpiSets = (DUAL && kAccStages == 1) ? 2 : 1;
+  static constexpr int kThreads = kGemmThreads + 128 * (kEpiSets - 1);
   static constexpr int kSmemBytes = kStages * kStageBytes + kStaging + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(kTmemNeeded <= 512, "TMEM budget exceeded");
   static_assert(kStages >= 2, "not enough shared memory for two stages");
@@ -158,7 +163,7 @@ __device__ __forceinline__ long long decode_tile(long long t, int m_tiles, int n
 }
 
 template <int BN, int KIND, int DUAL>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(GemmCfg<BN, KIND, DUAL>::kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ StoreMaps stm, GemmParams p) {
   using Cfg = GemmCfg<BN, KIND, DUAL>;
@@ -205,7 +210,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 4);
+      mbar_init(&acc_empty[a], 4 * Cfg::kEpiSets);
     }
     mbar_init(epi_bar, 4);
     mbar_init_fence();
@@ -411,8 +416,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       acc = (acc + 1 == Cfg::kAccStages) ? 0 : acc + 1;
       if (acc == 0) acc_phase ^= 1;
     }
-  } else if (warp >= 2 && warp < 6) {
-    // ------------------------------------------------------------ epilogue (4 warps)
+  } else if ((warp >= 2 && warp < 6) || warp >= 8) {
+    // ------------------------------------------------------------ epilogue (4 warps, or two sets that take chunks in turn)
     const int quad = warp & 3;                 // TMEM lane quadrant this warp may read
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -430,12 +435,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       // per-column metadata (route weight / return address) of the first chunk, fetched while the MMAs still run;
       // every chunk then fetches the next chunk's before it starts its own stores
       constexpr int kChunkPre = BN >= 32 ? 32 : BN;
+      constexpr int kStep = kChunkPre * Cfg::kEpiSets;
+      const int c_first = Cfg::kEpiSets > 1 && warp >= 8 ? kChunkPre : 0;
       const float* rw_base = (p.out_mode == 4 || p.out_mode == 5) ? p.row_w + (table ? 0ll : 1ll * b * p.row_w_ld) : nullptr;
       float rw_next = 0.f;
       int2 meta_next = make_int2(-1, -1);
-      if (lane < kChunkPre && n_base + lane < n_lim) {
-        if (rw_base != nullptr) rw_next = __ldcg(rw_base + n_base + lane);
-        if (p.out_mode == 7) meta_next = __ldcg(p.scatter_meta + n_base + lane);
+      if (lane < kChunkPre && n_base + c_first + lane < n_lim) {
+        if (rw_base != nullptr) rw_next = __ldcg(rw_base + n_base + c_first + lane);
+        if (p.out_mode == 7) meta_next = __ldcg(p.scatter_meta + n_base + c_first + lane);
       }
       if (!mbar_wait(&acc_full[acc], acc_phase, p.status, 300)) { ok = false; break; }
       tc_fence_after();
@@ -456,7 +463,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       // columns the tensor cores wrote for this tile (see n_mma in the issuer), in whole chunks
       const int n_cols = (table && p.out_mode != 6) ? min(BN, (max(n_lim - n_base, 0) + kChunk - 1) / kChunk * kChunk) : BN;
 #pragma unroll 1
-      for (int c = 0; c < n_cols; c += kChunk) {
+      for (int c = c_first; c < n_cols; c += kStep) {
         uint32_t v[32];
         if constexpr (kChunk == 32) {
           tmem_ld_32x32(t_row + c, v);
@@ -487,9 +494,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int2 meta_lane = meta_next;
         rw_next = 0.f;
         meta_next = make_int2(-1, -1);
-        if (c + kChunk < BN && lane < kChunk && n0 + kChunk + lane < n_lim) {
-          if (rw_base != nullptr) rw_next = __ldcg(rw_base + n0 + kChunk + lane);
-          if (p.out_mode == 7) meta_next = __ldcg(p.scatter_meta + n0 + kChunk + lane);
+        if (c + kStep < BN && lane < kChunk && n0 + kStep + lane < n_lim) {
+          if (rw_base != nullptr) rw_next = __ldcg(rw_base + n0 + kStep + lane);
+          if (p.out_mode == 7) meta_next = __ldcg(p.scatter_meta + n0 + kStep + lane);
         }
         if (p.out_mode == 0) {
           if (m < p.M) {
@@ -810,7 +817,7 @@ static cudaError_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, c
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_pdl(gemm_tc_kernel<BN, KIND, DUAL>, dim3(grid), dim3(kGemmThreads), Cfg::kSmemBytes, stream, tmA, tmB, peer, p);
+  return launch_pdl(gemm_tc_kernel<BN, KIND, DUAL>, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tmA, tmB, peer, p);
 }
 
 template <int KIND>
