@@ -720,3 +720,32 @@ def test_expert_tile_width_by_pass_size(tokens):
         assert ep.bn == (192 if tile is None and (124 <= tokens / 2 <= 192 or tokens / 2 >= 288) else 128)
         got.append(out)
     assert torch.equal(got[0], got[1]) and float(got[0].abs().max()) > 0
+
+
+@pytest.mark.parametrize("H,rows,expand,tap", [(128, 256, True, True), (5120, 300, True, False), (5120, 1000, False, False),
+                                               (6144, 450, True, True)])
+def test_expand_of_long_passes_matches_short_ones(H, rows, expand, tap):
+    """Rows through the ring of bulk copies (in place, uneven rows per CTA) are the rows of a block each, bit for bit."""
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    torch.manual_seed(H + rows)
+    start = torch.randn(rows, 4, H, device="cuda").bfloat16()
+    plane, post, comb = torch.randn(rows, H, device="cuda"), torch.rand(rows, 4, device="cuda"), torch.rand(rows, 16, device="cuda")
+    pre, norm_w, st = torch.rand(rows, 4, device="cuda"), torch.rand(H, device="cuda"), lib.new_status(torch.device("cuda", 0))
+    got = []
+    for most in (rows, 150):                               # one pass; passes that are too small for the ring
+        s, xn = start.clone(), torch.zeros(rows, H, device="cuda", dtype=torch.bfloat16)
+        partial, mean = torch.zeros(rows, 25, device="cuda"), torch.zeros(rows, H, device="cuda")
+        for r0 in range(0, rows, most):
+            n = min(most, rows - r0)
+            bases = (C.c_void_p * 1)(plane[r0:].data_ptr())
+            lib.check(k.ds41_hc_post_mix(lib.ptr(s[r0:]), lib.ptr(s[r0:]), bases, int(expand), 1, C.c_longlong(0),
+                                         lib.ptr(post[r0:]), lib.ptr(comb[r0:]), lib.ptr(None), lib.ptr(partial[r0:]), n, H,
+                                         lib.ptr(None), lib.ptr(None), lib.ptr(st), lib.ptr(pre[r0:]), lib.ptr(norm_w),
+                                         lib.ptr(xn[r0:]), lib.ptr(mean[r0:] if tap else None), C.c_float(1e-6), lib.stream()), "expand")
+        torch.cuda.synchronize()
+        assert int(st[0]) == 0
+        got.append((s, xn, partial, mean))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    assert float(got[0][1].float().abs().max()) > 0 and torch.equal(got[0][0], start) == (not expand)
