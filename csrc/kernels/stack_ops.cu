@@ -38,6 +38,14 @@ __device__ __forceinline__ Moments merge_lanes(Moments v) {          // result i
   return {__shfl_sync(0xffffffffu, v.mean, 0), __shfl_sync(0xffffffffu, v.m2, 0), __shfl_sync(0xffffffffu, v.n, 0)};
 }
 
+// Sum of the squared deviations of a piece's first `live` columns; products rounded before they are added, so that all forms of
+// a norm (whole pieces, ragged rows) give the same bits whatever the compiler would contract.
+__device__ __forceinline__ float piece_sq(float4 v, float mean, int live) {
+  const float a = v.x - mean, b = v.y - mean, c = v.z - mean, d = v.w - mean;
+  const float aa = __fmul_rn(a, a), bb = __fmul_rn(b, b), cc = __fmul_rn(c, c), dd = __fmul_rn(d, d);
+  return (live > 0 ? aa : 0.f) + (live > 1 ? bb : 0.f) + (live > 2 ? cc : 0.f) + (live > 3 ? dd : 0.f);
+}
+
 // Subtrahend and factor of a row's norm - layer norm (subtract the mean) or RMS norm (mean of squares) - from the pieces of
 // four columns that the threads hold; `n` columns of the row are in this CTA, piece i covers columns 4 (tid + i blockDim).
 // Deviations are taken from each thread's own mean and merged pairwise, over the warp, the CTA and the cluster, in an order
@@ -51,17 +59,17 @@ __device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, 
     float s = 0.f, q = 0.f;
 #pragma unroll
     for (int i = 0; i < NI; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
-    float mean = kind == 0 ? s * (1.0f / (4 * NI)) : 0.f;            // an RMS norm merges with zero means
+    float mean = kind == 0 ? s / (4 * NI) : 0.f;                     // an RMS norm merges with zero means
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
-      q += (a * a + b * b) + (c * c + d * d);
-    }
+    for (int i = 0; i < NI; ++i) q += piece_sq(v[i], mean, 4);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     float half = 2.0f * NI;                // half the number of columns that one side of a merge has
-    auto merge_over = [&](int o) {         // both sides compute the same
-      const float m = __shfl_xor_sync(0xffffffffu, mean, o), t = __shfl_xor_sync(0xffffffffu, q, o), d = m - mean;
+    auto merge_over = [&](int o) {         // merge() of the lower lane's columns and the upper one's, the same in both
+      const float m = __shfl_xor_sync(0xffffffffu, mean, o), t = __shfl_xor_sync(0xffffffffu, q, o);
+      const bool low = (lane & o) == 0;
+      const float d = low ? m - mean : mean - m;
       q = (q + t) + d * d * half;
-      mean = 0.5f * (mean + m);
+      mean = (low ? mean : m) + d * 0.5f;
       half *= 2.0f;
     };
     if (kind == 0) {
@@ -70,7 +78,6 @@ __device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, 
     } else {
       q = warp_sum(q);
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     if (lane == 0) {
       slot[warp] = mean;
       slot[32 + warp] = q;
@@ -96,8 +103,7 @@ __device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, 
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
     const int live = n - 4 * static_cast<int>(threadIdx.x + i * blockDim.x);
-    const float a = v[i].x - mean, b = v[i].y - mean, c = v[i].z - mean, d = v[i].w - mean;
-    q += (live > 0 ? a * a : 0.f) + (live > 1 ? b * b : 0.f) + (live > 2 ? c * c : 0.f) + (live > 3 ? d * d : 0.f);
+    q += piece_sq(v[i], mean, live);
   }
   Moments t{mean, q, cnt};
   if (kind == 0) t = merge_lanes(t);

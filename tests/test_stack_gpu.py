@@ -7,6 +7,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 import torch
 
@@ -351,6 +352,74 @@ def test_residual_step(rows, W, kind):
 def test_residual_step_of_whole_pieces(rows, W, kind):
     """Rows that fill every thread's pieces: no column is tested against the row's end, moments merge in equal halves."""
     test_residual_step(rows, W, kind)
+
+
+def norm_in_order(x, kind, eps):
+    """Mean and factor of every row as one block of the residual step sums them, in 32 bits: a thread's own moments, then the
+    lower half of the threads with the upper one, over a warp and over the warps."""
+    def fma(a, b, c):
+        return (a.astype(np.float64) * b.astype(np.float64) + c.astype(np.float64)).astype(np.float32)
+
+    def merge(a, b):
+        with np.errstate(divide="ignore", invalid="ignore"):
+            d, f = b[0] - a[0], b[2] / (a[2] + b[2])
+            both = fma(d, f, a[0]), fma(d * d, a[2] * f, a[1] + b[1]), a[2] + b[2]
+        return tuple(np.where(b[2] == 0, u, v) for u, v in zip(a, both))
+
+    def over(t):
+        while t[0].shape[-1] > 1:
+            o = t[0].shape[-1] // 2
+            t = merge([v[..., :o] for v in t], [v[..., o:] for v in t])
+        return [v[..., 0] for v in t]
+
+    rows, W = x.shape
+    pieces = (W + 3) // 4
+    width = lambda ni: ((pieces + ni - 1) // ni + 31) // 32 * 32
+    ni = next((n for n in (1, 2, 4) if width(n) <= 256), 8)
+    threads = width(ni)
+    v = np.zeros((rows, ni * threads * 4), np.float32)
+    v[:, :W] = x
+    live = (np.arange(v.shape[1]) < W).reshape(ni, threads, 4)
+    v, cnt = v.reshape(rows, ni, threads, 4), live.sum((0, 2)).astype(np.float32)
+    s = q = np.zeros((rows, threads), np.float32)
+    for p in range(ni):
+        s = s + ((v[:, p, :, 0] + v[:, p, :, 1]) + (v[:, p, :, 2] + v[:, p, :, 3]))
+    mean = np.where(cnt > 0, s / np.maximum(cnt, 1), 0).astype(np.float32) if kind == 0 else np.zeros_like(s)
+    for p in range(ni):
+        e = v[:, p] - mean[..., None]
+        e = np.where(live[p], e * e, np.float32(0))
+        q = q + (((e[..., 0] + e[..., 1]) + e[..., 2]) + e[..., 3])
+    t = [u.reshape(rows, -1, 32) for u in (mean, q, np.broadcast_to(cnt, mean.shape))]
+    warps = over(t)
+    t = [np.zeros((rows, 32), np.float32) for _ in range(3)]
+    for u, w in zip(t, warps):
+        u[:, :w.shape[1]] = w
+    mean, m2, _ = over(t)
+    return mean, np.float32(1) / np.sqrt(m2 / np.float32(W) + np.float32(eps))
+
+
+def check_norm_order(rows, W, kind):
+    lib, S, k = _stack()
+    g = gen(W + kind)
+    x, w = torch.randn(rows, W, generator=g) * 2 + 1, torch.randn(W, generator=g)
+    L = S.ceil_to(W, 8)
+    X, NW, h = torch.zeros(rows, L).cuda(), w.cuda(), torch.zeros(rows, L).cuda()
+    X[:, :W] = x.cuda()
+    a = S.ResidArgs()
+    a.y = a.gate = S.NO_PROJ
+    a.x_in, a.next_w, a.h, a.ldh, a.ldx = lib.ptr(X), lib.ptr(NW), lib.ptr(h), L, L
+    a.rows, a.W, a.norm_kind, a.eps, a.f32 = rows, W, kind, 1e-5, 1
+    _ok(k.ds41_resid_step(C.byref(a), lib.stream()))
+    mean, inv = norm_in_order(x.numpy(), kind, 1e-5)
+    want = (x.numpy() - mean[:, None]) * inv[:, None] * w.numpy()
+    assert torch.equal(h[:, :W].cpu(), torch.from_numpy(want))
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("W", [128, 1024, 2048, 4096, 8192, 16384])
+def test_norms_of_whole_pieces_sum_in_the_declared_order(W, kind):
+    """Bit for bit: the form without column tests sums as the general one does, so a row's width decides no rounding."""
+    check_norm_order(33, W, kind)
 
 
 @pytest.mark.parametrize("ff", [37, 640, 5000])
