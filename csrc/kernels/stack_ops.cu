@@ -23,12 +23,12 @@ struct Moments {
   float mean, m2, n;
 };
 __device__ __forceinline__ Moments merge(Moments a, Moments b) {
+  if (b.n == 0.f) return a;
   const float n = a.n + b.n;
-  if (n == 0.f) return a;
   // halves of equal size in all but a row's last pieces: no division in the chain of merges that every row waits for twice
   // (1 row of 2048 columns, layer norms: 11.1 us with the divisions, 10.0 without; 8 rows, RMS norms: 6.6 and 5.8)
-  const float d = b.mean - a.mean, f = b.n == a.n ? 0.5f : __fdividef(b.n, n);
-  return {a.mean + d * f, a.m2 + b.m2 + d * d * (a.n * f), n};
+  const float d = b.mean - a.mean, f = b.n == a.n ? 0.5f : b.n / n;
+  return {fmaf(d, f, a.mean), fmaf(d * d, a.n * f, a.m2 + b.m2), n};
 }
 __device__ __forceinline__ Moments merge_lanes(Moments v) {          // result in lane 0, then in every lane
 #pragma unroll

@@ -422,6 +422,13 @@ def test_norms_of_whole_pieces_sum_in_the_declared_order(W, kind):
     check_norm_order(33, W, kind)
 
 
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("W", [52, 90, 1032, 1501, 3000, 5124, 9000])
+def test_norms_of_ragged_rows_sum_in_the_declared_order(W, kind):
+    """Bit for bit, with the correctly rounded share of unequal halves (and none of an empty one)."""
+    check_norm_order(40, W, kind)
+
+
 @pytest.mark.parametrize("ff", [37, 640, 5000])
 def test_polynorm_and_gates(ff):
     lib, S, k = _stack()
