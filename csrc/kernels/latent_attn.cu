@@ -503,70 +503,57 @@ static int attend_mma_heads(const ds41_latent_attend_args& a) {
   return fits(1) ? 16 : 0;
 }
 
-// One block per (head, row): the splits' weights first, then G groups of 128 threads sum four columns per thread over every G-th
-// split.  A chain of latencies: four groups for many splits (one row's keys: 66 splits in 8.2 us, 32 in 7.5 with one group), one
-// group where few splits of many rows are better served by small blocks (32 rows x 32 heads, nine splits: 6.8 us, 12.3 with four).
-constexpr int kMaxSplits = 256, kMergeGroups = 4, kMergeFew = 16;
-template <typename T, int G>
-__global__ void __launch_bounds__(128 * G) latent_merge_kernel(const float* part_o, const float* part_ml, const float* sink,
-                                                               int n_splits, int heads, int kv_pad, T* out, int ld_out) {
+// One block per (head, row): the splits' weights first, a thread each, then every thread sums four columns over the splits in
+// their order.  A chain of latencies: 32 rows x 32 heads of nine splits 6.8 us, one row of 32 splits 7.5.
+constexpr int kMaxSplits = 256;
+template <typename T>
+__global__ void __launch_bounds__(128) latent_merge_kernel(const float* part_o, const float* part_ml, const float* sink,
+                                                           int n_splits, int heads, int kv_pad, T* out, int ld_out) {
   __shared__ float wt[kMaxSplits];
-  __shared__ float red[33], tops[4 * G];
-  __shared__ float4 sums[G > 1 ? G - 1 : 1][128];
-  const int h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x, group = tid / 128, t = tid % 128;
+  __shared__ float red[33], tops[4];
+  const int h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x;
   pdl_launch_dependents();
   pdl_wait();
   const long long cell0 = 1ll * r * n_splits * heads + h;
   const float sk = sink != nullptr ? sink[h] : -INFINITY;
-  static_assert(kMergeFew <= 128 && kMaxSplits <= 128 * kMergeGroups, "one split per thread");
-  float2 ml = make_float2(-INFINITY, 0.f);
-  if (tid < n_splits) ml = *reinterpret_cast<const float2*>(part_ml + 2 * (cell0 + 1ll * tid * heads));
-  float m = fmaxf(sk, ml.x);
+  float2 ml[kMaxSplits / 128];
+  float m = sk;
+#pragma unroll
+  for (int j = 0; j < kMaxSplits / 128; ++j) {
+    const int s = tid + 128 * j;
+    ml[j] = make_float2(-INFINITY, 0.f);
+    if (s < n_splits) ml[j] = *reinterpret_cast<const float2*>(part_ml + 2 * (cell0 + 1ll * s * heads));
+    m = fmaxf(m, ml[j].x);
+  }
 #pragma unroll
   for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if ((tid & 31) == 0) tops[tid >> 5] = m;
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < 4 * G; ++w) m = fmaxf(m, tops[w]);
+  for (int w = 0; w < 4; ++w) m = fmaxf(m, tops[w]);
   float den = 0.f;
-  if (tid < n_splits) {
-    const float e = ml.y > 0.f ? expf(ml.x - m) : 0.f;
-    wt[tid] = e;
-    den = e * ml.y;
+#pragma unroll
+  for (int j = 0; j < kMaxSplits / 128; ++j) {
+    const float e = ml[j].y > 0.f ? expf(ml[j].x - m) : 0.f;
+    if (tid + 128 * j < n_splits) wt[tid + 128 * j] = e;
+    den += e * ml[j].y;
   }
   den = block_sum(den, red) + (sink != nullptr ? expf(sk - m) : 0.f);
   const float inv = den > 0.f ? 1.0f / den : 0.f;
-  for (int i0 = 0; i0 < kv_pad; i0 += 512) {
-    const int i = i0 + 4 * t;
+  for (int i = 4 * tid; i < kv_pad; i += 512) {
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (i < kv_pad)
 #pragma unroll 8
-      for (int s = group; s < n_splits; s += G) {
-        const float e = wt[s];
-        if (e > 0.f) {
-          const float4 o = *reinterpret_cast<const float4*>(part_o + (cell0 + 1ll * s * heads) * kv_pad + i);
-          a.x += e * o.x;
-          a.y += e * o.y;
-          a.z += e * o.z;
-          a.w += e * o.w;
-        }
+    for (int s = 0; s < n_splits; ++s) {
+      const float e = wt[s];
+      if (e > 0.f) {
+        const float4 o = *reinterpret_cast<const float4*>(part_o + (cell0 + 1ll * s * heads) * kv_pad + i);
+        a.x += e * o.x;
+        a.y += e * o.y;
+        a.z += e * o.z;
+        a.w += e * o.w;
       }
-    if constexpr (G > 1) {
-      if (group > 0) sums[group - 1][t] = a;
-      __syncthreads();
     }
-    if (group == 0 && i < kv_pad) {
-#pragma unroll
-      for (int q = 0; q < G - 1; ++q) {
-        const float4 b = sums[q][t];
-        a.x += b.x;
-        a.y += b.y;
-        a.z += b.z;
-        a.w += b.w;
-      }
-      store4(out + 1ll * r * ld_out + h * kv_pad + i, make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv));
-    }
-    if constexpr (G > 1) __syncthreads();
+    store4(out + 1ll * r * ld_out + h * kv_pad + i, make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv));
   }
 }
 
@@ -662,15 +649,9 @@ extern "C" int ds41_latent_merge(const float* part_o, const float* part_ml, cons
     return cudaErrorInvalidValue;
   const dim3 grid(heads, rows);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  auto launch = [&](auto kernel, int groups, auto* to) {
-    return launch_pdl(kernel, grid, dim3(128 * groups), 0, st, part_o, part_ml, sink, n_splits, heads, kv_pad, to, ld_out);
-  };
-  const bool few = n_splits <= kMergeFew;
-  if (f32) {
-    float* to = static_cast<float*>(out);
-    return few ? launch(latent_merge_kernel<float, 1>, 1, to) : launch(latent_merge_kernel<float, kMergeGroups>, kMergeGroups, to);
-  }
-  __nv_bfloat16* to = static_cast<__nv_bfloat16*>(out);
-  return few ? launch(latent_merge_kernel<__nv_bfloat16, 1>, 1, to)
-             : launch(latent_merge_kernel<__nv_bfloat16, kMergeGroups>, kMergeGroups, to);
+  if (f32)
+    return launch_pdl(latent_merge_kernel<float>, grid, dim3(128), 0, st, part_o, part_ml, sink, n_splits, heads, kv_pad,
+                      static_cast<float*>(out), ld_out);
+  return launch_pdl(latent_merge_kernel<__nv_bfloat16>, grid, dim3(128), 0, st, part_o, part_ml, sink, n_splits, heads,
+                    kv_pad, static_cast<__nv_bfloat16*>(out), ld_out);
 }

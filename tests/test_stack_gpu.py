@@ -551,6 +551,33 @@ def test_absorbed_attention_over_pages(case, splits, dtype):
     torch.testing.assert_close(got, c.want(), rtol=tol, atol=tol)
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("splits", [17, 32, 130])
+def test_absorbed_attention_over_many_splits(splits, dtype):
+    test_absorbed_attention_over_pages(1, splits, dtype)
+
+
+@pytest.mark.parametrize("sink", [False, True])
+@pytest.mark.parametrize("splits,kvp", [(9, 144), (17, 512), (32, 512), (66, 576), (128, 16), (130, 144), (256, 48)])
+def test_merge_adds_the_splits_in_their_order(splits, kvp, sink):
+    """Bit for bit: the splits of one row weigh the same, so only the order of the additions decides the rounding."""
+    lib, S, k = _stack()
+    rows, H, g = 3, 5, gen(splits)
+    part = torch.randn(rows, splits, H, kvp, generator=g)
+    ml = torch.tensor([0.5, 2.0]).expand(rows, splits, H, 2).contiguous()
+    ml[0, ::3] = torch.tensor([float("-inf"), 0.0])                       # splits without a key
+    want = torch.zeros(rows, H, kvp)
+    for s in range(splits):
+        want += torch.where(ml[:, s, :, 1:] > 0, part[:, s], 0.0)
+    den = ml[..., 1].sum(1) + (1.0 if sink else 0.0)                      # the sink's logit is the largest one: whole numbers
+    want *= 1.0 / den[..., None]
+    part, ml, out = part.cuda(), ml.cuda(), torch.zeros(rows, H * kvp).cuda()
+    sk = torch.full((H,), 0.5).cuda() if sink else None
+    _ok(k.ds41_latent_merge(lib.ptr(part), lib.ptr(ml), lib.ptr(sk), splits, rows, H, kvp, lib.ptr(out), H * kvp, 1,
+                            lib.stream()))
+    assert torch.equal(out.cpu().view(rows, H, kvp), want)
+
+
 @pytest.mark.parametrize("case", [dict(heads=2, dim=48, rot=16, vdim=48, rank=64, n_keys=129, rows=129),
                                   dict(heads=3, dim=128, rot=64, vdim=128, rank=64, n_keys=700, rows=257),
                                   dict(heads=1, dim=16, rot=16, vdim=16, rank=32, n_keys=1000, rows=64),
