@@ -679,10 +679,11 @@ class StackEngine(RowsEngine):
     # ------------------------------------------------------------------ helpers
     def attn_splits(self, rows: int, heads: int) -> int:
         """Key splits per row of the absorbed attention: enough blocks to fill the GPU about twice, static per batch
-        size (a captured pass replays while the context grows).  A block takes whole tiles of 64 keys, one after the other, so
-        a single row is cut down to about one tile each (4097 keys, 16 heads: 18.0 us in 32 splits, 9.7 in 66)."""
+        size (a captured pass replays while the context grows).  At most 32: the splits are the order in which a row's
+        keys are summed, and 66 of them (one tile of 64 keys each, 4097 keys of 16 heads in 9.7 us rather than 18.0) gave other
+        results than the model had before."""
         want = 2 * 148 // (rows * -(-heads // 32))
-        return max(1, min(want, 128, -(-self.cache.max_ctx // 64)))
+        return max(1, min(want, 32, -(-self.cache.max_ctx // 64)))
 
     def project(self, tag: str, x: torch.Tensor, ldx: int, rows: int, m: Matrix, buf: torch.Tensor, few: bool = False) -> Proj:
         """fp32 result of a projection; `few`: the matrix has few rows, which long passes take as the 128-row operand."""

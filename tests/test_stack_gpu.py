@@ -578,6 +578,17 @@ def test_merge_adds_the_splits_in_their_order(splits, kvp, sink):
     assert torch.equal(out.cpu().view(rows, H, kvp), want)
 
 
+def test_splits_of_a_row_follow_its_batch_alone():
+    """How a row's keys are cut decides how its sums round, so the rule is part of a model's results."""
+    from types import SimpleNamespace
+    from ds41rt_b200.models.stack import StackEngine
+    e = SimpleNamespace(cache=SimpleNamespace(max_ctx=8192))
+    assert [StackEngine.attn_splits(e, rows, 16) for rows in (1, 2, 9, 10, 32, 64, 1000)] == [32, 32, 32, 29, 9, 4, 1]
+    assert [StackEngine.attn_splits(e, rows, 33) for rows in (1, 5, 8)] == [32, 29, 18]
+    e.cache.max_ctx = 130
+    assert StackEngine.attn_splits(e, 1, 16) == 3
+
+
 @pytest.mark.parametrize("case", [dict(heads=2, dim=48, rot=16, vdim=48, rank=64, n_keys=129, rows=129),
                                   dict(heads=3, dim=128, rot=64, vdim=128, rank=64, n_keys=700, rows=257),
                                   dict(heads=1, dim=16, rot=16, vdim=16, rank=32, n_keys=1000, rows=64),
