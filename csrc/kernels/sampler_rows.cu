@@ -15,6 +15,7 @@
 #include <cooperative_groups.h>
 
 #include <atomic>
+#include <utility>
 
 #include "ds41_api.h"
 #include "ds41_launch.cuh"
@@ -392,6 +393,8 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   };
   if (!(p.temperature >= 0.0f) || isinf(p.temperature)) return finish(kSampleBadTemperature, 0);
   if (!(p.top_p > 0.0f) || !(p.min_p >= 0.0f) || p.min_p > 1.0f) return finish(kSampleBadParameter, 0);
+  // a peer's shared memory may be touched once all CTAs of the cluster run: the wait hides behind the slice's loads
+  auto started = cl.barrier_arrive();
   const bool greedy = p.temperature < 1e-5f || p.top_k == 1;
   const float inv_t = greedy ? 1.0f : 1.0f / p.temperature;
 
@@ -463,6 +466,7 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   merge_warp(mine);
   if (lane == 0) sh.warp_part[warp] = mine;
   __syncthreads();
+  cl.barrier_wait(std::move(started));
   if (warp == 0) {
     mine = sh.warp_part[lane];
     merge_warp(mine);

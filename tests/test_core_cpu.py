@@ -1,8 +1,13 @@
 """Host runtime (C++ core) unit tests: sampler oracle, verification rule, Engram hashing, prefix banks, KV leases."""
+import re
+from pathlib import Path
+
 import numpy as np
 import pytest
 
 from ds41rt_b200.runtime import core as K
+
+ROOT = Path(__file__).resolve().parent.parent
 
 
 # ---------------------------------------------------------------------------------------------- sampler
@@ -398,3 +403,36 @@ def test_kv_allocator_against_a_reference_model_under_random_traffic():
         check()
     low = {k: v for k, v in steps.items() if v < 5}
     assert not low, low
+
+
+def _kernels_without_lambdas(text):
+    """(name, body) of every __global__ function, the bodies of the lambdas in it left out."""
+    def end_of(t, at):               # index behind the brace that closes the one at `at`
+        depth = 0
+        for i in range(at, len(t)):
+            depth += {"{": 1, "}": -1}.get(t[i], 0)
+            if depth == 0:
+                return i + 1
+        raise AssertionError("unbalanced braces")
+
+    text = re.sub(r"//[^\n]*", "", text)
+    for m in re.finditer(r"__global__[^;{]*?(\w+_kernel)\s*\([^;{]*\)\s*\{", text):
+        body = text[m.end() - 1:end_of(text, m.end() - 1)]
+        while (lam := re.search(r"\[[&=]?\]\s*\([^)]*\)[^;{]*\{", body)) is not None:
+            body = body[:lam.start()] + body[end_of(body, lam.end() - 1):]
+        yield m.group(1), body
+
+
+def test_clusters_cross_a_barrier_before_they_touch_a_peers_memory():
+    """A CTA's shared memory exists for its peers once it is known to run: a kernel that reads or writes a peer's has waited
+    on a cluster barrier first, in the kernel itself and not only in what it calls on its way out."""
+    seen = []
+    for src in sorted((ROOT / "csrc" / "kernels").glob("*.cu")):
+        for name, body in _kernels_without_lambdas(src.read_text()):
+            remote = body.find("map_shared_rank")
+            if remote < 0:
+                continue
+            seen.append(name)
+            barrier = re.search(r"\b(cl|cluster)\.(sync\(\)|barrier_wait\()", body)
+            assert barrier is not None and barrier.start() < remote, name
+    assert {"sample_rows_kernel", "argmax_rows_kernel"} <= set(seen), seen
