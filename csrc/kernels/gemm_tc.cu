@@ -959,12 +959,14 @@ extern "C" int ds41_gemm_tc(const ds41_gemm_args* a, void* stream) {
   p.ldo = a->ldo; p.out_batch_stride = a->out_batch_stride;
   p.out = k_splits > 1 ? a->split_workspace : a->out;
   if (p.out == nullptr && a->rs_world == 0) return cudaErrorInvalidValue;
-  if (out_mode == 1 && kind == 0 && k_splits == 1 && bn >= 64 && a->rs_world == 0 && a->softcap == 0.f && (a->ldo & 3) == 0 &&
-      (reinterpret_cast<uintptr_t>(a->out) & 15) == 0 && (batch == 1 || (a->out_batch_stride & 3) == 0)) {
-    e = make_tensor_map_3d(&peer.m[0], a->out, TmaDtype::kF32, N, M, batch, a->ldo * 4, a->out_batch_stride * 4, 32, 32, true);
-    if (e != cudaSuccess) return e;
+  // A tile table keeps plain stores: its tiles begin at any column (a TMA store begins on 16 bytes), end before the next group,
+  // and share one plane.  So does an output that no tensor map describes.
+  if (out_mode == 1 && kind == 0 && k_splits == 1 && bn >= 64 && a->rs_world == 0 && a->softcap == 0.f &&
+      a->tile_group == nullptr && (a->ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(a->out) & 15) == 0 &&
+      (batch == 1 || (a->out_batch_stride & 3) == 0) &&
+      make_tensor_map_3d(&peer.m[0], a->out, TmaDtype::kF32, N, M, batch, a->ldo * 4, a->out_batch_stride * 4, 32, 32, true) ==
+          cudaSuccess)
     p.out_mode = kModeF32Staged;
-  }
   // split planes are laid out [split][batch][rows][ldo]
   const long long plane = (out_mode == 1 ? 1ll * M : 1ll * N) * a->ldo;
   p.out_split_stride = k_splits > 1 ? plane * batch : 0;

@@ -143,3 +143,35 @@ def test_nvfp4_both_operands(rows, N, K):
     torch.cuda.synchronize()
     lib.raise_on_status(st, "gemm nvfp4")
     assert _rel(out, ref) < 2e-3
+
+
+@pytest.mark.parametrize("bn", [64, 128, 256])
+def test_fp32_rows_of_a_tile_table_end_with_their_group(bn):
+    """bf16 groups at any column, in one plane: columns between and behind the groups stay as they were, whatever the
+    (unused) stride between batches."""
+    import ctypes as C
+    from ds41rt_b200.ops import lib
+    g = torch.Generator().manual_seed(bn)
+    E, M, K, cap = 3, 200, 320, 700
+    groups = [(0, 37), (37, 37 + 150), (301, 301 + 257)]                 # first column, end
+    x, w = torch.randn(cap, K, generator=g).bfloat16(), (torch.randn(E, M, K, generator=g) * 0.05).bfloat16()
+    tiles = [(e, r, min(r + bn, b)) for e, (a, b) in enumerate(groups) for r in range(a, b, bn)]
+    tab = torch.tensor(tiles + [(0, 0, cap)] * 2, dtype=torch.int32).T.contiguous().cuda()
+    n = torch.tensor([len(tiles)], dtype=torch.int32).cuda()
+    X, W, st = x.cuda(), w.cuda(), lib.new_status("cuda")
+    out = torch.full((2 * M, cap), 7.0, device="cuda")                   # a plane more than the product has
+    a = lib.GemmArgs()
+    a.A, a.B, a.out, a.status = lib.ptr(W), lib.ptr(X), lib.ptr(out), lib.ptr(st)
+    a.lda, a.ldb, a.ldo, a.M, a.N, a.K, a.batch, a.a_batches, a.a_batch_stride = K, K, cap, M, cap, K, E, E, M * K
+    a.out_batch_stride, a.kind, a.out_mode, a.k_splits, a.b_batch_kind, a.bn = M * cap, 0, 1, 1, 1, bn
+    a.tile_group, a.tile_row0, a.tile_end = (lib.ptr(t) for t in tab)
+    a.n_tiles_dev, a.max_tiles = lib.ptr(n), len(tiles) + 2
+    lib.check(lib.kernels().ds41_gemm_tc(C.byref(a), lib.stream()), "gemm")
+    torch.cuda.synchronize()
+    lib.raise_on_status(st, "gemm tile table")
+    got, want, held = out.cpu(), torch.full((2 * M, cap), 7.0), torch.zeros(cap, dtype=torch.bool)
+    for e, (c0, c1) in enumerate(groups):
+        want[:M, c0:c1] = _ref(w[e], x[c0:c1])
+        held[c0:c1] = True
+    assert _rel(got[:M, held], want[:M, held]) < 2e-3
+    assert bool((got[:, ~held] == 7.0).all()) and bool((got[M:] == 7.0).all())
