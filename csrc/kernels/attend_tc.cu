@@ -238,6 +238,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attend_tc_kernel(AttendTcParams
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();
 
+  bool ok = true;                                // false: a wait of this thread gave up
   if (warp >= 4 && warp < 8) {
     // ------------------------------------------------------------ gather: Q rows and 16 keys of every tile per warp
     const int lw = warp - 4;
@@ -285,7 +286,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) attend_tc_kernel(AttendTcParams
     const uint8_t* my_ptr = nullptr;
     int my_fp4 = 0;
     if (live) lookup(s, j, my_ptr, my_fp4);
-    bool ok = true;
     int g = 0, it = 0;                           // tiles / items with keys so far
     while (live && ok) {
       if (j == 0) {
@@ -470,7 +470,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) attend_tc_kernel(AttendTcParams
       }
     };
     int g0 = 0, it = 0;
-    bool ok = true;
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const ItemShape s = item_shape(p, item);
       if (s.n_my == 0) continue;
@@ -545,7 +544,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) attend_tc_kernel(AttendTcParams
     // product has run: lanes 0-15 stage half 0 in buffer 0, lanes 16-31 half 1 in buffer 1
     const uint32_t stage_row = smem_u32(sP) + half * kPanelBytes + (warp * 16 + hsel) * 128;
     const uint8_t* stage_base = sP + warp * 16 * 128;
-    bool ok = true;
     int g = 0, it = 0;
     for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
       const ItemShape s = item_shape(p, item);
@@ -781,8 +779,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attend_tc_kernel(AttendTcParams
 
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
-  __syncthreads();
-  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != kStatusOk) {
+  if (__syncthreads_or(!ok)) {                    // one answer for the block, whatever other CTAs report meanwhile
     // a wait gave up: let copies and MMAs that may still be in flight finish before the CTA's memory goes away
     const long long start = clock64();
     while (clock64() - start < 2000000ll) __nanosleep(1000);

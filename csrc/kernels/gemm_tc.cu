@@ -225,13 +225,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  bool ok = true;                              // false: a wait of this thread gave up
   if (warp == 0 && lane == 0) {
     // ------------------------------------------------------------ TMA producer
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
     int stage = 0;
     uint32_t phase = 0;
-    bool ok = true;
     // 4-bit A tiles occupy one byte per element in shared memory but the copy engine accounts the packed bytes
     const uint32_t kStageTx = (p.a_fp4 ? Cfg::kABytes / 2 : Cfg::kABytes) + Cfg::kBBytes +
                               (Cfg::kScaled ? 512 * (Cfg::kAtomsA + Cfg::kAtomsB) : 0);
@@ -335,7 +335,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint32_t phase = 0;
     int acc = 0;
     uint32_t acc_phase = 0;
-    bool ok = true;
     constexpr uint32_t kFmt = (KIND == 0) ? 1u : 0u;   // bf16 / e4m3
     for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
       int mt_unused, nt;
@@ -421,7 +420,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int quad = warp & 3;                 // TMEM lane quadrant this warp may read
     int acc = 0;
     uint32_t acc_phase = 0;
-    bool ok = true;
     uint32_t st_pair = 0;                      // mode 6: staging buffer parity of this warp
     uint32_t epi_count = 0;                    // mode 7: chunks staged so far (buffer = count & 1, barrier phase)
     for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
@@ -777,7 +775,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
   if (p.sig_counter != nullptr) __threadfence();          // this CTA's output stores, before it is counted as done
-  __syncthreads();
+  const bool failed = __syncthreads_or(!ok);   // one answer for the block, whatever other CTAs report meanwhile
   if (p.sig_counter != nullptr && warp == 0) {
     unsigned int last = 0;
     if (lane == 0) last = atomicAdd(p.sig_counter, 1u) == gridDim.x - 1 ? 1u : 0u;
@@ -795,7 +793,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (lane < p.sig_world) flag_store_release(const_cast<uint32_t*>(p.sig_flags[lane]), e);   // release at system scope
     }
   }
-  if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != kStatusOk) {
+  if (failed) {
     // A wait gave up: let copies that may still be in flight land before the CTA's memory goes away.
     const long long start = clock64();
     while (clock64() - start < 2000000ll) __nanosleep(1000);

@@ -442,6 +442,7 @@ hc_expand_stream_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_
   __syncthreads();
   pdl_wait();
   const int mine = (rows - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  bool gave_up = false;
   if (warp == 8 * kStreamGroups) {
     if (lane == 0) {
       const uint32_t row_bytes = kHcMaxMult * H * 2;
@@ -449,7 +450,7 @@ hc_expand_stream_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_
       for (int i = 0; i < mine; ++i) {
         const int s = i % ring.stages;
         const long long r = blockIdx.x + 1ll * i * gridDim.x;
-        if (!mbar_wait(&empty[s], ((i / ring.stages) & 1) ^ 1, status, 410)) break;
+        if (!mbar_wait(&empty[s], ((i / ring.stages) & 1) ^ 1, status, 410)) { gave_up = true; break; }
         uint8_t* to = smem + s * ring.stage_bytes;
         mbar_expect_tx(&full[s], tx);
         bulk_load(to, streams_in + r * kHcMaxMult * H, row_bytes, &full[s]);
@@ -468,7 +469,7 @@ hc_expand_stream_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_
     for (int i = group; i < mine; i += kStreamGroups, parity ^= 1) {
       const int s = i % ring.stages;
       const long long r = blockIdx.x + 1ll * i * gridDim.x;
-      mbar_wait(&full[s], (i / ring.stages) & 1, status, 411);
+      if (!mbar_wait(&full[s], (i / ring.stages) & 1, status, 411)) gave_up = true;
       const uint8_t* row = smem + s * ring.stage_bytes;
       const float* coef = reinterpret_cast<const float*>(row + ring.coef_off);
       float cm[16], pw[4], p_in[kHcMaxMult], keep[kMaxItems][8];
@@ -531,12 +532,11 @@ hc_expand_stream_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_
       }
     }
   }
-  __syncthreads();
-  if (status != nullptr && *reinterpret_cast<volatile int*>(status) != kStatusOk) {
-    // a wait gave up: copies that may still be in flight land before the CTA's memory goes away
+  // a wait gave up: every thread stays until copies that may be in flight have landed in the CTA's memory.  One answer for the
+  // block, since other CTAs may report in the status word at any moment
+  if (__syncthreads_or(gave_up)) {
     const long long start = clock64();
     while (clock64() - start < 2000000ll) __nanosleep(1000);
-    __syncthreads();
   }
 }
 

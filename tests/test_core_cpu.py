@@ -405,21 +405,26 @@ def test_kv_allocator_against_a_reference_model_under_random_traffic():
     assert not low, low
 
 
+def _end_of_block(t, at):
+    """Index behind the brace that closes the one at `at`."""
+    depth = 0
+    for i in range(at, len(t)):
+        depth += {"{": 1, "}": -1}.get(t[i], 0)
+        if depth == 0:
+            return i + 1
+    raise AssertionError("unbalanced braces")
+
+
+def _sources():
+    return {src.name: re.sub(r"//[^\n]*", "", src.read_text()) for src in sorted((ROOT / "csrc" / "kernels").glob("*.cu"))}
+
+
 def _kernels_without_lambdas(text):
     """(name, body) of every __global__ function, the bodies of the lambdas in it left out."""
-    def end_of(t, at):               # index behind the brace that closes the one at `at`
-        depth = 0
-        for i in range(at, len(t)):
-            depth += {"{": 1, "}": -1}.get(t[i], 0)
-            if depth == 0:
-                return i + 1
-        raise AssertionError("unbalanced braces")
-
-    text = re.sub(r"//[^\n]*", "", text)
     for m in re.finditer(r"__global__[^;{]*?(\w+_kernel)\s*\([^;{]*\)\s*\{", text):
-        body = text[m.end() - 1:end_of(text, m.end() - 1)]
+        body = text[m.end() - 1:_end_of_block(text, m.end() - 1)]
         while (lam := re.search(r"\[[&=]?\]\s*\([^)]*\)[^;{]*\{", body)) is not None:
-            body = body[:lam.start()] + body[end_of(body, lam.end() - 1):]
+            body = body[:lam.start()] + body[_end_of_block(body, lam.end() - 1):]
         yield m.group(1), body
 
 
@@ -427,8 +432,8 @@ def test_clusters_cross_a_barrier_before_they_touch_a_peers_memory():
     """A CTA's shared memory exists for its peers once it is known to run: a kernel that reads or writes a peer's has waited
     on a cluster barrier first, in the kernel itself and not only in what it calls on its way out."""
     seen = []
-    for src in sorted((ROOT / "csrc" / "kernels").glob("*.cu")):
-        for name, body in _kernels_without_lambdas(src.read_text()):
+    for text in _sources().values():
+        for name, body in _kernels_without_lambdas(text):
             remote = body.find("map_shared_rank")
             if remote < 0:
                 continue
@@ -436,3 +441,12 @@ def test_clusters_cross_a_barrier_before_they_touch_a_peers_memory():
             barrier = re.search(r"\b(cl|cluster)\.(sync\(\)|barrier_wait\()", body)
             assert barrier is not None and barrier.start() < remote, name
     assert {"sample_rows_kernel", "argmax_rows_kernel"} <= set(seen), seen
+
+
+def test_no_barrier_behind_a_condition_that_threads_read_for_themselves():
+    """The status word may change under a block's eyes: a branch on it holds a barrier only if one vote has decided for all."""
+    for name, text in _sources().items():
+        for m in re.finditer(r"\bif \(((?:[^{};()]|\((?:[^{};()]|\([^{};()]*\))*\))*)\) \{", text):
+            if "status" in m.group(1) and "__syncthreads_or" not in m.group(1):
+                body = text[m.end() - 1:_end_of_block(text, m.end() - 1)]
+                assert "__syncthreads" not in body and "named_barrier" not in body, (name, m.group(0))
