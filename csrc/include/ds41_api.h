@@ -425,6 +425,10 @@ int ds41_vis_softmax(const float* s, long long ld, long long rows, int n_valid, 
 int ds41_vis_merge(const void* x, void* out, int gh, int gw, int m, int W, void* stream);
 int ds41_vis_scatter(const void* src, const int* rows, void* dst, int n, int H, int copies, void* stream);
 
+// Prefill-sized activation quantiser (1x128 scales, one warp per row); rows >= *rows_dev (if given) are skipped.
+int ds41_act_quant_mx_rows(const void* x, long long ldx, void* q, long long ldq, void* sf, int rows, int K,
+                           const int* rows_dev, void* stream);
+
 // Activation quantisers of grouped passes: only rows that a tile table names (tile t: rows [tile_row0[t], tile_end[t]), the
 // first *n_tiles of at most max_tiles tiles) are read and written.  E4M3 with 1x128 scales, or NVFP4 (as below).
 int ds41_act_quant_mx_tiles(const void* x, long long ldx, void* q, long long ldq, void* sf, int rows, int K,

@@ -81,6 +81,11 @@ struct QuantTiles {
 };
 constexpr int kTileCols = 512;      // columns of a tile's rows that one block takes: a few rows still spread over the GPU
 
+// Scale bytes of row r begin here; `atoms` 512-byte atoms per 128 rows.
+__device__ __forceinline__ uint8_t* atom_row_of(uint8_t* sf, int r, int atoms) {
+  return sf + 1ll * (r / 128) * atoms * 512 + (r % 32) * 16 + ((r / 32) % 4) * 4;
+}
+
 // 256 columns from k0 of one row, 1x128 scales: 16 bytes per lane, one scale per half warp.  A whole warp calls.
 __device__ __forceinline__ void mx_row_step(const __nv_bfloat16* src, uint8_t* dst, uint8_t* atom_row, int k0, int K, int lane) {
   const int k = k0 + lane * 8;
@@ -112,6 +117,18 @@ __device__ __forceinline__ void mx_row_step(const __nv_bfloat16* src, uint8_t* d
     *reinterpret_cast<uint2*>(dst + k) = o;
     if ((lane & 15) == 0) *reinterpret_cast<uint32_t*>(atom_row + 1ll * (k / 128) * 512) = e * 0x01010101u;
   }
+}
+
+// All rows below *rows_dev (a device count, e.g. the rows a rank received), a warp per row.
+__global__ void __launch_bounds__(256)
+act_quant_mx_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ q, long long ldq,
+                         uint8_t* __restrict__ sf, int rows, int K, const int* __restrict__ rows_dev) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int live = rows_dev != nullptr ? min(rows, *rows_dev) : rows;
+  for (int r = blockIdx.x * 8 + warp; r < live; r += gridDim.x * 8)
+    for (int k0 = 0; k0 < K; k0 += 256) mx_row_step(x + 1ll * r * ldx, q + 1ll * r * ldq, atom_row_of(sf, r, K / 128), k0, K, lane);
 }
 
 // NVFP4 activation rows: e2m1 values (two per byte, even element in the low nibble) with one E4M3 scale per 16
@@ -147,11 +164,6 @@ __device__ __forceinline__ void nvfp4_row_step(const __nv_bfloat16* src, uint8_t
     *reinterpret_cast<uint32_t*>(dst + k / 2) = packed;
     if ((lane & 1) == 0) atom_row[1ll * (k / 64) * 512 + ((k / 16) & 3)] = bs.__x;
   }
-}
-
-// Scale bytes of row r begin here; `atoms` 512-byte atoms per 128 rows.
-__device__ __forceinline__ uint8_t* atom_row_of(uint8_t* sf, int r, int atoms) {
-  return sf + 1ll * (r / 128) * atoms * 512 + (r % 32) * 16 + ((r / 32) % 4) * 4;
 }
 
 __global__ void __launch_bounds__(256)
@@ -224,6 +236,15 @@ extern "C" int ds41_act_quant_nvfp4_rows(const void* x, long long ldx, void* q, 
   return launch_pdl(act_quant_nvfp4_rows_kernel, dim3(blocks, batch), dim3(256), 0, static_cast<cudaStream_t>(stream),
                     static_cast<const __nv_bfloat16*>(x), ldx, static_cast<uint8_t*>(q), ldq, static_cast<uint8_t*>(sf),
                     rows, K, global_scale, rows_dev, x_batch_stride, q_batch_stride, sf_batch_stride, n_active);
+}
+
+extern "C" int ds41_act_quant_mx_rows(const void* x, long long ldx, void* q, long long ldq, void* sf, int rows, int K,
+                                      const int* rows_dev, void* stream) {
+  if (rows <= 0 || K <= 0 || K % 128 != 0 || (ldx & 7) || (ldq & 7)) return cudaErrorInvalidValue;
+  const int blocks = min((rows + 7) / 8, 8 * sm_count_cached());
+  return launch_pdl(act_quant_mx_rows_kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                    static_cast<const __nv_bfloat16*>(x), ldx, static_cast<uint8_t*>(q), ldq, static_cast<uint8_t*>(sf),
+                    rows, K, rows_dev);
 }
 
 extern "C" int ds41_act_quant_mx_tiles(const void* x, long long ldx, void* q, long long ldq, void* sf, int rows, int K,

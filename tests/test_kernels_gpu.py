@@ -620,6 +620,28 @@ def test_tile_quantisers_touch_the_rows_of_the_table(kind, K):
     assert torch.equal(got_s[live], want_s[live]) and bool((got_s[dead] == 0xAB).all())
 
 
+@pytest.mark.parametrize("rows,live,K,pad", [(1, None, 128, 0), (9, 5, 640, 8), (300, None, 384, 0), (1500, 1291, 256, 16)])
+def test_row_quantiser_of_long_passes(rows, live, K, pad):
+    """Rows below the device count as the general quantiser gives them, bit for bit; what lies behind stays as it was."""
+    from ds41rt_b200.ops import lib
+    from ds41rt_b200.ops.mx import unpack_sf_atoms
+    k = lib.kernels()
+    torch.manual_seed(rows)
+    x = (torch.randn(rows, K + pad, device="cuda") * torch.exp(torch.randn(rows, 1, device="cuda"))).bfloat16()
+    q, want = (torch.full((rows, K), 0xAB, dtype=torch.uint8, device="cuda") for _ in range(2))
+    sf, want_sf = (torch.full(((rows + 127) // 128, K // 128, 512), 0xAB, dtype=torch.uint8, device="cuda") for _ in range(2))
+    n = None if live is None else torch.tensor([live], dtype=torch.int32, device="cuda")
+    lib.check(k.ds41_act_quant_mx_rows(lib.ptr(x), C.c_longlong(K + pad), lib.ptr(q), C.c_longlong(K), lib.ptr(sf), rows, K,
+                                       lib.ptr(n), lib.stream()), "quant")
+    m = rows if live is None else live
+    lib.check(k.ds41_act_quant_mx(lib.ptr(x), C.c_longlong(K + pad), C.c_longlong(0), lib.ptr(want), C.c_longlong(K),
+                                  C.c_longlong(0), lib.ptr(want_sf), C.c_longlong(0), m, K, 1, 128, None, lib.stream()), "quant")
+    torch.cuda.synchronize()
+    assert torch.equal(q, want)
+    a, b = unpack_sf_atoms(sf.cpu(), rows), unpack_sf_atoms(want_sf.cpu(), rows)
+    assert torch.equal(a[:m], b[:m]) and bool((a[m:] == 0xAB).all())
+
+
 @pytest.mark.parametrize("vocab,ld,rows", [(3, 3, 1), (31, 32, 2), (4096, 4096, 3), (65537, 65540, 2), (129280, 129280, 5)])
 def test_argmax_rows_over_a_cluster(vocab, ld, rows):
     """Largest allowed logit, lowest id among equals, at the edges of the eight parts of a row; statuses."""
