@@ -29,17 +29,21 @@ struct ArgmaxParams {
   int* row_status;        // optional [rows]: 1 = non-finite logit seen, 2 = no allowed candidate
 };
 
-// A cluster of eight CTAs shares a row: one CTA keeps too few loads in flight for half a megabyte (129280 columns, 1 row: 17.6 us
-// with one CTA of 1024 threads, 5 with the cluster; 32 rows 18.0 and 8.4).  Every thread has kArgmaxDeep 16-byte loads in flight.
-constexpr int kArgmaxCtas = 8, kArgmaxThreads = 512, kArgmaxDeep = 4;
-__global__ void __launch_bounds__(kArgmaxThreads) argmax_rows_kernel(ArgmaxParams p) {
-  __shared__ float wv[kArgmaxThreads / 32];
-  __shared__ int wi[kArgmaxThreads / 32];
+// Where rows are long and few, a cluster of eight CTAs shares one: one CTA keeps too few loads in flight for half a megabyte.
+// Short rows do not pay for the cluster and many rows fill the GPU by themselves.  us, one CTA of 1024 threads / a cluster of
+// eight of 512: 4096 columns 1 row 2.2 / 2.5, 128 rows 3.0 / 8.8; 32000 columns 16 rows 4.4 / 3.3, 64 rows 5.5 / 6.7; 129280
+// columns 1 row 11.1 / 3.8, 128 rows 19.5 / 16.7, 300 rows 38.0 / 39.6; 262144 columns 128 rows 40.1 / 30.2, 1024 rows 164 / 198.
+constexpr int kArgmaxCtas = 8;
+static bool argmax_in_cluster(int rows, int vocab) { return vocab >= 16384 && rows <= 128 && rows <= vocab / 1024; }
+
+template <int CTAS, int THREADS, int DEEP>                 // every thread has DEEP 16-byte loads in flight
+__global__ void __launch_bounds__(THREADS) argmax_rows_kernel(ArgmaxParams p) {
+  __shared__ float wv[THREADS / 32];
+  __shared__ int wi[THREADS / 32];
   __shared__ int bad;
   __shared__ float cta_v;
   __shared__ int cta_i;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int r = blockIdx.x / kArgmaxCtas, part = blockIdx.x % kArgmaxCtas;
+  const int r = blockIdx.x / CTAS, part = blockIdx.x % CTAS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_launch_dependents();
   pdl_wait();
@@ -57,66 +61,70 @@ __global__ void __launch_bounds__(kArgmaxThreads) argmax_rows_kernel(ArgmaxParam
     if (mrow != nullptr) ok = (mrow[tok >> 5] >> (tok & 31)) & 1u;
     if (ok && (x > v || (x == v && tok < idx))) { v = x; idx = tok; }
   };
-  const int per = ((p.vocab_local + kArgmaxCtas - 1) / kArgmaxCtas + 3) / 4 * 4;       // whole 16-byte pieces
+  const int per = CTAS == 1 ? p.vocab_local : ((p.vocab_local + CTAS - 1) / CTAS + 3) / 4 * 4;       // whole 16-byte pieces
   const int i0 = min(p.vocab_local, part * per), i1 = min(p.vocab_local, i0 + per);
   int i = i0 + tid;
   if ((p.ld & 3) == 0 && (reinterpret_cast<uintptr_t>(p.logits) & 15) == 0) {
     const int g1 = i1 >> 2;
-    for (int g0 = (i0 >> 2) + tid; g0 < g1; g0 += kArgmaxThreads * kArgmaxDeep) {
-      float4 a[kArgmaxDeep];
+    for (int g0 = (i0 >> 2) + tid; g0 < g1; g0 += THREADS * DEEP) {
+      float4 a[DEEP];
+      a[0] = *reinterpret_cast<const float4*>(row + 4 * g0);
 #pragma unroll
-      for (int u = 0; u < kArgmaxDeep; ++u)
-        if (g0 + u * kArgmaxThreads < g1) a[u] = *reinterpret_cast<const float4*>(row + 4 * (g0 + u * kArgmaxThreads));
+      for (int u = 1; u < DEEP; ++u)
+        if (g0 + u * THREADS < g1) a[u] = *reinterpret_cast<const float4*>(row + 4 * (g0 + u * THREADS));
 #pragma unroll
-      for (int u = 0; u < kArgmaxDeep; ++u) {
-        const int g = g0 + u * kArgmaxThreads;
+      for (int u = 0; u < DEEP; ++u) {
+        const int g = g0 + u * THREADS;
         if (g < g1) { take(4 * g, a[u].x); take(4 * g + 1, a[u].y); take(4 * g + 2, a[u].z); take(4 * g + 3, a[u].w); }
       }
     }
     i = max(i0, 4 * g1) + tid;
   }
-  for (; i < i1; i += kArgmaxThreads) take(i, row[i]);
+  for (; i < i1; i += THREADS) take(i, row[i]);
   if (nonfinite) bad = 1;
   auto better = [&](float ov, int oi) {
     if (ov > v || (ov == v && oi < idx)) { v = ov; idx = oi; }
   };
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-    better(ov, oi);
-  }
-  if (lane == 0) { wv[warp] = v; wi[warp] = idx; }
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < kArgmaxThreads / 32; ++w) better(wv[w], wi[w]);
-    cta_v = v;
-    cta_i = idx;
-  }
-  cluster.sync();
-  if (part == 0 && warp == 0) {
-    int any_bad = 0;
-    v = -INFINITY;
-    idx = 0x7fffffff;
-    if (lane < kArgmaxCtas) {
-      v = *cluster.map_shared_rank(&cta_v, lane);
-      idx = *cluster.map_shared_rank(&cta_i, lane);
-      any_bad = *cluster.map_shared_rank(&bad, lane);
-    }
-    any_bad = __any_sync(0xffffffffu, any_bad);
+  auto better_of_warp = [&]() {
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
       const float ov = __shfl_xor_sync(0xffffffffu, v, o);
       const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
       better(ov, oi);
     }
-    if (lane == 0) {
-      p.best_val[r] = v;
-      p.best_idx[r] = idx == 0x7fffffff ? -1 : idx;
-      if (p.row_status != nullptr) p.row_status[r] = any_bad ? 1 : (idx == 0x7fffffff ? 2 : 0);
-    }
+  };
+  auto finish = [&](int any_bad) {
+    p.best_val[r] = v;
+    p.best_idx[r] = idx == 0x7fffffff ? -1 : idx;
+    if (p.row_status != nullptr) p.row_status[r] = any_bad ? 1 : (idx == 0x7fffffff ? 2 : 0);
+  };
+  better_of_warp();
+  if (lane == 0) { wv[warp] = v; wi[warp] = idx; }
+  __syncthreads();
+  if (tid == 0) {
+    for (int w = 1; w < THREADS / 32; ++w) better(wv[w], wi[w]);
+    if (CTAS == 1) finish(bad);
+    cta_v = v;
+    cta_i = idx;
   }
-  cluster.sync();            // the first CTA may still read the others' shared memory
+  if constexpr (CTAS > 1) {
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    if (part == 0 && warp == 0) {
+      int any_bad = 0;
+      v = -INFINITY;
+      idx = 0x7fffffff;
+      if (lane < CTAS) {
+        v = *cluster.map_shared_rank(&cta_v, lane);
+        idx = *cluster.map_shared_rank(&cta_i, lane);
+        any_bad = *cluster.map_shared_rank(&bad, lane);
+      }
+      any_bad = __any_sync(0xffffffffu, any_bad);
+      better_of_warp();
+      if (lane == 0) finish(any_bad);
+    }
+    cluster.sync();            // the first CTA may still read the others' shared memory
+  }
 }
 
 // candidates from `n_ranks` shards: vals[k][rows], idxs[k][rows] (pointer tables, possibly peer memory)
@@ -219,8 +227,10 @@ extern "C" int ds41_argmax_rows(const float* logits, long long ld, int rows, int
                                 int* row_status, void* stream) {
   if (rows <= 0 || vocab_local <= 0) return cudaErrorInvalidValue;
   ArgmaxParams p{logits, ld, vocab_local, vocab_offset, mask, mask_words, best_val, best_idx, row_status};
-  return launch_pdl_cluster(argmax_rows_kernel, dim3(rows * kArgmaxCtas), dim3(kArgmaxThreads), kArgmaxCtas, 0,
-                            static_cast<cudaStream_t>(stream), p);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (argmax_in_cluster(rows, vocab_local))
+    return launch_pdl_cluster(argmax_rows_kernel<kArgmaxCtas, 512, 4>, dim3(rows * kArgmaxCtas), dim3(512), kArgmaxCtas, 0, st, p);
+  return launch_pdl(argmax_rows_kernel<1, 1024, 2>, dim3(rows), dim3(1024), 0, st, p);
 }
 
 extern "C" int ds41_argmax_merge(const float* const* vals, const int* const* idxs, int n_ranks, int rows, int* out,

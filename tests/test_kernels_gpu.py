@@ -771,3 +771,10 @@ def test_expand_of_long_passes_matches_short_ones(H, rows, expand, tap):
     for a, b in zip(*got):
         assert torch.equal(a, b)
     assert float(got[0][1].float().abs().max()) > 0 and torch.equal(got[0][0], start) == (not expand)
+
+
+@pytest.mark.parametrize("vocab,ld,rows", [(16383, 16384, 5), (16384, 16384, 16), (16384, 16384, 17), (4096, 4096, 3), (131072, 131072, 128),
+                                           (131072, 131072, 129)])
+def test_argmax_rows_on_both_sides_of_the_rule(vocab, ld, rows):
+    """A cluster for few long rows, one block for short or many ones."""
+    test_argmax_rows_over_a_cluster(vocab, ld, rows)
