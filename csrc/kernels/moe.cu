@@ -113,7 +113,10 @@ __device__ __forceinline__ uint32_t order_key(float v) {
 // Many rows: bound by the bytes of the planes.  The first `sel_blocks` blocks choose experts, a warp per row with its scores in
 // registers (no block barriers: a choice is a maximum over a lane's scores and two warp reductions); the others compute the
 // shared expert's activation, four columns per thread.  8192 rows of 384 + 2 x 2304 columns: 189 us as a block per row, 67 so.
-constexpr int kRouterRows = 512;       // passes from here on (64 rows of several planes: 7 us as a block per row, 13 as a warp)
+// Where a warp walks many planes by itself the block form stays the better one until rows fill the GPU.  us, block / warp form:
+// 511 rows of one plane 11.1 / 7.5; 512 rows of 960 columns, 3 planes 10.2 / 9.6, 8 planes 10.7 / 13.6; 384 columns, 12 planes, 512
+// rows 11.0 / 14.2, 1024 rows 17.0 / 15.7; 16 planes, 1024 rows 17.8 / 18.5.  Below 320 rows the block form wins or ties throughout.
+static bool router_by_warps(int rows, int splits) { return rows >= 512 && rows >= 160 * splits; }
 __global__ void __launch_bounds__(256) router_rows_kernel(RouterParams p, int sel_blocks) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_launch_dependents();
@@ -513,7 +516,7 @@ extern "C" int ds41_router_select(const float* planes, int splits, int rows, int
                  static_cast<__nv_bfloat16*>(shared_act)};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // four columns per thread: every piece of a row starts on 16 bytes
-  if (rows >= kRouterRows && topk >= 1 && splits >= 1 && ((E | I_sh | ntot) & 3) == 0 &&
+  if (router_by_warps(rows, splits) && topk >= 1 && splits >= 1 && ((E | I_sh | ntot) & 3) == 0 &&
       (reinterpret_cast<uintptr_t>(planes) & 15) == 0 && (reinterpret_cast<uintptr_t>(shared_act) & 7) == 0) {
     const int sel_blocks = (rows + 7) / 8;
     const long long act_blocks = (1ll * rows * (I_sh / 4) + 255) / 256;

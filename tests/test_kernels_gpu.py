@@ -778,3 +778,29 @@ def test_expand_of_long_passes_matches_short_ones(H, rows, expand, tap):
 def test_argmax_rows_on_both_sides_of_the_rule(vocab, ld, rows):
     """A cluster for few long rows, one block for short or many ones."""
     test_argmax_rows_over_a_cluster(vocab, ld, rows)
+
+
+@pytest.mark.parametrize("rows,splits,E,I_sh", [(512, 3, 384, 64), (512, 4, 384, 64), (640, 4, 36, 4), (1919, 12, 64, 0), (1920, 12, 64, 0)])
+def test_router_rows_do_not_depend_on_the_pass(rows, splits, E, I_sh):
+    """A long pass, by warps or (with many planes) by blocks, gives every row what a short pass gives it, bit for bit."""
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    torch.manual_seed(rows)
+    topk, ntot = 6, E + 2 * I_sh
+    planes, bias = torch.randn(splits, rows, ntot, device="cuda"), torch.randn(E, device="cuda") * 0.1
+    planes[:, 3, :E] = 0.5
+    planes[0, 5, 0] = float("inf")
+
+    def run(part):
+        n = part.shape[1]
+        part = part.contiguous()
+        ids, wts = torch.zeros(n, topk, dtype=torch.int32, device="cuda"), torch.zeros(n, topk, device="cuda")
+        act = torch.zeros(n, max(I_sh, 1), device="cuda", dtype=torch.bfloat16)
+        lib.check(k.ds41_router_select(lib.ptr(part), splits, n, ntot, E, I_sh, topk, lib.ptr(bias), C.c_float(1.5), C.c_float(10.0),
+                                       lib.ptr(ids), lib.ptr(wts), lib.ptr(act), lib.stream()), "router")
+        torch.cuda.synchronize()
+        return ids, wts.view(torch.int32), act.view(torch.int16)
+
+    whole, parts = run(planes), [run(planes[:, r:r + 100]) for r in range(0, rows, 100)]
+    for i, w in enumerate(whole):
+        assert torch.equal(w, torch.cat([p[i] for p in parts]))
