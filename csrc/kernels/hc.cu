@@ -406,7 +406,6 @@ hc_expand_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_out, Pa
 // row's two barriers.  Here a producer thread brings whole rows (streams, plane, coefficients) into a ring by bulk copies and
 // two groups of 256 threads take them in turn, one CTA per SM: 179 us, 5.2 TB/s.  A thread's columns and every sum's order are
 // those of hc_expand_kernel, so the results are the same bits.
-constexpr int kStreamRows = 256;       // passes from here on (333 rows: 20.8 us as a block per row, 15.6 so)
 constexpr int kStreamGroups = 2, kStreamThreads = 256 * kStreamGroups + 32;
 struct StreamRing {
   int plane_off, coef_off, stage_bytes, stages;
@@ -778,11 +777,14 @@ extern "C" int ds41_hc_post_mix(const void* streams_in, void* streams_out, const
   const int slices = H / kHcSlice;
   int rpb = rows * slices / (2 * 148) / kHcRowsPerBlock * kHcRowsPerBlock;
   rpb = rpb < kHcRowsPerBlock ? kHcRowsPerBlock : (rpb > 64 ? 64 : rpb);
-  // long passes of one rank: rows through a ring in shared memory, where copies of whole rows are possible (16-byte pieces)
+  // long passes of one rank: rows through a ring in shared memory, where copies of whole rows are possible (16-byte pieces) and
+  // blocks of a row each no longer run all at once (two an SM; 5120 columns, us as blocks / through the ring: 256 rows without
+  // a plane 5.3 / 5.6, 300 rows 8.9 / 7.6 and with a plane 15.2 / 12.3)
   const bool aligned = ((reinterpret_cast<uintptr_t>(streams_in) | reinterpret_cast<uintptr_t>(post) |
                          reinterpret_cast<uintptr_t>(comb) | reinterpret_cast<uintptr_t>(pre_in) |
                          reinterpret_cast<uintptr_t>(n_ranks > 0 ? parts.base[0] : nullptr)) & 15) == 0;
-  if (fn == nullptr && xn != nullptr && n_ranks <= 1 && (n_ranks == 0 || n_splits == 1) && rows >= kStreamRows && aligned) {
+  if (fn == nullptr && xn != nullptr && n_ranks <= 1 && (n_ranks == 0 || n_splits == 1) && rows > 2 * sm_count() &&
+      aligned) {
     const StreamRing ring = stream_ring(H, n_ranks > 0);
     static std::atomic<bool> ready[64];
     int dev = 0;

@@ -804,3 +804,10 @@ def test_router_rows_do_not_depend_on_the_pass(rows, splits, E, I_sh):
     whole, parts = run(planes), [run(planes[:, r:r + 100]) for r in range(0, rows, 100)]
     for i, w in enumerate(whole):
         assert torch.equal(w, torch.cat([p[i] for p in parts]))
+
+
+@pytest.mark.parametrize("rows", [296, 297])
+@pytest.mark.parametrize("expand", [False, True])
+def test_expand_on_both_sides_of_the_rule(rows, expand):
+    """Two blocks an SM still hold 296 rows at once on 148 SMs; one more goes through the ring."""
+    test_expand_of_long_passes_matches_short_ones(1024, rows, expand, True)
