@@ -18,6 +18,7 @@
 #include "ds41_api.h"
 #include "ds41_launch.cuh"
 #include "ds41_ptx.cuh"
+#include "ds41_tma.h"
 
 namespace ds41 {
 
@@ -60,7 +61,12 @@ struct HcStepParams {
   int* status;
 };
 
-__global__ void __launch_bounds__(256, 3) hc_step_kernel(HcStepParams p) {
+// EARLY: the whole grid is on the GPU at once (three blocks an SM) and the launch is one chain of latencies, so every step's
+// operands are fetched ahead and held in registers.  Larger grids want more blocks an SM instead.  us, held / not: 8 rows of
+// 5120 columns 14.6 / 16.8, 16 rows of 16 planes 22.4 / 21.4, 64 rows 40.6 / 36.0; 16 rows of 7168 columns 23.3 / 21.4.
+constexpr int kEarlyBlocks = 3;
+template <bool EARLY>
+__global__ void __launch_bounds__(256, EARLY ? kEarlyBlocks : 4) hc_step_kernel(HcStepParams p) {
   __shared__ float xs[kMult][kSlice];
   __shared__ float sqc[kSlice];
   __shared__ float proj[kStride];
@@ -69,17 +75,19 @@ __global__ void __launch_bounds__(256, 3) hc_step_kernel(HcStepParams p) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_slices = gridDim.x;
   pdl_launch_dependents();
-  // The launch is one chain of latencies (H 5120: 17.9 us for 1 row and 22.8 for 16 when each step loaded what it needed, 15.1
-  // and 20.9 now), so what does not depend on the previous kernel is fetched while that one ends: this warp's three rows of the
-  // mixing matrix (2 MB in all, from HBM when much weight has passed since the last layer).
+  // What does not depend on the previous kernel is fetched while that one ends: this warp's three rows of the mixing matrix
+  // (2 MB in all, from HBM when much weight has passed since the last layer).
   constexpr int kMixSteps = kMult * kSlice / 32;
-  float fn[3][kMixSteps];
-#pragma unroll
-  for (int i = 0; i < kMixSteps; ++i) {
+  float fn[3][EARLY ? kMixSteps : 1];
+  auto mix_row = [&](int j, int i) {
     const int idx = lane + 32 * i;
+    return __ldg(p.fn + 1ll * (warp + 8 * j) * (kMult * H) + 1ll * (idx / kSlice) * H + c0 + idx % kSlice);
+  };
+  if constexpr (EARLY) {
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      fn[j][i] = __ldg(p.fn + 1ll * (warp + 8 * j) * (kMult * H) + 1ll * (idx / kSlice) * H + c0 + idx % kSlice);
+    for (int i = 0; i < kMixSteps; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) fn[j][i] = mix_row(j, i);
   }
   pdl_wait();
   if (p.wait_flags != nullptr && p.parts.n_ranks > 1) {
@@ -143,12 +151,12 @@ __global__ void __launch_bounds__(256, 3) hc_step_kernel(HcStepParams p) {
   {
     float dot[3] = {0.f, 0.f, 0.f};
     float sq = 0.f;
-#pragma unroll
+#pragma unroll (EARLY ? kMixSteps : 8)
     for (int i = 0; i < kMixSteps; ++i) {
       const int idx = lane + 32 * i;
       const float x = xs[idx / kSlice][idx % kSlice];
 #pragma unroll
-      for (int j = 0; j < 3; ++j) dot[j] = fmaf(x, fn[j][i], dot[j]);
+      for (int j = 0; j < 3; ++j) dot[j] = fmaf(x, EARLY ? fn[j][EARLY ? i : 0] : mix_row(j, i), dot[j]);
       sq = fmaf(x, x, sq);
     }
 #pragma unroll
@@ -175,10 +183,10 @@ __global__ void __launch_bounds__(256, 3) hc_step_kernel(HcStepParams p) {
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // all that the finish reads is asked for at once: this warp's sums over the slices, the collapsed row, the norm weight
+  // EARLY: all that the finish reads is asked for at once: this warp's sums over the slices, the collapsed row, the norm weight
   const int n_items = H / 8;
-  constexpr int kHeld = 3;                 // pieces of eight columns that a thread holds from here on
-  float4 xa[kHeld], xb[kHeld], wa[kHeld], wb[kHeld];
+  constexpr int kHeld = EARLY ? 3 : 0;     // pieces of eight columns that a thread holds from here on
+  float4 xa[kHeld + 1], xb[kHeld + 1], wa[kHeld + 1], wb[kHeld + 1];
   auto fetch = [&](int i, float4& a, float4& b, float4& u, float4& v) {
     a = b = make_float4(0.f, 0.f, 0.f, 0.f);
     u = v = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -336,7 +344,10 @@ extern "C" int ds41_hc_step(const ds41_hc_step_args* a, void* stream) {
   p.rows = a->rows; p.H = a->H; p.iters = a->iters;
   p.hc_eps = a->hc_eps; p.norm_eps = a->norm_eps;
   p.wait_flags = a->wait_flags; p.wait_epoch = a->wait_epoch; p.status = a->status;
-  return launch_pdl(hc_step_kernel, dim3(a->H / kSlice, a->rows), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
+  const dim3 grid(a->H / kSlice, a->rows);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (1ll * grid.x * grid.y <= 1ll * kEarlyBlocks * sm_count()) return launch_pdl(hc_step_kernel<true>, grid, dim3(256), 0, st, p);
+  return launch_pdl(hc_step_kernel<false>, grid, dim3(256), 0, st, p);
 }
 
 // ---------------------------------------------------------------------------------------------------

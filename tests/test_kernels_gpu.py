@@ -811,3 +811,49 @@ def test_router_rows_do_not_depend_on_the_pass(rows, splits, E, I_sh):
 def test_expand_on_both_sides_of_the_rule(rows, expand):
     """Two blocks an SM still hold 296 rows at once on 148 SMs; one more goes through the ring."""
     test_expand_of_long_passes_matches_short_ones(1024, rows, expand, True)
+
+
+@pytest.mark.parametrize("rows,H,splits", [(55, 1024, 1), (56, 1024, 16), (11, 5120, 4), (12, 5120, 4), (3, 6272, 2), (9, 6272, 2),
+                                           (7, 7168, 1), (8, 7168, 16)])
+def test_hc_step_rows_do_not_depend_on_the_pass(rows, H, splits):
+    """Small grids hold their operands in registers, larger ones load them when needed; rows beyond 6144 columns go on in
+    further pieces.  Every row is what a launch of its own gives, bit for bit, and what the plain statement gives."""
+    from ds41rt_b200.models import reference as R
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    torch.manual_seed(rows + H)
+    streams, sub = torch.randn(rows, 4, H, device="cuda").bfloat16(), torch.randn(splits, rows, H, device="cuda")
+    fn, scale, base = torch.randn(24, 4 * H, device="cuda") * 0.02, torch.tensor([1.0, 0.7, 1.3], device="cuda"), torch.randn(24, device="cuda") * 0.5
+    pre, post = torch.rand(rows, 4, device="cuda"), torch.rand(rows, 4, device="cuda") * 2
+    comb, norm_w = torch.rand(rows, 16, device="cuda") * 0.5, torch.rand(H, device="cuda") + 0.5
+    st = lib.new_status("cuda")
+
+    def run(r0, r1):
+        n = r1 - r0
+        part = sub[:, r0:r1].contiguous()
+        bases = (C.c_void_p * 1)(part.data_ptr())
+        src, p_in, p_out, cb = (t[r0:r1].contiguous() for t in (streams, pre, post, comb))
+        z = lambda *s, dt=torch.float32: torch.zeros(*s, device="cuda", dtype=dt)
+        out = [torch.empty_like(src), z(n, 4), z(n, 4), z(n, 16), z(n, H, dt=torch.bfloat16), z(n, H, dt=torch.uint8), z(n, H)]
+        scratch = [z(H // 128, n, 26), z(n, H), z(n, dt=torch.int32), z(1, H // 128, 512, dt=torch.uint8)]
+        a = lib.HcStepArgs()
+        a.streams_in, a.part_bases = lib.ptr(src), C.cast(bases, C.c_void_p)
+        a.streams_out, a.next_pre, a.post_out, a.comb_out, a.xn, a.xq, a.tap_mean = (lib.ptr(t) for t in out)
+        a.partial, a.xc, a.tickets, a.xq_sf = (lib.ptr(t) for t in scratch)
+        a.post, a.comb, a.pre_in, a.fn, a.scale, a.base, a.norm_w = (lib.ptr(t) for t in (p_out, cb, p_in, fn, scale, base, norm_w))
+        a.status, a.split_stride, a.n_ranks, a.n_splits = lib.ptr(st), n * H, 1, splits
+        a.rows, a.H, a.iters, a.hc_eps, a.norm_eps = n, H, 20, 1e-6, 1e-20
+        lib.check(k.ds41_hc_step(C.byref(a), lib.stream()), "hc_step")
+        torch.cuda.synchronize()
+        assert not bool(scratch[2].any())
+        return out
+
+    whole, single = run(0, rows), [run(r, r + 1) for r in range(rows)]
+    for i, w in enumerate(whole):
+        assert torch.equal(w, torch.cat([s[i] for s in single])), i
+    y = sub.sum(0).bfloat16().double()
+    new = torch.einsum("rsd,rsh->rdh", comb.view(rows, 4, 4).double(), streams.double()) + post.double()[..., None] * y[:, None]
+    x = torch.einsum("rs,rsh->rh", pre.double(), whole[0].double())
+    xn = x * torch.rsqrt((x * x).mean(-1, keepdim=True)) * norm_w.double()
+    assert float((whole[0].double() - new).abs().max()) < 2.0 ** -7 * float(new.abs().max())
+    assert float((whole[4].double() - xn).abs().max()) < 2.0 ** -6 * float(xn.abs().max())
