@@ -347,7 +347,9 @@ extern "C" int ds41_qkv_post(const float* planes, int splits, int rows, int ntot
   QkvPostParams p{planes, splits, rows, ntot, Q, D, rope_dim, extra_f32, index_heads, index_scale, q_norm_w,
                   kv_norm_w, inv_freq, row_pos, row_slot, static_cast<__nv_bfloat16*>(q_lat),
                   static_cast<__nv_bfloat16*>(win), ring, kv_row_bytes, extras, eps};
-  if ((Q + D) & 1) return cudaErrorInvalidValue;   // kv columns are read as aligned float2
+  // kv columns are read as aligned float2
+  if (((Q + D) & 1) || ((ntot & 1) && (rows > 1 || splits > 1)) || (reinterpret_cast<uintptr_t>(planes) & 7))
+    return cudaErrorInvalidValue;
   return launch_pdl(qkv_post_kernel, dim3(rows, p.extra_f32 > 0 ? 3 : 2), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
 }
 

@@ -857,3 +857,23 @@ def test_hc_step_rows_do_not_depend_on_the_pass(rows, H, splits):
     xn = x * torch.rsqrt((x * x).mean(-1, keepdim=True)) * norm_w.double()
     assert float((whole[0].double() - new).abs().max()) < 2.0 ** -7 * float(new.abs().max())
     assert float((whole[4].double() - xn).abs().max()) < 2.0 ** -6 * float(xn.abs().max())
+
+
+def test_qkv_post_refuses_rows_at_odd_columns():
+    """kv columns are read in pairs: an odd row length with further rows or planes, or a base between pairs, is refused."""
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    Q, D = 64, 64
+
+    def call(splits, rows, ntot, offset=0):
+        planes, one = torch.zeros(splits * rows * ntot + 4, device="cuda"), torch.ones(256, device="cuda")
+        i32 = torch.zeros(4, dtype=torch.int32, device="cuda")
+        out = torch.zeros(4, 2048, device="cuda")
+        err = k.ds41_qkv_post(C.c_void_p(planes.data_ptr() + offset), splits, rows, ntot, Q, D, 32, 0, 0, C.c_float(1.0), lib.ptr(one),
+                              lib.ptr(one), lib.ptr(one), lib.ptr(i32), lib.ptr(i32), lib.ptr(out[0]), lib.ptr(out[1]), 4,
+                              lib.ptr(out[2]), C.c_float(1e-6), 0, lib.stream())
+        torch.cuda.synchronize()
+        return err
+
+    assert call(1, 2, 129) != 0 and call(2, 1, 129) != 0 and call(1, 1, 128, offset=4) != 0
+    assert call(1, 1, 129) == 0 and call(2, 3, 130) == 0
