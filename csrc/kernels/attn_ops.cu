@@ -89,7 +89,10 @@ struct QkvPostParams {
   float eps;
 };
 
-// grid (rows, 2): block y == 0 normalises the q latent, y == 1 handles kv (norm + RoPE + ring write) and extras.
+constexpr int kFewPlanes = 7;
+constexpr int kOwnExtras = 256;       // up to one column a thread: 200 rows, 8 columns of 10 planes 7.0 us in the kv block, 7.5 in a third
+// grid (rows, 2 or 3): block y == 0 normalises the q latent, y == 1 handles kv (norm + RoPE + ring write), and the extras unless
+// there are enough for a block y == 2.
 __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
   __shared__ float scratch[8];
   const int r = blockIdx.x, tid = threadIdx.x;
@@ -99,17 +102,27 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
   const float* row0 = p.planes + 1ll * r * p.ntot;
   if (blockIdx.y == 0) {
     // ---- q latent (Q <= 2048: up to 8 columns per thread, all split loads issued together)
-    // the planes outside, the columns inside: four planes of all columns in flight (a decode pass waits for little else:
-    // 10.7 -> 9.0 us on average, 8192 rows 78 -> 55)
+    // Few planes: the planes outside, the columns inside, four planes of all columns in flight.  Many planes: one column after
+    // the other, which the compiler pipelines better.  The order of a column's sum is the same.  16 rows of 1280 + 512 columns,
+    // us with columns / planes inside: 1 plane 2.3 / 3.4, 6 planes 4.2 / 5.4, 8 planes 4.8 / 4.6, 12 planes 6.1 / 5.5.
     float vals[8];
     float sq = 0.f;
 #pragma unroll
     for (int n = 0; n < 8; ++n) vals[n] = 0.f;
+    if (p.splits <= kFewPlanes) {
 #pragma unroll 4
-    for (int s = 0; s < p.splits; ++s)
+      for (int s = 0; s < p.splits; ++s)
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+          if (tid + 256 * n < p.Q) vals[n] += row0[s * plane + tid + 256 * n];
+    } else {
 #pragma unroll
       for (int n = 0; n < 8; ++n)
-        if (tid + 256 * n < p.Q) vals[n] += row0[s * plane + tid + 256 * n];
+        if (tid + 256 * n < p.Q) {
+#pragma unroll 4
+          for (int s = 0; s < p.splits; ++s) vals[n] += row0[s * plane + tid + 256 * n];
+        }
+    }
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       vals[n] = bf16_round(vals[n]);
@@ -124,8 +137,8 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
     }
     return;
   }
-  if (blockIdx.y == 2) {
-    // ---- extras (fp32 pass-through; index weights scaled)
+  // ---- extras (fp32 pass-through; index weights scaled): in a block of their own, or a few by the kv block
+  auto extras = [&]() {
     for (int c0 = tid; c0 < p.extra_f32; c0 += 256 * 4) {
       float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
@@ -140,8 +153,8 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
         p.extras[1ll * r * p.extra_f32 + c] = c >= p.extra_f32 - p.index_heads ? a[n] * p.index_scale : a[n];
       }
     }
-    return;
-  }
+  };
+  if (blockIdx.y == 2) return extras();
   // ---- kv: thread handles adjacent pairs so RoPE stays in-thread (D <= 2048)
   const int pos = p.row_pos[r], slot = p.row_slot[r];
   float2 kvv[4];
@@ -194,6 +207,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
       reinterpret_cast<__nv_bfloat162*>(dst)[i] = __floats2bfloat162_rn(a, b);
     }
   }
+  if (gridDim.y == 2) extras();
 }
 
 struct CompressParams {
@@ -350,7 +364,7 @@ extern "C" int ds41_qkv_post(const float* planes, int splits, int rows, int ntot
   // kv columns are read as aligned float2
   if (((Q + D) & 1) || ((ntot & 1) && (rows > 1 || splits > 1)) || (reinterpret_cast<uintptr_t>(planes) & 7))
     return cudaErrorInvalidValue;
-  return launch_pdl(qkv_post_kernel, dim3(rows, p.extra_f32 > 0 ? 3 : 2), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
+  return launch_pdl(qkv_post_kernel, dim3(rows, extra_f32 > kOwnExtras ? 3 : 2), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
 }
 
 extern "C" int ds41_compress(const float* extras, int extra_stride, int rows, int D, int ID, int rope_dim, int ratio,

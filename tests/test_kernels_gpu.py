@@ -877,3 +877,41 @@ def test_qkv_post_refuses_rows_at_odd_columns():
 
     assert call(1, 2, 129) != 0 and call(2, 1, 129) != 0 and call(1, 1, 128, offset=4) != 0
     assert call(1, 1, 129) == 0 and call(2, 3, 130) == 0
+
+
+@pytest.mark.parametrize("rows,Q,extra", [(1, 1280, 0), (3, 2048, 6), (2, 96, 256), (2, 1280, 258), (2, 300, 1300)])
+def test_qkv_post_sums_planes_in_their_order(rows, Q, extra):
+    """Few planes (columns inside) and many (planes inside), extras in the kv block and in one of their own: the same bits, since
+    further planes of zeros change no sum."""
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    torch.manual_seed(Q + extra)
+    D, rope, heads = 512, 64, min(extra, 4)
+    ntot = Q + D + extra
+    planes = torch.randn(5, rows, ntot, device="cuda")
+    qn, kn, inv = torch.rand(Q, device="cuda") + 0.5, torch.rand(D, device="cuda") + 0.5, torch.rand(rope // 2, device="cuda")
+    pos, slot = torch.arange(7, 7 + rows, dtype=torch.int32, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda")
+    got = []
+    for n in (5, 7, 8, 16):
+        pl = torch.zeros(n, rows, ntot, device="cuda")
+        pl[:5] = planes
+        ql, win = torch.zeros(rows, Q, device="cuda", dtype=torch.bfloat16), torch.zeros(1, 32, D, device="cuda", dtype=torch.bfloat16)
+        ex = torch.full((rows, extra + 1), 7.0, device="cuda")
+        lib.check(k.ds41_qkv_post(lib.ptr(pl), n, rows, ntot, Q, D, rope, extra, heads, C.c_float(0.25), lib.ptr(qn), lib.ptr(kn),
+                                  lib.ptr(inv), lib.ptr(pos), lib.ptr(slot), lib.ptr(ql), lib.ptr(win), 32, lib.ptr(ex),
+                                  C.c_float(1e-6), 0, lib.stream()), "qkv_post")
+        torch.cuda.synchronize()
+        got.append((ql, win, ex))
+    for g in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], g))
+    total = planes[0].clone()
+    for p in planes[1:]:
+        total += p
+    want = total[:, Q + D:].clone()
+    want[:, extra - heads:] *= 0.25
+    ql, win, ex = got[0]
+    assert torch.equal(ex.view(-1)[: rows * extra].view(rows, extra), want) and bool((ex.view(-1)[rows * extra:] == 7.0).all())
+    q = total[:, :Q].bfloat16().double()
+    ref = q * torch.rsqrt((q * q).mean(-1, keepdim=True) + 1e-6) * qn.double()
+    assert float((ql.double() - ref).abs().max()) < 2.0 ** -7 * float(ref.abs().max())
+    assert bool(win[0, 7:7 + rows].any(-1).all()) and not bool(win[0, :7].any())
