@@ -1,4 +1,4 @@
-// Grammar-mask token sampler on the GPU: a cluster of eight 1024-thread CTAs per row.
+// Grammar-mask token sampler on the GPU: one, two, four or eight 1024-thread CTAs per row.
 //
 // Same rule as the host oracle (csrc/core/sampler.cc): allow-mask -> temperature -> min_p -> top_k -> top_p ->
 // categorical draw with a SplitMix64 (seed, position) uniform; greedy when T < 1e-5 or top_k == 1 (strict whole-row
@@ -15,7 +15,6 @@
 #include <cooperative_groups.h>
 
 #include <atomic>
-#include <utility>
 
 #include "ds41_api.h"
 #include "ds41_launch.cuh"
@@ -58,13 +57,13 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
   return static_cast<float>(static_cast<uint32_t>(x >> 40)) * (1.0f / 16777216.0f);
 }
 
-// A row is shared by a cluster of eight CTAs.  One CTA per row walked 517 KB up to fifteen times from L2 with a fraction of one
-// SM's bandwidth: 780 us for sixteen rows of 129280 logits.  Now each CTA reads its eighth once, keeps the order keys of the
+// A row is shared by a cluster of up to eight CTAs.  One CTA per row walked 517 KB up to fifteen times from L2 with a fraction of
+// one SM's bandwidth: 780 us for sixteen rows of 129280 logits.  Now each CTA reads its part once, keeps the order keys of the
 // scaled logits in shared memory, and only histograms, sums and short lists travel, through distributed shared memory: 68 us for
-// the same rows.  Every CTA draws the same conclusions from the same integers, so there is no broadcast step and all control
-// flow is uniform in the cluster.  What is left is a chain of cluster barriers (2000 cycles each) and of passes over the keys
-// (5000 to 7000 cycles); the reads from memory are 2 % of it.
-constexpr int kSampleCluster = 8;
+// the same rows, eight CTAs each.  Every CTA draws the same conclusions from the same integers, so there is no broadcast step and
+// all control flow is uniform in the cluster.  What is left is a chain of cluster barriers (2000 cycles each) and of passes over
+// the keys (5000 to 7000 cycles); the reads from memory are 2 % of it.
+constexpr int kSampleMaxCluster = 8;
 constexpr int kSampleMaxSlice = 49152;     // keys per CTA that fit its shared memory; longer slices are read again from L2
 
 struct SamplePart {                        // what one CTA found in its slice
@@ -88,15 +87,15 @@ struct SampleShared {
   alignas(8) unsigned int mass[2][3][256];
   unsigned int tot_cnt[256];
   unsigned long long tot_mass[256];
-  SamplePart part[kSampleCluster];
-  unsigned long long slot[3][kSampleCluster];      // one exchange each
+  SamplePart part[kSampleMaxCluster];
+  unsigned long long slot[3][kSampleMaxCluster];      // one exchange each
   unsigned long long warp[kSampleThreads / 32];
   SamplePart warp_part[kSampleThreads / 32];
   unsigned long long total;                        // weight of a selection's candidates
   double remaining;
   unsigned int digit, tie_count, best_key, n_above;
   int token;
-  unsigned int own_n, far_n[kSampleCluster];
+  unsigned int own_n, far_n[kSampleMaxCluster];
   uint2 own_list[kSampleList];                     // {key, token} of this CTA's members
   int n_list;                                      // members of the last selection that were gathered; -1: too many
   int list_id[kSampleList + 1];
@@ -126,19 +125,35 @@ struct CandSet {
   unsigned long long tie_mult;
 };
 
+// The CTAs that share a row: a cluster, or one CTA by itself.
+template <int CL>
+struct SamplePeers {
+  __device__ __forceinline__ unsigned rank() const { return CL == 1 ? 0u : cg::this_cluster().block_rank(); }
+  __device__ __forceinline__ void sync() const {
+    if constexpr (CL == 1) __syncthreads();
+    else cg::this_cluster().sync();
+  }
+  template <class T>
+  __device__ __forceinline__ T* of(T* mine, int rank) const {
+    if constexpr (CL == 1) return mine;
+    else return cg::this_cluster().map_shared_rank(mine, rank);
+  }
+};
+
 // Sum over the cluster; `slot` is used once per launch, so no second barrier protects it.
-__device__ unsigned long long cluster_sum(SampleShared& sh, cg::cluster_group& cl, int slot, unsigned long long v) {
+template <int CL>
+__device__ unsigned long long cluster_sum(SampleShared& sh, SamplePeers<CL> cl, int slot, unsigned long long v) {
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   if ((threadIdx.x & 31) == 0) sh.warp[threadIdx.x >> 5] = v;
   __syncthreads();
   if (threadIdx.x < 32) {
     unsigned long long mine = sh.warp[threadIdx.x];
     for (int off = 16; off > 0; off >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, off);
-    if (threadIdx.x < kSampleCluster) *cl.map_shared_rank(&sh.slot[slot][cl.block_rank()], threadIdx.x) = mine;
+    if (threadIdx.x < CL) *cl.of(&sh.slot[slot][cl.rank()], threadIdx.x) = mine;
   }
   cl.sync();
   unsigned long long all = 0;
-  for (int c = 0; c < kSampleCluster; ++c) all += sh.slot[slot][c];
+  for (int c = 0; c < CL; ++c) all += sh.slot[slot][c];
   return all;
 }
 
@@ -150,9 +165,10 @@ __device__ __forceinline__ uint32_t bucket_of(uint32_t key, float max_scaled) {
   return 255u - (d >= 255.0f ? 255u : static_cast<uint32_t>(d));
 }
 
-// Every CTA gathers the members of all slices that `is_member` names (fewer than kSampleList) and the tie group, if it takes part.
-template <class F>
-__device__ void gather_members(SampleShared& sh, cg::cluster_group& cl, const SampleSlice& row, float max_scaled,
+// Every CTA gathers the members of all slices that `is_member` names (fewer than kSampleList) and the tie group, if it takes
+// part.
+template <int CL, class F>
+__device__ void gather_members(SampleShared& sh, SamplePeers<CL> cl, const SampleSlice& row, float max_scaled,
                                const CandSet& set, bool by_mass, bool tie, F is_member) {
   const int tid = threadIdx.x;
   for (int i = tid; i < row.n; i += kSampleThreads) {
@@ -163,19 +179,19 @@ __device__ void gather_members(SampleShared& sh, cg::cluster_group& cl, const Sa
     }
   }
   cl.sync();
-  if (tid < kSampleCluster) sh.far_n[tid] = *cl.map_shared_rank(&sh.own_n, tid);
+  if (tid < CL) sh.far_n[tid] = *cl.of(&sh.own_n, tid);
   __syncthreads();
-  constexpr int kPer = kSampleThreads / kSampleCluster;      // threads that read one peer's members
+  constexpr int kPer = kSampleThreads / CL;      // threads that read one peer's members
   const int from = tid / kPer;
   int before = 0, n = 0;
 #pragma unroll
-  for (int r = 0; r < kSampleCluster; ++r) {
+  for (int r = 0; r < CL; ++r) {
     before = r == from ? n : before;
     n += static_cast<int>(sh.far_n[r]);
   }
   n = min(n, kSampleList);
   for (int i = tid % kPer; i < static_cast<int>(sh.far_n[from]) && before + i < kSampleList; i += kPer) {
-    const uint2 m = *cl.map_shared_rank(&sh.own_list[i], from);
+    const uint2 m = *cl.of(&sh.own_list[i], from);
     sh.list[before + i] = {m.x, 1u, by_mass ? weight_fx(key_value(m.x), max_scaled) : 1ull};
     sh.list_id[before + i] = static_cast<int>(m.y);
   }
@@ -224,11 +240,13 @@ __device__ uint32_t solve_list(SampleShared& sh, bool tie, double target, double
   return best;
 }
 
-// Selection by five digits (the bucket, then the bytes of the key), high keys first.  by_mass: find the key at which the running weight reaches the target; else the key at
-// which the running count reaches it.  `frac` >= 0: the target is that share of the set's weight, which is left in sh.total.
+// Selection by five digits (the bucket, then the bytes of the key), high keys first.  by_mass: find the key at which the running
+// weight reaches the target; else the key at which the running count reaches it.  `frac` >= 0: the target is that share of the
+// set's weight, which is left in sh.total.
 // On return sh.remaining is what the ties at the returned key must still supply and sh.tie_count how many candidates carry it.
 // `pass` counts the histograms of the launch.
-__device__ uint32_t radix_select(SampleShared& sh, cg::cluster_group& cl, const SampleSlice& row, float max_scaled, CandSet set,
+template <int CL>
+__device__ uint32_t radix_select(SampleShared& sh, SamplePeers<CL> cl, const SampleSlice& row, float max_scaled, CandSet set,
                                  bool by_mass, double target, double frac, int& pass) {
   const int tid = threadIdx.x, lane = tid & 31;
   uint32_t prefix = 0, prefix_mask = 0, bucket = 0;
@@ -273,7 +291,7 @@ __device__ uint32_t radix_select(SampleShared& sh, cg::cluster_group& cl, const 
         if (lane == __ffs(peers) - 1) atomicAdd(&cnt[d], static_cast<unsigned>(__popc(peers)));
       }
     }
-    if (cl.block_rank() == 0 && tid == 0 && set.tie_mult > 0 && member(set.tie_key)) {
+    if (cl.rank() == 0 && tid == 0 && set.tie_mult > 0 && member(set.tie_key)) {
       const uint32_t d = digit(set.tie_key);
       atomicAdd(&cnt[d], static_cast<unsigned int>(set.tie_mult));
     }
@@ -282,13 +300,13 @@ __device__ uint32_t radix_select(SampleShared& sh, cg::cluster_group& cl, const 
       unsigned int c = 0;
       unsigned long long m = 0;
 #pragma unroll
-      for (int r = 0; r < kSampleCluster; ++r) {
-        c += *cl.map_shared_rank(&cnt[tid], r);
+      for (int r = 0; r < CL; ++r) {
+        c += *cl.of(&cnt[tid], r);
         if (by_mass && row.wide)
-          m += *cl.map_shared_rank(reinterpret_cast<unsigned long long*>(mass[0]) + tid, r);
+          m += *cl.of(reinterpret_cast<unsigned long long*>(mass[0]) + tid, r);
         else if (by_mass)
-          m += *cl.map_shared_rank(&mass[0][tid], r) + (static_cast<unsigned long long>(*cl.map_shared_rank(&mass[1][tid], r)) << 14) +
-               (static_cast<unsigned long long>(*cl.map_shared_rank(&mass[2][tid], r)) << 28);
+          m += *cl.of(&mass[0][tid], r) + (static_cast<unsigned long long>(*cl.of(&mass[1][tid], r)) << 14) +
+               (static_cast<unsigned long long>(*cl.of(&mass[2][tid], r)) << 28);
       }
       if (by_mass && set.tie_mult > 0 && member(set.tie_key) && digit(set.tie_key) == static_cast<uint32_t>(tid))
         m += set.tie_mult * weight_fx(key_value(set.tie_key), max_scaled);
@@ -370,6 +388,7 @@ __device__ uint32_t radix_select(SampleShared& sh, cg::cluster_group& cl, const 
   return prefix;
 }
 
+template <int CL>
 __global__ void __launch_bounds__(kSampleThreads)
 sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, const uint32_t* __restrict__ masks,
                    int mask_words, const ds41_sample_row* __restrict__ rows, int* __restrict__ tokens,
@@ -378,8 +397,8 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   extern __shared__ uint32_t key_store[];
   pdl_launch_dependents();
   pdl_wait();
-  cg::cluster_group cl = cg::this_cluster();
-  const int rank = static_cast<int>(cl.block_rank()), row = blockIdx.x / kSampleCluster;
+  const SamplePeers<CL> cl;
+  const int rank = static_cast<int>(cl.rank()), row = blockIdx.x / CL;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const ds41_sample_row p = rows[row];
   const uint32_t* mask = (masks != nullptr && p.mask_row >= 0) ? masks + 1ll * p.mask_row * mask_words : nullptr;
@@ -394,19 +413,19 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   if (!(p.temperature >= 0.0f) || isinf(p.temperature)) return finish(kSampleBadTemperature, 0);
   if (!(p.top_p > 0.0f) || !(p.min_p >= 0.0f) || p.min_p > 1.0f) return finish(kSampleBadParameter, 0);
   // a peer's shared memory may be touched once all CTAs of the cluster run: the wait hides behind the slice's loads
-  auto started = cl.barrier_arrive();
+  if constexpr (CL > 1) cg::cluster_group::barrier_arrive();
   const bool greedy = p.temperature < 1e-5f || p.top_k == 1;
   const float inv_t = greedy ? 1.0f : 1.0f / p.temperature;
 
   // ---- the slice: order keys, finiteness, allowed count, maximum (greedy: arg max with the lowest id on ties)
-  const int slice = ((vocab + kSampleCluster - 1) / kSampleCluster + 31) & ~31;
+  const int slice = ((vocab + CL - 1) / CL + 31) & ~31;
   SampleSlice own;
   own.id0 = min(vocab, rank * slice);
   own.n = min(vocab, own.id0 + slice) - own.id0;
   own.logits = logits + 1ll * row * ld + own.id0;
   own.mask = mask;
   own.inv_t = inv_t;
-  own.keys = slice <= kSampleMaxSlice ? key_store : nullptr;
+  own.keys = slice <= kSampleMaxSlice && (CL > 1 || !greedy) ? key_store : nullptr;
   own.wide = slice > kSampleMostPieces;
   SamplePart mine{-INFINITY, -1, 0u, 0u};
   auto take = [&](int i, float v) {
@@ -466,15 +485,15 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   merge_warp(mine);
   if (lane == 0) sh.warp_part[warp] = mine;
   __syncthreads();
-  cl.barrier_wait(std::move(started));
+  if constexpr (CL > 1) cg::cluster_group::barrier_wait();
   if (warp == 0) {
     mine = sh.warp_part[lane];
     merge_warp(mine);
-    if (lane < kSampleCluster) *cl.map_shared_rank(&sh.part[rank], lane) = mine;
+    if (lane < CL) *cl.of(&sh.part[rank], lane) = mine;
   }
   cl.sync();
   SamplePart all = sh.part[0];
-  for (int c = 1; c < kSampleCluster; ++c) merge(all, sh.part[c]);
+  for (int c = 1; c < CL; ++c) merge(all, sh.part[c]);
   if (all.bad != 0u) return finish(kSampleNonFinite, 0);
   if (all.best_i < 0 || all.allowed == 0) return finish(kSampleEmpty, 0);
   if (greedy) return finish(kSampleOk, all.best_i);
@@ -487,6 +506,48 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   const uint32_t excl0 = p.min_p > 0.0f ? order_key(min_scaled) - 1u : 0u;
   const bool filtered = p.top_k > 0 || p.top_p < 1.0f;
 
+  if (CL == 1 && !filtered) {
+    // ---- categorical over the survivors in token order: every thread owns consecutive tokens, an odd number of them, so that
+    // the threads of a warp read different banks
+    const int seg = ((own.n + kSampleThreads - 1) / kSampleThreads) | 1;
+    const int i0 = min(own.n, tid * seg), i1 = min(own.n, i0 + seg);
+    auto weight = [&](int i) -> unsigned long long {
+      const uint32_t k = own[i];
+      return k > excl0 ? weight_fx(key_value(k), max_scaled) : 0ull;
+    };
+    unsigned long long sum = 0;
+    for (int i = i0; i < i1; ++i) sum += weight(i);
+    unsigned long long before = sum;
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned long long up = __shfl_up_sync(0xffffffffu, before, off);
+      if (lane >= off) before += up;
+    }
+    before -= sum;
+    const unsigned long long total = cluster_sum(sh, cl, 0, sum);
+    for (int w = 0; w < warp; ++w) before += sh.warp[w];
+    const double target = static_cast<double>(u) * static_cast<double>(total);
+    if (tid == 0) sh.token = -1;
+    __syncthreads();
+    // the first thread whose running sum reaches the target owns the draw
+    if (sum > 0 && static_cast<double>(before + sum) >= target && (static_cast<double>(before) < target || before == 0)) {
+      for (int i = i0; i < i1; ++i) {
+        before += weight(i);
+        if (before > 0 && static_cast<double>(before) >= target) {
+          sh.token = i;
+          break;
+        }
+      }
+    }
+    __syncthreads();
+    if (sh.token < 0) {                              // rounding left the target above every sum: the last survivor wins
+      int last = -1;
+      for (int i = i1 - 1; i >= i0 && last < 0; --i)
+        if (own[i] > excl0) last = i;
+      if (last >= 0) atomicMax(&sh.token, last);
+      __syncthreads();
+    }
+    return finish(sh.token >= 0 ? kSampleOk : kSampleEmpty, sh.token);
+  }
   if (!filtered) {
     // ---- categorical over the survivors in token order: a warp owns consecutive tokens, 32 at a time
     const int per_warp = ((own.n + kSampleThreads / 32 - 1) / (kSampleThreads / 32) + 31) & ~31;
@@ -532,11 +593,11 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
     last = __reduce_max_sync(0xffffffffu, last);
     if (lane == 0) atomicMax(&sh.token, last);
     __syncthreads();
-    if (tid < kSampleCluster)
-      *cl.map_shared_rank(&sh.slot[2][rank], tid) = sh.token >= 0 ? 1ull + own.id0 + sh.token : 0ull;
+    if (tid < CL)
+      *cl.of(&sh.slot[2][rank], tid) = sh.token >= 0 ? 1ull + own.id0 + sh.token : 0ull;
     cl.sync();
     unsigned long long top = 0;
-    for (int c = 0; c < kSampleCluster; ++c) top = max(top, sh.slot[2][c]);
+    for (int c = 0; c < CL; ++c) top = max(top, sh.slot[2][c]);
     return finish(top > 0 ? kSampleOk : kSampleEmpty, static_cast<int>(top) - 1);
   }
 
@@ -616,7 +677,7 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   cluster_sum(sh, cl, 1, eq);
   long long before = 0;
   int holder = -1;
-  for (int c = 0; c < kSampleCluster; ++c) {
+  for (int c = 0; c < CL; ++c) {
     const long long here = static_cast<long long>(sh.slot[1][c]);
     if (holder < 0 && tie_index < before + here) holder = c;
     if (holder < 0) before += here;
@@ -646,21 +707,61 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
 
 using namespace ds41;
 
-extern "C" int ds41_sample_rows(const float* logits, long long ld, int rows, int vocab, const uint32_t* masks,
-                                int mask_words, const ds41_sample_row* params, int* tokens, int* status, void* stream) {
-  if (logits == nullptr || params == nullptr || tokens == nullptr || status == nullptr || rows <= 0 || vocab <= 0)
-    return cudaErrorInvalidValue;
-  if (masks != nullptr && mask_words != (vocab + 31) / 32) return cudaErrorInvalidValue;
-  const int slice = ((vocab + kSampleCluster - 1) / kSampleCluster + 31) & ~31;
+template <int CL>
+static int launch_sample(const float* logits, long long ld, int rows, int vocab, const uint32_t* masks, int mask_words,
+                         const ds41_sample_row* params, int* tokens, int* status, cudaStream_t stream) {
+  const int slice = ((vocab + CL - 1) / CL + 31) & ~31;
   const size_t smem = slice <= kSampleMaxSlice ? 4ull * slice : 0;
   static std::atomic<bool> configured[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev].load(std::memory_order_acquire)) {
-    const cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kSampleMaxSlice);
+    const cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               4 * kSampleMaxSlice);
     if (e != cudaSuccess) return e;
     configured[dev].store(true, std::memory_order_release);
   }
-  return launch_pdl_cluster(sample_rows_kernel, dim3(rows * kSampleCluster), dim3(kSampleThreads), kSampleCluster, smem,
-                            static_cast<cudaStream_t>(stream), logits, ld, vocab, masks, mask_words, params, tokens, status);
+  if constexpr (CL == 1)
+    return launch_pdl(sample_rows_kernel<CL>, dim3(rows), dim3(kSampleThreads), smem, stream, logits, ld, vocab, masks,
+                      mask_words, params, tokens, status);
+  else
+    return launch_pdl_cluster(sample_rows_kernel<CL>, dim3(rows * CL), dim3(kSampleThreads), CL, smem, stream, logits, ld, vocab,
+                              masks, mask_words, params, tokens, status);
+}
+
+// CTAs that share a row.  A row alone is fastest over eight; but about 15 clusters of eight run at once, 36 of four, 74 of two
+// and 148 single CTAs, and every CTA more costs its barriers, which short rows do not earn back.  Slices should stay in shared
+// memory.  What the rows ask for is known on the device alone, so the line is drawn by mixed passes; greedy rows by themselves,
+// which have a kernel of their own (argmax_rows), and min-p rows lose by it where many rows are long (64 x 129280: 17 -> 32 and
+// 57 -> 64 us).  us for rows that ask for plain temperature, nucleus, top-k and min-p in turn, over 8 / 4 / 2 / 1 CTAs (and one
+// CTA that reads its row from L2 up to fifteen times):
+//   2000 columns    8 rows  17 /  16 /  16 /   13  (67)     64 rows   61 /  35 /  30 /   27  (72)
+//   16000 columns                                           64 rows   84 /  52 /  38 /   41 (152)
+//   30000 columns  16 rows  34 /  38 /  47 /   64 (244)     64 rows   83 /  60 /  62 /   78 (253)
+//                                                          148 rows  196 / 119 /  88 /   72 (250)
+//   65536 columns  20 rows  51 /  61 /  99 /  213 (476)     64 rows  105 /  94 / 189 /  407 (480)
+//   129280 columns 16 rows  68 / 100 / 235 /  419 (761)     64 rows  144 / 197 / 766 / 1508 (853)
+//                                                          100 rows  222 / 178 / 393 / 1141 (855)
+static int sample_ctas(int rows, int vocab) {
+  if (vocab <= 4096) return 1;
+  if (vocab <= kSampleMaxSlice) {
+    if (vocab > 16384 && rows <= (vocab <= 32768 ? 15 : 24)) return 8;
+    return rows <= 36 ? 4 : rows <= 74 ? 2 : 1;
+  }
+  if (vocab <= 2 * kSampleMaxSlice) return rows <= 40 ? 8 : rows <= 100 ? 4 : 2;
+  return rows <= 64 || vocab > 4 * kSampleMaxSlice ? 8 : 4;
+}
+
+extern "C" int ds41_sample_rows(const float* logits, long long ld, int rows, int vocab, const uint32_t* masks,
+                                int mask_words, const ds41_sample_row* params, int* tokens, int* status, void* stream) {
+  if (logits == nullptr || params == nullptr || tokens == nullptr || status == nullptr || rows <= 0 || vocab <= 0)
+    return cudaErrorInvalidValue;
+  if (masks != nullptr && mask_words != (vocab + 31) / 32) return cudaErrorInvalidValue;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  switch (sample_ctas(rows, vocab)) {
+    case 8: return launch_sample<8>(logits, ld, rows, vocab, masks, mask_words, params, tokens, status, st);
+    case 4: return launch_sample<4>(logits, ld, rows, vocab, masks, mask_words, params, tokens, status, st);
+    case 2: return launch_sample<2>(logits, ld, rows, vocab, masks, mask_words, params, tokens, status, st);
+    default: return launch_sample<1>(logits, ld, rows, vocab, masks, mask_words, params, tokens, status, st);
+  }
 }

@@ -434,12 +434,12 @@ def test_clusters_cross_a_barrier_before_they_touch_a_peers_memory():
     seen = []
     for text in _sources().values():
         for name, body in _kernels_without_lambdas(text):
-            remote = body.find("map_shared_rank")
-            if remote < 0:
+            remote = re.search(r"map_shared_rank|\bcl\.of\(", body)
+            if remote is None:
                 continue
             seen.append(name)
-            barrier = re.search(r"\b(cl|cluster)\.(sync\(\)|barrier_wait\()", body)
-            assert barrier is not None and barrier.start() < remote, name
+            barrier = re.search(r"\b(cl|cluster)\.sync\(\)|\bcluster_group::barrier_wait\(", body)
+            assert barrier is not None and barrier.start() < remote.start(), name
     assert {"sample_rows_kernel", "argmax_rows_kernel"} <= set(seen), seen
 
 

@@ -164,3 +164,26 @@ def test_sampler_slices_of_a_row(vocab, offset):
             assert (int(st[r]) == 0) == (err == 0)
             wrong += err == 0 and int(tok[r]) != want
     assert wrong <= 1, wrong
+
+
+@pytest.mark.parametrize("vocab,counts", [(4096, (8,)), (4097, (36, 37, 75)), (20000, (15, 16, 37, 74, 75, 150)), (40000, (24, 25, 75)),
+                                          (60000, (40, 41, 101)), (100000, (64, 65))])
+def test_a_row_gets_its_token_whatever_is_sampled_beside_it(vocab, counts):
+    """How many CTAs share a row follows the number of rows and their length; sums are whole numbers, so the token does not."""
+    from ds41rt_b200.ops.sampling import RowParams, pack_params, sample_rows
+    rng = np.random.default_rng(vocab)
+    asked = [dict(temperature=0.0), dict(temperature=1.0), dict(temperature=0.7, top_p=0.8), dict(temperature=0.9, top_k=7),
+             dict(temperature=1.1, min_p=0.1), dict(temperature=1.0, top_k=2000, top_p=0.95), dict(temperature=1.4, top_p=0.999)]
+    n = max(counts)
+    dev = torch.device("cuda")
+    logits = torch.from_numpy(rng.normal(0, 2, size=(n, vocab)).astype(np.float32)).to(dev)
+    logits[1] = 0.0                                          # all equal
+    logits[2, ::2] = 3.0
+    masks = torch.from_numpy(rng.integers(0, 2 ** 32, size=(1, (vocab + 31) // 32), dtype=np.uint64).astype(np.uint32).view(np.int32)).to(dev)
+    rows = [RowParams(seed=5 + i, position=i, mask_row=0 if i % 3 == 2 else -1, **asked[i % len(asked)]) for i in range(n)]
+    alone = [sample_rows(logits[i:i + 1], pack_params([rows[i]], dev), masks) for i in range(n)]
+    tok, st = (torch.cat([a[j] for a in alone]) for j in (0, 1))
+    assert not bool(st.any())
+    for m in counts:
+        t, s = sample_rows(logits[:m], pack_params(rows[:m], dev), masks)
+        assert torch.equal(t, tok[:m]) and not bool(s.any())
