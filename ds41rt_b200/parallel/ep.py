@@ -142,12 +142,23 @@ class ExpertParallelMoE:
         """Width of this pass's expert tiles in tokens (block-scaled FP8).  Every tile streams its expert's weights, so what
         counts is how many tiles an expert of the mean size needs: around 128 rows half of the experts need a second, nearly
         empty 128-token tile, and up to 192 all of them, while one 192-token tile holds the expert and multiplies only the
-        columns it has.  Below, and where both widths need the same number, the narrow tile is cheaper.  FC1 + FC2 of 128
-        experts, 5120 x 2304, us with 128 / 192 tokens: 96 rows each 1005 / 1067, 112 1059 / 1141, 128 1334 / 1226, 150 1774 /
-        1266, 170 1770 / 1359, 192 1763 / 1700, 230 1850 / 2163, 256 2194 / 2212, 320 2549 / 2394, 384 3176 / 3032, 512 4291 /
-        3594."""
+        columns it has.  Below, and where both widths need the same number, the narrow tile is cheaper.  Experts differ around
+        their mean, and with small ones a second wide tile costs more than its weights save; a layer whose wide tiles leave
+        SMs without one keeps the narrow ones.  Whole layers, time with 128-token tiles / time with 192, at 112, 128, 152, 176,
+        192, 230, 300, 420 and 700 rows per expert:
+          128 experts of 5120 x 2304   0.95 1.14 1.35 1.29 1.05 0.89 1.16 1.09 1.17
+          48 of 5120 x 2304            1.01 1.12 1.26 1.15 1.00 0.91 1.11 1.08 1.16
+          8 of 4096 x 2048             0.99 1.13 1.12 1.08 0.92 0.89 1.03 0.98 1.10
+          32 of 4096 x 1408            0.97 1.04 1.08 1.04 0.94 0.89 1.11 0.96 1.07
+          64 of 2048 x 1024            0.95 1.04 1.06 1.02 0.89 0.98 1.04 0.95 1.04
+          16 of 2048 x 1024            1.01 1.06 1.02 1.04 0.88 0.89 0.99 0.90 1.03
+          8 of 2048 x 1024             0.94 0.93 0.93 0.90 0.87 0.87 1.06 0.86 0.98"""
         rows = tokens * self.topk / self.e_local          # every rank sends about this pass's tokens
-        self.bn = self.bn2 = 192 if 124 <= rows <= 192 or rows >= 288 else 128
+        size = self.H * self.I
+        one = 124 <= rows <= (192 if size >= 10 << 20 else 176)        # most experts fit one wide tile
+        many = rows >= 288 and size >= 4 << 20
+        fills = self.e_local * -(-self.I // 128) * -(-rows // 192) >= 128
+        self.bn = self.bn2 = 192 if (one or many) and fills else 128
 
     # ------------------------------------------------------------------ argument blocks
     def _ep_args(self, x, ids, weights, tokens) -> lib.EpArgs:

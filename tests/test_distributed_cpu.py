@@ -201,3 +201,23 @@ def test_a_failing_follower_leaves_and_the_leader_stops_launching():
     assert res[1][0] == "follower" and "site 201" in res[1][3][0], res[1]
     assert res[0][0] == "rank failure", res[0]
     assert res[0][1] == [1] and "forward failed" in res[0][2][1]
+
+
+def test_width_of_expert_tiles_follows_rows_and_the_size_of_the_layer():
+    """192 tokens where the mean expert fills one such tile but not two of 128, or many when experts are large; never where the
+    layer's wide tiles would leave SMs without one."""
+    from types import SimpleNamespace
+    from ds41rt_b200.parallel.ep import ExpertParallelMoE
+
+    def width(experts, hidden, inter, rows, topk=6):
+        ep = SimpleNamespace(topk=topk, e_local=experts, H=hidden, I=inter)
+        ExpertParallelMoE._tile(ep, -(-experts * rows // topk))
+        assert ep.bn == ep.bn2
+        return ep.bn
+
+    flagship = [width(384, 5120, 2304, r) for r in (1, 64, 123, 124, 128, 192, 193, 287, 288, 1000)]
+    assert flagship == [128] * 3 + [192] * 3 + [128] * 2 + [192] * 2
+    assert [width(32, 4096, 1408, r) for r in (64, 150, 170, 180, 192, 230, 512)] == [128, 192, 192, 128, 128, 128, 192]
+    assert [width(64, 2048, 1024, r) for r in (64, 150, 180, 230, 512)] == [128, 192, 128, 128, 128]
+    assert {width(8, 2048, 1024, r) for r in (128, 170, 192, 300, 512, 1000)} == {128}
+    assert width(4, 512, 256, 150, topk=2) == 128
