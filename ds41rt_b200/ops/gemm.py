@@ -16,6 +16,7 @@ from . import lib
 
 KIND = {"bf16": 0, "fp8": 1, "mxfp8": 2}
 _ELEM = {0: 2, 1: 1, 2: 1}
+SMS = 148                     # of a B200: splits and forms are chosen by it, so that a result does not depend on the device found
 
 
 def pick_bn(rows: int) -> int:
@@ -25,7 +26,7 @@ def pick_bn(rows: int) -> int:
     return 128
 
 
-def pick_splits(m: int, k: int, kind: int = 0, max_ctas: int = 148, max_splits: int = 16, n_tiles: int = 1,
+def pick_splits(m: int, k: int, kind: int = 0, max_ctas: int = SMS, max_splits: int = 16, n_tiles: int = 1,
                 batch: int = 1) -> int:
     """Largest split-K factor that keeps the grid within one wave of `max_ctas` CTAs (no empty split)."""
     bk = 128 // _ELEM[kind]
@@ -93,7 +94,7 @@ def wide(rows: int, n: int, batch: int = 1) -> bool:
     and activation byte then serves twice the products of a 128 x 128 tile of the swapped form, and results leave in TMA
     stores (8192 rows x 33k x 1280: 954 us swapped, 545 us wide; 333 rows: 65 and 47) - once such tiles fill the GPU;
     below that the swapped form's smaller tiles and its split over K keep more SMs busy."""
-    return rows > 128 and -(-rows // 128) * -(-n // 256) * batch >= 148
+    return rows > 128 and -(-rows // 128) * -(-n // 256) * batch >= SMS
 
 
 def linear_planes(x: torch.Tensor, w: torch.Tensor, planes: torch.Tensor, splits: int, *, status=None, signal=None):

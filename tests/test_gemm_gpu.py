@@ -175,3 +175,92 @@ def test_fp32_rows_of_a_tile_table_end_with_their_group(bn):
         held[c0:c1] = True
     assert _rel(got[:M, held], want[:M, held]) < 2e-3
     assert bool((got[:, ~held] == 7.0).all()) and bool((got[M:] == 7.0).all())
+
+
+def _swapped_and_wide(rows, N, K, seed=0):
+    g = torch.Generator().manual_seed(rows + N + seed)
+    x, w = torch.randn(rows, K, generator=g).bfloat16().cuda(), (torch.randn(N, K, generator=g) * 0.05).bfloat16().cuda()
+    return x, w
+
+
+@pytest.mark.parametrize("rows,N,K", [(129, 18944, 136), (333, 12676, 192), (333, 12801, 72), (1025, 4250, 320), (2049, 2306, 64)])
+def test_planes_of_long_passes_are_those_of_the_swapped_form(rows, N, K):
+    """Rows as the 128-row operand and 256 weight rows as the other one, stored by TMA where the rows allow it: the same products
+    in the same order, bit for bit, at ragged rows, columns and depths."""
+    from ds41rt_b200.ops import gemm as G, lib
+    assert G.wide(rows, N) and not G.wide(128, 1 << 20) and not G.wide(rows, 256)
+    x, w = _swapped_and_wide(rows, N, K)
+    st = lib.new_status("cuda")
+    flat = torch.full((rows * N + 64,), 7.0, device="cuda")
+    planes = flat[: rows * N].view(1, rows, N)
+    G.linear_planes(x, w, planes, 1, status=st)
+    want = torch.zeros(rows, N, device="cuda")
+    G.gemm_raw(w, x, want, N, rows, K, lda=K, ldb=K, ldo=N, out_mode=3, status=st)
+    torch.cuda.synchronize()
+    lib.raise_on_status(st, "gemm wide")
+    assert torch.equal(planes[0], want) and bool((flat[rows * N:] == 7.0).all())
+    assert _rel(want, _ref(x, w)) < 2e-3
+
+
+@pytest.mark.parametrize("mode", [1, 6])
+@pytest.mark.parametrize("rows,N,K,pad,batch", [(333, 1000, 192, 24, 1), (1025, 264, 128, 8, 1), (300, 200, 72, 0, 3), (129, 72, 64, 8, 4),
+                                                (40, 328, 256, 0, 2)])
+def test_stores_of_wide_forms_keep_to_their_columns(mode, rows, N, K, pad, batch):
+    """fp32 and bf16 rows through TMA stores: longer output rows than the product has columns, and batches side by side in one
+    row.  Bit for bit what the swapped form stores; what lies between stays as it was."""
+    from ds41rt_b200.ops import gemm as G, lib
+    g = torch.Generator().manual_seed(rows + mode)
+    x = torch.randn(rows, batch * K, generator=g).bfloat16().cuda()
+    w = (torch.randn(batch, N, K, generator=g) * 0.05).bfloat16().cuda()
+    dt, ld, st = (torch.float32 if mode == 1 else torch.bfloat16), batch * (N + pad), lib.new_status("cuda")
+    got, want = (torch.full((rows + 2, ld), 7.0, device="cuda", dtype=dt) for _ in range(2))
+    G.gemm_raw(x, w, got, rows, N, K, lda=batch * K, ldb=K, ldo=ld, out_mode=mode, bn=256, batch=batch, a_batch_stride=K,
+               b_batch_stride=N * K, out_batch_stride=N + pad, status=st, static_operand=2)
+    G.gemm_raw(w, x, want, N, rows, K, lda=K, ldb=batch * K, ldo=ld, out_mode=3 if mode == 1 else 2, batch=batch,
+               a_batch_stride=N * K, b_batch_stride=K, out_batch_stride=N + pad, status=st)
+    torch.cuda.synchronize()
+    lib.raise_on_status(st, "gemm wide")
+    assert torch.equal(got, want)
+    held = want.view(rows + 2, batch, N + pad)
+    assert bool((held[rows:] == 7.0).all()) and bool((held[:, :, N:] == 7.0).all())
+    ref = torch.einsum("rbk,bnk->rbn", x.float().view(rows, batch, K), w.float())
+    assert _rel(held[:rows, :, :N], ref) < (2e-3 if mode == 1 else 1e-2)
+
+
+def test_outputs_that_no_tensor_map_describes_take_plain_stores():
+    """fp32 rows at odd lengths, off 16 bytes, and one row whose length says nothing."""
+    from ds41rt_b200.ops import gemm as G, lib
+    rows, N, K = 300, 72, 64
+    x, w = _swapped_and_wide(rows, N, K)
+    st = lib.new_status("cuda")
+    ref = _ref(x, w)
+    for ld, off, m in ((75, 0, rows), (76, 1, rows), (0, 0, 1)):
+        flat = torch.full((rows * 80,), 7.0, device="cuda")
+        G.gemm_raw(x, w, flat[off:], m, N, K, lda=K, ldb=K, ldo=ld, out_mode=1, bn=64, status=st)
+        torch.cuda.synchronize()
+        lib.raise_on_status(st, "gemm")
+        step = max(ld, N)
+        out = flat[off: off + m * step].view(m, step)
+        assert _rel(out[:, :N], ref[:m]) < 2e-3 and bool((out[:, N:] == 7.0).all()) and bool((flat[off + m * step:] == 7.0).all())
+
+
+def test_gathered_rows_of_one_rank_through_staged_stores():
+    """The all-gather form with a world of one (no waits, no copies): the same rows as without it."""
+    import ctypes as C
+    from ds41rt_b200.ops import gemm as G, lib
+    rows, N, K = 384, 200, 192
+    x, w = _swapped_and_wide(rows, N, K)
+    st = lib.new_status("cuda")
+    got, want = torch.full((rows, 208), 7.0, device="cuda"), torch.full((rows, 208), 7.0, device="cuda")
+    arrive, epoch = torch.zeros(8, dtype=torch.int32, device="cuda"), torch.ones(1, dtype=torch.int32, device="cuda")
+    a = lib.GemmArgs()
+    a.B, a.out, a.status = lib.ptr(w), lib.ptr(got), lib.ptr(st)
+    a.lda, a.ldb, a.ldo, a.M, a.N, a.K, a.batch, a.a_batches = K, K, 208, rows, N, K, 1, 1
+    a.kind, a.out_mode, a.k_splits, a.bn = 0, 1, 1, 128
+    a.ag_world, a.ag_rank, a.ag_rows, a.ag_epoch = 1, 0, rows, lib.ptr(epoch)
+    a.a_peers[0], a.ag_arrive[0] = x.data_ptr(), arrive.data_ptr()
+    lib.check(lib.kernels().ds41_gemm_tc(C.byref(a), lib.stream()), "gemm")
+    G.gemm_raw(w, x, want, N, rows, K, lda=K, ldb=K, ldo=208, out_mode=3, status=st)
+    torch.cuda.synchronize()
+    lib.raise_on_status(st, "gemm gathered")
+    assert torch.equal(got, want)
