@@ -90,7 +90,7 @@ struct QkvPostParams {
 };
 
 constexpr int kFewPlanes = 7;
-constexpr int kOwnExtras = 256;       // up to one column a thread: 200 rows, 8 columns of 10 planes 7.0 us in the kv block, 7.5 in a third
+constexpr int kOwnExtras = 256;       // up to one column a thread (200 rows, 8 columns of 10 planes: 7.0 us by the kv block, 7.5)
 // grid (rows, 2 or 3): block y == 0 normalises the q latent, y == 1 handles kv (norm + RoPE + ring write), and the extras unless
 // there are enough for a block y == 2.
 __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
@@ -364,7 +364,8 @@ extern "C" int ds41_qkv_post(const float* planes, int splits, int rows, int ntot
   // kv columns are read as aligned float2
   if (((Q + D) & 1) || ((ntot & 1) && (rows > 1 || splits > 1)) || (reinterpret_cast<uintptr_t>(planes) & 7))
     return cudaErrorInvalidValue;
-  return launch_pdl(qkv_post_kernel, dim3(rows, extra_f32 > kOwnExtras ? 3 : 2), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
+  return launch_pdl(qkv_post_kernel, dim3(rows, extra_f32 > kOwnExtras ? 3 : 2), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                    p);
 }
 
 extern "C" int ds41_compress(const float* extras, int extra_stride, int rows, int D, int ID, int rope_dim, int ratio,

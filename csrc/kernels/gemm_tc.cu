@@ -732,7 +732,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       acc = (acc + 1 == Cfg::kAccStages) ? 0 : acc + 1;
       if (acc == 0) acc_phase ^= 1;
     }
-    if ((p.out_mode == 6 || p.out_mode == kModeF32Staged) && lane == 0) bulk_wait_group<0>();   // every TMA store of this warp has been performed
+    // every TMA store of this warp has been performed
+    if ((p.out_mode == 6 || p.out_mode == kModeF32Staged) && lane == 0) bulk_wait_group<0>();
   } else if (warp >= 6) {
     // ------------------------------------------------------------ all-gather copiers (2 warps)
     if (p.ag_world > 1) {

@@ -796,8 +796,9 @@ extern "C" int ds41_hc_post_mix(const void* streams_in, void* streams_out, const
       ready[dev].store(true, std::memory_order_release);
     }
     const int grid = rows < sm_count() ? rows : sm_count();
-    return launch_pdl(hc_expand_stream_kernel, dim3(grid), dim3(kStreamThreads), static_cast<size_t>(ring.stages) * ring.stage_bytes,
-                      static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(streams_in),
+    return launch_pdl(hc_expand_stream_kernel, dim3(grid), dim3(kStreamThreads),
+                      static_cast<size_t>(ring.stages) * ring.stage_bytes, static_cast<cudaStream_t>(stream),
+                      static_cast<const __nv_bfloat16*>(streams_in),
                       static_cast<__nv_bfloat16*>(streams_out), n_ranks > 0 ? parts.base[0] : static_cast<const float*>(nullptr),
                       post, comb, partial, rows, H, status, pre_in, norm_w, static_cast<__nv_bfloat16*>(xn), tap_mean,
                       norm_eps, ring);

@@ -63,7 +63,7 @@ struct HcStepParams {
 
 // EARLY: the whole grid is on the GPU at once (three blocks an SM) and the launch is one chain of latencies, so every step's
 // operands are fetched ahead and held in registers.  Larger grids want more blocks an SM instead.  us, held / not: 8 rows of
-// 5120 columns 14.6 / 16.8, 16 rows of 16 planes 22.4 / 21.4, 64 rows 40.6 / 36.0; 16 rows of 7168 columns 23.3 / 21.4.
+// 5120 columns 14.6 / 16.8, 16 rows of 16 planes 22.4 / 19.3, 64 rows 40.6 / 34.8; 16 rows of 7168 columns 23.3 / 20.7.
 constexpr int kEarlyBlocks = 3;
 template <bool EARLY>
 __global__ void __launch_bounds__(256, EARLY ? kEarlyBlocks : 4) hc_step_kernel(HcStepParams p) {
@@ -346,7 +346,8 @@ extern "C" int ds41_hc_step(const ds41_hc_step_args* a, void* stream) {
   p.wait_flags = a->wait_flags; p.wait_epoch = a->wait_epoch; p.status = a->status;
   const dim3 grid(a->H / kSlice, a->rows);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (1ll * grid.x * grid.y <= 1ll * kEarlyBlocks * sm_count()) return launch_pdl(hc_step_kernel<true>, grid, dim3(256), 0, st, p);
+  if (1ll * grid.x * grid.y <= 1ll * kEarlyBlocks * sm_count())
+    return launch_pdl(hc_step_kernel<true>, grid, dim3(256), 0, st, p);
   return launch_pdl(hc_step_kernel<false>, grid, dim3(256), 0, st, p);
 }
 

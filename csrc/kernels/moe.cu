@@ -114,8 +114,8 @@ __device__ __forceinline__ uint32_t order_key(float v) {
 // registers (no block barriers: a choice is a maximum over a lane's scores and two warp reductions); the others compute the
 // shared expert's activation, four columns per thread.  8192 rows of 384 + 2 x 2304 columns: 189 us as a block per row, 67 so.
 // Where a warp walks many planes by itself the block form stays the better one until rows fill the GPU.  us, block / warp form:
-// 511 rows of one plane 11.1 / 7.5; 512 rows of 960 columns, 3 planes 10.2 / 9.6, 8 planes 10.7 / 13.6; 384 columns, 12 planes, 512
-// rows 11.0 / 14.2, 1024 rows 17.0 / 15.7; 16 planes, 1024 rows 17.8 / 18.5.  Below 320 rows the block form wins or ties throughout.
+// 511 rows of one plane 11.1 / 7.5; 512 rows of 960 columns, 8 planes 10.7 / 13.6; 384 columns, 12 planes, 512 rows 11.0 / 14.2,
+// 768 rows 14.1 / 14.8; 16 planes, 1024 rows 17.8 / 18.5.  Below 320 rows the block form wins or ties throughout.
 static bool router_by_warps(int rows, int splits) { return rows >= 512 && rows >= 160 * splits; }
 __global__ void __launch_bounds__(256) router_rows_kernel(RouterParams p, int sel_blocks) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

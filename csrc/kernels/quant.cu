@@ -128,7 +128,8 @@ act_quant_mx_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uin
   pdl_wait();
   const int live = rows_dev != nullptr ? min(rows, *rows_dev) : rows;
   for (int r = blockIdx.x * 8 + warp; r < live; r += gridDim.x * 8)
-    for (int k0 = 0; k0 < K; k0 += 256) mx_row_step(x + 1ll * r * ldx, q + 1ll * r * ldq, atom_row_of(sf, r, K / 128), k0, K, lane);
+    for (int k0 = 0; k0 < K; k0 += 256)
+      mx_row_step(x + 1ll * r * ldx, q + 1ll * r * ldq, atom_row_of(sf, r, K / 128), k0, K, lane);
 }
 
 // NVFP4 activation rows: e2m1 values (two per byte, even element in the low nibble) with one E4M3 scale per 16
@@ -203,8 +204,10 @@ act_quant_tiles_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8
     for (int r = t.row0[tile] + warp; r < end; r += 8)
 #pragma unroll
       for (int k0 = c0; k0 < c0 + kTileCols; k0 += 256) {
-        if constexpr (NV) nvfp4_row_step(x + 1ll * r * ldx, q + 1ll * r * (ldq / 2), atom_row_of(sf, r, K / 64), k0, c1, global_scale, lane);
-        else mx_row_step(x + 1ll * r * ldx, q + 1ll * r * ldq, atom_row_of(sf, r, K / 128), k0, c1, lane);
+        if constexpr (NV)
+          nvfp4_row_step(x + 1ll * r * ldx, q + 1ll * r * (ldq / 2), atom_row_of(sf, r, K / 64), k0, c1, global_scale, lane);
+        else
+          mx_row_step(x + 1ll * r * ldx, q + 1ll * r * ldq, atom_row_of(sf, r, K / 128), k0, c1, lane);
       }
   }
 }

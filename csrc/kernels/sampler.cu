@@ -229,7 +229,8 @@ extern "C" int ds41_argmax_rows(const float* logits, long long ld, int rows, int
   ArgmaxParams p{logits, ld, vocab_local, vocab_offset, mask, mask_words, best_val, best_idx, row_status};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (argmax_in_cluster(rows, vocab_local))
-    return launch_pdl_cluster(argmax_rows_kernel<kArgmaxCtas, 512, 4>, dim3(rows * kArgmaxCtas), dim3(512), kArgmaxCtas, 0, st, p);
+    return launch_pdl_cluster(argmax_rows_kernel<kArgmaxCtas, 512, 4>, dim3(rows * kArgmaxCtas), dim3(512), kArgmaxCtas, 0, st,
+                              p);
   return launch_pdl(argmax_rows_kernel<1, 1024, 2>, dim3(rows), dim3(1024), 0, st, p);
 }
 

@@ -148,9 +148,10 @@ __device__ __forceinline__ float4 routed_at4(const ds41_resid_args& p, int r, in
   return s;
 }
 
-// Many rows: bound by the instructions of a row rather than its bytes (ncu: 45 % of issue slots at 22 % of the memory's rate; more
-// threads or more rows an SM made it slower), so rows that fill the threads' pieces (FULL) drop every test of a column against
-// the row's end.  2048 rows x 4096 columns: 75 -> 57 us on average in a model with kept streams, 49 -> 39 without; 953 rows 28 -> 22.
+// Many rows: bound by latency, a block's loads and its two chains of merges one after the other (ncu: 45 % of issue slots and
+// 22 % of the memory's rate; more threads or more rows an SM made it slower), so rows that fill the threads' pieces (FULL) shorten
+// the chain by every test of a column against the row's end.  2048 rows x 4096 columns: 75 -> 57 us on average in a model with
+// kept streams, 49 -> 39 without; 953 rows 28 -> 22.
 template <typename T, int CL, int NI, bool FULL>
 __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_step_kernel(ds41_resid_args p) {
   __shared__ float slots[2][96];
