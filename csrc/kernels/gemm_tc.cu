@@ -1,7 +1,7 @@
 // Tensor-core GEMM for sm_100a:  D[m,n] = sum_k A[m,k] * B[n,k]   (both operands K-major)
 //
-// One persistent warp-specialised kernel: warp 0 streams A/B tiles with TMA into a multi-stage
-// shared-memory ring, warp 1 issues tcgen05.mma into double-buffered TMEM accumulators, warps 2-5
+// One persistent warp-specialised kernel: warp 0 (block-scaled kinds: and the last warp) streams A/B tiles with TMA into a
+// multi-stage shared-memory ring, warp 1 issues tcgen05.mma into double-buffered TMEM accumulators, warps 2-5
 // drain TMEM with tcgen05.ld and write the result.  Kinds: bf16, fp8 e4m3 (unscaled) and MX
 // block-scaled fp8 (UE8M0 scale per 32 elements, scale factors copied into TMEM with tcgen05.cp).
 // Split-K writes fp32 partial planes; "transposed" output serves the swap-AB decode orientation
@@ -10,6 +10,8 @@
 // Capability parity: replaces the reference's AOT block-scaled dense GEMMs
 // (native/include/ds41rt_v41_fp8.h:6-47) and its cuBLAS fallbacks (native/cuda/kernels/v41_attention_ops.cu:130-155).
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "ds41_api.h"
 #include "ds41_launch.cuh"
@@ -24,7 +26,8 @@ namespace ds41 {
 
 constexpr int kBM = 128;
 constexpr int kTileKBytes = 128;       // one 128-byte swizzle span of K per stage
-constexpr int kGemmThreads = 256;      // warps: 0 TMA, 1 MMA, 2-5 epilogue, 6-7 all-gather copiers, 8-11 second epilogue set
+constexpr int kGemmThreads = 256;      // warps: 0 TMA, 1 MMA, 2-5 epilogue, 6-7 all-gather copiers, 8-11 second epilogue set,
+                                       // last: second producer of block-scaled kinds
 constexpr int kStagingBytes = 32768;   // TMA-store staging: 4 epilogue warps x 2 buffers x [32 rows][128 B]
 
 constexpr int kModeF32Staged = 16;
@@ -138,7 +141,7 @@ struct GemmCfg {
   // instructions per column and thread), so two sets of four warps share its columns.  FC1 of 384 experts x 128 rows, 5120 x
   // 2304: 2445 us with one set, 2198 with two.
   static constexpr int kEpiSets = (DUAL && kAccStages == 1) ? 2 : 1;
-  static constexpr int kThreads = kGemmThreads + 128 * (kEpiSets - 1);
+  static constexpr int kThreads = kGemmThreads + 128 * (kEpiSets - 1) + (kScaled ? 32 : 0);    // + the second producer
   static constexpr int kSmemBytes = kStages * kStageBytes + kStaging + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(kTmemNeeded <= 512, "TMEM budget exceeded");
   static_assert(kStages >= 2, "not enough shared memory for two stages");
@@ -205,7 +208,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], Cfg::kScaled ? 2 : 1);       // one arrival per producer
       mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -226,42 +229,53 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const uint32_t tmem_base = *tmem_slot;
 
   bool ok = true;                              // false: a wait of this thread gave up
-  if (warp == 0 && lane == 0) {
-    // ------------------------------------------------------------ TMA producer
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
+  // ------------------------------------------------------------ TMA producers
+  // One warp per role, walking its loop with uniform control flow; `leader` predicates the copies.  A scaled kind asks for three to
+  // five copies a stage, and one thread that issued them all (from a one-lane branch, whose descriptors and coordinates take
+  // a detour) was what a stage waited for: warp 0 then copies A tiles, the last warp B tiles and scale factors.  85 experts of
+  // 5120 x 2304 for 16 rows, FC1 and FC2: e2m1 weights 228 and 177 us with one thread, 195 and 125 so; e4m3 329 and 185, 324 and 175.
+  auto produce = [&](auto takes_a, auto takes_b) {
+    constexpr bool kA = decltype(takes_a)::value, kB = decltype(takes_b)::value;
+    const bool leader = elect_one();
+    if (leader) {
+      if constexpr (kA) tma_prefetch_desc(&tmA);
+      if constexpr (kB) tma_prefetch_desc(&tmB);
+    }
     int stage = 0;
     uint32_t phase = 0;
     // 4-bit A tiles occupy one byte per element in shared memory but the copy engine accounts the packed bytes
-    const uint32_t kStageTx = (p.a_fp4 ? Cfg::kABytes / 2 : Cfg::kABytes) + Cfg::kBBytes +
-                              (Cfg::kScaled ? 512 * (Cfg::kAtomsA + Cfg::kAtomsB) : 0);
+    const uint32_t tx = (kA ? (p.a_fp4 ? Cfg::kABytes / 2 : Cfg::kABytes) : 0) +
+                        (kB ? Cfg::kBBytes + (Cfg::kScaled ? 512 * (Cfg::kAtomsA + Cfg::kAtomsB) : 0) : 0);
     // Weight tiles of the first stages do not depend on the previous kernel: fetch them before waiting for it.
     int prefetched = 0;
-    if (p.static_operand != 0 && p.n_active == nullptr && p.batch_map == nullptr && !table && blockIdx.x < tiles) {
-      long long r = blockIdx.x;
-      int mt, nt;
-      r = decode_tile(r, m_tiles, n_tiles, band_tiles, mt, nt);
-      const int sp = static_cast<int>(r % p.k_splits); r /= p.k_splits;
-      const int b = static_cast<int>(r);
-      const int kb0 = sp * kb_per_split;
-      const int kb1 = min(kb_total, kb0 + kb_per_split);
-      prefetched = min(S, kb1 - kb0);
-      for (int i = 0; i < prefetched; ++i) {
-        uint8_t* sa = smem + i * Cfg::kStageBytes;
-        mbar_expect_tx(&full[i], kStageTx);
-        if (p.static_operand == 1) {
-          tma_load_3d(sa, &tmA, &full[i], (kb0 + i) * Cfg::kBK, mt * kBM, b);
-          if constexpr (DUAL)
-            tma_load_3d(sa + Cfg::kATile, &tmA, &full[i], (kb0 + i) * Cfg::kBK, p.up_row_offset + mt * kBM, b);
-        } else {
-          tma_load_3d(sa + Cfg::kABytes, &tmB, &full[i], (kb0 + i) * Cfg::kBK, nt * BN, p.b_batch_kind == 1 ? 0 : b);
+    if ((kA && p.static_operand == 1) || (kB && p.static_operand == 2)) {
+      if (p.n_active == nullptr && p.batch_map == nullptr && !table && blockIdx.x < tiles) {
+        long long r = blockIdx.x;
+        int mt, nt;
+        r = decode_tile(r, m_tiles, n_tiles, band_tiles, mt, nt);
+        const int sp = static_cast<int>(r % p.k_splits); r /= p.k_splits;
+        const int b = static_cast<int>(r);
+        const int kb0 = sp * kb_per_split;
+        const int kb1 = min(kb_total, kb0 + kb_per_split);
+        prefetched = min(S, kb1 - kb0);
+        for (int i = 0; i < prefetched; ++i) {
+          uint8_t* sa = smem + i * Cfg::kStageBytes;
+          mbar_expect_tx_if(leader, &full[i], tx);
+          if (kA && p.static_operand == 1) {
+            tma_load_3d_if(leader, sa, &tmA, &full[i], (kb0 + i) * Cfg::kBK, mt * kBM, b);
+            if constexpr (DUAL)
+              tma_load_3d_if(leader, sa + Cfg::kATile, &tmA, &full[i], (kb0 + i) * Cfg::kBK, p.up_row_offset + mt * kBM, b);
+          } else {
+            tma_load_3d_if(leader, sa + Cfg::kABytes, &tmB, &full[i], (kb0 + i) * Cfg::kBK, nt * BN,
+                           p.b_batch_kind == 1 ? 0 : b);
+          }
         }
       }
     }
     pdl_wait();
     if (p.wait_flags != nullptr && p.wait_world > 1) {
       for (int k = 0; k < p.wait_world && ok; ++k)
-        if (!flag_wait_ge(p.wait_flags[k], *p.wait_epoch, p.status, 120 + k)) ok = false;
+        ok = __all_sync(0xffffffffu, flag_wait_ge(p.wait_flags[k], *p.wait_epoch, p.status, 120 + k));
     }
     for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
       long long r = t;
@@ -272,58 +286,69 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int n_base = table ? p.tile_row0[nt] : nt * BN;
       const int kb0 = sp * kb_per_split;
       const int kb1 = min(kb_total, kb0 + kb_per_split);
-      const int mt_eff = rot ? (mt + rot) % m_tiles : mt;
-      const int a_row = mt_eff * kBM;
-      if (p.ag_world > 1) {
+      const int ba = p.batch_map != nullptr ? p.batch_map[b] : b;
+      const int bb = p.b_batch_kind == 0 ? ba : (p.b_batch_kind == 1 ? 0 : b);
+      const int a_row = (rot ? (mt + rot) % m_tiles : mt) * kBM;
+      if (kA && p.ag_world > 1) {
         const int src = a_row / p.ag_rows;
         if (src != p.ag_rank) {
           // the rows were pushed by rank src's copier warps: wait for all K chunks of this 128-row tile
           const int j = (a_row - src * p.ag_rows) / kBM;
           const uint32_t need = *p.ag_epoch * static_cast<uint32_t>(p.ag_chunks);
-          if (!flag_wait_ge(p.ag_arrive[p.ag_rank] + src * (p.ag_rows / kBM) + j, need, p.status, 110 + src)) {
-            ok = false;
-            break;
-          }
+          ok = __all_sync(0xffffffffu, flag_wait_ge(p.ag_arrive[p.ag_rank] + src * (p.ag_rows / kBM) + j, need, p.status,
+                                                    110 + src));
+          if (!ok) break;
           asm volatile("fence.proxy.async;" ::: "memory");
         }
+      }
+      // scale-factor atoms: [row_atom][k_atom][512 B]; kSfPerTile consecutive k_atoms per stage and 128 rows
+      // (MX: one atom = 128 K elements with a UE8M0 scale per 32; NVFP4: four atoms of 64 K elements, E4M3 per 16)
+      constexpr uint32_t kSf = 512 * Cfg::kSfPerTile;
+      [[maybe_unused]] const uint8_t *sf_a = nullptr, *sf_up = nullptr, *sf_b[Cfg::kTilesB] = {};
+      if constexpr (kB && Cfg::kScaled) {
+        const long long row_atoms = 1ll * kb_total * kSf, at = 1ll * kb0 * kSf;
+        const uint8_t* of_a = p.sfa + ba * p.sfa_batch_stride + at;
+        sf_a = of_a + mt * row_atoms;
+        if constexpr (DUAL) sf_up = of_a + (p.up_row_offset / 128 + mt) * row_atoms;
+#pragma unroll
+        for (int a = 0; a < Cfg::kTilesB; ++a)
+          sf_b[a] = p.sfb + bb * p.sfb_batch_stride + at + (n_base / 128 + a) * row_atoms;
       }
       for (int kb = kb0; kb < kb1; ++kb) {
         const bool early = prefetched > 0;      // this stage's barrier is armed and its weight tile is in flight
         if (early) --prefetched;
-        if (!early && !mbar_wait(&empty[stage], phase ^ 1, p.status, 100)) { ok = false; break; }
+        if (!early) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, p.status, 100));
+          if (!ok) break;
+          mbar_expect_tx_if(leader, &full[stage], tx);
+        }
         uint8_t* sa = smem + stage * Cfg::kStageBytes;
         uint8_t* sb = sa + Cfg::kABytes;
-        if (!early) mbar_expect_tx(&full[stage], kStageTx);
-        const int ba = p.batch_map != nullptr ? p.batch_map[b] : b;
-        const int bb = p.b_batch_kind == 0 ? ba : (p.b_batch_kind == 1 ? 0 : b);
-        if (!early || p.static_operand != 1) {
-          tma_load_3d(sa, &tmA, &full[stage], kb * Cfg::kBK, a_row, ba);
+        if (kA && (!early || p.static_operand != 1)) {
+          tma_load_3d_if(leader, sa, &tmA, &full[stage], kb * Cfg::kBK, a_row, ba);
           if constexpr (DUAL)
-            tma_load_3d(sa + Cfg::kATile, &tmA, &full[stage], kb * Cfg::kBK, p.up_row_offset + mt * kBM, ba);
+            tma_load_3d_if(leader, sa + Cfg::kATile, &tmA, &full[stage], kb * Cfg::kBK, p.up_row_offset + mt * kBM, ba);
         }
-        if (!early || p.static_operand != 2) tma_load_3d(sb, &tmB, &full[stage], kb * Cfg::kBK, n_base, bb);
-        if constexpr (Cfg::kScaled) {
-          // scale-factor atoms: [row_atom][k_atom][512 B]; kSfPerTile consecutive k_atoms per stage and 128 rows
-          // (MX: one atom = 128 K elements with a UE8M0 scale per 32; NVFP4: four atoms of 64 K elements, E4M3 per 16)
-          constexpr int kSf = Cfg::kSfPerTile;
+        if (kB && (!early || p.static_operand != 2))
+          tma_load_3d_if(leader, sb, &tmB, &full[stage], kb * Cfg::kBK, n_base, bb);
+        if constexpr (kB && Cfg::kScaled) {
           uint8_t* ssf = sb + Cfg::kBBytes;
-          const long long ka = 1ll * kb * kSf;
-          const long long n_ka = 1ll * kb_total * kSf;
-          bulk_load(ssf, p.sfa + ba * p.sfa_batch_stride + (1ll * mt * n_ka + ka) * 512, 512 * kSf, &full[stage]);
-          if constexpr (DUAL) {
-            const long long mt_up = p.up_row_offset / 128 + mt;
-            bulk_load(ssf + 512 * kSf, p.sfa + ba * p.sfa_batch_stride + (mt_up * n_ka + ka) * 512, 512 * kSf, &full[stage]);
-          }
+          const uint32_t at = static_cast<uint32_t>(kb - kb0) * kSf;
+          bulk_load_if(leader, ssf, sf_a + at, kSf, &full[stage]);
+          if constexpr (DUAL) bulk_load_if(leader, ssf + kSf, sf_up + at, kSf, &full[stage]);
 #pragma unroll
-          for (int a = 0; a < Cfg::kTilesB; ++a) {
-            const long long ra = n_base / 128 + a;
-            bulk_load(ssf + 512 * (Cfg::kAtomsA + a * kSf), p.sfb + bb * p.sfb_batch_stride + (ra * n_ka + ka) * 512,
-                      512 * kSf, &full[stage]);
-          }
+          for (int a = 0; a < Cfg::kTilesB; ++a)
+            bulk_load_if(leader, ssf + 512 * (Cfg::kAtomsA + a * Cfg::kSfPerTile), sf_b[a] + at, kSf, &full[stage]);
         }
         if (++stage == S) { stage = 0; phase ^= 1; }
       }
     }
+  };
+  if (warp == 0) {
+    if constexpr (Cfg::kScaled) produce(std::true_type{}, std::false_type{});
+    else produce(std::true_type{}, std::true_type{});
+  } else if (Cfg::kScaled && warp == Cfg::kThreads / 32 - 1) {
+    if constexpr (Cfg::kScaled) produce(std::false_type{}, std::true_type{});
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     // The whole warp walks the loop with uniform control flow; `leader` predicates the tensor-core instructions
