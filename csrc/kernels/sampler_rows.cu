@@ -59,12 +59,16 @@ __device__ __forceinline__ float uniform01(unsigned long long seed, unsigned lon
 
 // A row is shared by a cluster of up to eight CTAs.  One CTA per row walked 517 KB up to fifteen times from L2 with a fraction of
 // one SM's bandwidth: 780 us for sixteen rows of 129280 logits.  Now each CTA reads its part once, keeps the order keys of the
-// scaled logits in shared memory, and only histograms, sums and short lists travel, through distributed shared memory: 68 us for
-// the same rows, eight CTAs each.  Every CTA draws the same conclusions from the same integers, so there is no broadcast step and
-// all control flow is uniform in the cluster.  What is left is a chain of cluster barriers (2000 cycles each) and of passes over
-// the keys (5000 to 7000 cycles); the reads from memory are 2 % of it.
+// scaled logits in shared memory, and only histograms, sums and short lists travel, through distributed shared memory.  Every CTA
+// draws the same conclusions from the same integers, so there is no broadcast step and all control flow is uniform in the cluster.
+// What is left is a chain of cluster barriers (2000 cycles each) and of passes over the keys (5000 to 7000 cycles); the reads from
+// memory are 2 % of it.  So a selection sorts the row into 1024 bins of its own, of which the CTAs exchange 256 sums and then the
+// four bins of one, and the draw looks at the nucleus' histogram again instead of making one: 16 rows with mixed filters 80 us
+// with 256 bins and a histogram for every selection, 52 so; nucleus rows alone 109 and 72.
 constexpr int kSampleMaxCluster = 8;
 constexpr int kSampleMaxSlice = 49152;     // keys per CTA that fit its shared memory; longer slices are read again from L2
+// A slice's first histogram has PER bins for each of the 256 that the CTAs exchange: four, or one beside the longest slices
+constexpr int kSampleFineSlice = 45056;
 
 struct SamplePart {                        // what one CTA found in its slice
   float best;
@@ -79,10 +83,16 @@ struct SampleMember {
   unsigned long long mass;                 // by count: the count
 };
 
+template <int PER>
 struct SampleShared {
-  // histograms of the even and odd passes: the other one may still be read by peers.  A weight is counted in pieces of
-  // 14 bits, whose sums over a slice of up to 2^18 tokens fit 32 bits (64-bit additions in shared memory are compare-and-swap
-  // loops: 22 us a pass); longer slices take the first 512 words as 64-bit sums.
+  static constexpr int kFineBins = 256 * PER;
+  // A weight is counted in pieces of 14 bits, whose sums over a slice of up to 2^18 tokens fit 32 bits (64-bit additions in shared
+  // memory are compare-and-swap loops: 22 us a pass); longer slices take the first words as 64-bit sums.
+  // The first histogram of a selection, this slice's: 32nds (PER = 4) below the maximum, and the same added up to
+  // eighths.
+  unsigned int fine_cnt[kFineBins];
+  alignas(8) unsigned int fine_mass[3][kFineBins];
+  // histograms of the even and odd passes that follow: the other one may still be read by peers
   unsigned int cnt[2][256];
   alignas(8) unsigned int mass[2][3][256];
   unsigned int tot_cnt[256];
@@ -92,7 +102,10 @@ struct SampleShared {
   unsigned long long warp[kSampleThreads / 32];
   SamplePart warp_part[kSampleThreads / 32];
   unsigned long long total;                        // weight of a selection's candidates
+  unsigned long long total_list;
+  unsigned int low_key;
   double remaining;
+  unsigned long long above_mass;
   unsigned int digit, tie_count, best_key, n_above;
   int token;
   unsigned int own_n, far_n[kSampleMaxCluster];
@@ -141,8 +154,8 @@ struct SamplePeers {
 };
 
 // Sum over the cluster; `slot` is used once per launch, so no second barrier protects it.
-template <int CL>
-__device__ unsigned long long cluster_sum(SampleShared& sh, SamplePeers<CL> cl, int slot, unsigned long long v) {
+template <int CL, int PER>
+__device__ unsigned long long cluster_sum(SampleShared<PER>& sh, SamplePeers<CL> cl, int slot, unsigned long long v) {
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
   if ((threadIdx.x & 31) == 0) sh.warp[threadIdx.x >> 5] = v;
   __syncthreads();
@@ -157,18 +170,20 @@ __device__ unsigned long long cluster_sum(SampleShared& sh, SamplePeers<CL> cl, 
   return all;
 }
 
-// Eighths below the maximum, highest first, the last bucket open: the first digit of a selection.  It spreads the tokens of a
-// row over the bins, where the top byte of a key (sign and exponent) put a row into half a dozen: the lanes of a warp then met
+// 32nds (PER = 4) below the maximum, highest first, the last bucket open: the first digit of a selection.  It spreads the tokens of
+// a row over the bins, where the top byte of a key (sign and exponent) put a row into half a dozen: the lanes of a warp then met
 // in the same counters and a pass took 40 us.
+template <int PER>
 __device__ __forceinline__ uint32_t bucket_of(uint32_t key, float max_scaled) {
-  const float d = (max_scaled - key_value(key)) * 8.0f;
-  return 255u - (d >= 255.0f ? 255u : static_cast<uint32_t>(d));
+  constexpr uint32_t kLast = 256u * PER - 1u;
+  const float d = (max_scaled - key_value(key)) * (8.0f * PER);
+  return kLast - (d >= static_cast<float>(kLast) ? kLast : static_cast<uint32_t>(d));
 }
 
 // Every CTA gathers the members of all slices that `is_member` names (fewer than kSampleList) and the tie group, if it takes
 // part.
-template <int CL, class F>
-__device__ void gather_members(SampleShared& sh, SamplePeers<CL> cl, const SampleSlice& row, float max_scaled,
+template <int CL, int PER, class F>
+__device__ void gather_members(SampleShared<PER>& sh, SamplePeers<CL> cl, const SampleSlice& row, float max_scaled,
                                const CandSet& set, bool by_mass, bool tie, F is_member) {
   const int tid = threadIdx.x;
   for (int i = tid; i < row.n; i += kSampleThreads) {
@@ -182,7 +197,7 @@ __device__ void gather_members(SampleShared& sh, SamplePeers<CL> cl, const Sampl
   if (tid < CL) sh.far_n[tid] = *cl.of(&sh.own_n, tid);
   __syncthreads();
   constexpr int kPer = kSampleThreads / CL;      // threads that read one peer's members
-  const int from = tid / kPer;
+  const int from = min(tid / kPer, CL - 1);      // the last one's may be a few more
   int before = 0, n = 0;
 #pragma unroll
   for (int r = 0; r < CL; ++r) {
@@ -190,7 +205,7 @@ __device__ void gather_members(SampleShared& sh, SamplePeers<CL> cl, const Sampl
     n += static_cast<int>(sh.far_n[r]);
   }
   n = min(n, kSampleList);
-  for (int i = tid % kPer; i < static_cast<int>(sh.far_n[from]) && before + i < kSampleList; i += kPer) {
+  for (int i = tid - from * kPer; i < static_cast<int>(sh.far_n[from]) && before + i < kSampleList && tid < CL * kPer; i += kPer) {
     const uint2 m = *cl.of(&sh.own_list[i], from);
     sh.list[before + i] = {m.x, 1u, by_mass ? weight_fx(key_value(m.x), max_scaled) : 1ull};
     sh.list_id[before + i] = static_cast<int>(m.y);
@@ -204,37 +219,67 @@ __device__ void gather_members(SampleShared& sh, SamplePeers<CL> cl, const Sampl
   __syncthreads();
 }
 
-// The highest key whose members and the ones above weigh at least the target (`frac` >= 0: that share of the list's weight),
-// each thread summing what lies above its own member.
-__device__ uint32_t solve_list(SampleShared& sh, bool tie, double target, double frac) {
+// The highest key whose members and the ones above weigh at least the target (`frac` >= 0: that share of the list's weight).
+// Several lanes share a member and sum what is not below it, each over a part of the list.
+template <int PER>
+__device__ uint32_t solve_list(SampleShared<PER>& sh, bool tie, double target, double frac) {
   const int tid = threadIdx.x, total = sh.n_list + (tie ? 1 : 0);
-  uint32_t key = 0, equal = 0, higher = 0, low = 0xFFFFFFFFu;
-  unsigned long long above = 0, same = 0, all = 0;
-  if (tid == 0) sh.best_key = 0;
-  __syncthreads();
-  if (tid < total) {
-    key = sh.list[tid].key;
-#pragma unroll 4
-    for (int j = 0; j < total; ++j) {
-      const SampleMember m = sh.list[j];
-      all += m.mass;
-      above += m.key > key ? m.mass : 0ull;
-      same += m.key == key ? m.mass : 0ull;
-      higher += m.key > key ? m.count : 0u;
-      equal += m.key == key ? m.count : 0u;
-      low = min(low, m.key);
-    }
-    if (frac >= 0.0) target = frac * static_cast<double>(all);
-    // rounding can leave the target just above the total: then the lowest key present is the one
-    if (static_cast<double>(above + same) >= target || key == low) atomicMax(&sh.best_key, key);
+  int per = 32;                                  // lanes per member
+  while (per > 1 && total * per > kSampleThreads) per >>= 1;
+  const int member = tid / per, part = tid % per;
+  const bool live = member < total;
+  const uint32_t key = live ? sh.list[member].key : 0u;
+  unsigned long long upto = 0, all = 0;
+  uint32_t low = 0xFFFFFFFFu;
+  if (tid == 0) {
+    sh.best_key = 0;
+    sh.low_key = 0xFFFFFFFFu;
+    sh.total_list = 0;
   }
   __syncthreads();
+  if (live) {
+#pragma unroll 4
+    for (int j = part; j < total; j += per) {
+      const SampleMember m = sh.list[j];
+      upto += m.key >= key ? m.mass : 0ull;
+    }
+  }
+  for (int o = per >> 1; o > 0; o >>= 1) upto += __shfl_xor_sync(0xffffffffu, upto, o);
+  if (tid < total) {
+    all = sh.list[tid].mass;
+    low = sh.list[tid].key;
+  }
+  low = __reduce_min_sync(0xffffffffu, low);
+  for (int o = 16; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+  if ((tid & 31) == 0 && tid < total) {
+    atomicMin(&sh.low_key, low);
+    atomicAdd(&sh.total_list, all);
+  }
+  __syncthreads();
+  all = sh.total_list;
+  if (frac >= 0.0) target = frac * static_cast<double>(all);
+  // rounding can leave the target just above the total: then the lowest key present is the one
+  if (live && (static_cast<double>(upto) >= target || key == sh.low_key)) atomicMax(&sh.best_key, key);
+  __syncthreads();
   const uint32_t best = sh.best_key;
-  if (tid < total && key == best) {              // members of one key write the same
-    sh.remaining = target - static_cast<double>(above);
-    sh.tie_count = equal;
-    sh.n_above = higher;
-    if (frac >= 0.0) sh.total = all;
+  if (tid < 32) {                                // what lies above it
+    unsigned long long above = 0;
+    uint32_t equal = 0, higher = 0;
+    for (int j = tid; j < total; j += 32) {
+      const SampleMember m = sh.list[j];
+      above += m.key > best ? m.mass : 0ull;
+      equal += m.key == best ? m.count : 0u;
+      higher += m.key > best ? m.count : 0u;
+    }
+    equal = __reduce_add_sync(0xffffffffu, equal);
+    higher = __reduce_add_sync(0xffffffffu, higher);
+    for (int o = 16; o > 0; o >>= 1) above += __shfl_xor_sync(0xffffffffu, above, o);
+    if (tid == 0) {
+      sh.remaining = target - static_cast<double>(above);
+      sh.tie_count = equal;
+      sh.n_above = higher;
+      if (frac >= 0.0) sh.total = all;
+    }
   }
   __syncthreads();
   return best;
@@ -243,57 +288,161 @@ __device__ uint32_t solve_list(SampleShared& sh, bool tie, double target, double
 // Selection by five digits (the bucket, then the bytes of the key), high keys first.  by_mass: find the key at which the running
 // weight reaches the target; else the key at which the running count reaches it.  `frac` >= 0: the target is that share of the
 // set's weight, which is left in sh.total.
+// `narrowed`: the set is what the selection before this one, by weight too, left of its own: whole bins above the bin of
+// set.excl, whose histogram stands, and a part of that bin; one look at the histogram then takes the place of a pass.
 // On return sh.remaining is what the ties at the returned key must still supply and sh.tie_count how many candidates carry it.
 // `pass` counts the histograms of the launch.
-template <int CL>
-__device__ uint32_t radix_select(SampleShared& sh, SamplePeers<CL> cl, const SampleSlice& row, float max_scaled, CandSet set,
-                                 bool by_mass, double target, double frac, int& pass) {
+template <int CL, int PER>
+__device__ uint32_t radix_select(SampleShared<PER>& sh, SamplePeers<CL> cl, const SampleSlice& row, float max_scaled, CandSet set,
+                                 bool by_mass, double target, double frac, bool narrowed, int& pass) {
   const int tid = threadIdx.x, lane = tid & 31;
-  uint32_t prefix = 0, prefix_mask = 0, bucket = 0;
-  for (int shift = 32; shift >= 0; shift -= 8, ++pass) {
-    unsigned int* cnt = sh.cnt[pass & 1];
-    unsigned int(*mass)[256] = sh.mass[pass & 1];
-    const bool first = shift == 32;
-    if (tid < 256) cnt[tid] = mass[0][tid] = mass[1][tid] = mass[2][tid] = 0;
-    auto add_mass = [&](uint32_t d, unsigned long long w) {
-      if (row.wide) {
-        atomicAdd(reinterpret_cast<unsigned long long*>(mass[0]) + d, w);
-        return;
-      }
-      constexpr unsigned kPiece = (1u << 14) - 1;
-      const unsigned a = static_cast<unsigned>(w) & kPiece, b = static_cast<unsigned>(w >> 14) & kPiece;
-      const unsigned c = static_cast<unsigned>(w >> 28);
-      if (a != 0) atomicAdd(&mass[0][d], a);
-      if (b != 0) atomicAdd(&mass[1][d], b);
-      if (c != 0) atomicAdd(&mass[2][d], c);
-    };
-    __syncthreads();
-    auto member = [&](uint32_t k) { return first || (bucket_of(k, max_scaled) == bucket && (k & prefix_mask) == prefix); };
-    auto digit = [&](uint32_t k) { return first ? bucket_of(k, max_scaled) : (k >> shift) & 255u; };
-    // Integer sums: the result does not depend on the order or the grouping of the additions.  After the first digit lanes of
-    // a warp that hit the same one add once, since the tokens that are left share their top bytes.
-    for (int base = 0; base < row.n; base += kSampleThreads) {
-      const uint32_t k = base + tid < row.n ? row[base + tid] : 0u;
-      const bool act = k > set.excl && member(k);
-      if (!__any_sync(0xffffffffu, act)) continue;
-      if (first) {
-        if (act) {
-          const uint32_t d = digit(k);
-          atomicAdd(&cnt[d], 1u);
-          if (by_mass) add_mass(d, weight_fx(key_value(k), max_scaled));
-        }
-        continue;
-      }
-      const uint32_t d = digit(k);
-      const unsigned peers = __match_any_sync(0xffffffffu, act ? d : 256u);
-      if (act) {
-        if (by_mass) add_mass(d, weight_fx(key_value(k), max_scaled));
-        if (lane == __ffs(peers) - 1) atomicAdd(&cnt[d], static_cast<unsigned>(__popc(peers)));
+  constexpr int kFineBins = 256 * PER;
+  auto add_mass = [&](unsigned int* mass, int bins, uint32_t d, unsigned long long w) {
+    if (row.wide) {
+      atomicAdd(reinterpret_cast<unsigned long long*>(mass) + d, w);
+      return;
+    }
+    constexpr unsigned kPiece = (1u << 14) - 1;
+    const unsigned a = static_cast<unsigned>(w) & kPiece, b = static_cast<unsigned>(w >> 14) & kPiece;
+    const unsigned c = static_cast<unsigned>(w >> 28);
+    if (a != 0) atomicAdd(mass + d, a);
+    if (b != 0) atomicAdd(mass + bins + d, b);
+    if (c != 0) atomicAdd(mass + 2 * bins + d, c);
+  };
+  auto whole = [&](const unsigned int* mass, int bins, uint32_t d) -> unsigned long long {
+    if (row.wide) return reinterpret_cast<const unsigned long long*>(mass)[d];
+    return mass[d] + (static_cast<unsigned long long>(mass[bins + d]) << 14) +
+           (static_cast<unsigned long long>(mass[2 * bins + d]) << 28);
+  };
+  const uint32_t floor_bin = narrowed ? bucket_of<PER>(set.excl, max_scaled) : 0u;
+  // Warp 0: the first of the 256 bins, from the highest down, whose running weight reaches the target.
+  auto scan = [&](bool first) {
+    // eight bins per lane from the highest down: the first bin in use whose running sum reaches the target
+    unsigned long long sum = 0;
+    unsigned members = 0;
+    auto bin_of = [&](int j) { return 255 - 8 * lane - j; };
+    auto out = [&](int d) { return first && d < static_cast<int>(floor_bin / PER); };
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (out(bin_of(j))) continue;
+      sum += sh.tot_mass[bin_of(j)];
+      members += sh.tot_cnt[bin_of(j)];
+    }
+    const bool used = members != 0;
+    unsigned long long incl = sum;
+    unsigned higher = members;
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, off);
+      const unsigned more = __shfl_up_sync(0xffffffffu, higher, off);
+      if (lane >= off) {
+        incl += up;
+        higher += more;
       }
     }
-    if (cl.rank() == 0 && tid == 0 && set.tie_mult > 0 && member(set.tie_key)) {
-      const uint32_t d = digit(set.tie_key);
-      atomicAdd(&cnt[d], static_cast<unsigned int>(set.tie_mult));
+    higher -= members;
+    const unsigned long long all = __shfl_sync(0xffffffffu, incl, 31);
+    if (first && frac >= 0.0) target = frac * static_cast<double>(all);
+    const unsigned reach = __ballot_sync(0xffffffffu, used && static_cast<double>(incl) >= target);
+    const unsigned any = __ballot_sync(0xffffffffu, used);
+    // rounding can leave the target just above the total: then the selection ends on the lowest key present
+    const int owner = reach != 0 ? __ffs(reach) - 1 : (any != 0 ? 31 - __clz(any) : 0);
+    if (lane == owner) {
+      unsigned long long acc = incl - sum, at = acc;
+      int pick = -1;
+      for (int j = 0; j < 8; ++j) {
+        const int d = bin_of(j);
+        if (out(d) || sh.tot_cnt[d] == 0) continue;
+        if (pick >= 0) higher += sh.tot_cnt[pick];
+        pick = d;
+        at = acc;
+        acc += sh.tot_mass[d];
+        if (reach != 0 && static_cast<double>(acc) >= target) break;
+      }
+      if (pick < 0) pick = 0;
+      sh.digit = static_cast<unsigned int>(pick);
+      sh.above_mass = at;
+      sh.tie_count = sh.tot_cnt[pick];
+      sh.n_above = first ? higher : sh.n_above + higher;
+      if (first) sh.total = all;
+    }
+    __syncwarp();
+    if (!first) {
+      if (lane == 0) sh.remaining = target - static_cast<double>(sh.above_mass);
+      return;
+    }
+    // the bin that the four bins of its eighth hide: lane (peer, bin) reads, all lanes add
+    const uint32_t coarse = sh.digit;
+    const int sub = lane & (PER - 1);
+    const uint32_t d = coarse * PER + sub;
+    unsigned c = 0;
+    unsigned long long m = 0;
+    for (int r = lane / PER; r < CL; r += 32 / PER) {
+      c += *cl.of(&sh.fine_cnt[d], r);
+      if (by_mass) m += whole(cl.of(sh.fine_mass[0], r), kFineBins, d);
+    }
+#pragma unroll
+    for (int o = PER; o < 32; o <<= 1) {
+      c += __shfl_xor_sync(0xffffffffu, c, o);
+      m += __shfl_xor_sync(0xffffffffu, m, o);
+    }
+    // (narrowed: the lowest bin counts more than the set has of it, and nothing below it is looked at)
+    if (set.tie_mult > 0 && bucket_of<PER>(set.tie_key, max_scaled) == d) {
+      c += static_cast<unsigned>(set.tie_mult);
+      m += set.tie_mult * weight_fx(key_value(set.tie_key), max_scaled);
+    }
+    if (!by_mass) m = c;
+    unsigned long long acc = sh.above_mass, at = acc;
+    unsigned above = sh.n_above, before = above, count = 0;
+    int pick = -1;
+#pragma unroll
+    for (int k = PER - 1; k >= 0; --k) {
+      const unsigned ck = __shfl_sync(0xffffffffu, c, k);
+      const unsigned long long mk = __shfl_sync(0xffffffffu, m, k);
+      const bool done = pick >= 0 && reach != 0 && static_cast<double>(acc) >= target;
+      if (!done && ck != 0 && coarse * PER + k >= floor_bin) {
+        pick = k;
+        at = acc;
+        before = above;
+        count = ck;
+        acc += mk;
+        above += ck;
+      }
+    }
+    if (lane == 0) {
+      if (pick < 0) pick = 0;
+      sh.remaining = target - static_cast<double>(at);
+      sh.digit = coarse * PER + pick;
+      sh.tie_count = count;
+      sh.n_above = before;
+    }
+  };
+  // ---- the first digit
+  if (!narrowed) {
+    for (int i = tid; i < kFineBins; i += kSampleThreads)
+      sh.fine_cnt[i] = sh.fine_mass[0][i] = sh.fine_mass[1][i] = sh.fine_mass[2][i] = 0;
+    __syncthreads();
+    // Integer sums: the result does not depend on the order or the grouping of the additions.
+    for (int base = 0; base < row.n; base += kSampleThreads) {
+      const uint32_t k = base + tid < row.n ? row[base + tid] : 0u;
+      if (k <= set.excl) continue;
+      const uint32_t d = bucket_of<PER>(k, max_scaled);
+      atomicAdd(&sh.fine_cnt[d], 1u);
+      if (by_mass) add_mass(sh.fine_mass[0], kFineBins, d, weight_fx(key_value(k), max_scaled));
+    }
+    __syncthreads();
+    unsigned int* cnt = sh.cnt[pass & 1];
+    unsigned long long* mass = reinterpret_cast<unsigned long long*>(sh.mass[pass & 1][0]);
+    ++pass;
+    if (tid < 256) {
+      unsigned c = 0;
+      unsigned long long m = 0;
+#pragma unroll
+      for (int k = 0; k < PER; ++k) {
+        c += sh.fine_cnt[tid * PER + k];
+        if (by_mass) m += whole(sh.fine_mass[0], kFineBins, tid * PER + k);
+      }
+      cnt[tid] = c;
+      mass[tid] = m;
     }
     cl.sync();
     if (tid < 256) {
@@ -302,98 +451,90 @@ __device__ uint32_t radix_select(SampleShared& sh, SamplePeers<CL> cl, const Sam
 #pragma unroll
       for (int r = 0; r < CL; ++r) {
         c += *cl.of(&cnt[tid], r);
-        if (by_mass && row.wide)
-          m += *cl.of(reinterpret_cast<unsigned long long*>(mass[0]) + tid, r);
-        else if (by_mass)
-          m += *cl.of(&mass[0][tid], r) + (static_cast<unsigned long long>(*cl.of(&mass[1][tid], r)) << 14) +
-               (static_cast<unsigned long long>(*cl.of(&mass[2][tid], r)) << 28);
+        if (by_mass) m += *cl.of(&mass[tid], r);
+      }
+      if (set.tie_mult > 0 && bucket_of<PER>(set.tie_key, max_scaled) / PER == static_cast<uint32_t>(tid)) {
+        c += static_cast<unsigned int>(set.tie_mult);
+        if (by_mass) m += set.tie_mult * weight_fx(key_value(set.tie_key), max_scaled);
+      }
+      sh.tot_cnt[tid] = c;
+      sh.tot_mass[tid] = by_mass ? m : c;
+    }
+  } else {
+    cl.sync();                                   // peers are done with this CTA's former members
+  }
+  if (tid == 0) {
+    sh.own_n = 0;
+    sh.n_list = -1;
+  }
+  __syncthreads();
+  if (tid < 32) scan(true);
+  __syncthreads();
+  target = sh.remaining;
+  const uint32_t bucket = sh.digit;
+  if (sh.tie_count < kSampleList) {
+    const bool tie = set.tie_mult > 0 && bucket_of<PER>(set.tie_key, max_scaled) == bucket;
+    const unsigned above = sh.n_above;
+    gather_members(sh, cl, row, max_scaled, set, by_mass, tie,
+                   [&](uint32_t k) { return bucket_of<PER>(k, max_scaled) == bucket; });
+    const uint32_t key = solve_list(sh, tie, target, -1.0);
+    if (tid == 0) sh.n_above += above;
+    __syncthreads();
+    return key;
+  }
+  // ---- too many tokens in one bin: the bytes of their keys
+  uint32_t prefix = 0, prefix_mask = 0;
+  for (int shift = 24; shift >= 0; shift -= 8, ++pass) {
+    unsigned int* cnt = sh.cnt[pass & 1];
+    unsigned int(*mass)[256] = sh.mass[pass & 1];
+    if (tid < 256) cnt[tid] = mass[0][tid] = mass[1][tid] = mass[2][tid] = 0;
+    __syncthreads();
+    auto member = [&](uint32_t k) { return bucket_of<PER>(k, max_scaled) == bucket && (k & prefix_mask) == prefix; };
+    auto digit = [&](uint32_t k) { return (k >> shift) & 255u; };
+    // Lanes of a warp that hit the same digit add once, since the tokens that are left share their top bytes.
+    for (int base = 0; base < row.n; base += kSampleThreads) {
+      const uint32_t k = base + tid < row.n ? row[base + tid] : 0u;
+      const bool act = k > set.excl && member(k);
+      if (!__any_sync(0xffffffffu, act)) continue;
+      const uint32_t d = digit(k);
+      const unsigned peers = __match_any_sync(0xffffffffu, act ? d : 256u);
+      if (act) {
+        if (by_mass) add_mass(mass[0], 256, d, weight_fx(key_value(k), max_scaled));
+        if (lane == __ffs(peers) - 1) atomicAdd(&cnt[d], static_cast<unsigned>(__popc(peers)));
+      }
+    }
+    if (cl.rank() == 0 && tid == 0 && set.tie_mult > 0 && member(set.tie_key))
+      atomicAdd(&cnt[digit(set.tie_key)], static_cast<unsigned int>(set.tie_mult));
+    cl.sync();
+    if (tid < 256) {
+      unsigned int c = 0;
+      unsigned long long m = 0;
+#pragma unroll
+      for (int r = 0; r < CL; ++r) {
+        c += *cl.of(&cnt[tid], r);
+        if (by_mass) m += whole(cl.of(mass[0], r), 256, tid);
       }
       if (by_mass && set.tie_mult > 0 && member(set.tie_key) && digit(set.tie_key) == static_cast<uint32_t>(tid))
         m += set.tie_mult * weight_fx(key_value(set.tie_key), max_scaled);
       sh.tot_cnt[tid] = c;
       sh.tot_mass[tid] = by_mass ? m : c;
     }
-    if (tid == 0) {
-      sh.own_n = 0;
-      sh.n_list = -1;
-    }
     __syncthreads();
-    if (tid < 32) {
-      // eight bins per lane from the highest down: the first bin in use whose running sum reaches the target
-      unsigned long long sum = 0;
-      unsigned members = 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        sum += sh.tot_mass[255 - 8 * lane - j];
-        members += sh.tot_cnt[255 - 8 * lane - j];
-      }
-      const bool used = members != 0;
-      unsigned long long incl = sum;
-      unsigned higher = members;
-      for (int off = 1; off < 32; off <<= 1) {
-        const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, off);
-        const unsigned more = __shfl_up_sync(0xffffffffu, higher, off);
-        if (lane >= off) {
-          incl += up;
-          higher += more;
-        }
-      }
-      higher -= members;
-      const unsigned long long all = __shfl_sync(0xffffffffu, incl, 31);
-      if (first && frac >= 0.0) target = frac * static_cast<double>(all);
-      const unsigned reach = __ballot_sync(0xffffffffu, used && static_cast<double>(incl) >= target);
-      const unsigned any = __ballot_sync(0xffffffffu, used);
-      // rounding can leave the target just above the total: then the selection ends on the lowest key present
-      const int owner = reach != 0 ? __ffs(reach) - 1 : (any != 0 ? 31 - __clz(any) : 0);
-      if (lane == owner) {
-        unsigned long long acc = incl - sum, at = acc;
-        int pick = -1;
-        for (int j = 0; j < 8; ++j) {
-          const int d = 255 - 8 * lane - j;
-          if (sh.tot_cnt[d] == 0) continue;
-          if (pick >= 0) higher += sh.tot_cnt[pick];
-          pick = d;
-          at = acc;
-          acc += sh.tot_mass[d];
-          if (reach != 0 && static_cast<double>(acc) >= target) break;
-        }
-        if (pick < 0) pick = 0;
-        sh.remaining = target - static_cast<double>(at);
-        sh.digit = static_cast<unsigned int>(pick);
-        sh.tie_count = sh.tot_cnt[pick];
-        sh.n_above = first ? higher : sh.n_above + higher;
-        if (first) sh.total = all;
-      }
-    }
+    if (tid < 32) scan(false);
     __syncthreads();
     target = sh.remaining;
-    if (first) {
-      bucket = sh.digit;
-      if (sh.tie_count < kSampleList) {
-        ++pass;
-        const bool tie = set.tie_mult > 0 && member(set.tie_key) && bucket_of(set.tie_key, max_scaled) == bucket;
-        const unsigned above = sh.n_above;
-        gather_members(sh, cl, row, max_scaled, set, by_mass, tie,
-                       [&](uint32_t k) { return bucket_of(k, max_scaled) == bucket; });
-        const uint32_t key = solve_list(sh, tie, target, -1.0);
-        if (tid == 0) sh.n_above += above;
-        __syncthreads();
-        return key;
-      }
-    } else {
-      prefix |= sh.digit << shift;
-      prefix_mask |= 255u << shift;
-    }
+    prefix |= sh.digit << shift;
+    prefix_mask |= 255u << shift;
   }
   return prefix;
 }
 
-template <int CL>
+template <int CL, int PER>
 __global__ void __launch_bounds__(kSampleThreads)
 sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, const uint32_t* __restrict__ masks,
                    int mask_words, const ds41_sample_row* __restrict__ rows, int* __restrict__ tokens,
                    int* __restrict__ status) {
-  __shared__ SampleShared sh;
+  __shared__ SampleShared<PER> sh;
   extern __shared__ uint32_t key_store[];
   pdl_launch_dependents();
   pdl_wait();
@@ -616,8 +757,10 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
     gather_members(sh, cl, own, max_scaled, set, true, true, [](uint32_t) { return true; });
     gathered = true;
   };
+  bool narrowed = false;                           // the last selection's histogram holds the set's bins
   auto select = [&](double target, double frac) {
-    return gathered ? solve_list(sh, true, target, frac) : radix_select(sh, cl, own, max_scaled, set, true, target, frac, pass);
+    return gathered ? solve_list(sh, true, target, frac)
+                    : radix_select(sh, cl, own, max_scaled, set, true, target, frac, narrowed, pass);
   };
   unsigned long long survivors = all.allowed;
   if (p.min_p > 0.0f) {
@@ -627,7 +770,8 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   }
   if (survivors == 0) return finish(kSampleEmpty, 0);
   if (p.top_k > 0 && static_cast<unsigned long long>(p.top_k) < survivors) {
-    const uint32_t pk = radix_select(sh, cl, own, max_scaled, set, false, static_cast<double>(p.top_k), -1.0, pass);
+    const uint32_t pk = radix_select(sh, cl, own, max_scaled, set, false, static_cast<double>(p.top_k), -1.0, false,
+                                     pass);
     set.excl = pk;
     set.tie_key = pk;
     set.tie_mult = static_cast<unsigned long long>(fmin(fmax(sh.remaining, 1.0), static_cast<double>(sh.tie_count)));
@@ -636,6 +780,8 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
   double draw_of = -1.0, draw_frac = static_cast<double>(u);
   if (p.top_p < 1.0f) {
     const uint32_t pp = select(0.0, static_cast<double>(p.top_p));
+    // tot_* keep the first histogram unless the selection went on to the bytes of the keys, or had a list to begin with
+    narrowed = !gathered && sh.n_list >= 0;
     const double target = static_cast<double>(p.top_p) * static_cast<double>(sh.total);
     const double need = sh.remaining;
     const unsigned long long ties = sh.tie_count;
@@ -707,26 +853,35 @@ sample_rows_kernel(const float* __restrict__ logits, long long ld, int vocab, co
 
 using namespace ds41;
 
-template <int CL>
-static int launch_sample(const float* logits, long long ld, int rows, int vocab, const uint32_t* masks, int mask_words,
-                         const ds41_sample_row* params, int* tokens, int* status, cudaStream_t stream) {
+template <int CL, int PER>
+static int launch_sample_as(const float* logits, long long ld, int rows, int vocab, const uint32_t* masks, int mask_words,
+                            const ds41_sample_row* params, int* tokens, int* status, cudaStream_t stream) {
   const int slice = ((vocab + CL - 1) / CL + 31) & ~31;
   const size_t smem = slice <= kSampleMaxSlice ? 4ull * slice : 0;
+  constexpr int kMost = PER > 1 ? kSampleFineSlice : kSampleMaxSlice;
   static std::atomic<bool> configured[64];
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev].load(std::memory_order_acquire)) {
-    const cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel<CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               4 * kSampleMaxSlice);
+    const cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel<CL, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kMost);
     if (e != cudaSuccess) return e;
     configured[dev].store(true, std::memory_order_release);
   }
   if constexpr (CL == 1)
-    return launch_pdl(sample_rows_kernel<CL>, dim3(rows), dim3(kSampleThreads), smem, stream, logits, ld, vocab, masks,
+    return launch_pdl(sample_rows_kernel<CL, PER>, dim3(rows), dim3(kSampleThreads), smem, stream, logits, ld, vocab, masks,
                       mask_words, params, tokens, status);
   else
-    return launch_pdl_cluster(sample_rows_kernel<CL>, dim3(rows * CL), dim3(kSampleThreads), CL, smem, stream, logits, ld, vocab,
-                              masks, mask_words, params, tokens, status);
+    return launch_pdl_cluster(sample_rows_kernel<CL, PER>, dim3(rows * CL), dim3(kSampleThreads), CL, smem, stream, logits, ld,
+                              vocab, masks, mask_words, params, tokens, status);
+}
+
+template <int CL>
+static int launch_sample(const float* logits, long long ld, int rows, int vocab, const uint32_t* masks, int mask_words,
+                         const ds41_sample_row* params, int* tokens, int* status, cudaStream_t stream) {
+  const int slice = ((vocab + CL - 1) / CL + 31) & ~31;
+  return slice > kSampleFineSlice && slice <= kSampleMaxSlice
+             ? launch_sample_as<CL, 1>(logits, ld, rows, vocab, masks, mask_words, params, tokens, status, stream)
+             : launch_sample_as<CL, 4>(logits, ld, rows, vocab, masks, mask_words, params, tokens, status, stream);
 }
 
 // CTAs that share a row.  A row alone is fastest over eight; but about 15 clusters of eight run at once, 36 of four, 74 of two
