@@ -39,6 +39,13 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Address of the same shared variable in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t mine, uint32_t rank) {
+  uint32_t there;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(mine), "r"(rank));
+  return there;
+}
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

@@ -54,6 +54,64 @@ __device__ __forceinline__ float2 proj_at2(const ds41_proj& a, long long row, in
   }
   return s;
 }
+
+__device__ __forceinline__ void operator+=(float4& a, const float4& b) {
+  a.x += b.x;
+  a.y += b.y;
+  a.z += b.z;
+  a.w += b.w;
+}
+__device__ __forceinline__ void operator+=(float2& a, const float2& b) {
+  a.x += b.x;
+  a.y += b.y;
+}
+// The same places in passes of few rows, which are chains of latencies: eight planes are under way at once, whatever their number,
+// and added in their order.  The loops above have the first, then four together, then the rest one after the other (of eight
+// planes five round trips to L2, 0.4 us each); in kernels of many rows the registers are worth more.
+constexpr int kPlanes = 8;
+template <typename V>
+__device__ __forceinline__ void fetch_planes(V (&t)[kPlanes], const float* p, long long plane, int n) {
+#pragma unroll
+  for (int u = 0; u < kPlanes; ++u)
+    if (u < n) t[u] = *reinterpret_cast<const V*>(p + u * plane);
+}
+template <typename V>
+__device__ __forceinline__ V add_planes(V (&t)[kPlanes], const float* p, long long plane, int n) {
+  V s = t[0];
+#pragma unroll
+  for (int u = 1; u < kPlanes; ++u)
+    if (u < n) s += t[u];
+  for (int k = kPlanes; k < n; k += kPlanes) {
+    fetch_planes(t, p + k * plane, plane, n - k);
+#pragma unroll
+    for (int u = 0; u < kPlanes; ++u)
+      if (k + u < n) s += t[u];
+  }
+  return s;
+}
+template <typename V>
+__device__ __forceinline__ V sum_planes(const float* p, long long plane, int n) {
+  if (n == 1) return *reinterpret_cast<const V*>(p);
+  V t[kPlanes];
+  fetch_planes(t, p, plane, n);
+  return add_planes(t, p, plane, n);
+}
+
+__device__ __forceinline__ float few_at(const ds41_proj& a, long long row, int col) {
+  const long long i = row * a.ld + a.col + col;
+  if (a.bf16) return proj_at(a, row, col);
+  return sum_planes<float>(static_cast<const float*>(a.data) + i, a.plane, a.splits);
+}
+__device__ __forceinline__ float2 few_at2(const ds41_proj& a, long long row, int col) {
+  const long long i = row * a.ld + a.col + col;
+  if (a.bf16) return proj_at2(a, row, col);
+  return sum_planes<float2>(static_cast<const float*>(a.data) + i, a.plane, a.splits);
+}
+__device__ __forceinline__ float4 few_at4(const ds41_proj& a, long long row, int col) {
+  const long long i = row * a.ld + a.col + col;
+  if (a.bf16) return proj_at4(a, row, col);
+  return sum_planes<float4>(static_cast<const float*>(a.data) + i, a.plane, a.splits);
+}
 __device__ __forceinline__ void store2(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
 __device__ __forceinline__ void store2(__nv_bfloat16* p, float x, float y) {
   *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y);

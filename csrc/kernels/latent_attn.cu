@@ -31,7 +31,7 @@ __device__ __forceinline__ void norm_row(const ds41_proj& p, int r, int n, const
   float q = 0.f;
   int c = 0;
   for (int i = 4 * threadIdx.x; i < n; i += 4 * blockDim.x, ++c) {
-    float4 v = proj_at4(p, r, i);
+    float4 v = few_at4(p, r, i);
     if (i + 1 >= n) v.y = 0.f;
     if (i + 2 >= n) v.z = 0.f;
     if (i + 3 >= n) v.w = 0.f;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256) latent_query_kernel(ds41_proj q, const in
   const int first = in_place ? dim_pad : 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < heads * half; i += gridDim.x * blockDim.x) {
     const int h = i / half, j = 2 * (i - h * half) + first, c = h * hs + j;
-    const float2 ab = proj_at2(q, r, c);
+    const float2 ab = few_at2(q, r, c);
     float a = ab.x, b = ab.y;
     const int t = j - dim_pad;
     if (t >= 0 && t < rot_dim) {

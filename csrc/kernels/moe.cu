@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kRouteThreads) route_softmax_kernel(ds41_route
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
       const int e = lane + 32 * i;
-      z[i] = e < p.experts ? proj_at(p.z, r, e) + (p.bias != nullptr ? p.bias[e] : 0.f) : -INFINITY;
+      z[i] = e < p.experts ? few_at(p.z, r, e) + (p.bias != nullptr ? p.bias[e] : 0.f) : -INFINITY;
     }
     float my_z = -INFINITY, best = -INFINITY;
     int my_id = -1;

@@ -49,20 +49,19 @@ __device__ __forceinline__ float piece_sq(float4 v, float mean, int live) {
 // Subtrahend and factor of a row's norm - layer norm (subtract the mean) or RMS norm (mean of squares) - from the pieces of
 // four columns that the threads hold; `n` columns of the row are in this CTA, piece i covers columns 4 (tid + i blockDim).
 // Deviations are taken from each thread's own mean and merged pairwise, over the warp, the CTA and the cluster, in an order
-// that is the same in every thread.  `slot` holds 3 x 32 floats; at most 32 warps (4 per CTA of a cluster of 8).
+// that is the same in every thread.
 // FULL: every thread holds whole pieces and the warps' number is a power of two, so that both halves of every merge count the
 // same and nothing but means and deviations travels.
-template <int CL, int NI, bool FULL>
-__device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, int kind, float eps, float* slot) {
+template <int NI, bool FULL, class EXCHANGE>
+__device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, int kind, float eps, EXCHANGE exchange) {
+  const int lane = threadIdx.x & 31;
   if constexpr (FULL) {
-    static_assert(CL == 1, "one CTA per row");
     float s = 0.f, q = 0.f;
 #pragma unroll
     for (int i = 0; i < NI; ++i) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
     float mean = kind == 0 ? s / (4 * NI) : 0.f;                     // an RMS norm merges with zero means
 #pragma unroll
     for (int i = 0; i < NI; ++i) q += piece_sq(v[i], mean, 4);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     float half = 2.0f * NI;                // half the number of columns that one side of a merge has
     auto merge_over = [&](int o) {         // merge() of the lower lane's columns and the upper one's, the same in both
       const float m = __shfl_xor_sync(0xffffffffu, mean, o), t = __shfl_xor_sync(0xffffffffu, q, o);
@@ -78,14 +77,10 @@ __device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, 
     } else {
       q = warp_sum(q);
     }
-    if (lane == 0) {
-      slot[warp] = mean;
-      slot[32 + warp] = q;
-    }
-    __syncthreads();
-    mean = slot[lane & (n_warps - 1)];
-    q = slot[32 + (lane & (n_warps - 1))];
-    for (int o = n_warps >> 1; o; o >>= 1) {
+    const Moments t = exchange(Moments{mean, q, 0.f});
+    mean = t.mean;
+    q = t.m2;
+    for (int o = exchange.warps >> 1; o; o >>= 1) {
       if (kind == 0) merge_over(o);
       else q += __shfl_xor_sync(0xffffffffu, q, o);
     }
@@ -108,29 +103,61 @@ __device__ __forceinline__ float2 row_norm(const float4 (&v)[NI], int n, int W, 
   Moments t{mean, q, cnt};
   if (kind == 0) t = merge_lanes(t);
   else t.m2 = warp_sum(q);                 // no means to merge
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
-  if (lane == 0) {
-    slot[warp] = t.mean;
-    slot[32 + warp] = t.m2;
-    slot[64 + warp] = t.n;
-  }
-  t = {0.f, 0.f, 0.f};
-  if constexpr (CL == 1) {
-    __syncthreads();
-    if (lane < n_warps) t = {slot[lane], slot[32 + lane], slot[64 + lane]};
-  } else {
-    cg::cluster_group cluster = cg::this_cluster();
-    cluster.sync();
-    if (lane < CL * n_warps) {
-      const float* far = cluster.map_shared_rank(slot, lane / n_warps);
-      const int w = lane % n_warps;
-      t = {far[w], far[32 + w], far[64 + w]};
-    }
-  }
+  t = exchange(t);
+  if (lane >= exchange.warps) t = {0.f, 0.f, 0.f};
   if (kind == 0) t = merge_lanes(t);
   else t.m2 = warp_sum(t.m2);
   return make_float2(t.mean, 1.0f / sqrtf(t.m2 / W + eps));
 }
+
+// What row_norm asks of the threads that share a row: every warp's moments in, lane l gets those of warp l % warps (of `warps`,
+// at most 32) out.  One CTA: through shared memory, one barrier.  `slot` holds 3 x 32 floats.
+struct BlockExchange {
+  float* slot;
+  int warps;
+  __device__ __forceinline__ Moments operator()(Moments t) const {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+      slot[warp] = t.mean;
+      slot[32 + warp] = t.m2;
+      slot[64 + warp] = t.n;
+    }
+    __syncthreads();
+    const int w = lane < warps ? lane : lane & (warps - 1);      // the lanes beyond are read where `warps` is a power of two
+    return {slot[w], slot[32 + w], slot[64 + w]};
+  }
+};
+
+// The CTAs of a cluster: every warp sends its moments to all of them, 16 bytes each, and counts on a barrier there; a warp waits for
+// its own CTA's copy alone.  (A barrier of the cluster and loads from the peers afterwards: 2000 cycles a norm instead of 1000.)
+constexpr int kShare = 8;              // CTAs that share a row
+struct RowShare {
+  float4 moments[32];
+  uint64_t bar;
+};
+struct ClusterExchange {
+  RowShare* sh;
+  int rank, warps;
+  __device__ __forceinline__ Moments operator()(Moments t) const {
+    const int lane = threadIdx.x & 31, at = rank * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (lane < kShare) {
+      const uint32_t to = cluster_addr(smem_u32(&sh->moments[at]), lane), bar = cluster_addr(smem_u32(&sh->bar), lane);
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                   ::"r"(to), "r"(__float_as_uint(t.mean)), "r"(__float_as_uint(t.m2)), "r"(__float_as_uint(t.n)), "r"(0u), "r"(bar)
+                   : "memory");
+    }
+    __syncwarp();
+    mbar_wait(&sh->bar, 0, nullptr, 0);
+    const float4 m = sh->moments[lane < warps ? lane : lane & (warps - 1)];
+    return {m.x, m.y, m.z};
+  }
+  // sh->bar counts the stores of all warps; peers may send once the cluster has met after this
+  __device__ __forceinline__ static void prepare(RowShare& sh, int warps) {
+    mbar_init(&sh.bar, 1);
+    mbar_init_fence();
+    mbar_expect_tx(&sh.bar, 16 * warps);
+  }
+};
 
 // Four columns of the sum of a row's routed results, in route order.
 __device__ __forceinline__ float4 routed_at4(const ds41_resid_args& p, int r, int col) {
@@ -152,13 +179,10 @@ __device__ __forceinline__ float4 routed_at4(const ds41_resid_args& p, int r, in
 // 22 % of the memory's rate; more threads or more rows an SM made it slower), so rows that fill the threads' pieces (FULL) shorten
 // the chain by every test of a column against the row's end.  2048 rows x 4096 columns: 75 -> 57 us on average in a model with
 // kept streams, 49 -> 39 without; 953 rows 28 -> 22.
-template <typename T, int CL, int NI, bool FULL>
-__global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_step_kernel(ds41_resid_args p) {
+template <typename T, int NI, bool FULL>
+__global__ void __launch_bounds__(NI <= 4 ? 256 : 512) resid_step_kernel(ds41_resid_args p) {
   __shared__ float slots[2][96];
-  const int per = ((p.W + CL - 1) / CL + 3) / 4 * 4;
-  const int part = CL > 1 ? blockIdx.x % CL : 0;
-  const int r = CL > 1 ? blockIdx.x / CL : blockIdx.x;
-  const int c0 = min(p.W, part * per), n = min(p.W, c0 + per) - c0;
+  const int r = blockIdx.x, n_warps = blockDim.x >> 5;
   pdl_launch_dependents();
   pdl_wait();
   float4 x[NI];
@@ -166,33 +190,70 @@ __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_s
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
     at[i] = 4 * (threadIdx.x + i * blockDim.x);
-    live[i] = FULL ? 4 : n - at[i];
+    live[i] = FULL ? 4 : p.W - at[i];
     x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (p.tokens != nullptr) {
     const int tok = p.tokens[r];
-    const ds41_proj e{p.embed, 0, static_cast<int>(p.embed_ld), 1, 1, c0};
+    const ds41_proj e{p.embed, 0, static_cast<int>(p.embed_ld), 1, 1, 0};
     if (tok >= 0 && tok < p.vocab)
 #pragma unroll
       for (int i = 0; i < NI; ++i)
         if (live[i] > 0) x[i] = proj_at4(e, tok, at[i]);
   } else {
-    const float* in = p.x_in + r * p.ldx + c0;
+    const float* in = p.x_in + r * p.ldx;
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (live[i] > 0) x[i] = *reinterpret_cast<const float4*>(in + at[i]);
   }
-  // Few rows (clusters): what does not depend on the sublayer is loaded first - the weighted sum of the older kept streams,
-  // the norm weight - since the launch is a chain of latencies.  Many rows: the registers are worth more.
-  constexpr bool kEarly = CL > 1;
-  float4 older[NI], w_next[NI];
+  auto clip = [&](float4& v, int i) {         // columns beyond the row hold zeros
+    if (FULL) return;
+    if (live[i] < 4) v.w = 0.f;
+    if (live[i] < 3) v.z = 0.f;
+    if (live[i] < 2) v.y = 0.f;
+  };
+  if (p.y.data != nullptr) {
+    float4 y[NI];
 #pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    older[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (kEarly) w_next[i] = p.next_w != nullptr && live[i] > 0 ? load4(p.next_w + c0 + at[i], live[i]) : older[i];
+    for (int i = 0; i < NI; ++i) {
+      y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (live[i] > 0) {
+        y[i] = p.y_route != nullptr ? routed_at4(p, r, at[i]) : proj_at4(p.y, r, at[i]);
+        if (p.gate.data != nullptr) {
+          const float4 g = proj_at4(p.gate, r, at[i]), b = load4(p.gate_bias + at[i], live[i]);
+          y[i].x *= sigmoid_f32(g.x + b.x);
+          y[i].y *= sigmoid_f32(g.y + b.y);
+          y[i].z *= sigmoid_f32(g.z + b.z);
+          y[i].w *= sigmoid_f32(g.w + b.w);
+        }
+        clip(y[i], i);
+      }
+    }
+    float2 s = make_float2(0.f, 1.f);
+    if (p.post_w != nullptr) s = row_norm<NI, FULL>(y, p.W, p.W, p.post_rms ? 1 : p.norm_kind, p.eps, BlockExchange{slots[0], n_warps});
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (live[i] > 0) {
+        const float4 w = p.post_w != nullptr ? load4(p.post_w + at[i], live[i]) : make_float4(1.f, 1.f, 1.f, 1.f);
+        x[i].x += (y[i].x - s.x) * s.y * w.x;
+        x[i].y += (y[i].y - s.x) * s.y * w.y;
+        x[i].z += (y[i].z - s.x) * s.y * w.z;
+        x[i].w += (y[i].w - s.x) * s.y * w.w;
+      }
   }
-  auto add_older = [&]() {
-    const float* k0 = p.kept + r * p.ldx + c0;
+#pragma unroll
+  for (int i = 0; i < NI; ++i) clip(x[i], i);
+  if (p.x_out != nullptr) {
+    float* o = p.x_out + r * p.ldx;
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (live[i] > 0) store4(o + at[i], x[i]);
+  }
+  if (p.mix != nullptr) {
+    float4 older[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) older[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* k0 = p.kept + r * p.ldx;
 #pragma unroll 4
     for (int j = 0; j < p.n_mix - 1; ++j) {
       const float c = p.mix[j];
@@ -206,53 +267,6 @@ __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_s
           older[i].w += c * k.w;
         }
     }
-  };
-  if (kEarly && p.mix != nullptr) add_older();
-  auto clip = [&](float4& v, int i) {         // columns beyond the row hold zeros
-    if (FULL) return;
-    if (live[i] < 4) v.w = 0.f;
-    if (live[i] < 3) v.z = 0.f;
-    if (live[i] < 2) v.y = 0.f;
-  };
-  if (p.y.data != nullptr) {
-    float4 y[NI];
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (live[i] > 0) {
-        y[i] = p.y_route != nullptr ? routed_at4(p, r, c0 + at[i]) : proj_at4(p.y, r, c0 + at[i]);
-        if (p.gate.data != nullptr) {
-          const float4 g = proj_at4(p.gate, r, c0 + at[i]), b = load4(p.gate_bias + c0 + at[i], live[i]);
-          y[i].x *= sigmoid_f32(g.x + b.x);
-          y[i].y *= sigmoid_f32(g.y + b.y);
-          y[i].z *= sigmoid_f32(g.z + b.z);
-          y[i].w *= sigmoid_f32(g.w + b.w);
-        }
-        clip(y[i], i);
-      }
-    }
-    float2 s = make_float2(0.f, 1.f);
-    if (p.post_w != nullptr) s = row_norm<CL, NI, FULL>(y, n, p.W, p.post_rms ? 1 : p.norm_kind, p.eps, slots[0]);
-#pragma unroll
-    for (int i = 0; i < NI; ++i)
-      if (live[i] > 0) {
-        const float4 w = p.post_w != nullptr ? load4(p.post_w + c0 + at[i], live[i]) : make_float4(1.f, 1.f, 1.f, 1.f);
-        x[i].x += (y[i].x - s.x) * s.y * w.x;
-        x[i].y += (y[i].y - s.x) * s.y * w.y;
-        x[i].z += (y[i].z - s.x) * s.y * w.z;
-        x[i].w += (y[i].w - s.x) * s.y * w.w;
-      }
-  }
-#pragma unroll
-  for (int i = 0; i < NI; ++i) clip(x[i], i);
-  if (p.x_out != nullptr) {
-    float* o = p.x_out + r * p.ldx + c0;
-#pragma unroll
-    for (int i = 0; i < NI; ++i)
-      if (live[i] > 0) store4(o + at[i], x[i]);
-  }
-  if (p.mix != nullptr) {
-    if (!kEarly) add_older();
     const float last = p.mix[p.n_mix - 1];    // the newest kept stream is the row this block holds
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
@@ -261,30 +275,214 @@ __global__ void __launch_bounds__(CL == 8 ? 128 : (NI <= 4 ? 256 : 512)) resid_s
       clip(x[i], i);
     }
     if (p.x_avg != nullptr) {
-      float* o = p.x_avg + r * p.ldx + c0;
+      float* o = p.x_avg + r * p.ldx;
 #pragma unroll
       for (int i = 0; i < NI; ++i)
         if (live[i] > 0) store4(o + at[i], x[i]);
     }
   }
   if (p.next_w != nullptr) {
-    const float2 s = row_norm<CL, NI, FULL>(x, n, p.W, p.norm_kind, p.eps, slots[1]);
-    T* h = static_cast<T*>(p.h) + 1ll * r * p.ldh + c0;
+    const float2 s = row_norm<NI, FULL>(x, p.W, p.W, p.norm_kind, p.eps, BlockExchange{slots[1], n_warps});
+    T* h = static_cast<T*>(p.h) + 1ll * r * p.ldh;
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (live[i] > 0) {
-        const float4 w = kEarly ? w_next[i] : load4(p.next_w + c0 + at[i], live[i]);
+        const float4 w = load4(p.next_w + at[i], live[i]);
         store4(h + at[i], make_float4((x[i].x - s.x) * s.y * w.x, (x[i].y - s.x) * s.y * w.y, (x[i].z - s.x) * s.y * w.z,
                                       (x[i].w - s.x) * s.y * w.w));
       }
   }
   if (p.next_w == nullptr && p.raw_h) {
-    T* h = static_cast<T*>(p.h) + 1ll * r * p.ldh + c0;
+    T* h = static_cast<T*>(p.h) + 1ll * r * p.ldh;
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (live[i] > 0) store4(h + at[i], x[i]);
   }
-  if constexpr (CL > 1) cg::this_cluster().sync();      // peers may still read this CTA's moments
+}
+
+// A place of a projection whose loads are under way: all planes (up to eight), or the bf16 value.
+struct Ahead {
+  float4 t[kPlanes];
+  __device__ __forceinline__ void ask(const ds41_proj& a, long long row, int col) {
+    const long long i = row * a.ld + a.col + col;
+    if (a.bf16) t[0] = proj_at4(a, row, col);
+    else fetch_planes(t, static_cast<const float*>(a.data) + i, a.plane, a.splits);
+  }
+  __device__ __forceinline__ float4 get(const ds41_proj& a, long long row, int col) {
+    if (a.bf16 || a.splits == 1) return t[0];
+    return add_planes(t, static_cast<const float*>(a.data) + row * a.ld + a.col + col, a.plane, a.splits);
+  }
+};
+
+// A row's routed results again, ids and rows under way together.
+__device__ __forceinline__ float4 routed_few4(const ds41_resid_args& p, int r, int col) {
+  constexpr int kMost = 8;
+  if (p.y_top > kMost || p.y.bf16 || p.y.splits != 1) return routed_at4(p, r, col);
+  int e[kMost];
+  float4 v[kMost], s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int k = 0; k < kMost; ++k) e[k] = k < p.y_top ? p.y_route[r * p.y_top + k] : -1;
+  const float* base = static_cast<const float*>(p.y.data) + p.y.col + col;
+#pragma unroll
+  for (int k = 0; k < kMost; ++k)
+    if (e[k] >= 0)
+      v[k] = *reinterpret_cast<const float4*>(base + (p.y_rows > 0 ? 1ll * e[k] * p.y_rows + r : 1ll * r * p.y_top + k) * p.y.ld);
+#pragma unroll
+  for (int k = 0; k < kMost; ++k)
+    if (e[k] >= 0) s += v[k];
+  return s;
+}
+
+// Few rows: a cluster of eight CTAs shares a row, so that its loads do not queue on one SM.  The launch is a chain of latencies:
+// weights are read before the wait for the previous kernel, everything else is asked for at once behind it (rows of up to 4096
+// columns, a piece of four a thread), and each norm costs one way to the peers.  Inside a graph, one row of 2048 columns with
+// kept streams and eight planes of result and gate: 10.3 us with loads plane by plane, divisions in every merge of moments and a
+// cluster barrier with loads from the peers behind it, 6.5 so; eight rows without kept streams 5.0 and 4.2.
+template <typename T, int NI, bool FULL>
+__global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
+  __shared__ RowShare share[2];
+  const int per = ((p.W + kShare - 1) / kShare + 3) / 4 * 4;
+  const int part = blockIdx.x % kShare, r = blockIdx.x / kShare, lane = threadIdx.x & 31;
+  const int c0 = min(p.W, part * per), n = min(p.W, c0 + per) - c0, warps = kShare * (blockDim.x >> 5);
+  if (threadIdx.x == 0) {
+    ClusterExchange::prepare(share[0], warps);
+    ClusterExchange::prepare(share[1], warps);
+  }
+  cg::cluster_group::barrier_arrive();
+  pdl_launch_dependents();
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
+  float4 x[NI], y[NI], older[NI], w_next[NI], w_post[NI], bias[NI];
+  int at[NI], live[NI];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int c = 4 * (threadIdx.x + i * blockDim.x);
+    live[i] = FULL ? 4 : n - c;
+    at[i] = c0 + c;
+    x[i] = y[i] = older[i] = zero;
+    w_next[i] = p.next_w != nullptr && live[i] > 0 ? load4(p.next_w + at[i], live[i]) : zero;
+    w_post[i] = p.post_w != nullptr && live[i] > 0 ? load4(p.post_w + at[i], live[i]) : one;
+    bias[i] = p.gate.data != nullptr && live[i] > 0 ? load4(p.gate_bias + at[i], live[i]) : zero;
+  }
+  const int n_old = p.mix != nullptr ? p.n_mix - 1 : 0;
+  const float mix_lane = lane <= n_old && p.mix != nullptr ? p.mix[lane] : 0.f;
+  auto weight = [&](int j) { return j < 32 ? __shfl_sync(0xffffffffu, mix_lane, j) : p.mix[j]; };
+  cg::cluster_group::barrier_wait();
+  pdl_wait();
+  // ---- loads
+  const float* kept = p.kept + r * p.ldx;
+  const bool plain = p.y.data != nullptr && p.y_route == nullptr;
+  constexpr bool kAhead = NI == 1;         // one piece a thread: everything is under way before the first sum
+  Ahead ya, ga, ka;
+  if (p.tokens != nullptr) {
+    const int tok = p.tokens[r];
+    const ds41_proj e{p.embed, 0, static_cast<int>(p.embed_ld), 1, 1, 0};
+    if (tok >= 0 && tok < p.vocab)
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        if (live[i] > 0) x[i] = proj_at4(e, tok, at[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (live[i] > 0) x[i] = *reinterpret_cast<const float4*>(p.x_in + r * p.ldx + at[i]);
+  }
+  if (kAhead && live[0] > 0) {
+    if (plain) ya.ask(p.y, r, at[0]);
+    if (p.y.data != nullptr && p.gate.data != nullptr) ga.ask(p.gate, r, at[0]);
+    fetch_planes(ka.t, kept + at[0], p.kept_stride, n_old);
+  }
+  if (p.y.data != nullptr && p.y_route != nullptr)
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (live[i] > 0) y[i] = routed_few4(p, r, at[i]);
+  // ---- the weighted sum of the older kept streams
+  auto add_old = [&](int i, float c, float4 k) {
+    older[i].x += c * k.x;
+    older[i].y += c * k.y;
+    older[i].z += c * k.z;
+    older[i].w += c * k.w;
+  };
+  if constexpr (kAhead) {
+    for (int j0 = 0; j0 < n_old; j0 += kPlanes) {
+      if (j0 > 0 && live[0] > 0) fetch_planes(ka.t, kept + j0 * p.kept_stride + at[0], p.kept_stride, n_old - j0);
+#pragma unroll
+      for (int u = 0; u < kPlanes; ++u)
+        if (j0 + u < n_old) {
+          const float c = weight(j0 + u);
+          if (live[0] > 0) add_old(0, c, ka.t[u]);
+        }
+    }
+  } else {
+#pragma unroll 4
+    for (int j = 0; j < n_old; ++j) {
+      const float c = weight(j);
+#pragma unroll
+      for (int i = 0; i < NI; ++i)
+        if (live[i] > 0) add_old(i, c, *reinterpret_cast<const float4*>(kept + j * p.kept_stride + at[i]));
+    }
+  }
+  auto clip = [&](float4& v, int i) {         // columns beyond the row hold zeros
+    if (FULL) return;
+    if (live[i] < 4) v.w = 0.f;
+    if (live[i] < 3) v.z = 0.f;
+    if (live[i] < 2) v.y = 0.f;
+  };
+  // ---- the sublayer's result
+  if (p.y.data != nullptr) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (live[i] > 0) {
+        if (plain) y[i] = kAhead ? ya.get(p.y, r, at[i]) : few_at4(p.y, r, at[i]);
+        if (p.gate.data != nullptr) {
+          const float4 g = kAhead ? ga.get(p.gate, r, at[i]) : few_at4(p.gate, r, at[i]);
+          y[i].x *= sigmoid_f32(g.x + bias[i].x);
+          y[i].y *= sigmoid_f32(g.y + bias[i].y);
+          y[i].z *= sigmoid_f32(g.z + bias[i].z);
+          y[i].w *= sigmoid_f32(g.w + bias[i].w);
+        }
+        clip(y[i], i);
+      }
+    float2 s = make_float2(0.f, 1.f);
+    if (p.post_w != nullptr)
+      s = row_norm<NI, FULL>(y, n, p.W, p.post_rms ? 1 : p.norm_kind, p.eps, ClusterExchange{&share[0], part, warps});
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (live[i] > 0) {
+        x[i].x += (y[i].x - s.x) * s.y * w_post[i].x;
+        x[i].y += (y[i].y - s.x) * s.y * w_post[i].y;
+        x[i].z += (y[i].z - s.x) * s.y * w_post[i].z;
+        x[i].w += (y[i].w - s.x) * s.y * w_post[i].w;
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < NI; ++i) clip(x[i], i);
+  const float4(&stream)[NI] = x;
+  float4 avg[NI];
+  const float last = p.mix != nullptr ? weight(n_old) : 0.f;      // the newest kept stream is the row this block holds
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    avg[i] = x[i];
+    if (p.mix != nullptr) {
+      avg[i] = make_float4(older[i].x + last * x[i].x, older[i].y + last * x[i].y, older[i].z + last * x[i].z,
+                           older[i].w + last * x[i].w);
+      clip(avg[i], i);
+    }
+  }
+  float2 s = make_float2(0.f, 1.f);
+  if (p.next_w != nullptr) s = row_norm<NI, FULL>(avg, n, p.W, p.norm_kind, p.eps, ClusterExchange{&share[1], part, warps});
+  cg::cluster_group::barrier_arrive();
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    if (live[i] <= 0) continue;
+    if (p.x_out != nullptr) store4(p.x_out + r * p.ldx + at[i], stream[i]);
+    if (p.mix != nullptr && p.x_avg != nullptr) store4(p.x_avg + r * p.ldx + at[i], avg[i]);
+    T* h = static_cast<T*>(p.h) + 1ll * r * p.ldh + at[i];
+    if (p.next_w != nullptr)
+      store4(h, make_float4((avg[i].x - s.x) * s.y * w_next[i].x, (avg[i].y - s.x) * s.y * w_next[i].y,
+                            (avg[i].z - s.x) * s.y * w_next[i].z, (avg[i].w - s.x) * s.y * w_next[i].w));
+    else if (p.raw_h)
+      store4(h, avg[i]);
+  }
+  cg::cluster_group::barrier_wait();           // no CTA leaves while a peer may still send to it
 }
 
 template <typename T>
@@ -344,7 +542,7 @@ __global__ void __launch_bounds__(256) gate_mul_kernel(ds41_proj y, ds41_proj ga
   pdl_launch_dependents();
   pdl_wait();
   if (i >= n) return;
-  const float4 v = proj_at4(y, r, i), g = proj_at4(gate, r, i);
+  const float4 v = few_at4(y, r, i), g = few_at4(gate, r, i);
   store4(out + 1ll * r * ld_out + i, make_float4(v.x * sigmoid_f32(g.x), v.y * sigmoid_f32(g.y), v.z * sigmoid_f32(g.z),
                                                  v.w * sigmoid_f32(g.w)));
 }
@@ -365,7 +563,7 @@ __global__ void __launch_bounds__(128) head_norm_gate_kernel(const float* o, int
     const float4 v = load4(src + i, width - i);
     if (i < 4 * static_cast<int>(blockDim.x)) {
       v0 = v;
-      g0 = proj_at4(gate, r, h * stride + i);
+      g0 = few_at4(gate, r, h * stride + i);
       w0 = load4(w + h * stride + i, width - i);
     }
     q += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
@@ -436,7 +634,7 @@ __global__ void __launch_bounds__(128) side_act_kernel(ds41_proj z, const int* t
   for (int j = threadIdx.x; j < ld_out; j += blockDim.x) {
     float v = 0.f;
     if (j < n) {
-      const float a = proj_at(z, r, j);
+      const float a = few_at(z, r, j);
       const float e = known ? __bfloat162float(embed[tok * embed_ld + col + j]) : 0.f;
       v = 0.5f * a * (1.0f + tanhf(0.7978845608028654f * (a + 0.044715f * a * a * a))) * e;
     }
@@ -461,26 +659,30 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const T* src, int ld, 
   dst[1ll * r * ld + i] = s >= 0 && s < n_src ? src[1ll * s * ld + i] : from_f32<T>(0.f);
 }
 
-template <typename T, int CL, int NI>
+// FULL: a row fills the pieces of the threads that share it, whose warps' number is a power of two
+template <typename T, bool FEW, int NI>
 static cudaError_t launch_resid_ni(const ds41_resid_args& a, int threads, cudaStream_t st) {
-  if constexpr (CL == 1) {
-    if (a.W == 4 * NI * threads && (threads & (threads - 1)) == 0)
-      return launch_pdl(resid_step_kernel<T, CL, NI, true>, dim3(a.rows), dim3(threads), 0, st, a);
-    return launch_pdl(resid_step_kernel<T, CL, NI, false>, dim3(a.rows), dim3(threads), 0, st, a);
+  const bool even = (threads & (threads - 1)) == 0;
+  if constexpr (!FEW) {
+    if (even && a.W == 4 * NI * threads)
+      return launch_pdl(resid_step_kernel<T, NI, true>, dim3(a.rows), dim3(threads), 0, st, a);
+    return launch_pdl(resid_step_kernel<T, NI, false>, dim3(a.rows), dim3(threads), 0, st, a);
   } else {
-    return launch_pdl_cluster(resid_step_kernel<T, CL, NI, false>, dim3(a.rows * CL), dim3(threads), CL, 0, st, a);
+    if (even && a.W == kShare * 4 * NI * threads)
+      return launch_pdl_cluster(resid_few_kernel<T, NI, true>, dim3(a.rows * kShare), dim3(threads), kShare, 0, st, a);
+    return launch_pdl_cluster(resid_few_kernel<T, NI, false>, dim3(a.rows * kShare), dim3(threads), kShare, 0, st, a);
   }
 }
 
-template <typename T, int CL>
+template <typename T, bool FEW>
 static cudaError_t launch_resid(const ds41_resid_args& a, cudaStream_t st) {
-  const int pieces = ((a.W + CL - 1) / CL + 3) / 4;
+  const int ctas = FEW ? kShare : 1, pieces = ((a.W + ctas - 1) / ctas + 3) / 4;
   const auto width = [&](int ni) { return ((pieces + ni - 1) / ni + 31) / 32 * 32; };
-  constexpr int kMost = CL == 8 ? 128 : 256;        // the moments of a cluster's warps fit one warp
-  if (width(1) <= kMost) return launch_resid_ni<T, CL, 1>(a, width(1), st);
-  if (width(2) <= kMost) return launch_resid_ni<T, CL, 2>(a, width(2), st);
-  if (width(4) <= kMost) return launch_resid_ni<T, CL, 4>(a, width(4), st);
-  if (width(8) <= (CL == 8 ? 128 : 512)) return launch_resid_ni<T, CL, 8>(a, width(8), st);
+  constexpr int kMost = FEW ? 128 : 256;            // the moments of a cluster's warps fit one warp
+  if (width(1) <= kMost) return launch_resid_ni<T, FEW, 1>(a, width(1), st);
+  if (width(2) <= kMost) return launch_resid_ni<T, FEW, 2>(a, width(2), st);
+  if (width(4) <= kMost) return launch_resid_ni<T, FEW, 4>(a, width(4), st);
+  if (width(8) <= (FEW ? 128 : 512)) return launch_resid_ni<T, FEW, 8>(a, width(8), st);
   return cudaErrorInvalidValue;
 }
 
@@ -504,8 +706,8 @@ extern "C" int ds41_resid_step(const ds41_resid_args* a, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // few rows: a cluster of eight CTAs shares a row, so that its loads do not queue on one SM
   const bool wide = (a->rows <= 32 && a->W >= 1024) || a->W > 16384;
-  if (a->f32) return wide ? launch_resid<float, 8>(*a, st) : launch_resid<float, 1>(*a, st);
-  return wide ? launch_resid<__nv_bfloat16, 8>(*a, st) : launch_resid<__nv_bfloat16, 1>(*a, st);
+  if (a->f32) return wide ? launch_resid<float, true>(*a, st) : launch_resid<float, false>(*a, st);
+  return wide ? launch_resid<__nv_bfloat16, true>(*a, st) : launch_resid<__nv_bfloat16, false>(*a, st);
 }
 
 template <typename T>

@@ -354,6 +354,53 @@ def test_residual_step_of_whole_pieces(rows, W, kind):
     test_residual_step(rows, W, kind)
 
 
+@pytest.mark.parametrize("rows,W,planes,n_mix,top,kind", [(1, 1024, 1, 1, 0, 0), (2, 2048, 8, 9, 0, 0), (1, 2048, 9, 10, 0, 1),
+                                                          (3, 4096, 17, 33, 0, 0), (1, 4096, 2, 34, 0, 0), (2, 3000, 9, 10, 0, 0),
+                                                          (1, 8192, 9, 4, 0, 1), (4, 2048, 1, 0, 4, 1), (3, 1032, 1, 0, 9, 0)])
+def test_residual_step_of_few_rows(rows, W, planes, n_mix, top, kind):
+    """A cluster shares a row: any number of planes and of kept streams, around those whose loads are under way together, and
+    results of routed experts, some of which are absent.  Sums of up to 34 terms in 32 bits."""
+    lib, S, k = _stack()
+    g = gen(W + planes)
+    r = lambda *s: torch.randn(*s, generator=g)
+    L, eps = S.ceil_to(W, 8), 1e-5
+    norm = layer_norm if kind == 0 else (lambda v, w, e: rms_unit(v, e) * w)
+
+    def wide(t):
+        o = torch.full(t.shape[:-1] + (L,), float("nan"), device="cuda")
+        o[..., :W] = t.cuda()
+        return o
+
+    x, pw, nw, b, gt = r(rows, W), r(W), r(W), r(W), r(planes, rows, W)
+    a = S.ResidArgs()
+    if top:
+        y, route = r(6, rows, W), torch.randint(-1, 6, (rows, top), generator=g)
+        Y, R = wide(y), route.int().cuda()
+        a.y, a.y_route, a.y_top, a.y_rows = S.Proj(Y, L).args(), lib.ptr(R), top, rows
+        sub = torch.stack([sum((y[e, i].double() for e in route[i].tolist() if e >= 0), torch.zeros(W).double()) for i in range(rows)])
+    else:
+        y = r(planes, rows, W)
+        Y = wide(y)
+        a.y = S.Proj(Y, L, planes, rows * L).args()
+        sub = y.double().sum(0)
+    GT, X, PW, NW, B = wide(gt), wide(x), pw.cuda(), nw.cuda(), b.cuda()
+    a.gate = S.Proj(GT, L, planes, rows * L).args()
+    full = avg = x.double() + norm(sub * torch.sigmoid(gt.double().sum(0) + b.double()), pw.double(), eps)
+    out, x_avg, h = (torch.zeros(rows, L).cuda() for _ in range(3))
+    if n_mix:
+        kept, mix = r(max(n_mix - 1, 1), rows, W), r(n_mix)
+        KEPT, MIX = wide(kept), mix.cuda()
+        a.mix, a.kept, a.kept_stride, a.n_mix, a.x_avg = lib.ptr(MIX), lib.ptr(KEPT), rows * L, n_mix, lib.ptr(x_avg)
+        avg = sum((m * t for m, t in zip(mix.double(), [*kept.double()[:n_mix - 1], full])), torch.zeros(rows, W).double())
+    a.gate_bias, a.post_w, a.next_w, a.x_in, a.x_out = (lib.ptr(t) for t in (B, PW, NW, X, out))
+    a.h, a.ldh, a.ldx, a.rows, a.W, a.norm_kind, a.eps, a.f32 = lib.ptr(h), L, L, rows, W, kind, eps, 1
+    _ok(k.ds41_resid_step(C.byref(a), lib.stream()))
+    torch.testing.assert_close(out[:, :W].cpu().double(), full, rtol=2e-5, atol=2e-5)
+    if n_mix:
+        torch.testing.assert_close(x_avg[:, :W].cpu().double(), avg, rtol=2e-5, atol=1e-4)
+    torch.testing.assert_close(h[:, :W].cpu().double(), norm(avg, nw.double(), eps), rtol=2e-5, atol=5e-5)
+
+
 def norm_in_order(x, kind, eps):
     """Mean and factor of every row as one block of the residual step sums them, in 32 bits: a thread's own moments, then the
     lower half of the threads with the upper one, over a warp and over the warps."""
