@@ -23,6 +23,7 @@
 #include <atomic>
 
 #include "ds41_api.h"
+#include "ds41_hc.cuh"
 #include "ds41_launch.cuh"
 #include "ds41_ptx.cuh"
 #include "ds41_tma.h"
@@ -542,7 +543,7 @@ hc_expand_stream_kernel(const __nv_bfloat16* streams_in, __nv_bfloat16* streams_
 // One block per row.  Produces next_pre/post/comb from the slice partials, then the collapsed,
 // normalised row.  `norm_w` may be null (no weight).  When `xq` is given the normalised row is also emitted
 // as E4M3 with one power-of-two scale per 128 columns, written in the MX GEMM's scale-atom layout.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256 + 32)
 hc_finish_kernel(const float* __restrict__ partial, int n_slices, const float* __restrict__ scale,
                  const float* __restrict__ base, const float* __restrict__ pre_in,
                  const __nv_bfloat16* __restrict__ streams, const float* __restrict__ norm_w,
@@ -552,13 +553,14 @@ hc_finish_kernel(const float* __restrict__ partial, int n_slices, const float* _
                  const float* __restrict__ mix_planes, int mix_splits, long long mix_split_stride, int mix_ld) {
   __shared__ float proj[kHcProj + 1];
   __shared__ float warp_part[8];
-  __shared__ float inv_rms;
   const int r = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // the ninth warp derives the mixes, a chain of divisions, while the other eight collapse and normalise the row
+  constexpr int kWorkers = 256;
   pdl_launch_dependents();
   pdl_wait();
   // ---- slice partials: warp w reduces values w, w+8, w+16 (+24); fixed shuffle tree -> deterministic
-  for (int j = warp; j <= kHcProj; j += 8) {
+  for (int j = warp; j <= kHcProj && warp < 8; j += 8) {
     float acc = 0.f;
     if (mix_planes != nullptr && j < kHcProj) {
       // tensor-core projection: split-K planes [split][rows][mix_ld], columns j (high part) and 24 + j (low part)
@@ -573,7 +575,7 @@ hc_finish_kernel(const float* __restrict__ partial, int n_slices, const float* _
     if (lane == 0) proj[j] = acc;
   }
   __syncthreads();
-  if (warp == 0) {
+  if (warp == 8) {
     const float inv = rsqrtf(proj[kHcProj] / (4.0f * H) + norm_eps);
     if (lane < 4) {
       const float a = fmaf(proj[lane] * inv, scale[0], base[lane]);
@@ -583,24 +585,9 @@ hc_finish_kernel(const float* __restrict__ partial, int n_slices, const float* _
     }
     // comb: lane = s*4 + d for lanes < 16
     float v = lane < 16 ? fmaf(proj[8 + lane] * inv, scale[2], base[8 + lane]) : 0.f;
-    float mx = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    v = __expf(v - mx);
-    float sum = v + __shfl_xor_sync(0xffffffffu, v, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    v = v / sum + hc_eps;
-    sum = v + __shfl_xor_sync(0xffffffffu, v, 4);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-    v /= sum + hc_eps;
-    for (int it = 1; it < iters; ++it) {
-      sum = v + __shfl_xor_sync(0xffffffffu, v, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      v /= sum + hc_eps;
-      sum = v + __shfl_xor_sync(0xffffffffu, v, 4);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-      v /= sum + hc_eps;
-    }
+    v = sinkhorn_4x4(v, iters, hc_eps);
     if (lane < 16) comb[r * 16 + lane] = v;
+    return;
   }
   if (xn == nullptr) return;        // the expand kernel already collapsed and normalised the row
   // ---- collapse with the incoming pre + RMSNorm; each thread owns up to 3 groups of 8 columns
@@ -639,14 +626,11 @@ hc_finish_kernel(const float* __restrict__ partial, int n_slices, const float* _
   }
   local_sq = warp_sum(local_sq);
   if (lane == 0) warp_part[warp] = local_sq;
-  __syncthreads();
-  if (tid == 0) {
-    float t = 0.f;
-    for (int w = 0; w < 8; ++w) t += warp_part[w];
-    inv_rms = rsqrtf(t / H + norm_eps);
-  }
-  __syncthreads();
-  const float inv = inv_rms;
+  named_barrier(1, kWorkers);
+  float total = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) total += warp_part[w];
+  const float inv = rsqrtf(total / H + norm_eps);
 #pragma unroll
   for (int n = 0; n < kMaxItems; ++n) {
     const int i = tid + 256 * n;
@@ -728,23 +712,7 @@ hc_mixes_kernel(const float* __restrict__ partial, const float* __restrict__ sca
   }
   // comb: lane = s*4 + d for lanes < 16
   float v = lane < 16 ? fmaf(p_comb, scale[2], base[8 + lane]) : 0.f;
-  float mx = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
-  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-  v = __expf(v - mx);
-  float sum = v + __shfl_xor_sync(0xffffffffu, v, 1);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-  v = v / sum + hc_eps;
-  sum = v + __shfl_xor_sync(0xffffffffu, v, 4);
-  sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-  v /= sum + hc_eps;
-  for (int it = 1; it < iters; ++it) {
-    sum = v + __shfl_xor_sync(0xffffffffu, v, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    v /= sum + hc_eps;
-    sum = v + __shfl_xor_sync(0xffffffffu, v, 4);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-    v /= sum + hc_eps;
-  }
+  v = sinkhorn_4x4(v, iters, hc_eps);
   if (lane < 16) comb[r * 16 + lane] = v;
 }
 
@@ -836,7 +804,7 @@ extern "C" int ds41_hc_finish(const float* partial, int n_slices, const float* s
     return launch_pdl(hc_mixes_kernel, dim3((rows + 7) / 8), dim3(256), 0, static_cast<cudaStream_t>(stream), partial,
                       scale, base, next_pre, post, comb, rows, H, iters, hc_eps, norm_eps, mix_planes, mix_splits,
                       mix_split_stride, mix_ld);
-  return launch_pdl(hc_finish_kernel, dim3(rows), dim3(256), 0, static_cast<cudaStream_t>(stream), partial, n_slices,
+  return launch_pdl(hc_finish_kernel, dim3(rows), dim3(256 + 32), 0, static_cast<cudaStream_t>(stream), partial, n_slices,
                     scale, base, pre_in, static_cast<const __nv_bfloat16*>(streams), norm_w, next_pre, post, comb,
                     static_cast<__nv_bfloat16*>(xn), tap_mean, static_cast<uint8_t*>(xq),
                     static_cast<uint8_t*>(xq_sf), rows, H, iters, hc_eps, norm_eps, mix_planes, mix_splits,

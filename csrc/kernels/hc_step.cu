@@ -16,6 +16,7 @@
 // Mathematics: native/cuda/kernels/v41_hc.cu:6-29,70-120 and rust/crates/ds41rt-daemon/src/v41_hc.rs:153-225 of the
 // reference; the fusion and the one-shot cross-rank sum are this design's.
 #include "ds41_api.h"
+#include "ds41_hc.cuh"
 #include "ds41_launch.cuh"
 #include "ds41_ptx.cuh"
 #include "ds41_tma.h"
@@ -69,6 +70,8 @@ template <bool EARLY>
 __global__ void __launch_bounds__(256, EARLY ? kEarlyBlocks : 4) hc_step_kernel(HcStepParams p) {
   __shared__ float xs[kMult][kSlice];
   __shared__ float sqc[kSlice];
+  constexpr int kCoef = 2 * kMult + kMult * kMult;
+  __shared__ float coef[kCoef];                       // collapse weights, post, comb of the row
   __shared__ float proj[kStride];
   __shared__ int s_last;
   const int c0 = blockIdx.x * kSlice, r = blockIdx.y, H = p.H;
@@ -89,6 +92,12 @@ __global__ void __launch_bounds__(256, EARLY ? kEarlyBlocks : 4) hc_step_kernel(
 #pragma unroll
       for (int j = 0; j < 3; ++j) fn[j][i] = mix_row(j, i);
   }
+  // and what the block that finishes will read, into L2
+  if (p.norm_w != nullptr && tid < kSlice / 32) prefetch_l2(p.norm_w + c0 + 32 * tid);
+  if (blockIdx.x == 0 && tid == 32) {
+    prefetch_l2(p.scale);
+    prefetch_l2(p.base);
+  }
   pdl_wait();
   if (p.wait_flags != nullptr && p.parts.n_ranks > 1) {
     if (tid < p.parts.n_ranks) flag_wait_ge(p.wait_flags[tid], *p.wait_epoch, p.status, 400 + tid);
@@ -96,16 +105,17 @@ __global__ void __launch_bounds__(256, EARLY ? kEarlyBlocks : 4) hc_step_kernel(
   }
   float* my_partial = p.partial + (1ll * blockIdx.x * p.rows + r) * kStride;
   // ---------------------------------------------------------------- 1+2: expand and collapse one column per thread
+  // The row's coefficients by threads that hold no column, before the first store, which loads may not be moved across.
+  const int c = c0 + tid;
+  float s_in[kMult], sub = 0.f;
+  const bool closing = p.parts.n_ranks > 0;
   if (tid < kSlice) {
-    const int c = c0 + tid;
-    float s_in[kMult], out[kMult];
 #pragma unroll
     for (int s = 0; s < kMult; ++s) s_in[s] = __bfloat162float(p.streams_in[(1ll * r * kMult + s) * H + c]);
-    if (p.parts.n_ranks > 0) {
+    if (closing) {
       // Partial planes of every rank, summed in rank-major, split-minor order.  The loads of 32 planes are issued
       // before the first add: a load from a peer takes a few microseconds, and one at a time they were most of this
       // kernel's time on 8 GPUs.
-      float sub = 0.f;
       const int n_sp = p.parts.n_splits, total = p.parts.n_ranks * n_sp;
       if (p.parts.n_ranks == 1) {
         const float* plane = p.parts.base[0] + 1ll * r * H + c;
@@ -133,23 +143,30 @@ __global__ void __launch_bounds__(256, EARLY ? kEarlyBlocks : 4) hc_step_kernel(
         }
       }
       sub = bf16_round(sub);
+    }
+  } else if (tid < kSlice + kCoef) {
+    const int k = tid - kSlice;
+    coef[k] = k < 4 ? p.pre_in[r * 4 + k] : !closing ? 0.f : k < 8 ? p.post[r * 4 + k - 4] : p.comb[r * 16 + k - 8];
+  }
+  __syncthreads();
+  if (tid < kSlice) {
+    const float *pre = coef, *post = coef + 4, *comb = coef + 8;
+    float out[kMult];
 #pragma unroll
-      for (int d = 0; d < kMult; ++d) {
-        float acc = 0.f;
+    for (int d = 0; d < kMult; ++d) {
+      out[d] = s_in[d];
+      if (!closing) continue;
+      float acc = 0.f;
 #pragma unroll
-        for (int s = 0; s < kMult; ++s) acc = fmaf(p.comb[r * 16 + s * 4 + d], s_in[s], acc);
-        out[d] = bf16_round(fmaf(p.post[r * 4 + d], sub, acc));
-        p.streams_out[(1ll * r * kMult + d) * H + c] = __float2bfloat16_rn(out[d]);
-      }
-    } else {
-#pragma unroll
-      for (int d = 0; d < kMult; ++d) out[d] = s_in[d];
+      for (int s = 0; s < kMult; ++s) acc = fmaf(comb[s * 4 + d], s_in[s], acc);
+      out[d] = bf16_round(fmaf(post[d], sub, acc));
+      p.streams_out[(1ll * r * kMult + d) * H + c] = __float2bfloat16_rn(out[d]);
     }
     float col = 0.f, mean = 0.f;
 #pragma unroll
     for (int d = 0; d < kMult; ++d) {
       xs[d][tid] = out[d];
-      col = fmaf(p.pre_in[r * 4 + d], out[d], col);
+      col = fmaf(pre[d], out[d], col);
       mean += out[d];
     }
     col = bf16_round(col);
@@ -259,23 +276,7 @@ __global__ void __launch_bounds__(256, EARLY ? kEarlyBlocks : 4) hc_step_kernel(
       p.post_out[r * 4 + lane] = 2.0f / (1.0f + __expf(-b));
     }
     float v = lane < 16 ? fmaf(proj[8 + lane] * inv, p.scale[2], p.base[8 + lane]) : 0.f;   // lane = s*4 + d
-    float mx = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    v = __expf(v - mx);
-    float sum = v + __shfl_xor_sync(0xffffffffu, v, 1);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    v = v / sum + p.hc_eps;
-    sum = v + __shfl_xor_sync(0xffffffffu, v, 4);
-    sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-    v /= sum + p.hc_eps;
-    for (int it = 1; it < p.iters; ++it) {
-      sum = v + __shfl_xor_sync(0xffffffffu, v, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      v /= sum + p.hc_eps;
-      sum = v + __shfl_xor_sync(0xffffffffu, v, 4);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 8);
-      v /= sum + p.hc_eps;
-    }
+    v = sinkhorn_4x4(v, p.iters, p.hc_eps);
     if (lane < 16) p.comb_out[r * 16 + lane] = v;
     if (lane == 0) p.tickets[r] = 0u;
     return;
