@@ -39,6 +39,9 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// A line of 128 bytes on its way to L2.  Nothing is read: it may be asked for before the wait for the previous kernel.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Address of the same shared variable in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t mine, uint32_t rank) {
   uint32_t there;

@@ -69,22 +69,22 @@ __device__ __forceinline__ void operator+=(float2& a, const float2& b) {
 // and added in their order.  The loops above have the first, then four together, then the rest one after the other (of eight
 // planes five round trips to L2, 0.4 us each); in kernels of many rows the registers are worth more.
 constexpr int kPlanes = 8;
-template <typename V>
-__device__ __forceinline__ void fetch_planes(V (&t)[kPlanes], const float* p, long long plane, int n) {
+template <typename V, int N>
+__device__ __forceinline__ void fetch_planes(V (&t)[N], const float* p, long long plane, int n) {
 #pragma unroll
-  for (int u = 0; u < kPlanes; ++u)
+  for (int u = 0; u < N; ++u)
     if (u < n) t[u] = *reinterpret_cast<const V*>(p + u * plane);
 }
-template <typename V>
-__device__ __forceinline__ V add_planes(V (&t)[kPlanes], const float* p, long long plane, int n) {
+template <typename V, int N>
+__device__ __forceinline__ V add_planes(V (&t)[N], const float* p, long long plane, int n) {
   V s = t[0];
 #pragma unroll
-  for (int u = 1; u < kPlanes; ++u)
+  for (int u = 1; u < N; ++u)
     if (u < n) s += t[u];
-  for (int k = kPlanes; k < n; k += kPlanes) {
+  for (int k = N; k < n; k += N) {
     fetch_planes(t, p + k * plane, plane, n - k);
 #pragma unroll
-    for (int u = 0; u < kPlanes; ++u)
+    for (int u = 0; u < N; ++u)
       if (k + u < n) s += t[u];
   }
   return s;

@@ -267,70 +267,105 @@ __global__ void __launch_bounds__(128) latent_attend_plain_kernel(ds41_latent_at
 }
 
 // bf16 form on the warp-level tensor cores: one CTA per (row, MT x 16 heads, split) walks its keys 64 at a time through two
-// shared-memory buffers; the key tile is the value tile as well.  Four warps per 16 heads: each scores 16 of the 64 keys,
-// then accumulates a quarter of the latent columns (NP pairs of 8 columns).
+// shared-memory buffers; the key tile is the value tile as well.  PW warps per 16 heads: the first four score 16 of the 64 keys each,
+// then each accumulates its share of the latent columns (NP pairs of 8 columns).
+// A thread per key copies its whole row by one bulk copy, the rows of the first tiles being on their way to L2 before the wait for the
+// previous kernel.  Pieces of 16 bytes by all threads (four to five thousand cp.async a tile) kept a CTA waiting 8 us for its
+// first tile.  In a graph, one row over 4097 keys, 16 heads: 18.5 us with those, 10.7 so; 32 rows over 1100 keys, 32 heads 33 and 30.
 constexpr int kKeyTile = 64;
 constexpr int kProbStride = kKeyTile + 8;
 
-template <int MT, int NP>
-__global__ void __launch_bounds__(MT * 128) latent_attend_mma_kernel(ds41_latent_attend_args p) {
+__host__ __device__ constexpr int attend_mma_bytes(int mt, int row_len) {
+  return (mt * 16 + 2 * kKeyTile) * (row_len + 8) * 2 + mt * 16 * kProbStride * 2 + mt * 64 * 4 + 3 * 8;
+}
+
+template <int MT, int PW, int NP>
+__global__ void __launch_bounds__(MT * PW * 32) latent_attend_mma_kernel(ds41_latent_attend_args p) {
   extern __shared__ __align__(16) uint8_t la_smem[];
   const int RL = p.row_len, RS = RL + 8;
   __nv_bfloat16* sq = reinterpret_cast<__nv_bfloat16*>(la_smem);              // [MT * 16][RS]
   __nv_bfloat16* sk = sq + MT * 16 * RS;                                      // [2][64][RS]
   __nv_bfloat16* sp = sk + 2 * kKeyTile * RS;                                 // [MT][16][72]
   float* tops = reinterpret_cast<float*>(sp + MT * 16 * kProbStride);         // [MT][4][16] maxima, then sums
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mt = warp >> 2, w = warp & 3;
+  uint64_t* full = reinterpret_cast<uint64_t*>(tops + MT * 64);               // [2] key tiles, [1] the queries
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mt = warp / PW, w = warp % PW;
   const int g = lane >> 2, q2 = 2 * (lane & 3);
   const int split = blockIdx.x, r = blockIdx.y, h0 = blockIdx.z * MT * 16;
+  if (tid == 0) {
+    mbar_init(&full[0], kKeyTile);
+    mbar_init(&full[1], kKeyTile);
+    mbar_init(&full[2], MT * 16);
+    mbar_init_fence();
+  }
   pdl_launch_dependents();
+  int slot, k0, k1;
+  auto find = [&]() {
+    slot = p.row_slot[r];
+    const int n_keys = slot < 0 ? 0 : p.row_pos[r] + 1;
+    const int per = ((n_keys + kKeyTile - 1) / kKeyTile + p.n_splits - 1) / p.n_splits * kKeyTile;
+    k0 = split * per;
+    k1 = min(n_keys, k0 + per);
+  };
+  auto locate = [&](int key) {           // threads of the first two warps: where the row of a key lies
+    return key < k1 ? cache_row(static_cast<__nv_bfloat16*>(p.pool), p.page_table, p.max_pages, p.page_tokens, RL, slot, key)
+                    : nullptr;
+  };
+  find();
+  if (tid < kKeyTile) {                  // the cache's rows have left L2 since the last pass
+    constexpr int kTiles = 4;
+    const __nv_bfloat16* row[kTiles];
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i) row[i] = locate(k0 + i * kKeyTile + tid);
+#pragma unroll
+    for (int i = 0; i < kTiles; ++i)
+      if (row[i] != nullptr)
+        for (int d = 0; d < RL; d += 64) prefetch_l2(row[i] + d);
+  }
+  __syncthreads();                       // the barriers are ready
   pdl_wait();
-  const int slot = p.row_slot[r];
-  const int n_keys = slot < 0 ? 0 : p.row_pos[r] + 1;
-  const int per = ((n_keys + kKeyTile - 1) / kKeyTile + p.n_splits - 1) / p.n_splits * kKeyTile;
-  const int k0 = split * per, k1 = min(n_keys, k0 + per);
+  find();
   const long long cell0 = (1ll * r * p.n_splits + split) * p.heads;
   if (k0 >= k1) {
-    for (int h = tid; h < MT * 16; h += MT * 128)
+    for (int h = tid; h < MT * 16; h += MT * PW * 32)
       if (h0 + h < p.heads) {
         p.part_ml[2 * (cell0 + h0 + h)] = -INFINITY;
         p.part_ml[2 * (cell0 + h0 + h) + 1] = 0.f;
       }
     return;
   }
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  // lane i knows where the warp's i-th key of a tile lies; looked up one tile ahead of the copies
-  constexpr int kMine = kKeyTile / (MT * 4);
-  auto locate = [&](int key0) {
-    const int key = key0 + warp + (lane % kMine) * MT * 4;
-    return key < k1 ? cache_row(static_cast<__nv_bfloat16*>(p.pool), p.page_table, p.max_pages, p.page_tokens, RL, slot, key)
-                    : nullptr;
-  };
-  auto load = [&](__nv_bfloat16* where, int buf) {
-    __nv_bfloat16* dst = sk + buf * kKeyTile * RS + warp * RS;
-#pragma unroll 4
-    for (int i = 0; i < kMine; ++i) {
-      const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(
-          __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(where), i));
-      for (int d = lane * 8; d < RL; d += 256) {
-        if (src != nullptr) cp_async_16(dst + i * MT * 4 * RS + d, src + d);
-        else *reinterpret_cast<uint4*>(dst + i * MT * 4 * RS + d) = zero;
-      }
+  // one row of `bytes` at `src` (null: zeros) into shared memory, counted by `bar`
+  auto copy = [&](__nv_bfloat16* dst, const __nv_bfloat16* src, int values, uint64_t* bar) {
+    if (src != nullptr) {
+      bulk_load(dst, src, 2 * values, bar);
+    } else {
+      for (int d = 0; d < values; d += 8) *reinterpret_cast<uint4*>(dst + d) = make_uint4(0, 0, 0, 0);
     }
-    cp_async_commit();
   };
-  __nv_bfloat16* where = locate(k0);
-  for (int i = warp; i < MT * 16; i += MT * 4) {
-    const int h = h0 + i;
-    const __nv_bfloat16* qa = static_cast<const __nv_bfloat16*>(p.q_abs) + r * p.ld_q_abs + 1ll * h * p.kv_pad;
-    const __nv_bfloat16* qr = static_cast<const __nv_bfloat16*>(p.q_rot) + r * p.ld_q_rot + 1ll * h * p.q_rot_stride;
-    for (int d = lane * 8; d < RL; d += 256) {
-      if (h < p.heads) cp_async_16(sq + i * RS + d, d < p.kv_pad ? qa + d : qr + (d - p.kv_pad));
-      else *reinterpret_cast<uint4*>(sq + i * RS + d) = zero;
+  auto load = [&](const __nv_bfloat16* src, int buf) {
+    if (tid >= kKeyTile) return;
+    if (src != nullptr) mbar_expect_tx(&full[buf], 2 * RL);
+    copy(sk + (buf * kKeyTile + tid) * RS, src, RL, &full[buf]);
+    if (src == nullptr) mbar_arrive(&full[buf]);
+  };
+  {
+    const __nv_bfloat16 *first = nullptr, *second = nullptr;
+    if (tid < kKeyTile) {
+      first = locate(k0 + tid);
+      second = locate(k0 + kKeyTile + tid);
     }
+    load(first, 0);
+    if (tid >= kKeyTile && tid < kKeyTile + MT * 16) {
+      const int i = tid - kKeyTile, h = h0 + i;
+      const bool in = h < p.heads;
+      const __nv_bfloat16* qa = static_cast<const __nv_bfloat16*>(p.q_abs) + r * p.ld_q_abs + 1ll * h * p.kv_pad;
+      const __nv_bfloat16* qr = static_cast<const __nv_bfloat16*>(p.q_rot) + r * p.ld_q_rot + 1ll * h * p.q_rot_stride;
+      if (in) mbar_expect_tx(&full[2], 2 * RL);
+      copy(sq + i * RS, in ? qa : nullptr, p.kv_pad, &full[2]);
+      if (RL > p.kv_pad) copy(sq + i * RS + p.kv_pad, in ? qr : nullptr, RL - p.kv_pad, &full[2]);
+      if (!in) mbar_arrive(&full[2]);
+    }
+    if (k0 + kKeyTile < k1) load(second, 1);
   }
-  load(where, 0);
-  where = locate(k0 + kKeyTile);
   float acc[NP][2][4];
 #pragma unroll
   for (int i = 0; i < NP; ++i)
@@ -341,23 +376,19 @@ __global__ void __launch_bounds__(MT * 128) latent_attend_mma_kernel(ds41_latent
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   const float scale2 = p.scale * 1.4426950408889634f;
   const int n_pairs = p.kv_pad / 16;
-  int buf = 0;
-  for (int t0 = k0; t0 < k1; t0 += kKeyTile, buf ^= 1) {
-    if (t0 + kKeyTile < k1) {
-      load(where, buf ^ 1);
-      where = locate(t0 + 2 * kKeyTile);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
+  bool ok = mbar_wait(&full[2], 0, nullptr, 0);
+  int tile = 0;
+  for (int t0 = k0; t0 < k1; t0 += kKeyTile, ++tile) {
+    const int buf = tile & 1;
+    const __nv_bfloat16* later = tid < kKeyTile ? locate(t0 + 2 * kKeyTile + tid) : nullptr;      // looked up ahead of its copy
+    ok &= mbar_wait(&full[buf], (tile >> 1) & 1, nullptr, 0);
     const __nv_bfloat16* kt = sk + buf * kKeyTile * RS;
     float s[2][4] = {}, s_odd[2][4] = {};       // two chains: consecutive products into one accumulator wait for each other
-    {
+    if (w < 4) {
       const __nv_bfloat16* arow = sq + (mt * 16 + (lane & 15)) * RS + (lane >> 4) * 8;
       const __nv_bfloat16* brow = kt + (w * 16 + (lane & 7) + (lane >> 4) * 8) * RS + ((lane >> 3) & 1) * 8;
       int k = 0;
-#pragma unroll 3
+#pragma unroll 6
       for (; k + 32 <= RL; k += 32) {
         uint32_t a[4], b[4], c[4], d[4];
         ldmatrix_x4(a[0], a[1], a[2], a[3], arow + k);
@@ -376,21 +407,21 @@ __global__ void __launch_bounds__(MT * 128) latent_attend_mma_kernel(ds41_latent
         mma_bf16_16816(s[0], a, b[0], b[1]);
         mma_bf16_16816(s[1], a, b[2], b[3]);
       }
-    }
-    float top[2] = {-INFINITY, -INFINITY};
+      float top[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int key = t0 + w * 16 + 8 * j + q2 + (e & 1);
-        s[j][e] = key < k1 ? (s[j][e] + s_odd[j][e]) * scale2 : -INFINITY;
-        top[e >> 1] = fmaxf(top[e >> 1], s[j][e]);
+        for (int e = 0; e < 4; ++e) {
+          const int key = t0 + w * 16 + 8 * j + q2 + (e & 1);
+          s[j][e] = key < k1 ? (s[j][e] + s_odd[j][e]) * scale2 : -INFINITY;
+          top[e >> 1] = fmaxf(top[e >> 1], s[j][e]);
+        }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 1));
+        top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 2));
+        if ((lane & 3) == 0) tops[(mt * 4 + w) * 16 + g + 8 * u] = top[u];
       }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 1));
-      top[u] = fmaxf(top[u], __shfl_xor_sync(0xffffffffu, top[u], 2));
-      if ((lane & 3) == 0) tops[(mt * 4 + w) * 16 + g + 8 * u] = top[u];
     }
     __syncthreads();
     float keep[2];
@@ -404,14 +435,16 @@ __global__ void __launch_bounds__(MT * 128) latent_attend_mma_kernel(ds41_latent
       l[u] *= keep[u];
     }
     // the tile holds at least one visible key, so m is finite here
+    if (w < 4) {
 #pragma unroll
-    for (int j = 0; j < 2; ++j)
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const float x = ex2_approx(s[j][2 * u] - m[u]), y = ex2_approx(s[j][2 * u + 1] - m[u]);
-        l[u] += x + y;
-        *reinterpret_cast<uint32_t*>(sp + (mt * 16 + g + 8 * u) * kProbStride + w * 16 + 8 * j + q2) = pack_bf16(x, y);
-      }
+        for (int u = 0; u < 2; ++u) {
+          const float x = ex2_approx(s[j][2 * u] - m[u]), y = ex2_approx(s[j][2 * u + 1] - m[u]);
+          l[u] += x + y;
+          *reinterpret_cast<uint32_t*>(sp + (mt * 16 + g + 8 * u) * kProbStride + w * 16 + 8 * j + q2) = pack_bf16(x, y);
+        }
+    }
 #pragma unroll
     for (int i = 0; i < NP; ++i)
 #pragma unroll
@@ -427,7 +460,7 @@ __global__ void __launch_bounds__(MT * 128) latent_attend_mma_kernel(ds41_latent
       const __nv_bfloat16* brow = kt + (k + (lane & 15)) * RS + (lane >> 4) * 8;
 #pragma unroll
       for (int i = 0; i < NP; ++i) {
-        const int pair = w + 4 * i;
+        const int pair = w + PW * i;
         if (pair < n_pairs) {
           uint32_t b[4];
           ldmatrix_x4_trans(b[0], b[1], b[2], b[3], brow + 16 * pair);
@@ -437,14 +470,19 @@ __global__ void __launch_bounds__(MT * 128) latent_attend_mma_kernel(ds41_latent
       }
     }
     __syncthreads();
+    if (t0 + 2 * kKeyTile < k1) load(later, buf);
   }
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     l[u] += __shfl_xor_sync(0xffffffffu, l[u], 1);
     l[u] += __shfl_xor_sync(0xffffffffu, l[u], 2);
-    if ((lane & 3) == 0) tops[(mt * 4 + w) * 16 + g + 8 * u] = l[u];
+    if (w < 4 && (lane & 3) == 0) tops[(mt * 4 + w) * 16 + g + 8 * u] = l[u];
   }
-  __syncthreads();
+  if (__syncthreads_or(!ok)) {           // a wait gave up: let the copies in flight land before the memory changes hands
+    const long long start = clock64();
+    while (clock64() - start < 2000000ll) __nanosleep(1000);
+    __syncthreads();
+  }
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const int h = h0 + mt * 16 + g + 8 * u;
@@ -459,7 +497,7 @@ __global__ void __launch_bounds__(MT * 128) latent_attend_mma_kernel(ds41_latent
     }
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-      const int pair = w + 4 * i;
+      const int pair = w + PW * i;
       if (pair < n_pairs)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
@@ -469,25 +507,27 @@ __global__ void __launch_bounds__(MT * 128) latent_attend_mma_kernel(ds41_latent
   }
 }
 
-template <int MT, int NP>
+template <int MT, int PW, int NP>
 static int launch_attend_mma(const ds41_latent_attend_args& a, cudaStream_t st) {
-  const int smem = (MT * 16 + 2 * kKeyTile) * (a.row_len + 8) * 2 + MT * 16 * kProbStride * 2 + MT * 64 * 4;
+  const int smem = attend_mma_bytes(MT, a.row_len);
   static int allowed = 47 * 1024;
   if (smem > allowed) {
-    const cudaError_t e = cudaFuncSetAttribute(latent_attend_mma_kernel<MT, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(latent_attend_mma_kernel<MT, PW, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     allowed = smem;
   }
   const dim3 grid(a.n_splits, a.rows, (a.heads + MT * 16 - 1) / (MT * 16));
-  return launch_pdl(latent_attend_mma_kernel<MT, NP>, grid, dim3(MT * 128), smem, st, a);
+  return launch_pdl(latent_attend_mma_kernel<MT, PW, NP>, grid, dim3(MT * PW * 32), smem, st, a);
 }
 
+// eight warps in every form: for 16 heads the second four share the latent columns only
 template <int MT>
 static int dispatch_attend_mma(const ds41_latent_attend_args& a, cudaStream_t st) {
-  if (a.kv_pad <= 64) return launch_attend_mma<MT, 1>(a, st);
-  if (a.kv_pad <= 128) return launch_attend_mma<MT, 2>(a, st);
-  if (a.kv_pad <= 256) return launch_attend_mma<MT, 4>(a, st);
-  return launch_attend_mma<MT, 8>(a, st);
+  constexpr int PW = 8 / MT;
+  if (a.kv_pad <= 16 * PW) return launch_attend_mma<MT, PW, 1>(a, st);
+  if (a.kv_pad <= 32 * PW) return launch_attend_mma<MT, PW, 2>(a, st);
+  if (MT == 1 || a.kv_pad <= 64 * PW) return launch_attend_mma<MT, PW, 4>(a, st);      // at most 512 values
+  return launch_attend_mma<MT, MT == 1 ? 8 : PW, MT == 1 ? 4 : 8>(a, st);
 }
 
 // heads per CTA of the tensor-core form for this row length (0: it does not fit, the plain form runs)
@@ -496,16 +536,15 @@ static int attend_mma_heads(const ds41_latent_attend_args& a) {
       (a.q_rot_stride & 7) || ((reinterpret_cast<uintptr_t>(a.q_abs) | reinterpret_cast<uintptr_t>(a.q_rot) |
                                 reinterpret_cast<uintptr_t>(a.pool)) & 15))
     return 0;
-  auto fits = [&](int mt) {
-    return (mt * 16 + 2 * kKeyTile) * (a.row_len + 8) * 2 + mt * 16 * kProbStride * 2 + mt * 256 <= 226 * 1024;
-  };
+  auto fits = [&](int mt) { return attend_mma_bytes(mt, a.row_len) <= 226 * 1024; };
   if (a.heads > 16 && fits(2)) return 32;
   return fits(1) ? 16 : 0;
 }
 
 // One block per (head, row): the splits' weights first, a thread each, then every thread sums four columns over the splits in
-// their order.  A chain of latencies: 32 rows x 32 heads of nine splits 6.8 us, one row of 32 splits 7.5.
+// their order.  A chain of latencies: in a graph one row of 32 splits 5.8 us with the splits one by one, 4.9 with sixteen under way.
 constexpr int kMaxSplits = 256;
+constexpr int kUnder = 16;             // splits whose loads are under way together
 template <typename T>
 __global__ void __launch_bounds__(128) latent_merge_kernel(const float* part_o, const float* part_ml, const float* sink,
                                                            int n_splits, int heads, int kv_pad, T* out, int ld_out) {
@@ -542,15 +581,22 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const float* part_o, 
   const float inv = den > 0.f ? 1.0f / den : 0.f;
   for (int i = 4 * tid; i < kv_pad; i += 512) {
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int s = 0; s < n_splits; ++s) {
-      const float e = wt[s];
-      if (e > 0.f) {
-        const float4 o = *reinterpret_cast<const float4*>(part_o + (cell0 + 1ll * s * heads) * kv_pad + i);
-        a.x += e * o.x;
-        a.y += e * o.y;
-        a.z += e * o.z;
-        a.w += e * o.w;
+    const float* part = part_o + cell0 * kv_pad + i;
+    const long long step = 1ll * heads * kv_pad;
+    for (int s0 = 0; s0 < n_splits; s0 += kUnder) {
+      float4 o[kUnder];
+#pragma unroll
+      for (int u = 0; u < kUnder; ++u)
+        if (s0 + u < n_splits && wt[s0 + u] > 0.f) o[u] = *reinterpret_cast<const float4*>(part + (s0 + u) * step);
+#pragma unroll
+      for (int u = 0; u < kUnder; ++u) {
+        const float e = s0 + u < n_splits ? wt[s0 + u] : 0.f;
+        if (e > 0.f) {
+          a.x += e * o[u].x;
+          a.y += e * o[u].y;
+          a.z += e * o[u].z;
+          a.w += e * o[u].w;
+        }
       }
     }
     store4(out + 1ll * r * ld_out + h * kv_pad + i, make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv));

@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(NI <= 4 ? 256 : 512) resid_step_kernel(ds41_re
   }
 }
 
-// A place of a projection whose loads are under way: all planes (up to eight), or the bf16 value.
+// A place of a projection whose loads are under way: its planes (up to eight; sixteen would leave room for one CTA beside a GEMM's),
+// or the bf16 value.
 struct Ahead {
   float4 t[kPlanes];
   __device__ __forceinline__ void ask(const ds41_proj& a, long long row, int col) {
@@ -372,7 +373,8 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
   const float* kept = p.kept + r * p.ldx;
   const bool plain = p.y.data != nullptr && p.y_route == nullptr;
   constexpr bool kAhead = NI == 1;         // one piece a thread: everything is under way before the first sum
-  Ahead ya, ga, ka;
+  Ahead ya, ga;
+  float4 ka[kPlanes];
   if (p.tokens != nullptr) {
     const int tok = p.tokens[r];
     const ds41_proj e{p.embed, 0, static_cast<int>(p.embed_ld), 1, 1, 0};
@@ -388,7 +390,7 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
   if (kAhead && live[0] > 0) {
     if (plain) ya.ask(p.y, r, at[0]);
     if (p.y.data != nullptr && p.gate.data != nullptr) ga.ask(p.gate, r, at[0]);
-    fetch_planes(ka.t, kept + at[0], p.kept_stride, n_old);
+    fetch_planes(ka, kept + at[0], p.kept_stride, n_old);
   }
   if (p.y.data != nullptr && p.y_route != nullptr)
 #pragma unroll
@@ -403,12 +405,12 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
   };
   if constexpr (kAhead) {
     for (int j0 = 0; j0 < n_old; j0 += kPlanes) {
-      if (j0 > 0 && live[0] > 0) fetch_planes(ka.t, kept + j0 * p.kept_stride + at[0], p.kept_stride, n_old - j0);
+      if (j0 > 0 && live[0] > 0) fetch_planes(ka, kept + j0 * p.kept_stride + at[0], p.kept_stride, n_old - j0);
 #pragma unroll
       for (int u = 0; u < kPlanes; ++u)
         if (j0 + u < n_old) {
           const float c = weight(j0 + u);
-          if (live[0] > 0) add_old(0, c, ka.t[u]);
+          if (live[0] > 0) add_old(0, c, ka[u]);
         }
     }
   } else {
