@@ -89,40 +89,63 @@ struct QkvPostParams {
   float eps;
 };
 
-constexpr int kFewPlanes = 7;
+// vals[n] += the planes of column c + n step, in their order, for the columns below `end`.  Four planes of all columns are under way
+// at once: with few rows the launch is a chain of round trips to L2.  One row of ten planes, 1280 + 512 columns, in a graph: 11 us
+// with a column after the other, 3.5 so (weights read before the wait).
+template <typename V, int N>
+__device__ __forceinline__ void add_columns(V (&vals)[N], const float* row, long long plane, int splits, int c, int step, int end) {
+  constexpr int kUnder = 4;
+  constexpr int kEach = sizeof(V) / sizeof(float);
+  auto at = [&](int s, int n) { return *reinterpret_cast<const V*>(row + s * plane + kEach * (c + n * step)); };
+  auto add = [](V& a, const V& b) {
+    if constexpr (kEach == 1) {
+      a += b;
+    } else {
+      a.x += b.x;
+      a.y += b.y;
+    }
+  };
+  if (splits == 1) {
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      if (c + n * step < end) add(vals[n], at(0, n));
+    return;
+  }
+  for (int s0 = 0; s0 < splits; s0 += kUnder) {
+    V t[kUnder][N];
+#pragma unroll
+    for (int u = 0; u < kUnder; ++u)
+#pragma unroll
+      for (int n = 0; n < N; ++n)
+        if (s0 + u < splits && c + n * step < end) t[u][n] = at(s0 + u, n);
+#pragma unroll
+    for (int u = 0; u < kUnder; ++u)
+#pragma unroll
+      for (int n = 0; n < N; ++n)
+        if (s0 + u < splits && c + n * step < end) add(vals[n], t[u][n]);
+  }
+}
+
 constexpr int kOwnExtras = 256;       // up to one column a thread (200 rows, 8 columns of 10 planes: 7.0 us by the kv block, 7.5)
 // grid (rows, 2 or 3): block y == 0 normalises the q latent, y == 1 handles kv (norm + RoPE + ring write), and the extras unless
 // there are enough for a block y == 2.
 __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
   __shared__ float scratch[8];
   const int r = blockIdx.x, tid = threadIdx.x;
-  pdl_launch_dependents();
-  pdl_wait();
   const long long plane = 1ll * p.rows * p.ntot;
   const float* row0 = p.planes + 1ll * r * p.ntot;
+  pdl_launch_dependents();
   if (blockIdx.y == 0) {
-    // ---- q latent (Q <= 2048: up to 8 columns per thread, all split loads issued together)
-    // Few planes: the planes outside, the columns inside, four planes of all columns in flight.  Many planes: one column after
-    // the other, which the compiler pipelines better.  The order of a column's sum is the same.  16 rows of 1280 + 512 columns,
-    // us with columns / planes inside: 1 plane 2.3 / 3.4, 6 planes 4.2 / 5.4, 8 planes 4.8 / 4.6, 12 planes 6.1 / 5.5.
-    float vals[8];
+    // ---- q latent (Q <= 2048: up to 8 columns per thread)
+    float vals[8], w[8];
     float sq = 0.f;
 #pragma unroll
-    for (int n = 0; n < 8; ++n) vals[n] = 0.f;
-    if (p.splits <= kFewPlanes) {
-#pragma unroll 4
-      for (int s = 0; s < p.splits; ++s)
-#pragma unroll
-        for (int n = 0; n < 8; ++n)
-          if (tid + 256 * n < p.Q) vals[n] += row0[s * plane + tid + 256 * n];
-    } else {
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-        if (tid + 256 * n < p.Q) {
-#pragma unroll 4
-          for (int s = 0; s < p.splits; ++s) vals[n] += row0[s * plane + tid + 256 * n];
-        }
+    for (int n = 0; n < 8; ++n) {
+      vals[n] = 0.f;
+      w[n] = tid + 256 * n < p.Q ? p.q_norm_w[tid + 256 * n] : 0.f;      // weights: read before the wait
     }
+    pdl_wait();
+    add_columns(vals, row0, plane, p.splits, tid, 256, p.Q);
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       vals[n] = bf16_round(vals[n]);
@@ -133,7 +156,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       const int c = tid + 256 * n;
-      if (c < p.Q) p.q_lat[1ll * r * p.Q + c] = __float2bfloat16_rn(vals[n] * inv * p.q_norm_w[c]);
+      if (c < p.Q) p.q_lat[1ll * r * p.Q + c] = __float2bfloat16_rn(vals[n] * inv * w[n]);
     }
     return;
   }
@@ -141,11 +164,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
   auto extras = [&]() {
     for (int c0 = tid; c0 < p.extra_f32; c0 += 256 * 4) {
       float a[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-      for (int s = 0; s < p.splits; ++s)
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-          if (c0 + 256 * n < p.extra_f32) a[n] += row0[s * plane + p.Q + p.D + c0 + 256 * n];
+      add_columns(a, row0 + p.Q + p.D, plane, p.splits, c0, 256, p.extra_f32);
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
         const int c = c0 + 256 * n;
@@ -154,27 +173,29 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
       }
     }
   };
-  if (blockIdx.y == 2) return extras();
+  if (blockIdx.y == 2) {
+    pdl_wait();
+    return extras();
+  }
   // ---- kv: thread handles adjacent pairs so RoPE stays in-thread (D <= 2048)
-  const int pos = p.row_pos[r], slot = p.row_slot[r];
-  float2 kvv[4];
+  float2 kvv[4], w[4];
+  float freq[4];
   float sq = 0.f;
 #pragma unroll
+  for (int n = 0; n < 4; ++n) {                         // weights: read before the wait
+    const int i = tid + 256 * n, t = 2 * i - (p.D - p.rope_dim);
+    const bool in = i < p.D / 2;
+    kvv[n] = make_float2(0.f, 0.f);
+    w[n] = in ? make_float2(p.kv_norm_w[2 * i], p.kv_norm_w[2 * i + 1]) : kvv[n];
+    freq[n] = in && t >= 0 ? p.inv_freq[t / 2] : 0.f;
+  }
+  pdl_wait();
+  const int pos = p.row_pos[r], slot = p.row_slot[r];
+  add_columns(kvv, row0 + p.Q, plane, p.splits, tid, 256, p.D / 2);
+#pragma unroll
   for (int n = 0; n < 4; ++n) {
-    const int i = tid + 256 * n;
-    float a = 0.f, b = 0.f;
-    if (i < p.D / 2) {
-#pragma unroll 4
-      for (int s = 0; s < p.splits; ++s) {
-        const float2 v = *reinterpret_cast<const float2*>(row0 + s * plane + p.Q + 2 * i);
-        a += v.x;
-        b += v.y;
-      }
-      a = bf16_round(a);
-      b = bf16_round(b);
-    }
-    kvv[n] = make_float2(a, b);
-    sq = fmaf(a, a, fmaf(b, b, sq));
+    kvv[n] = make_float2(bf16_round(kvv[n].x), bf16_round(kvv[n].y));
+    sq = fmaf(kvv[n].x, kvv[n].x, fmaf(kvv[n].y, kvv[n].y, sq));
   }
   const float tot = block_sum_256(sq, scratch);
   const float inv = rsqrtf(tot / p.D + p.eps);
@@ -188,12 +209,12 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
     const bool active = i < p.D / 2;
     float a = 0.f, b = 0.f;
     if (active) {
-      a = bf16_round(kvv[n].x * inv * p.kv_norm_w[2 * i]);
-      b = bf16_round(kvv[n].y * inv * p.kv_norm_w[2 * i + 1]);
+      a = bf16_round(kvv[n].x * inv * w[n].x);
+      b = bf16_round(kvv[n].y * inv * w[n].y);
       const int t = 2 * i - (p.D - p.rope_dim);
       if (t >= 0) {
         float c, s;
-        rope_cs(pos, p.inv_freq[t / 2], &c, &s);
+        rope_cs(pos, freq[n], &c, &s);
         const float ra = a * c - b * s;
         const float rb = b * c + a * s;
         a = ra;

@@ -566,6 +566,22 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
   const int g = lane >> 2, t4 = lane & 3;
   const int n_heads = min(kHeadsPerCta, p.heads - h_base);
   pdl_launch_dependents();
+  // While the previous kernel ends: the rotation's table and, on their way to L2, this CTA's rows of the window.  Both follow from the
+  // pass's inputs; the table is made again should the position turn out to be another one.  (One row in a graph: 12.5 us with
+  // both behind the wait and the queries loaded before the keys were asked for, 9.2 so.)
+  auto turns = [&](int at) {
+    if (tid < p.rope_dim / 2) rope_cs2(at, p.inv_freq[tid], &sCos[tid], &sSin[tid]);
+  };
+  const int early_pos = p.row_pos[r];
+  turns(early_pos);
+  {
+    const int lo = max(0, early_pos - p.window + 1), kp = lo + split * kKeysPerCta + (tid & 63), lane_slot = p.row_slot[r];
+    const int row_bytes = p.kv_row_bytes > 0 ? p.kv_row_bytes : 2 * D;
+    if (lane_slot >= 0 && kp <= early_pos) {
+      const uint8_t* row = reinterpret_cast<const uint8_t*>(p.win) + (1ll * lane_slot * p.ring + kp % p.ring) * row_bytes;
+      for (int b = 128 * (tid >> 6); b < row_bytes; b += 256) prefetch_l2(row + b);
+    }
+  }
   pdl_wait();
   const int pos = p.row_pos[r], slot = p.row_slot[r];
   float* ml_out = p.part_ml + ((1ll * r * p.n_splits + split) * p.heads + h_base) * 2;
@@ -589,32 +605,33 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
     }
     return;
   }
-  // ---- rope table and the Q tile with RoPE on the tail (zero rows for padding heads), once per CTA
-  if (tid < p.rope_dim / 2) rope_cs2(pos, p.inv_freq[tid], &sCos[tid], &sSin[tid]);
+  if (pos != early_pos) turns(pos);
   if (tid < kHeadsPerCta) {
     sM[tid] = -INFINITY;
     sL[tid] = 0.f;
   }
-  __syncthreads();
+  // the Q tile with RoPE on the tail (zero rows for padding heads), once per CTA, while its first keys are on their way
   const int rope0 = D - p.rope_dim;
+  auto load_q = [&]() {
 #pragma unroll 4
-  for (int idx = tid; idx < kHeadsPerCta * (D / 8); idx += 128) {
-    const int h = idx / (D / 8), ch = idx % (D / 8);
-    uint4 raw = make_uint4(0, 0, 0, 0);
-    if (h < n_heads)
-      raw = *reinterpret_cast<const uint4*>(p.q + 1ll * r * p.ldq + p.q_off + 1ll * (h_base + h) * D + ch * 8);
-    if (ch * 8 >= rope0 && h < n_heads) {
-      __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(&raw);
+    for (int idx = tid; idx < kHeadsPerCta * (D / 8); idx += 128) {
+      const int h = idx / (D / 8), ch = idx % (D / 8);
+      uint4 raw = make_uint4(0, 0, 0, 0);
+      if (h < n_heads)
+        raw = *reinterpret_cast<const uint4*>(p.q + 1ll * r * p.ldq + p.q_off + 1ll * (h_base + h) * D + ch * 8);
+      if (ch * 8 >= rope0 && h < n_heads) {
+        __nv_bfloat162* v = reinterpret_cast<__nv_bfloat162*>(&raw);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float2 f = __bfloat1622float2(v[q]);
-        const int t = (ch * 8 + 2 * q - rope0) / 2;
-        const float c = sCos[t], sn = sSin[t];
-        v[q] = __floats2bfloat162_rn(f.x * c - f.y * sn, f.y * c + f.x * sn);
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = __bfloat1622float2(v[q]);
+          const int t = (ch * 8 + 2 * q - rope0) / 2;
+          const float c = sCos[t], sn = sSin[t];
+          v[q] = __floats2bfloat162_rn(f.x * c - f.y * sn, f.y * c + f.x * sn);
+        }
       }
+      *reinterpret_cast<uint4*>(sQ + h * LD + ch * 8) = raw;
     }
-    *reinterpret_cast<uint4*>(sQ + h * LD + ch * 8) = raw;
-  }
+  };
   constexpr int NT = D / 32;
   float acc[NT][4];
 #pragma unroll
@@ -657,12 +674,14 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
         if (src != nullptr) cp_async_16(dst, src + ch * 8);
         else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
       }
+      if (tile == split) load_q();
       cp_async_wait_all();
       __syncthreads();
     } else {
       // FP8 rows: copy payload + scales as they are, then expand to bf16 (exact: e4m3 value times a power of two)
       const int chunks = p.kv_row_bytes / 16;
       const int comp_chunks = p.comp_row_bytes > 0 ? p.comp_row_bytes / 16 : chunks;
+#pragma unroll 4
       for (int idx = tid; idx < kKeysPerCta * chunks; idx += 128) {
         const int key = idx / chunks, ch = idx - key * chunks;
         const uint8_t* src = reinterpret_cast<const uint8_t*>(sPtr[key]);
@@ -670,6 +689,7 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
         if (src == nullptr) *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
         else if (ch < (k0 + key >= n_w ? comp_chunks : chunks)) cp_async_16(dst, src + ch * 16);   // FP4 rows are shorter
       }
+      if (tile == split) load_q();
       cp_async_wait_all();
       __syncthreads();
 #pragma unroll 4
@@ -1089,12 +1109,20 @@ __global__ void __launch_bounds__(128) attend_merge_kernel(MergeParams p) {
   const bool live = p.row_slot[r] >= 0;
   for (int i = tid; i < p.D / 2; i += 128) {
     float a = 0.f, b = 0.f;
-    for (int s = 0; s < p.n_splits; ++s) {
-      const float w = s_w[s];
-      if (w > 0.f) {
-        const float2 v = *reinterpret_cast<const float2*>(p.part_o + ((1ll * r * p.n_splits + s) * p.heads + h) * p.D + 2 * i);
-        a = fmaf(w, v.x, a);
-        b = fmaf(w, v.y, b);
+    const float* part = p.part_o + (1ll * r * p.n_splits * p.heads + h) * p.D + 2 * i;
+    const long long step = 1ll * p.heads * p.D;
+    for (int s0 = 0; s0 < p.n_splits; s0 += 8) {          // eight splits under way, added in their order
+      float2 v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (s0 + u < p.n_splits && s_w[s0 + u] > 0.f) v[u] = *reinterpret_cast<const float2*>(part + (s0 + u) * step);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float w = s0 + u < p.n_splits ? s_w[s0 + u] : 0.f;
+        if (w > 0.f) {
+          a = fmaf(w, v[u].x, a);
+          b = fmaf(w, v[u].y, b);
+        }
       }
     }
     a *= inv_denom;
