@@ -117,6 +117,8 @@ struct GemmCfg {
   static constexpr int kBBytes = BN * kTileKBytes;
   static constexpr int kTilesA = DUAL ? 2 : 1;
   static constexpr int kTilesB = (BN + 127) / 128;
+  static constexpr bool kPieces = kScaled && BN > 32;                  // B tiles of the expert table are copied in pieces
+  static constexpr int kPieceRows = 32;
   static constexpr int kAtomsA = kTilesA * kSfPerTile;
   static constexpr int kAtomsB = kTilesB * kSfPerTile;
   // scale-factor atoms (512 B each), padded so every stage keeps its 1024-byte tile alignment
@@ -244,8 +246,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     int stage = 0;
     uint32_t phase = 0;
     // 4-bit A tiles occupy one byte per element in shared memory but the copy engine accounts the packed bytes
-    const uint32_t tx = (kA ? (p.a_fp4 ? Cfg::kABytes / 2 : Cfg::kABytes) : 0) +
-                        (kB ? Cfg::kBBytes + (Cfg::kScaled ? 512 * (Cfg::kAtomsA + Cfg::kAtomsB) : 0) : 0);
+    const uint32_t tx_fixed = (kA ? (p.a_fp4 ? Cfg::kABytes / 2 : Cfg::kABytes) : 0) +
+                              (kB && Cfg::kScaled ? 512 * (Cfg::kAtomsA + Cfg::kAtomsB) : 0);
+    // A tile of the expert table that holds fewer than BN rows is copied in pieces of kPieceRows, as many as hold them: the rest of
+    // its rows would come from L2 for nothing.  384 experts of 2304 x 5120, FC2 with five rows each (tiles of 128): 746 us with
+    // whole tiles, 704 so; with 128 rows each (tiles of 192) 1108 and 1100.  A second producer issues the pieces; bf16 tiles, which
+    // have none and are mostly full, were 1 % slower by them.
+    constexpr int kPieceBytes = Cfg::kPieceRows * kTileKBytes;
+    int pieces = 1;
+    uint32_t tx = tx_fixed + (kB ? Cfg::kBBytes : 0);
     // Weight tiles of the first stages do not depend on the previous kernel: fetch them before waiting for it.
     int prefetched = 0;
     if ((kA && p.static_operand == 1) || (kB && p.static_operand == 2)) {
@@ -289,6 +298,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int ba = p.batch_map != nullptr ? p.batch_map[b] : b;
       const int bb = p.b_batch_kind == 0 ? ba : (p.b_batch_kind == 1 ? 0 : b);
       const int a_row = (rot ? (mt + rot) % m_tiles : mt) * kBM;
+      if (kB && table && Cfg::kPieces) {
+        const int valid = min(BN, max(1, p.tile_end[nt] - n_base));
+        pieces = (valid + Cfg::kPieceRows - 1) / Cfg::kPieceRows;
+        tx = tx_fixed + pieces * kPieceBytes;
+      }
       if (kA && p.ag_world > 1) {
         const int src = a_row / p.ag_rows;
         if (src != p.ag_rank) {
@@ -329,8 +343,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if constexpr (DUAL)
             tma_load_3d_if(leader, sa + Cfg::kATile, &tmA, &full[stage], kb * Cfg::kBK, p.up_row_offset + mt * kBM, ba);
         }
-        if (kB && (!early || p.static_operand != 2))
-          tma_load_3d_if(leader, sb, &tmB, &full[stage], kb * Cfg::kBK, n_base, bb);
+        if (kB && (!early || p.static_operand != 2)) {
+          if (table && Cfg::kPieces) {
+#pragma unroll 1
+            for (int i = 0; i < pieces; ++i)
+              tma_load_3d_if(leader, sb + i * kPieceBytes, &tmB, &full[stage], kb * Cfg::kBK, n_base + i * Cfg::kPieceRows, bb);
+          } else {
+            tma_load_3d_if(leader, sb, &tmB, &full[stage], kb * Cfg::kBK, n_base, bb);
+          }
+        }
         if constexpr (kB && Cfg::kScaled) {
           uint8_t* ssf = sb + Cfg::kBBytes;
           const uint32_t at = static_cast<uint32_t>(kb - kb0) * kSf;
@@ -916,13 +937,14 @@ extern "C" int ds41_gemm_tc(const ds41_gemm_args* a, void* stream) {
   const int b_batches = a->b_batch_kind == 1 ? 1 : (a->b_batch_kind == 0 ? a_batches : batch);
   const void* a_base = a->ag_world > 0 ? a->a_peers[a->ag_rank] : a->A;
   // e2m1 operands: strides count elements, two per byte in memory
+  const int b_box = a->tile_group != nullptr && kind >= 2 && bn > 32 ? 32 : bn;        // GemmCfg::kPieces
   cudaError_t e;
   if (kind == 3) {
     // both operands e2m1, packed in memory and in shared memory
     e = make_tensor_map_3d(&tmA, a_base, TmaDtype::kU4x16Align8, K, a_rows, a_batches, a->lda / 2, a->a_batch_stride / 2,
                            bk, kBM, true);
     if (e != cudaSuccess) return e;
-    e = make_tensor_map_3d(&tmB, a->B, TmaDtype::kU4x16Align8, K, N, b_batches, a->ldb / 2, a->b_batch_stride / 2, bk, bn,
+    e = make_tensor_map_3d(&tmB, a->B, TmaDtype::kU4x16Align8, K, N, b_batches, a->ldb / 2, a->b_batch_stride / 2, bk, b_box,
                            true);
   } else {
     e = a_fp4 ? make_tensor_map_3d(&tmA, a_base, TmaDtype::kU4x16Align16, K, a_rows, a_batches, a->lda / 2,
@@ -930,7 +952,7 @@ extern "C" int ds41_gemm_tc(const ds41_gemm_args* a, void* stream) {
               : make_tensor_map_3d(&tmA, a_base, dt, K, a_rows, a_batches, a->lda * elem, a->a_batch_stride * elem, bk,
                                    kBM, true);
     if (e != cudaSuccess) return e;
-    e = make_tensor_map_3d(&tmB, a->B, dt, K, N, b_batches, a->ldb * elem, a->b_batch_stride * elem, bk, bn, true);
+    e = make_tensor_map_3d(&tmB, a->B, dt, K, N, b_batches, a->ldb * elem, a->b_batch_stride * elem, bk, b_box, true);
   }
   if (e != cudaSuccess) return e;
   StoreMaps peer{};
