@@ -1100,7 +1100,7 @@ class DS41Engine(RowsEngine):
                     w_off = lw.extra_cols - cfg.index_heads
                     self._run("index_score_gemm", G.gemm_raw, self.idx_q, self.idx_k, self.scores, R * cfg.index_heads,
                               n_keys, cfg.index_dim, lda=cfg.index_dim, ldb=cfg.index_dim, ldo=self.max_keys, out_mode=8,
-                              bn=256 if n_keys >= 256 else 64, row_w=self.extras[:, w_off:], row_w_ld=lw.extra_cols,
+                              bn=G.score_bn(R * cfg.index_heads, n_keys), row_w=self.extras[:, w_off:], row_w_ld=lw.extra_cols,
                               col_limit=self.idx_vis, status=self.status)
                 else:
                     self._run("index_score", k.ds41_index_score_cand,
@@ -1173,6 +1173,11 @@ class DS41Engine(RowsEngine):
                 self._moe_sorted(R, lw)
             else:
                 EL = lw.n_experts // self.world
+                # the shared expert's second product before the routed ones: its weights are fetched while the router ends,
+                # which an expert GEMM's CTAs leave no room for (a request's step: 10 to 13 us behind them, 4 here)
+                s_s = self._splits(H, self.I_sh, R)
+                self._run("gemm_shared_down", G.linear_planes, self.shared_act[:R], lw.w2_sh,
+                                self.planes_shared.view(-1)[: s_s * R * H].view(s_s, R, H), s_s, status=self.status)
                 self._run("moe_plan", k.ds41_moe_plan, 
                     lib.ptr(self.ids), lib.ptr(self.route_w), lib.ptr(self.row_slot), R, lw.topk, self.rank * EL,
                     (self.rank + 1) * EL, self.max_active, self.moe_rows, lib.ptr(self.active), lib.ptr(self.n_active),
@@ -1232,9 +1237,6 @@ class DS41Engine(RowsEngine):
                                batch=self.max_active, a_batches=EL, a_batch_stride=H * I, b_batch_stride=R * I,
                                out_batch_stride=R * H, batch_map=self.active, n_active=self.n_active, b_batch_kind=2,
                                row_w=self.row_w, row_w_ld=self.moe_rows, status=self.status)
-                s_s = self._splits(H, self.I_sh, R)
-                self._run("gemm_shared_down", G.linear_planes, self.shared_act[:R], lw.w2_sh,
-                                self.planes_shared.view(-1)[: s_s * R * H].view(s_s, R, H), s_s, status=self.status)
                 if self.world > 1:       # the block that finishes last publishes the expert plane
                     self._run("moe_combine", k.ds41_moe_combine_signal, lib.ptr(self.fc2), lib.ptr(self.slot_of),
                               lib.ptr(self.planes_shared), s_s, R, lw.topk, H, lib.ptr(self.moe_plane),

@@ -97,6 +97,15 @@ def wide(rows: int, n: int, batch: int = 1) -> bool:
     return rows > 128 and -(-rows // 128) * -(-n // 256) * batch >= SMS
 
 
+def score_bn(m: int, n_keys: int) -> int:
+    """Keys per tile of the indexer's product: as many as still give every SM a tile.  One row over 2112 keys is nine tiles of 256
+    and waits for eight chunks of one tile's epilogue (16 us); sixty-six of 32 take 8."""
+    for bn in (256, 128, 64):
+        if n_keys >= bn and -(-m // 128) * -(-n_keys // bn) >= SMS:
+            return bn
+    return 32
+
+
 def linear_planes(x: torch.Tensor, w: torch.Tensor, planes: torch.Tensor, splits: int, *, status=None, signal=None):
     """Swap-AB split-K projection: planes[s, rows, N] (fp32) partial sums of x @ w.T.  `signal`: see gemm_raw."""
     rows, K = x.shape
