@@ -300,8 +300,8 @@ __global__ void __launch_bounds__(MT * PW * 32) latent_attend_mma_kernel(ds41_la
   pdl_launch_dependents();
   int slot, k0, k1;
   auto find = [&]() {
-    slot = p.row_slot[r];
-    const int n_keys = slot < 0 ? 0 : p.row_pos[r] + 1;
+    slot = __ldcg(p.row_slot + r);       // again behind the wait: past L1, which may hold what stood there before
+    const int n_keys = slot < 0 ? 0 : __ldcg(p.row_pos + r) + 1;
     const int per = ((n_keys + kKeyTile - 1) / kKeyTile + p.n_splits - 1) / p.n_splits * kKeyTile;
     k0 = split * per;
     k1 = min(n_keys, k0 + per);

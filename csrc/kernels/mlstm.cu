@@ -122,8 +122,10 @@ __global__ void __launch_bounds__(256) mlstm_walk_kernel(ds41_mlstm_args p) {
   int r = blockIdx.z;
   // the state has left L2 since the last pass: its lines are asked for while the previous kernel ends (one row, 4 heads of 256 x 512:
   // 8.8 and 8.1 us; 32 rows, 8 heads 55 and 53)
-  if (segment_start(p.row_slot, r) && p.row_slot[r] < p.slots && p.row_pos[r] != 0) {
-    const long long head = 1ll * p.row_slot[r] * p.heads + h;
+  // (__ldcg: past L1, which would answer the reads behind the wait)
+  const int early = __ldcg(p.row_slot + r);
+  if (early >= 0 && (r == 0 || __ldcg(p.row_slot + r - 1) != early) && early < p.slots && __ldcg(p.row_pos + r) != 0) {
+    const long long head = 1ll * early * p.heads + h;
     for (int d = tid; d < p.dim_pad; d += 256)
       prefetch_l2(p.state_s + (head * p.dim_pad + d) * p.vdim_pad + vb * kStateCols);
     if (32 * tid < p.dim_pad) prefetch_l2(p.state_n + (head * gridDim.x + vb) * p.dim_pad + 32 * tid);

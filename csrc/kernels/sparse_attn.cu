@@ -572,10 +572,10 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
   auto turns = [&](int at) {
     if (tid < p.rope_dim / 2) rope_cs2(at, p.inv_freq[tid], &sCos[tid], &sSin[tid]);
   };
-  const int early_pos = p.row_pos[r];
+  const int early_pos = __ldcg(p.row_pos + r);      // past L1, which would answer the read behind the wait
   turns(early_pos);
   {
-    const int lo = max(0, early_pos - p.window + 1), kp = lo + split * kKeysPerCta + (tid & 63), lane_slot = p.row_slot[r];
+    const int lo = max(0, early_pos - p.window + 1), kp = lo + split * kKeysPerCta + (tid & 63), lane_slot = __ldcg(p.row_slot + r);
     const int row_bytes = p.kv_row_bytes > 0 ? p.kv_row_bytes : 2 * D;
     if (lane_slot >= 0 && kp <= early_pos) {
       const uint8_t* row = reinterpret_cast<const uint8_t*>(p.win) + (1ll * lane_slot * p.ring + kp % p.ring) * row_bytes;
