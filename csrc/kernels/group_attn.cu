@@ -482,6 +482,9 @@ __global__ void __launch_bounds__(128) group_attend_plain_kernel(ds41_group_atte
 // KD: 16-column pieces of the key width, NP: of the value width.  A warp's walk is a chain of latencies, so a CTA has eight
 // of them; four, and two CTAs share an SM, where there are more CTAs than SMs (or the value width takes the registers).
 constexpr int kMaxStages = 4;
+// Tiles of keys that a CTA asks for, on their way to L2, before the wait for the previous kernel.  With the gap between that wait and
+// the first copy (the producer waited for the queries, too), 8 rows over about 2200 keys, 4 heads: 22 us in a graph, 20.7 so.
+constexpr int kAheadTiles = 8;
 
 struct AttendPlan {
   int warps, kc, vc, stages, box;                     // 64-column chunks, ring length, rows per TMA box
@@ -538,8 +541,31 @@ group_attend_mma_kernel(const __grid_constant__ CUtensorMap pool, const ds41_gro
     tma_prefetch_desc(&pool);
   }
   pdl_launch_dependents();
+  int slot, pos, first, base, t0, t1;
+  auto find = [&]() {                    // this CTA's tiles of keys
+    slot = __ldcg(p.row_slot + r);       // again behind the wait: past L1, which may hold what stood there before
+    pos = __ldcg(p.row_pos + r);
+    first = chunk_start(pos, p.chunk);
+    base = first - first % plan.box;
+    const int tiles = (pos - base) / kTileKeys + 1, per = (tiles + p.n_splits - 1) / p.n_splits;
+    t0 = min(tiles, split * per);
+    t1 = min(tiles, t0 + per);
+  };
+  find();
+  if (slot >= 0) {                       // the cache's rows have left L2 since the last pass
+    const int k0 = base + t0 * kTileKeys, k1 = min(pos + 1, base + min(t1, t0 + kAheadTiles) * kTileKeys);
+    const int k_lines = (dp + 63) / 64, lines = k_lines + (vp + 63) / 64, row_len = p.kv_heads * (dp + vp);
+#pragma unroll 4
+    for (int i = tid; i < (k1 - k0) * lines; i += blockDim.x) {
+      const int key = i / lines, c = i - key * lines;
+      const __nv_bfloat16* kv = cache_row(static_cast<const __nv_bfloat16*>(p.pool), p.page_table, p.max_pages, p.page_tokens,
+                                          row_len, slot, k0 + key);
+      if (kv != nullptr) prefetch_l2(kv + (c < k_lines ? g * dp + 64 * c : p.kv_heads * dp + g * vp + 64 * (c - k_lines)));
+    }
+  }
+  __syncthreads();                       // the barriers are ready
   pdl_wait();
-  const int slot = p.row_slot[r], pos = p.row_pos[r];
+  find();
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out) + 1ll * r * p.ld_out;
   if (slot < 0) {                        // the same in every CTA of the cluster
     if (split == 0)
@@ -547,9 +573,6 @@ group_attend_mma_kernel(const __grid_constant__ CUtensorMap pool, const ds41_gro
         if (h0 + i / vp < h_end) out[(h0 + i / vp) * vp + i % vp] = __float2bfloat16_rn(0.f);
     return;
   }
-  const int first = chunk_start(pos, p.chunk), base = first - first % plan.box;
-  const int tiles = (pos - base) / kTileKeys + 1, per = (tiles + p.n_splits - 1) / p.n_splits;
-  const int t0 = min(tiles, split * per), t1 = min(tiles, t0 + per);
   if (warp < NW) {
     for (int i = warp; i < 16; i += NW) {
       const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(p.q) + r * p.ld_q + (h0 + i) * dp;
@@ -557,8 +580,8 @@ group_attend_mma_kernel(const __grid_constant__ CUtensorMap pool, const ds41_gro
         *reinterpret_cast<uint4*>(sq + i * KS + d) =
             h0 + i < h_end ? *reinterpret_cast<const uint4*>(q + d) : make_uint4(0, 0, 0, 0);
     }
+    named_barrier(1, 32 * NW);           // the producer does not wait for the queries
   }
-  __syncthreads();
   float acc[NP][2][4];
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   if (warp == NW) {
