@@ -241,6 +241,12 @@ int ds41_argmax_rows(const float* logits, long long ld, int rows, int vocab_loca
 int ds41_argmax_merge(const float* const* vals, const int* const* idxs, int n_ranks, int rows, int* out,
                       const uint32_t* const* wait_flags, const uint32_t* wait_epoch, int* status, void* stream);
 int ds41_decode_feedback(const int* chosen, int* tokens, int* pos, int rows, void* stream);
+// A step of a decode session.  `host`, `host_in`, `host_out`: pinned memory; inputs are [3][rows] tokens, positions, slots.
+// ds41_step_result and ds41_graph_step (inputs, the captured pass, result) return when the result is there.
+int ds41_step_inputs(const int* host, int* tokens, int* pos, int* slot, int rows, void* stream);
+int ds41_step_result(const int* chosen, int* host, int rows, void* stream);
+int ds41_graph_step(void* graph_exec, const int* host_in, int* tokens, int* pos, int* slot, const int* chosen, int* host_out,
+                    int rows, void* stream);
 int ds41_spec_accept(const int* inputs, const int* chosen, const int* first, const int* count, int reqs,
                      int max_emit, int eos, int* accepted, int* emit, int* n_emit, void* stream);
 

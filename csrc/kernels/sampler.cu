@@ -212,9 +212,49 @@ __global__ void decode_feedback_kernel(const int* chosen, int* tokens, int* pos,
   }
 }
 
+// Inputs of a step from pinned host memory (tokens, positions and slots of `rows` rows, one after the other), and its result back into
+// it.  The GPU reads and writes that memory itself: three copies by the copy engines and one back, each with a hand-over between
+// engines, cost a decode step some 20 us more, torch's share of them included
+// (one request of flash, three layers: 888 us a step with those, 870 so).  Neither kernel lets the next one start early, since those read the inputs before they
+// wait (a graph's first kernel does not start early in any case).
+__global__ void step_inputs_kernel(const int* host, int* tokens, int* pos, int* slot, int rows) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 3 * rows) return;
+  const int part = i / rows, r = i - part * rows;
+  (part == 0 ? tokens : part == 1 ? pos : slot)[r] = __ldcv(host + i);
+}
+__global__ void step_result_kernel(const int* chosen, int* host, int rows) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < rows) host[r] = chosen[r];
+}
+
 }  // namespace ds41
 
 using namespace ds41;
+
+extern "C" int ds41_step_inputs(const int* host, int* tokens, int* pos, int* slot, int rows, void* stream) {
+  if (host == nullptr || tokens == nullptr || pos == nullptr || slot == nullptr || rows <= 0 || rows > (1 << 28))
+    return cudaErrorInvalidValue;
+  step_inputs_kernel<<<(3 * rows + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(host, tokens, pos, slot, rows);
+  return cudaGetLastError();
+}
+
+extern "C" int ds41_step_result(const int* chosen, int* host, int rows, void* stream) {
+  if (chosen == nullptr || host == nullptr || rows <= 0) return cudaErrorInvalidValue;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  step_result_kernel<<<(rows + 255) / 256, 256, 0, st>>>(chosen, host, rows);
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : cudaStreamSynchronize(st);
+}
+
+extern "C" int ds41_graph_step(void* graph_exec, const int* host_in, int* tokens, int* pos, int* slot, const int* chosen,
+                               int* host_out, int rows, void* stream) {
+  if (graph_exec == nullptr) return cudaErrorInvalidValue;
+  int e = ds41_step_inputs(host_in, tokens, pos, slot, rows, stream);
+  if (e != cudaSuccess) return e;
+  e = cudaGraphLaunch(static_cast<cudaGraphExec_t>(graph_exec), static_cast<cudaStream_t>(stream));
+  return e != cudaSuccess ? e : ds41_step_result(chosen, host_out, rows, stream);
+}
 
 extern "C" int ds41_decode_feedback(const int* chosen, int* tokens, int* pos, int rows, void* stream) {
   if (rows <= 0) return cudaErrorInvalidValue;

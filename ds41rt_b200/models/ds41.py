@@ -30,7 +30,7 @@ from ..ops import attention as A
 from ..ops import gemm as G
 from ..ops import lib
 from ..parallel.fabric import Fabric, SymBuffer
-from .base import RowsEngine
+from .base import RowsEngine, row_values
 from .paged import PagedSlots
 
 BF16 = torch.bfloat16
@@ -806,15 +806,14 @@ class DS41Engine(RowsEngine):
         floor under the attention windows of the pass: positions below it are not attended."""
         n = len(positions)
         self._floor_on = row_lo is not None
+        assert all(x is None or len(x) == n for x in (row_lo, row_hi))
         if row_lo is not None:
-            self.row_lo.copy_(torch.tensor(list(row_lo) + [0] * (self.max_rows - n), dtype=I32), non_blocking=True)
-        assert n <= self.max_rows
-        pad = self.max_rows - n
-        p = torch.tensor(list(positions) + [0] * pad, dtype=I32)
-        s = torch.tensor(list(slots) + [-1] * pad, dtype=I32)
+            self.row_lo.copy_(row_values(row_lo, self.max_rows, 0), non_blocking=True)
+        assert n <= self.max_rows and n == len(slots)
+        p, s = row_values(positions, self.max_rows, 0), row_values(slots, self.max_rows, -1)
         if tokens is not None:        # None: the token ids are already on the device (fed by a kernel)
             assert len(tokens) == n
-            self.in_tokens.copy_(torch.tensor(list(tokens) + [0] * pad, dtype=I32), non_blocking=True)
+            self.in_tokens.copy_(row_values(tokens, self.max_rows, 0), non_blocking=True)
         self.row_pos.copy_(p, non_blocking=True)
         self.row_slot.copy_(s, non_blocking=True)
         # what the host knows about the pass it just described (used by the next forward_rows only): a long pass over
@@ -822,16 +821,14 @@ class DS41Engine(RowsEngine):
         # A decode-sized pass over one request (a speculative verification, a lone request's step) scores on the tensor
         # cores too; its launches may be replayed from a graph while the context grows, so the key count is the static
         # bound (-1) and the visible count per row is worked out on the device.
-        slot_list = list(slots)
-        one = n > 0 and len(set(slot_list)) == 1 and slot_list[0] >= 0
+        one = n > 0 and int(s[0]) >= 0 and bool((s[:n] == s[0]).all())
         self._pass_hint = None
         if one and n > self.moe_rows:
-            self._pass_hint = (n, int(max(positions)))
+            self._pass_hint = (n, int(p[:n].max()))
         elif one and getattr(self, "idx_q", None) is not None and self.max_keys <= 32768:
             self._pass_hint = (n, -1)
         if self.row_hi is not None:
-            h = torch.tensor(list(row_hi if row_hi is not None else positions) + [0] * pad, dtype=I32)
-            self.row_hi.copy_(h, non_blocking=True)
+            self.row_hi.copy_(row_values(row_hi if row_hi is not None else positions, self.max_rows, 0), non_blocking=True)
 
     # ------------------------------------------------------------------ Engram memory layers
     def attach_engram(self, layer: int, module) -> None:
@@ -1669,12 +1666,12 @@ class DS41Engine(RowsEngine):
         r0 = self.ced_replay_start(start, end)
         for c0 in range(start, end, chunk):
             c1 = min(end, c0 + chunk)
-            self.set_rows(tokens[c0 - start:c1 - start], list(range(c0, c1)), [slot] * (c1 - c0))
+            self.set_rows(tokens[c0 - start:c1 - start], range(c0, c1), [slot] * (c1 - c0))
             self.ced_encoder_slice(c0, c1, r0)
         nxt = -1
         for c0 in range(r0, end, chunk):
             c1 = min(end, c0 + chunk)
-            self.set_rows(tokens[c0 - start:c1 - start], list(range(c0, c1)), [slot] * (c1 - c0),
+            self.set_rows(tokens[c0 - start:c1 - start], range(c0, c1), [slot] * (c1 - c0),
                           row_lo=[r0] * (c1 - c0))
             self.ced_replay_slice(c0, c1, r0, head=c1 >= end)
             if c1 >= end:

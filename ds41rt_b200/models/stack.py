@@ -22,7 +22,7 @@ from ..ops import lib
 from ..ops import stack as S
 from ..ops.stack import Matrix, Proj, ceil_to
 from ..stack_config import GroupedAttentionSpec, LatentAttentionSpec, MLSTMSpec, MoESpec, StackConfig
-from .base import RowsEngine
+from .base import RowsEngine, row_values
 from .paged import PagedSlots
 
 BF16, F32, I32 = torch.bfloat16, torch.float32, torch.int32
@@ -713,24 +713,23 @@ class StackEngine(RowsEngine):
         assert row_lo is None and row_hi is None, "a layer stack has no window floor"
         n = len(positions)
         assert n <= self.max_rows
-        slots, positions, seen = list(slots), list(positions), set()
-        for i in range(n):
-            if slots[i] < 0:
-                continue
-            if i and slots[i] == slots[i - 1]:
-                assert positions[i] == positions[i - 1] + 1, "rows of a request must follow one another"
-            else:
-                assert slots[i] not in seen, "rows of a request must be adjacent"
-                seen.add(slots[i])
+        assert n == len(slots)
+        pos, slot = row_values(positions, self.max_rows, 0), row_values(slots, self.max_rows, -1)
+        p, s = pos[:n], slot[:n]
+        follows = (s[1:] == s[:-1]) & (s[1:] >= 0)            # a row of the same request as the row before it
+        assert bool((p[1:] == p[:-1] + 1)[follows].all()), "rows of a request must follow one another"
+        first = s >= 0
+        first[1:] &= ~follows
+        seen = s[first].tolist()
+        assert len(set(seen)) == len(seen), "rows of a request must be adjacent"
         # what the host knows about the pass it just described: a long pass of one request
-        one = n >= self.long_rows and len(seen) == 1 and min(slots) >= 0 and not self.f32
-        self._hint = (n, positions[-1] + 1) if one else None
-        pad = self.max_rows - n
+        one = n >= self.long_rows and len(seen) == 1 and int(s.min()) >= 0 and not self.f32
+        self._hint = (n, int(p[-1]) + 1) if one else None
         if tokens is not None:
             assert len(tokens) == n
-            self.in_tokens.copy_(torch.tensor(list(tokens) + [0] * pad, dtype=I32), non_blocking=True)
-        self.row_pos.copy_(torch.tensor(positions + [0] * pad, dtype=I32), non_blocking=True)
-        self.row_slot.copy_(torch.tensor(slots + [-1] * pad, dtype=I32), non_blocking=True)
+            self.in_tokens.copy_(row_values(tokens, self.max_rows, 0), non_blocking=True)
+        self.row_pos.copy_(pos, non_blocking=True)
+        self.row_slot.copy_(slot, non_blocking=True)
 
     def _resid(self, R: int, *, y: Optional[Proj] = None, gate: Optional[Proj] = None, bias=None, post=None, x_in=None,
                x_out=None, layer: Optional[int] = None, next_w=None, post_rms: bool = False):

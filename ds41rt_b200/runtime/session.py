@@ -12,6 +12,7 @@ Reference behaviour being replaced: lazily captured per-shape CUDA graphs keyed 
 """
 from __future__ import annotations
 
+import ctypes as C
 from typing import Dict, List, Optional
 
 import torch
@@ -27,10 +28,10 @@ class DecodeSession:
         self.graphs: Dict[tuple, torch.cuda.CUDAGraph] = {}
         self.launches_per_graph: Dict[tuple, int] = {}
         R = engine.max_rows
-        self.h_tokens = torch.zeros(R, dtype=torch.int32).pin_memory()
-        self.h_pos = torch.zeros(R, dtype=torch.int32).pin_memory()
-        self.h_slot = torch.full((R,), -1, dtype=torch.int32).pin_memory()
+        # a step's inputs (tokens, positions, slots of its rows, one after the other) and its result
+        self.h_in = torch.zeros(3 * R, dtype=torch.int32).pin_memory()
         self.h_chosen = torch.zeros(R, dtype=torch.int32).pin_memory()
+        self._in, self._chosen = self.h_in.numpy(), self.h_chosen.numpy()
         self.h2d_bytes = 0
         self.d2h_bytes = 0
 
@@ -53,25 +54,26 @@ class DecodeSession:
 
     # ------------------------------------------------------------------ stepping
     def step(self, tokens: List[int], positions: List[int], slots: List[int]) -> List[int]:
-        """One pass through the public path: pinned H2D of the inputs, graph replay, D2H of the result."""
+        """One pass through the public path: the inputs from pinned memory, graph replay, the result back into it."""
         n = len(tokens)
         e = self.e
-        self.h_tokens[:n] = torch.tensor(tokens, dtype=torch.int32)
-        self.h_pos[:n] = torch.tensor(positions, dtype=torch.int32)
-        self.h_slot[:n] = torch.tensor(slots, dtype=torch.int32)
-        e.in_tokens[:n].copy_(self.h_tokens[:n], non_blocking=True)
-        e.row_pos[:n].copy_(self.h_pos[:n], non_blocking=True)
-        e.row_slot[:n].copy_(self.h_slot[:n], non_blocking=True)
+        if not 0 < n <= e.max_rows:
+            raise ValueError(f"a step has 1 to {e.max_rows} rows, not {n}")
+        for i, values in enumerate((tokens, positions, slots)):
+            self._in[i * n:(i + 1) * n] = values
         self.h2d_bytes += 3 * 4 * n
         g = self.graph(n)
+        src, dst, s = lib.ptr(self.h_in), lib.ptr(self.h_chosen), lib.stream()
+        rows = (lib.ptr(e.in_tokens), lib.ptr(e.row_pos), lib.ptr(e.row_slot))
         if g is not None:
-            g.replay()
+            lib.check(e.k.ds41_graph_step(C.c_void_p(g.raw_cuda_graph_exec()), src, *rows, lib.ptr(e.chosen), dst, n, s),
+                      "decode step")
         else:
+            lib.check(e.k.ds41_step_inputs(src, *rows, n, s), "step inputs")
             e.forward_rows(n)
-        self.h_chosen[:n].copy_(e.chosen[:n], non_blocking=True)
-        torch.cuda.current_stream().synchronize()
+            lib.check(e.k.ds41_step_result(lib.ptr(e.chosen), dst, n, s), "step result")
         self.d2h_bytes += 4 * n
-        return self.h_chosen[:n].tolist()
+        return self._chosen[:n].tolist()
 
     def run_device_loop(self, rows: int, steps: int):
         """`steps` decode steps with on-device token feedback (no host synchronisation inside)."""
