@@ -105,17 +105,19 @@ struct GemmParams {
   int* status;
 };
 
-template <int BN, int KIND, int DUAL = 0>
+// FORM: 0 plain, 1 dual (gate and up tiles of a gated product, mode 4), 2 indexer scores (mode 8)
+template <int BN, int KIND, int FORM = 0>
 struct GemmCfg {
+  static constexpr bool kDual = FORM == 1, kScore = FORM == 2;
   static constexpr int kElemBytes = (KIND == 0) ? 2 : 1;
   // elements of K per stage: one 128-byte swizzle span (kind 3 packs two e2m1 values per byte)
   static constexpr int kBK = (KIND == 3) ? 2 * kTileKBytes : kTileKBytes / kElemBytes;
   static constexpr int kSfPerTile = (KIND == 3) ? 4 : 1;               // 512-byte scale atoms per 128 rows per stage
   static constexpr bool kScaled = (KIND == 2 || KIND == 3);
   static constexpr int kATile = kBM * kTileKBytes;                     // 16 KiB
-  static constexpr int kABytes = kATile * (DUAL ? 2 : 1);
+  static constexpr int kABytes = kATile * (kDual ? 2 : 1);
   static constexpr int kBBytes = BN * kTileKBytes;
-  static constexpr int kTilesA = DUAL ? 2 : 1;
+  static constexpr int kTilesA = kDual ? 2 : 1;
   static constexpr int kTilesB = (BN + 127) / 128;
   static constexpr bool kPieces = kScaled && BN > 32;                  // B tiles of the expert table are copied in pieces
   static constexpr int kPieceRows = 32;
@@ -124,14 +126,14 @@ struct GemmCfg {
   // scale-factor atoms (512 B each), padded so every stage keeps its 1024-byte tile alignment
   static constexpr int kSfBytes = kScaled ? ((512 * (kAtomsA + kAtomsB) + 1023) / 1024 * 1024) : 0;
   static constexpr int kStageBytes = kABytes + kBBytes + kSfBytes;
-  static constexpr int kStaging = (!DUAL && BN >= 64) ? kStagingBytes : 0;
+  static constexpr int kStaging = (FORM == 0 && BN >= 64) ? kStagingBytes : 0;
   static constexpr int kStagesRaw = ((kStaging ? 194 : 200) * 1024) / kStageBytes;
   // Skinny decode tiles (BN <= 32) keep the ring short enough for two CTAs of consecutive launches to share an SM: the
   // next kernel's set-up and its weight prefetch then overlap the tail of the previous one (programmatic launch).
   static constexpr int kStageCap = (BN <= 32) ? DS41_SKINNY_STAGES : 8;
   static constexpr int kStages = kStagesRaw > kStageCap ? kStageCap : kStagesRaw;
   static constexpr int kSfCols = kScaled ? 4 * (kAtomsA + kAtomsB) : 0;               // TMEM columns per stage
-  static constexpr int kAccCols = (BN < 32 ? 32 : BN) * (DUAL ? 2 : 1);
+  static constexpr int kAccCols = (BN < 32 ? 32 : BN) * (kDual ? 2 : 1);
   // Two accumulator sets let the epilogue of one tile overlap the MMAs of the next.  The widest block-scaled dual tile
   // (128 tokens x gate + up) leaves room for only one beside its scale columns; it is still the better trade there:
   // each weight byte fetched from L2 serves twice the tokens of a 64-wide tile.
@@ -142,10 +144,12 @@ struct GemmCfg {
   // The widest block-scaled dual tile has a single accumulator set: the tensor cores wait for its epilogue (about 40
   // instructions per column and thread), so two sets of four warps share its columns.  FC1 of 384 experts x 128 rows, 5120 x
   // 2304: 2445 us with one set, 2198 with two.
-  static constexpr int kEpiSets = (DUAL && kAccStages == 1) ? 2 : 1;
+  // So do they with indexer scores, whose two K steps take a tenth of their epilogue's time.
+  static constexpr int kEpiSets = (kDual && kAccStages == 1) || kScore ? 2 : 1;
   static constexpr int kThreads = kGemmThreads + 128 * (kEpiSets - 1) + (kScaled ? 32 : 0);    // + the second producer
   static constexpr int kSmemBytes = kStages * kStageBytes + kStaging + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(kTmemNeeded <= 512, "TMEM budget exceeded");
+  static_assert(!kScore || BN >= 32, "a chunk of scores has 32 columns");
   static_assert(kStages >= 2, "not enough shared memory for two stages");
 };
 
@@ -167,11 +171,11 @@ __device__ __forceinline__ long long decode_tile(long long t, int m_tiles, int n
   return outer;
 }
 
-template <int BN, int KIND, int DUAL>
-__global__ void __launch_bounds__(GemmCfg<BN, KIND, DUAL>::kThreads, 1)
+template <int BN, int KIND, int FORM>
+__global__ void __launch_bounds__(GemmCfg<BN, KIND, FORM>::kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ StoreMaps stm, GemmParams p) {
-  using Cfg = GemmCfg<BN, KIND, DUAL>;
+  using Cfg = GemmCfg<BN, KIND, FORM>;
   constexpr int S = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
@@ -231,6 +235,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const uint32_t tmem_base = *tmem_slot;
 
   bool ok = true;                              // false: a wait of this thread gave up
+  // A tile of scores whose keys none of its four queries sees is neither loaded nor multiplied: the epilogue fills it.  Every role asks
+  // for itself, behind its wait for the kernel that wrote the limits.  8192 rows of one request, 32 heads, 4096 keys: 1406 us with
+  // all tiles and one set of epilogue warps, 428 without the hidden half and with two.
+  auto hidden = [&](int mt, int nt) {
+    if constexpr (Cfg::kScore) {
+      if (p.col_limit == nullptr || table) return false;
+      const int q0 = mt * (kBM / 32), q1 = min(q0 + kBM / 32, p.M / 32);
+      int lim = 0;
+      for (int q = q0; q < q1; ++q) lim = max(lim, __ldg(p.col_limit + q));
+      return nt * BN >= lim;
+    } else {
+      return false;
+    }
+  };
   // ------------------------------------------------------------ TMA producers
   // One warp per role, walking its loop with uniform control flow; `leader` predicates the copies.  A scaled kind asks for three to
   // five copies a stage, and one thread that issued them all (from a one-lane branch, whose descriptors and coordinates take
@@ -257,7 +275,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint32_t tx = tx_fixed + (kB ? Cfg::kBBytes : 0);
     // Weight tiles of the first stages do not depend on the previous kernel: fetch them before waiting for it.
     int prefetched = 0;
-    if ((kA && p.static_operand == 1) || (kB && p.static_operand == 2)) {
+    if (!Cfg::kScore && ((kA && p.static_operand == 1) || (kB && p.static_operand == 2))) {
       if (p.n_active == nullptr && p.batch_map == nullptr && !table && blockIdx.x < tiles) {
         long long r = blockIdx.x;
         int mt, nt;
@@ -272,7 +290,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           mbar_expect_tx_if(leader, &full[i], tx);
           if (kA && p.static_operand == 1) {
             tma_load_3d_if(leader, sa, &tmA, &full[i], (kb0 + i) * Cfg::kBK, mt * kBM, b);
-            if constexpr (DUAL)
+            if constexpr (Cfg::kDual)
               tma_load_3d_if(leader, sa + Cfg::kATile, &tmA, &full[i], (kb0 + i) * Cfg::kBK, p.up_row_offset + mt * kBM, b);
           } else {
             tma_load_3d_if(leader, sa + Cfg::kABytes, &tmB, &full[i], (kb0 + i) * Cfg::kBK, nt * BN,
@@ -290,6 +308,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       long long r = t;
       int mt, nt;
       r = decode_tile(r, m_tiles, n_tiles, band_tiles, mt, nt);
+      if (hidden(mt, nt)) continue;
       const int sp = static_cast<int>(r % p.k_splits); r /= p.k_splits;
       const int b = table ? p.tile_group[nt] : static_cast<int>(r);
       const int n_base = table ? p.tile_row0[nt] : nt * BN;
@@ -323,7 +342,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const long long row_atoms = 1ll * kb_total * kSf, at = 1ll * kb0 * kSf;
         const uint8_t* of_a = p.sfa + ba * p.sfa_batch_stride + at;
         sf_a = of_a + mt * row_atoms;
-        if constexpr (DUAL) sf_up = of_a + (p.up_row_offset / 128 + mt) * row_atoms;
+        if constexpr (Cfg::kDual) sf_up = of_a + (p.up_row_offset / 128 + mt) * row_atoms;
 #pragma unroll
         for (int a = 0; a < Cfg::kTilesB; ++a)
           sf_b[a] = p.sfb + bb * p.sfb_batch_stride + at + (n_base / 128 + a) * row_atoms;
@@ -340,7 +359,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         uint8_t* sb = sa + Cfg::kABytes;
         if (kA && (!early || p.static_operand != 1)) {
           tma_load_3d_if(leader, sa, &tmA, &full[stage], kb * Cfg::kBK, a_row, ba);
-          if constexpr (DUAL)
+          if constexpr (Cfg::kDual)
             tma_load_3d_if(leader, sa + Cfg::kATile, &tmA, &full[stage], kb * Cfg::kBK, p.up_row_offset + mt * kBM, ba);
         }
         if (kB && (!early || p.static_operand != 2)) {
@@ -356,7 +375,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           uint8_t* ssf = sb + Cfg::kBBytes;
           const uint32_t at = static_cast<uint32_t>(kb - kb0) * kSf;
           bulk_load_if(leader, ssf, sf_a + at, kSf, &full[stage]);
-          if constexpr (DUAL) bulk_load_if(leader, ssf + kSf, sf_up + at, kSf, &full[stage]);
+          if constexpr (Cfg::kDual) bulk_load_if(leader, ssf + kSf, sf_up + at, kSf, &full[stage]);
 #pragma unroll
           for (int a = 0; a < Cfg::kTilesB; ++a)
             bulk_load_if(leader, ssf + 512 * (Cfg::kAtomsA + a * Cfg::kSfPerTile), sf_b[a] + at, kSf, &full[stage]);
@@ -382,9 +401,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     int acc = 0;
     uint32_t acc_phase = 0;
     constexpr uint32_t kFmt = (KIND == 0) ? 1u : 0u;   // bf16 / e4m3
+    if constexpr (Cfg::kScore) pdl_wait();
     for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-      int mt_unused, nt;
-      const long long r = decode_tile(t, m_tiles, n_tiles, band_tiles, mt_unused, nt);
+      int mt, nt;
+      const long long r = decode_tile(t, m_tiles, n_tiles, band_tiles, mt, nt);
+      if (hidden(mt, nt)) continue;
       const int sp = static_cast<int>(r % p.k_splits);
       const int kb0 = sp * kb_per_split;
       const int kb1 = min(kb_total, kb0 + kb_per_split);
@@ -426,7 +447,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               // one atom per stage; instruction k uses byte k of every 32-bit scale cell
               const uint32_t id = umma_idesc_bs(kBM, n_mma, p.a_fp4 ? 5u : 0u, 0, 1, k, k);   // e2m1 = 5, e4m3 = 0
               umma_mxf8_if(leader, d_tmem, adesc + 2 * k, bdesc + 2 * k, id, accum, sf_t, sfb_t);
-              if constexpr (DUAL) {
+              if constexpr (Cfg::kDual) {
                 const uint64_t adesc2 = umma_desc_sw128(sa + Cfg::kATile);
                 umma_mxf8_if(leader, d_tmem + Cfg::kAccCols / 2, adesc2 + 2 * k, bdesc + 2 * k, id, accum, sf_t + 4, sfb_t);
               }
@@ -434,7 +455,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               // NVFP4: instruction k (64 K elements) uses atom k: four E4M3 scales per row fill one 32-bit cell
               const uint32_t id = umma_idesc_bs(kBM, n_mma, 1u, 1u, 0, 0, 0);                // e2m1 x e2m1, UE4M3 scales
               umma_nvf4_if(leader, d_tmem, adesc + 2 * k, bdesc + 2 * k, id, accum, sf_t + 4 * k, sfb_t + 4 * k);
-              if constexpr (DUAL) {
+              if constexpr (Cfg::kDual) {
                 const uint64_t adesc2 = umma_desc_sw128(sa + Cfg::kATile);
                 umma_nvf4_if(leader, d_tmem + Cfg::kAccCols / 2, adesc2 + 2 * k, bdesc + 2 * k, id, accum, sf_t + 16 + 4 * k,
                           sfb_t + 4 * k);
@@ -447,7 +468,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const uint32_t accum = (kb > kb0 || k > 0) ? 1u : 0u;
             if constexpr (KIND == 0) umma_bf16_if(leader, d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc_t, accum);
             else umma_f8_if(leader, d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc_t, accum);
-            if constexpr (DUAL) {
+            if constexpr (Cfg::kDual) {
               const uint64_t adesc2 = umma_desc_sw128(sa + Cfg::kATile);
               if constexpr (KIND == 0) umma_bf16_if(leader, d_tmem + Cfg::kAccCols / 2, adesc2 + 2 * k, bdesc + 2 * k, idesc_t, accum);
               else umma_f8_if(leader, d_tmem + Cfg::kAccCols / 2, adesc2 + 2 * k, bdesc + 2 * k, idesc_t, accum);
@@ -468,6 +489,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint32_t acc_phase = 0;
     uint32_t st_pair = 0;                      // mode 6: staging buffer parity of this warp
     uint32_t epi_count = 0;                    // mode 7: chunks staged so far (buffer = count & 1, barrier phase)
+    if constexpr (Cfg::kScore) pdl_wait();
     for (long long t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
       long long r = t;
       int mt, nt;
@@ -476,6 +498,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const int b = table ? p.tile_group[nt] : static_cast<int>(r);
       const int n_base = table ? p.tile_row0[nt] : nt * BN;
       const int n_lim = table ? p.tile_end[nt] : p.N;
+      // scores: a warp's 32 rows are the heads of one query
+      [[maybe_unused]] const int qrow = mt * (kBM / 32) + quad;
+      [[maybe_unused]] float head_w = 0.f;
+      [[maybe_unused]] int seen = n_lim;
+      if constexpr (Cfg::kScore) {
+        if (32 * qrow < p.M) {
+          head_w = __ldg(p.row_w + 1ll * qrow * p.row_w_ld + lane);
+          if (p.col_limit != nullptr) seen = __ldg(p.col_limit + qrow);
+        }
+        if (hidden(mt, nt)) {
+          float* o = static_cast<float*>(p.out) + b * p.out_batch_stride + 1ll * qrow * p.ldo;
+          if (32 * qrow < p.M)
+            for (int c = n_base + lane + (warp >= 8 ? 32 : 0); c < min(n_lim, n_base + BN); c += 32 * Cfg::kEpiSets) o[c] = -INFINITY;
+          continue;
+        }
+      }
       // per-column metadata (route weight / return address) of the first chunk, fetched while the MMAs still run;
       // every chunk then fetches the next chunk's before it starts its own stores
       constexpr int kChunkPre = BN >= 32 ? 32 : BN;
@@ -527,7 +565,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
           for (int j = 0; j < kChunk; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * alpha);
         }
-        if constexpr (KIND == 0 && !DUAL) {
+        if constexpr (KIND == 0 && FORM == 0) {
           if (p.softcap > 0.f) {
 #pragma unroll
             for (int j = 0; j < kChunk; ++j) v[j] = __float_as_uint(p.softcap * tanhf(__uint_as_float(v[j]) / p.softcap));
@@ -542,7 +580,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (rw_base != nullptr) rw_next = __ldcg(rw_base + n0 + kStep + lane);
           if (p.out_mode == 7) meta_next = __ldcg(p.scatter_meta + n0 + kStep + lane);
         }
-        if (p.out_mode == 0) {
+        if constexpr (Cfg::kScore) {
+          // relu x head weight, then a butterfly that leaves the sum over the heads of column l on lane l (31 shuffles for 32
+          // columns), then one coalesced row store
+          float f[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) f[j] = fmaxf(__uint_as_float(v[j]), 0.f) * head_w;
+#pragma unroll
+          for (int off = 16; off >= 1; off >>= 1) {
+            const bool upper = (lane & off) != 0;
+#pragma unroll
+            for (int i = 0; i < off; ++i) {
+              const float send = upper ? f[i] : f[i + off];
+              const float keep = upper ? f[i + off] : f[i];
+              f[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+            }
+          }
+          if (m < p.M && n0 + lane < n_lim)
+            reinterpret_cast<float*>(p.out)[obase + 1ll * qrow * p.ldo + n0 + lane] = n0 + lane < seen ? f[0] : -INFINITY;
+        } else if (p.out_mode == 0) {
           if (m < p.M) {
             __nv_bfloat16* o = rs_base != nullptr ? reinterpret_cast<__nv_bfloat16*>(rs_base) + rs_row * p.ldo + n0
                                                   : reinterpret_cast<__nv_bfloat16*>(p.out) + obase + 1ll * m * p.ldo + n0;
@@ -595,7 +651,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               if (n0 + j < n_lim) o[1ll * (n0 + j) * p.ldo] = __uint_as_float(v[j]);
           }
         } else if (p.out_mode == 4) {
-          if constexpr (DUAL) {
+          if constexpr (Cfg::kDual) {
             // v = gate chunk; fetch the matching up chunk from the second accumulator half
             uint32_t u[32];
             if constexpr (kChunk == 32) {
@@ -693,30 +749,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               bulk_commit_group();
             }
             ++st_pair;
-          }
-        } else if (p.out_mode == 8) {
-          // One epilogue warp = the 32 heads of one query row.  relu x head weight, then a butterfly that leaves the
-          // sum over heads of column l on lane l (31 shuffles for 32 columns), then one coalesced row store.
-          if constexpr (kChunk == 32) {
-            const int qrow = m >> 5;
-            const float wgt = m < p.M ? __ldg(p.row_w + 1ll * qrow * p.row_w_ld + lane) : 0.f;
-            float f[32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) f[j] = fmaxf(__uint_as_float(v[j]), 0.f) * wgt;
-#pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) {
-              const bool upper = (lane & off) != 0;
-#pragma unroll
-              for (int i = 0; i < off; ++i) {
-                const float send = upper ? f[i] : f[i + off];
-                const float keep = upper ? f[i + off] : f[i];
-                f[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-              }
-            }
-            if (m < p.M && n0 + lane < n_lim) {
-              const int lim = p.col_limit != nullptr ? __ldg(p.col_limit + qrow) : n_lim;
-              reinterpret_cast<float*>(p.out)[obase + 1ll * qrow * p.ldo + n0 + lane] = n0 + lane < lim ? f[0] : -INFINITY;
-            }
           }
         } else if (p.out_mode == 7) {
           // expert-parallel combine: column n is a received token row; its result row goes back to the rank it
@@ -849,20 +881,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   if (warp == 0) tmem_dealloc(tmem_base, Cfg::kTmemCols);
 }
 
-template <int BN, int KIND, int DUAL = 0>
+template <int BN, int KIND, int FORM = 0>
 static cudaError_t launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const StoreMaps& peer,
                                const GemmParams& p, int grid, cudaStream_t stream) {
-  using Cfg = GemmCfg<BN, KIND, DUAL>;
+  using Cfg = GemmCfg<BN, KIND, FORM>;
   static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, KIND, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel<BN, KIND, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
-  return launch_pdl(gemm_tc_kernel<BN, KIND, DUAL>, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tmA, tmB, peer, p);
+  return launch_pdl(gemm_tc_kernel<BN, KIND, FORM>, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, tmA, tmB, peer, p);
 }
 
 template <int KIND>
@@ -881,6 +913,23 @@ static cudaError_t dispatch_bn(int bn, const CUtensorMap& tmA, const CUtensorMap
         return cudaErrorInvalidValue;
       default: return cudaErrorInvalidValue;
     }
+  }
+  if (p.out_mode == 8) {
+    if constexpr (KIND < 3) {
+      switch (bn) {
+        case 32: return launch_gemm<32, KIND, 2>(tmA, tmB, peer, p, grid, stream);
+        case 64: return launch_gemm<64, KIND, 2>(tmA, tmB, peer, p, grid, stream);
+        case 128: return launch_gemm<128, KIND, 2>(tmA, tmB, peer, p, grid, stream);
+        case 192:
+          if constexpr (KIND == 2) return launch_gemm<192, KIND, 2>(tmA, tmB, peer, p, grid, stream);
+          return cudaErrorInvalidValue;
+        case 256:
+          if constexpr (KIND < 2) return launch_gemm<256, KIND, 2>(tmA, tmB, peer, p, grid, stream);
+          return cudaErrorInvalidValue;
+        default: return cudaErrorInvalidValue;
+      }
+    }
+    return cudaErrorInvalidValue;
   }
   switch (bn) {
     case 16: return launch_gemm<16, KIND>(tmA, tmB, peer, p, grid, stream);

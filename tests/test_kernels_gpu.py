@@ -361,6 +361,33 @@ def test_index_scores_on_tensor_cores_match_the_scalar_kernel():
         assert torch.isinf(got[r, nv:n_keys]).all()
 
 
+@pytest.mark.parametrize("bn", [32, 64, 128, 256])
+@pytest.mark.parametrize("rows,n_keys,static", [(1, 70, 0), (5, 257, 2), (70, 1000, 0), (301, 640, 1)])
+def test_index_scores_by_tiles(rows, n_keys, static, bn):
+    """Scores whatever the queries of a tile see: nothing, part of a tile, keys beyond the last one; unordered limits."""
+    from ds41rt_b200.ops import gemm as G, lib
+    IH, ID, ld = 32, 128, 1024
+    torch.manual_seed(rows)
+    q = torch.randn(rows * IH, ID, device="cuda").bfloat16()
+    keys = torch.randn(n_keys, ID, device="cuda").bfloat16()
+    w = torch.randn(rows, IH, device="cuda")
+    limit = torch.randint(0, n_keys + 20, (rows,), device="cuda", dtype=torch.int32)
+    limit[rows // 2:rows // 2 + 9] = 0                     # whole tiles of queries that see nothing
+    for lim in (limit, None):
+        got = torch.full((rows, ld), float("nan"), device="cuda")
+        st = lib.new_status("cuda")
+        G.gemm_raw(q, keys, got, rows * IH, n_keys, ID, lda=ID, ldb=ID, ldo=ld, out_mode=8, bn=bn, row_w=w, row_w_ld=IH,
+                   col_limit=lim, status=st, static_operand=static)
+        torch.cuda.synchronize()
+        lib.raise_on_status(st, "index gemm")
+        qh = q.double().view(rows, IH, ID)
+        want = torch.einsum("rh,rhk->rk", w.double(), (qh @ keys.double().T).relu())
+        bound = torch.einsum("rh,rhk->rk", w.double().abs(), qh.abs() @ keys.double().abs().T) * (ID + IH + 2) * 2.0 ** -23
+        sees = torch.arange(n_keys, device="cuda")[None] < (lim if lim is not None else limit.new_full((rows,), n_keys))[:, None]
+        assert torch.isneginf(got[:, :n_keys][~sees]).all() and got[:, n_keys:].isnan().all()
+        assert ((got[:, :n_keys].double() - want).abs() <= bound)[sees].all()
+
+
 def test_fp4_index_keys_and_queries_follow_the_quantisation_oracle():
     """Index keys stored as FP4 rows (E2M1 pairs + UE8M0 per 32 values, 68 bytes for 128 values): the per-key kernel and
     the tensor-core path both score the dequantised keys against queries quantised the same way; the per-key kernel
