@@ -175,10 +175,59 @@ __device__ __forceinline__ float4 routed_at4(const ds41_resid_args& p, int r, in
   return s;
 }
 
-// Many rows: bound by latency, a block's loads and its two chains of merges one after the other (ncu: 45 % of issue slots and
-// 22 % of the memory's rate; more threads or more rows an SM made it slower), so rows that fill the threads' pieces (FULL) shorten
-// the chain by every test of a column against the row's end.  2048 rows x 4096 columns: 75 -> 57 us on average in a model with
-// kept streams, 49 -> 39 without; 953 rows 28 -> 22.
+// A thread's pieces of a row of a projection, all under way together: which form it has is asked once, not piece by piece, since a
+// test between two loads makes the second one wait for what the first one's value is used for.
+template <int NI>
+__device__ __forceinline__ void proj_pieces(const ds41_proj& a, long long row, const int (&at)[NI], float4 (&v)[NI]) {
+  const long long i0 = row * a.ld + a.col;
+  if (a.bf16) {
+    uint2 raw[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) raw[i] = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(a.data) + i0 + at[i]);
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      v[i] = make_float4(__uint_as_float(raw[i].x << 16), __uint_as_float(raw[i].x & 0xffff0000u), __uint_as_float(raw[i].y << 16),
+                         __uint_as_float(raw[i].y & 0xffff0000u));
+  } else if (a.splits == 1) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) v[i] = *reinterpret_cast<const float4*>(static_cast<const float*>(a.data) + i0 + at[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) v[i] = proj_at4(a, row, at[i]);
+  }
+}
+// The same of the sum of a row's routed results (bf16 rows, one per route, at most four routes), in route order.
+constexpr int kRoutes = 4;
+template <int NI>
+__device__ __forceinline__ void routed_pieces(const ds41_resid_args& p, int r, const int (&at)[NI], float4 (&v)[NI]) {
+  bool on[kRoutes];
+  uint2 raw[kRoutes][NI];
+#pragma unroll
+  for (int k = 0; k < kRoutes; ++k) on[k] = k < p.y_top && p.y_route[r * p.y_top + k] >= 0;
+#pragma unroll
+  for (int k = 0; k < kRoutes; ++k) {
+    const __nv_bfloat16* row = static_cast<const __nv_bfloat16*>(p.y.data) + (1ll * r * p.y_top + k) * p.y.ld + p.y.col;
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+      if (k < p.y_top) raw[k][i] = *reinterpret_cast<const uint2*>(row + at[i]);       // a dropped route's row is there too
+  }
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < kRoutes; ++k)
+      if (on[k])
+        v[i] += make_float4(__uint_as_float(raw[k][i].x << 16), __uint_as_float(raw[k][i].x & 0xffff0000u),
+                            __uint_as_float(raw[k][i].y << 16), __uint_as_float(raw[k][i].y & 0xffff0000u));
+  }
+}
+
+// Many rows: bound by latency, a block's loads and its two chains of merges one after the other.  Rows that fill the threads'
+// pieces (FULL) shorten the chain by every test of a column against the row's end, and ask for stream, result and gate at once.
+// Piece by piece, with a test of the projection's form between two loads, 2048 rows x 4096 columns took 28 us (plain result), 49
+// (gated, two norms), 73 (the same with four kept streams) and 54 (four routes); together 26, 44, 70 and 26; 953 rows with routes
+// 30 and 16.  Kept streams stay behind the first norm: asked for with the rest they cost the registers of a third block an SM
+// (kept streams 82 us).
 template <typename T, int NI, bool FULL>
 __global__ void __launch_bounds__(NI <= 4 ? 256 : 512) resid_step_kernel(ds41_resid_args p) {
   __shared__ float slots[2][96];
@@ -214,19 +263,35 @@ __global__ void __launch_bounds__(NI <= 4 ? 256 : 512) resid_step_kernel(ds41_re
   };
   if (p.y.data != nullptr) {
     float4 y[NI];
+    auto gated = [&](float4& v, const float4& g, const float4& b) {
+      v.x *= sigmoid_f32(g.x + b.x);
+      v.y *= sigmoid_f32(g.y + b.y);
+      v.z *= sigmoid_f32(g.z + b.z);
+      v.w *= sigmoid_f32(g.w + b.w);
+    };
+    bool whole = false;
+    if constexpr (FULL) {
+      const bool routed = p.y_route != nullptr;
+      whole = !routed || (p.y.bf16 && p.y_rows == 0 && p.y_top <= kRoutes);
+      if (whole) {
+        if (routed) routed_pieces(p, r, at, y);
+        else proj_pieces(p.y, r, at, y);
+        float4 g[NI];
+        if (p.gate.data != nullptr) proj_pieces(p.gate, r, at, g);
+        if (p.gate.data != nullptr)
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (live[i] > 0) {
-        y[i] = p.y_route != nullptr ? routed_at4(p, r, at[i]) : proj_at4(p.y, r, at[i]);
-        if (p.gate.data != nullptr) {
-          const float4 g = proj_at4(p.gate, r, at[i]), b = load4(p.gate_bias + at[i], live[i]);
-          y[i].x *= sigmoid_f32(g.x + b.x);
-          y[i].y *= sigmoid_f32(g.y + b.y);
-          y[i].z *= sigmoid_f32(g.z + b.z);
-          y[i].w *= sigmoid_f32(g.w + b.w);
+          for (int i = 0; i < NI; ++i) gated(y[i], g[i], load4(p.gate_bias + at[i], 4));
+      }
+    }
+    if (!whole) {
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (live[i] > 0) {
+          y[i] = p.y_route != nullptr ? routed_at4(p, r, at[i]) : proj_at4(p.y, r, at[i]);
+          if (p.gate.data != nullptr) gated(y[i], proj_at4(p.gate, r, at[i]), load4(p.gate_bias + at[i], live[i]));
+          clip(y[i], i);
         }
-        clip(y[i], i);
       }
     }
     float2 s = make_float2(0.f, 1.f);

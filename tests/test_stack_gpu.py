@@ -401,6 +401,43 @@ def test_residual_step_of_few_rows(rows, W, planes, n_mix, top, kind):
     torch.testing.assert_close(h[:, :W].cpu().double(), norm(avg, nw.double(), eps), rtol=2e-5, atol=5e-5)
 
 
+@pytest.mark.parametrize("W", [1024, 4096, 8192, 4000])
+@pytest.mark.parametrize("form,top,gate", [("f32", 0, "bf16"), ("f32", 0, "f32"), ("bf16", 0, None), ("bf16", 1, None), ("bf16", 4, "bf16"),
+                                           ("bf16", 5, None), ("f32", 3, None)])
+def test_residual_step_of_many_rows_by_form(W, form, top, gate):
+    """Results and gates in every form that a long pass has, with and without whole pieces; a dropped route's row holds anything."""
+    lib, S, k = _stack()
+    g, rows, eps = gen(W + top), 35, 1e-5
+    r = lambda *s: torch.randn(*s, generator=g)
+    dt = BF16 if form == "bf16" else torch.float32
+    x, pw, nw, b = r(rows, W), r(W), r(W), r(W)
+    a = S.ResidArgs()
+    if top:
+        y, route = r(rows * top, W).to(dt), torch.randint(-1, 3, (rows, top), generator=g)
+        y[(route < 0).flatten()] = float("nan")
+        Y, R = y.cuda(), route.int().cuda()
+        a.y, a.y_route, a.y_top = S.Proj(Y, W).args(), lib.ptr(R), top
+        sub = torch.where(route[..., None] >= 0, y.double().view(rows, top, W), 0.0).sum(1)
+    else:
+        y = r(rows, W).to(dt)
+        Y = y.cuda()
+        a.y, sub = S.Proj(Y, W).args(), y.double()
+    a.gate = S.NO_PROJ
+    if gate:
+        gt = r(rows, W).to(BF16 if gate == "bf16" else torch.float32)
+        GT, B = gt.cuda(), b.cuda()
+        a.gate, a.gate_bias = S.Proj(GT, W).args(), lib.ptr(B)
+        sub = sub * torch.sigmoid(gt.double() + b.double())
+    full = x.double() + rms_unit(sub, eps) * pw.double()
+    X, PW, NW, out, h = x.cuda(), pw.cuda(), nw.cuda(), torch.zeros(rows, W).cuda(), torch.zeros(rows, W, dtype=BF16).cuda()
+    a.post_w, a.next_w, a.x_in, a.x_out = (lib.ptr(t) for t in (PW, NW, X, out))
+    a.h, a.ldh, a.ldx, a.rows, a.W, a.norm_kind, a.eps = lib.ptr(h), W, W, rows, W, 1, eps
+    _ok(k.ds41_resid_step(C.byref(a), lib.stream()))
+    # sums of five 32-bit terms; the last step is one rounding to bf16
+    torch.testing.assert_close(out.cpu().double(), full, rtol=2e-5, atol=2e-5)
+    torch.testing.assert_close(h.cpu().double(), rms_unit(full, eps) * nw.double(), rtol=2.0 ** -8, atol=1e-4)
+
+
 def norm_in_order(x, kind, eps):
     """Mean and factor of every row as one block of the residual step sums them, in 32 bits: a thread's own moments, then the
     lower half of the threads with the upper one, over a warp and over the warps."""
