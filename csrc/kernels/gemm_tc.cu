@@ -146,8 +146,14 @@ struct GemmCfg {
   // 2304: 2445 us with one set, 2198 with two.
   // So do they with indexer scores, whose two K steps take a tenth of their epilogue's time.
   static constexpr int kEpiSets = (kDual && kAccStages == 1) || kScore ? 2 : 1;
+  // They empty it before they compute: a warp's chunks of (gate, up), rounded to bf16 as the product takes them, go into registers,
+  // a third one into shared memory.  With a chunk computed and stored before the next was read the FC1 above took 2100 us, 1865 so.
+  static constexpr bool kDrain = kDual && kAccStages == 1 && BN >= 64;
+  static constexpr int kDrainChunks = kDrain ? BN / 64 : 0;                            // chunks of 32 columns a warp holds
+  static constexpr int kDrainBytes = kDrainChunks > 2 ? 8 * (kDrainChunks - 2) * 4096 : 0;
+  static_assert(kDrainChunks <= 3, "chunks of a tile that is emptied first");
   static constexpr int kThreads = kGemmThreads + 128 * (kEpiSets - 1) + (kScaled ? 32 : 0);    // + the second producer
-  static constexpr int kSmemBytes = kStages * kStageBytes + kStaging + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int kSmemBytes = kStages * kStageBytes + kStaging + kDrainBytes + 1024 /*align*/ + 256 /*barriers*/;
   static_assert(kTmemNeeded <= 512, "TMEM budget exceeded");
   static_assert(!kScore || BN >= 32, "a chunk of scores has 32 columns");
   static_assert(kStages >= 2, "not enough shared memory for two stages");
@@ -181,7 +187,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
   uint8_t* staging = smem + S * Cfg::kStageBytes;
-  uint8_t* bar_base = staging + Cfg::kStaging;
+  uint8_t* drain = staging + Cfg::kStaging;
+  uint8_t* bar_base = drain + Cfg::kDrainBytes;
   uint64_t* full = reinterpret_cast<uint64_t*>(bar_base);
   uint64_t* empty = full + S;
   uint64_t* acc_full = empty + S;
@@ -544,6 +551,58 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (KIND == 3 && p.alpha_batch != nullptr) alpha *= __ldg(p.alpha_batch + (p.batch_map != nullptr ? p.batch_map[b] : b));
       // columns the tensor cores wrote for this tile (see n_mma in the issuer), in whole chunks
       const int n_cols = (table && p.out_mode != 6) ? min(BN, (max(n_lim - n_base, 0) + kChunk - 1) / kChunk * kChunk) : BN;
+      if constexpr (Cfg::kDrain) {
+        if (p.out_mode == 4 && p.act_alpha == 0.f) {
+          uint32_t held[2][32];                // (gate, up) pairs of the warp's first two chunks
+          uint32_t* third = reinterpret_cast<uint32_t*>(drain) + (quad + (warp >= 8 ? 4 : 0)) * 1024 + lane;
+          float rw[Cfg::kDrainChunks];
+#pragma unroll
+          for (int i = 0; i < Cfg::kDrainChunks; ++i) {
+            const int c = c_first + kStep * i;
+            rw[i] = i == 0 ? rw_next : 0.f;
+            if (c >= n_cols) continue;
+            if (i > 0 && n_base + c + lane < n_lim) rw[i] = __ldcg(rw_base + n_base + c + lane);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              uint32_t g[16], u[16];
+              tmem_ld_32x16(t_row + c + 16 * half, g);
+              tmem_ld_32x16(t_row + Cfg::kAccCols / 2 + c + 16 * half, u);
+              tmem_wait_ld();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const float a = KIND == 3 ? alpha : 1.f;
+                const __nv_bfloat162 pair = KIND == 3 ? __floats2bfloat162_rn(__uint_as_float(g[j]) * a, __uint_as_float(u[j]) * a)
+                                                      : __floats2bfloat162_rn(__uint_as_float(g[j]), __uint_as_float(u[j]));
+                const uint32_t bits = *reinterpret_cast<const uint32_t*>(&pair);
+                if (i < 2) held[i & 1][16 * half + j] = bits;
+                else third[(16 * half + j) * 32] = bits;
+              }
+            }
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[acc]);
+          acc = (acc + 1 == Cfg::kAccStages) ? 0 : acc + 1;
+          if (acc == 0) acc_phase ^= 1;
+          __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + obase + m;
+#pragma unroll
+          for (int i = 0; i < Cfg::kDrainChunks; ++i) {
+            const int n0 = n_base + c_first + kStep * i;
+            if (c_first + kStep * i >= n_cols) continue;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float rwj = __shfl_sync(0xffffffffu, rw[i], j);
+              const uint32_t bits = i < 2 ? held[i & 1][j] : third[j * 32];
+              if (m < p.M && n0 + j < n_lim) {
+                const float gte = fminf(__uint_as_float(bits << 16), p.act_limit);
+                const float upv = fminf(fmaxf(__uint_as_float(bits & 0xffff0000u), -p.act_limit), p.act_limit);
+                o[1ll * (n0 + j) * p.ldo] = __float2bfloat16_rn(gte / (1.0f + __expf(-gte)) * upv * rwj);
+              }
+            }
+          }
+          continue;
+        }
+      }
 #pragma unroll 1
       for (int c = c_first; c < n_cols; c += kStep) {
         uint32_t v[32];
