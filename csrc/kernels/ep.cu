@@ -58,6 +58,18 @@ struct EpParams {
 
 constexpr int kEpOverflow = 7;   // status code: received rows exceed the receive buffer
 
+// What a block wrote for the peers, and then its flag; a lone rank's next kernel waits for this one and needs neither.
+__device__ __forceinline__ void publish(const EpParams& p, uint32_t* flag, uint32_t epoch) {
+  if (p.world > 1) __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (p.world > 1) flag_store_release(flag, epoch);
+    else *flag = epoch;
+  }
+}
+
+// One block, bound by the round trips of its threads' loads: eight ids are under way at once (one after the other, and with fences for
+// peers that a lone rank does not have, 8192 tokens x 6 routes took 31 us and 2048 x 4 ten: now 10.6 and 4).
 __global__ void __launch_bounds__(1024) ep_count_kernel(EpParams p) {
   extern __shared__ int hist[];
   pdl_launch_dependents();
@@ -66,9 +78,17 @@ __global__ void __launch_bounds__(1024) ep_count_kernel(EpParams p) {
   for (int i = threadIdx.x; i < E; i += blockDim.x) hist[i] = 0;
   __syncthreads();
   const int n = p.tokens * p.topk;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const int id = p.ids[i];
-    if (id >= 0 && id < E) atomicAdd(&hist[id], 1);
+  constexpr int kIds = 8;
+  for (int i0 = threadIdx.x; i0 < n; i0 += kIds * blockDim.x) {
+    int id[kIds];
+#pragma unroll
+    for (int u = 0; u < kIds; ++u) {
+      const int i = i0 + u * static_cast<int>(blockDim.x);
+      id[u] = i < n ? p.ids[i] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kIds; ++u)
+      if (id[u] >= 0 && id[u] < E) atomicAdd(&hist[id[u]], 1);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < E; i += blockDim.x) {
@@ -76,15 +96,13 @@ __global__ void __launch_bounds__(1024) ep_count_kernel(EpParams p) {
     p.counts[dst][p.rank * p.e_local + (i - dst * p.e_local)] = hist[i];
     p.cursor[i] = 0;
   }
-  __threadfence_system();
-  __syncthreads();
+  uint32_t e = 0;
   if (threadIdx.x == 0) {
     *p.ticket = 0;
-    const uint32_t e = *p.epoch + 1;
+    e = *p.epoch + 1;
     *p.epoch = e;
-    __threadfence_system();
-    flag_store_release(p.flags[p.rank] + 0, e);
   }
+  publish(p, p.flags[p.rank] + 0, e);
 }
 
 __global__ void __launch_bounds__(256) ep_plan_kernel(EpParams p) {
@@ -202,9 +220,7 @@ __global__ void __launch_bounds__(256) ep_plan_kernel(EpParams p) {
     for (int s = 0; s < src; ++s) base += __ldcg(counts + s * p.e_local + e);
     p.send_base[src][p.rank * p.e_local + e] = s_ok ? base : -1;
   }
-  __threadfence_system();
-  __syncthreads();
-  if (threadIdx.x == 0) flag_store_release(p.flags[p.rank] + 1, epoch);
+  publish(p, p.flags[p.rank] + 1, epoch);
 }
 
 __global__ void __launch_bounds__(256) ep_dispatch_kernel(EpParams p) {
@@ -298,6 +314,10 @@ __global__ void __launch_bounds__(256) ep_dispatch_kernel(EpParams p) {
       p.recv_meta[dst][row] = make_int2(p.rank, i);
       p.recv_w[dst][row] = p.weights[i];
     }
+  }
+  if (p.world == 1) {                    // the kernel that follows waits for this one
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.flags[p.rank][2] = epoch;
+    return;
   }
   __threadfence_system();
   __syncthreads();

@@ -1500,7 +1500,7 @@ class DS41Engine(RowsEngine):
             ep.set_weights(lw.w13, lw.w2, getattr(lw, "w13_sf", None), getattr(lw, "w2_sf", None),
                            getattr(lw, "w13_gs", None), getattr(lw, "w2_gs", None))
             if self.only is None or "ep_moe" in self.only:
-                self.launches += 7
+                self.launches += 7 if self.world > 1 else 6
                 self._run("ep_moe", ep.forward, xn, self.ids[lo:lo + Rl], self.route_w[lo:lo + Rl], moe_rows, moe_rows)
             pending = (moe_rows.data_ptr(), 1, 0)
             if self.layer_timer is not None:
@@ -1566,7 +1566,7 @@ class DS41Engine(RowsEngine):
         ep.set_weights(lw.w13, lw.w2, getattr(lw, "w13_sf", None), getattr(lw, "w2_sf", None),
                        getattr(lw, "w13_gs", None), getattr(lw, "w2_gs", None))
         if self.only is None or "ep_moe" in self.only:
-            self.launches += 7
+            self.launches += 7 if self.world > 1 else 6
             self._run("ep_moe", ep.forward, self.xn[lo:hi], self.ids[lo:hi], self.route_w[lo:hi], self.moe_plane[lo:hi],
                       self.moe_plane[lo:hi])
 

@@ -288,7 +288,8 @@ class ExpertParallelMoE:
         if out is None:
             assert self.f.world == 1
             return None
-        lib.check(k.ds41_ep_mark(C.byref(a), 3, st()), "ep_mark")
+        if self.f.world > 1:            # a lone rank's combine waits for the kernel before it
+            lib.check(k.ds41_ep_mark(C.byref(a), 3, st()), "ep_mark")
         lib.check(k.ds41_ep_combine(C.byref(a), lib.ptr(self.comb), lib.ptr(extra),
                                     C.c_longlong(extra.stride(0) if extra is not None else 0), lib.ptr(out),
                                     1 if out.dtype == torch.bfloat16 else 0, st()), "ep_combine")
