@@ -14,6 +14,7 @@
 #include "ds41_launch.cuh"
 #include "ds41_mma.cuh"
 #include "ds41_ptx.cuh"
+#include "ds41_tma.h"
 
 namespace ds41 {
 
@@ -230,8 +231,9 @@ __device__ __forceinline__ void radix_pick(const int* hist, int need, uint32_t p
   *s_need = need - cum;
 }
 
-// exclusive scan over 1024 threads; returns this thread's exclusive prefix, *total gets the block sum
-__device__ __forceinline__ int block_excl_scan_1024(int v, int* warp_tot /*[32]*/, int* total) {
+// exclusive scan over T threads; returns this thread's exclusive prefix, *total gets the block sum
+template <int T>
+__device__ __forceinline__ int block_excl_scan(int v, int* warp_tot /*[32]*/, int* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int incl = v;
 #pragma unroll
@@ -243,29 +245,29 @@ __device__ __forceinline__ int block_excl_scan_1024(int v, int* warp_tot /*[32]*
   if (lane == 31) warp_tot[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    int t = warp_tot[lane];
+    int t = lane < T / 32 ? warp_tot[lane] : 0;
     int ti = t;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int n = __shfl_up_sync(0xffffffffu, ti, o);
       if (lane >= o) ti += n;
     }
-    warp_tot[lane] = ti - t;   // exclusive warp offsets
+    if (lane < T / 32) warp_tot[lane] = ti - t;   // exclusive warp offsets
     if (lane == 31) *total = ti;
   }
   __syncthreads();
   return warp_tot[warp] + incl - v;
 }
 
-// Exact top-k of one row by a block of 1024 threads.  key(i) is the order-preserving 32-bit key of element i, 0 for an
+// Exact top-k of one row by a block of T threads.  key(i) is the order-preserving 32-bit key of element i, 0 for an
 // element that must never be chosen.  Writes the chosen ids in ascending order (-1 padded) and their count.  With at most
 // k eligible elements all of them are chosen; otherwise a 4-pass radix select finds the k-th largest key and ties on it
 // go to the lowest ids.
-// Rows of at most 1024 * M elements: every thread keeps its M consecutive keys in registers, so the scores are read
+// Rows of at most T * M elements: every thread keeps its M consecutive keys in registers, so the scores are read
 // once, the four radix passes build their histograms from registers, and the ordered compaction needs two block scans
 // in all (one block scan per 1024 elements and six reads of the row made the streaming form below take 30-43 us for 2 K
 // to 16 K keys).
-template <int M, class Key>
+template <int T, int M, class Key>
 __device__ void select_topk_row_reg(Key key, int n, int k, int* out, int* n_out) {
   __shared__ int hist[256];
   __shared__ int warp_tot[32];
@@ -287,7 +289,7 @@ __device__ void select_topk_row_reg(Key key, int n, int k, int* out, int* n_out)
   if (mine) atomicAdd(&s_valid, mine);
   __syncthreads();
   const int valid = s_valid;
-  for (int i = valid + tid; i < k; i += 1024) out[i] = -1;
+  for (int i = valid + tid; i < k; i += T) out[i] = -1;
   uint32_t thr = 0;
   int need = 0;
   if (valid > k) {
@@ -314,7 +316,7 @@ __device__ void select_topk_row_reg(Key key, int n, int k, int* out, int* n_out)
   int n_eq = 0;
 #pragma unroll
   for (int j = 0; j < M; ++j) n_eq += (u[j] != 0u && u[j] == thr) ? 1 : 0;
-  int eq_rank = block_excl_scan_1024(n_eq, warp_tot, &s_total);
+  int eq_rank = block_excl_scan<T>(n_eq, warp_tot, &s_total);
   __syncthreads();
   int n_keep = 0;
   uint32_t keep_bits = 0;
@@ -326,7 +328,7 @@ __device__ void select_topk_row_reg(Key key, int n, int k, int* out, int* n_out)
     keep_bits |= keep ? (1u << j) : 0u;
     n_keep += keep ? 1 : 0;
   }
-  int at = block_excl_scan_1024(n_keep, warp_tot, &s_total);
+  int at = block_excl_scan<T>(n_keep, warp_tot, &s_total);
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < M; ++j)
@@ -337,7 +339,7 @@ __device__ void select_topk_row_reg(Key key, int n, int k, int* out, int* n_out)
   if (tid == 0) *n_out = min(s_total, k);
 }
 
-template <class Key>
+template <int T, class Key>
 __device__ void select_topk_row_stream(Key key, int n, int k, int* out, int* n_out) {
   __shared__ int hist[256];
   __shared__ int warp_tot[32];
@@ -349,11 +351,11 @@ __device__ void select_topk_row_stream(Key key, int n, int k, int* out, int* n_o
   if (tid == 0) s_valid = 0;
   __syncthreads();
   int mine = 0;
-  for (int i = tid; i < n; i += 1024) mine += key(i) != 0u;
+  for (int i = tid; i < n; i += T) mine += key(i) != 0u;
   if (mine) atomicAdd(&s_valid, mine);
   __syncthreads();
   const int valid = s_valid;
-  for (int i = valid + tid; i < k; i += 1024) out[i] = -1;
+  for (int i = valid + tid; i < k; i += T) out[i] = -1;
   uint32_t thr = 0;
   int need = 0;
   if (valid > k) {
@@ -363,7 +365,7 @@ __device__ void select_topk_row_stream(Key key, int n, int k, int* out, int* n_o
       const int shift = 24 - 8 * pass;
       if (tid < 256) hist[tid] = 0;
       __syncthreads();
-      for (int i = tid; i < n; i += 1024) {
+      for (int i = tid; i < n; i += T) {
         const uint32_t u = key(i);
         if (u != 0u && (u & mask) == prefix) atomicAdd(&hist[(u >> shift) & 255], 1);
       }
@@ -379,17 +381,17 @@ __device__ void select_topk_row_stream(Key key, int n, int k, int* out, int* n_o
   }
   // ---- ordered compaction (ascending id): keep key > thr, and the first `need` keys == thr
   int base = 0, eq_base = 0;
-  for (int c0 = 0; c0 < n; c0 += 1024) {
+  for (int c0 = 0; c0 < n; c0 += T) {
     const int i = c0 + tid;
     uint32_t u = 0;
     if (i < n) u = key(i);
     const int is_eq = (i < n && u != 0u && u == thr) ? 1 : 0;
     int eq_total;
-    const int eq_rank = eq_base + block_excl_scan_1024(is_eq, warp_tot, &s_total);
+    const int eq_rank = eq_base + block_excl_scan<T>(is_eq, warp_tot, &s_total);
     __syncthreads();
     eq_total = s_total;
     const int keep = (i < n && u != 0u && (u > thr || (is_eq && eq_rank < need))) ? 1 : 0;
-    const int at = base + block_excl_scan_1024(keep, warp_tot, &s_total);
+    const int at = base + block_excl_scan<T>(keep, warp_tot, &s_total);
     __syncthreads();
     if (keep && at < k) out[at] = i;
     base += s_total;
@@ -399,13 +401,24 @@ __device__ void select_topk_row_stream(Key key, int n, int k, int* out, int* n_o
   if (tid == 0) *n_out = min(base, k);
 }
 
-template <class Key>
+// Threads per row.  Many rows are bound by the barriers of their passes, so that what counts is the rows an SM has at a time: two of
+// 1024 threads, five of 256.  Few rows are better off with more threads each.  8192 rows of up to 4096 keys, 512 chosen: 307 us
+// with 1024, 153 with 256.
+constexpr int kRowThreads = 256, kRowKeys = 32 * kRowThreads;        // the most keys that those hold
+template <int T, class Key>
 __device__ void select_topk_row(Key key, int n, int k, int* out, int* n_out) {
-  if (n <= 4 * 1024) select_topk_row_reg<4>(key, n, k, out, n_out);
-  else if (n <= 8 * 1024) select_topk_row_reg<8>(key, n, k, out, n_out);
-  else if (n <= 16 * 1024) select_topk_row_reg<16>(key, n, k, out, n_out);
-  else if (n <= 24 * 1024) select_topk_row_reg<24>(key, n, k, out, n_out);
-  else select_topk_row_stream(key, n, k, out, n_out);
+  if constexpr (T == 1024) {
+    if (n <= 4 * T) select_topk_row_reg<T, 4>(key, n, k, out, n_out);
+    else if (n <= 8 * T) select_topk_row_reg<T, 8>(key, n, k, out, n_out);
+    else if (n <= 16 * T) select_topk_row_reg<T, 16>(key, n, k, out, n_out);
+    else if (n <= 24 * T) select_topk_row_reg<T, 24>(key, n, k, out, n_out);
+    else select_topk_row_stream<T>(key, n, k, out, n_out);
+  } else {
+    if (n <= 8 * T) select_topk_row_reg<T, 8>(key, n, k, out, n_out);
+    else if (n <= 16 * T) select_topk_row_reg<T, 16>(key, n, k, out, n_out);
+    else if (n <= 32 * T) select_topk_row_reg<T, 32>(key, n, k, out, n_out);
+    else select_topk_row_stream<T>(key, n, k, out, n_out);        // positions beyond the context
+  }
 }
 
 struct TopkParams {
@@ -420,27 +433,28 @@ struct TopkParams {
   int cand_words, cand_block;
 };
 
-__global__ void __launch_bounds__(1024) topk_select_kernel(TopkParams p) {
+template <int T>
+__global__ void __launch_bounds__(T) topk_select_kernel(TopkParams p) {
   const int r = blockIdx.x, tid = threadIdx.x;
   pdl_launch_dependents();
   pdl_wait();
   const int pos = p.row_pos[r];
   int* out = p.sel + 1ll * r * p.k;
   if (p.row_slot[r] < 0) {
-    for (int i = tid; i < p.k; i += 1024) out[i] = -1;
+    for (int i = tid; i < p.k; i += T) out[i] = -1;
     if (tid == 0) p.n_sel[r] = 0;
     return;
   }
   const int n = min((pos + 1) / p.ratio, p.max_keys);
   if (n <= p.k && p.cand_mask == nullptr) {
-    for (int i = tid; i < p.k; i += 1024) out[i] = i < n ? i : -1;
+    for (int i = tid; i < p.k; i += T) out[i] = i < n ? i : -1;
     if (tid == 0) p.n_sel[r] = n;
     return;
   }
   const float* sc = p.scores + 1ll * r * p.max_keys;
   const uint32_t* cm = p.cand_mask;
   const int words = p.cand_words, blk = p.cand_block;
-  select_topk_row(
+  select_topk_row<T>(
       [=](int i) -> uint32_t {
         if (!cand_allowed(cm, words, blk, r, i)) return 0u;
         const uint32_t u = orderable(sc[i]);
@@ -480,7 +494,7 @@ __global__ void __launch_bounds__(1024) candidate_select_kernel(CandParams p) {
   }
   const float* sc = p.scores + 1ll * r * p.max_keys;
   const int B = p.block, newest = (n_vis - 1) / B;
-  select_topk_row(
+  select_topk_row<1024>(
       [=](int b) -> uint32_t {
         if (b == newest) return 0xFFFFFFFFu;
         float m = -INFINITY;
@@ -1228,7 +1242,10 @@ extern "C" int ds41_topk_select_cand(const float* scores, int max_keys, const in
   if (cand_mask != nullptr && (cand_words <= 0 || cand_block <= 0)) return cudaErrorInvalidValue;
   TopkParams p{scores, max_keys, row_pos, row_slot, ratio, k, sel, n_sel,
                static_cast<const uint32_t*>(cand_mask), cand_words, cand_block};
-  return launch_pdl(topk_select_kernel, dim3(rows), dim3(1024), 0, static_cast<cudaStream_t>(stream), p);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (rows > 2 * sm_count() && ratio > 0 && max_keys / ratio <= kRowKeys)
+    return launch_pdl(topk_select_kernel<kRowThreads>, dim3(rows), dim3(kRowThreads), 0, st, p);
+  return launch_pdl(topk_select_kernel<1024>, dim3(rows), dim3(1024), 0, st, p);
 }
 
 extern "C" int ds41_topk_select(const float* scores, int max_keys, const int* row_pos, const int* row_slot,

@@ -38,6 +38,36 @@ def test_topk_select_exact(max_keys, positions):
     assert int(n_sel[3]) == 0
 
 
+@pytest.mark.parametrize("masked", [False, True])
+@pytest.mark.parametrize("max_keys,ratio", [(513, 1), (2048, 1), (2049, 1), (4097, 1), (8192, 1), (16000, 2)])
+def test_topk_of_many_rows(max_keys, ratio, masked):
+    """Passes of many rows choose what passes of few rows choose (which the test above compares with a sort)."""
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    rows, topk, block = 400, 512, 8
+    torch.manual_seed(max_keys)
+    scores = torch.randn(rows, max_keys, device="cuda")
+    scores[::3] = scores[::3].round()                      # many ties
+    scores[1] = float("-inf")
+    scores[2, ::2] = float("inf")
+    pos = torch.randint(0, ratio * max_keys + 5, (rows,), device="cuda", dtype=torch.int32)
+    pos[3:6] = torch.tensor([ratio * max_keys - 1, 511, 512], dtype=torch.int32)
+    slot = torch.where(torch.arange(rows, device="cuda") % 50 == 7, -1, 0).int()
+    words = (max_keys + 32 * block - 1) // (32 * block)
+    mask = torch.randint(-2 ** 31, 2 ** 31, (rows, words), device="cuda", dtype=torch.int64).int()
+    got = []
+    for step in (rows, 100):
+        sel, n_sel = torch.zeros(rows, topk, dtype=torch.int32, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda")
+        for r in range(0, rows, step):
+            lib.check(k.ds41_topk_select_cand(lib.ptr(scores[r:]), max_keys, lib.ptr(pos[r:]), lib.ptr(slot[r:]), ratio, topk,
+                                              lib.ptr(sel[r:]), lib.ptr(n_sel[r:]), step, lib.ptr(mask[r:]) if masked else None,
+                                              words if masked else 0, block if masked else 0, lib.stream()), "topk")
+        torch.cuda.synchronize()
+        got.append((sel, n_sel))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert masked or int(got[0][1].max()) == topk          # a mask of random bits leaves half of the keys
+
+
 def _attend_ref(q, keys, sink, scale):
     # q [H, D], keys [n, D]
     logits = (q @ keys.t()) * scale
