@@ -253,21 +253,37 @@ __global__ void __launch_bounds__(512) moe_plan_kernel(PlanParams p) {
   }
 }
 
-// one warp per row, lane l holds the logits of experts l, l + 32, ...; lane k keeps the k-th choice
+// one warp per row, lane l holds the logits of experts l, l + 32, ... (kMine of them); lane k keeps the k-th choice.
+// A block that has all rows (a decode step of up to eight) is a chain of round trips to L2 and of the choices' shuffles: the bias is
+// read before the wait, the plan takes the routes from shared memory, and lanes hold no more logits than there are experts.  8 rows,
+// 32 experts, 4 chosen, what the launch adds to a step in a graph: 8.2 us with sixteen logits a lane and the routes read
+// back twice, 2.4 so.
 constexpr int kRouteThreads = 256;
 constexpr int kRouteMax = 512;           // experts
+template <int kMine>
 __global__ void __launch_bounds__(kRouteThreads) route_softmax_kernel(ds41_route_args p) {
+  constexpr int kRows = kRouteThreads / 32;
+  __shared__ int chosen[kRows * 32];               // [row of the block][top]: routes of a block that has all rows
+  __shared__ float chosen_w[kRows * 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_launch_dependents();
+  float bias[kMine];
+#pragma unroll
+  for (int i = 0; i < kMine; ++i) {
+    const int e = lane + 32 * i;
+    bias[i] = p.bias != nullptr && e < p.experts ? p.bias[e] : 0.f;
+  }
   pdl_wait();
-  const int r = blockIdx.x * (kRouteThreads / 32) + warp;
+  const bool alone = gridDim.x == 1;
+  if (alone && p.active != nullptr)
+    for (int i = tid; i < p.max_active * p.row_w_ld; i += kRouteThreads) p.row_w[i] = 0.f;
+  const int r = blockIdx.x * kRows + warp;
   if (r < p.rows) {
-    constexpr int kMine = kRouteMax / 32;
     float z[kMine];
 #pragma unroll
     for (int i = 0; i < kMine; ++i) {
       const int e = lane + 32 * i;
-      z[i] = e < p.experts ? few_at(p.z, r, e) + (p.bias != nullptr ? p.bias[e] : 0.f) : -INFINITY;
+      z[i] = e < p.experts ? few_at(p.z, r, e) + bias[i] : -INFINITY;
     }
     float my_z = -INFINITY, best = -INFINITY;
     int my_id = -1;
@@ -300,8 +316,9 @@ __global__ void __launch_bounds__(kRouteThreads) route_softmax_kernel(ds41_route
     const float e = lane < p.top && my_id >= 0 ? expf(my_z - best) : 0.f;
     const float w = e / warp_sum(e);
     if (lane < p.top) {
-      p.ids[r * p.top + lane] = p.row_slot[r] >= 0 ? my_id : -1;
-      p.weights[r * p.top + lane] = w;
+      const int id = p.row_slot[r] >= 0 ? my_id : -1;
+      p.ids[r * p.top + lane] = chosen[warp * p.top + lane] = id;
+      p.weights[r * p.top + lane] = chosen_w[warp * p.top + lane] = w;
     }
   }
   if (p.active == nullptr) return;
@@ -310,20 +327,26 @@ __global__ void __launch_bounds__(kRouteThreads) route_softmax_kernel(ds41_route
   __shared__ int used[kRouteMax];
   __shared__ int slot_of_expert[kRouteMax];
   for (int e = tid; e < p.experts; e += kRouteThreads) used[e] = 0;
-  if (gridDim.x > 1) {
+  if (!alone) {
     __threadfence();
     __syncthreads();
     if (tid == 0) last = atomicAdd(p.ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
     __syncthreads();
     if (!last) return;
     __threadfence();
+    for (int i = tid; i < p.max_active * p.row_w_ld; i += kRouteThreads) p.row_w[i] = 0.f;
   }
-  for (int i = tid; i < p.max_active * p.row_w_ld; i += kRouteThreads) p.row_w[i] = 0.f;
   __syncthreads();
   const int n = p.rows * p.top;
+  auto route = [&](int i, int& e, float& w) {
+    e = alone ? chosen[i] : __ldcg(p.ids + i);
+    w = alone ? chosen_w[i] : __ldcg(p.weights + i);
+  };
   for (int i = tid; i < n; i += kRouteThreads) {
-    const int e = __ldcg(p.ids + i);
-    if (e >= 0 && __ldcg(p.weights + i) > 0.f) used[e] = 1;
+    int e;
+    float w;
+    route(i, e, w);
+    if (e >= 0 && w > 0.f) used[e] = 1;
   }
   __syncthreads();
   if (warp == 0) {
@@ -344,8 +367,9 @@ __global__ void __launch_bounds__(kRouteThreads) route_softmax_kernel(ds41_route
   }
   __syncthreads();
   for (int i = tid; i < n; i += kRouteThreads) {
-    const int e = __ldcg(p.ids + i);
-    const float w = __ldcg(p.weights + i);
+    int e;
+    float w;
+    route(i, e, w);
     const int s = e >= 0 && w > 0.f ? slot_of_expert[e] : -1;
     p.slot_of[i] = s;
     if (s >= 0) p.row_w[1ll * s * p.row_w_ld + i / p.top] = w;
@@ -541,8 +565,11 @@ extern "C" int ds41_route_softmax(const ds41_route_args* a, void* stream) {
                                a->max_active <= 0 || a->row_w_ld < a->rows))
     return cudaErrorInvalidValue;
   constexpr int kWarps = kRouteThreads / 32;
-  return launch_pdl(route_softmax_kernel, dim3((a->rows + kWarps - 1) / kWarps), dim3(kRouteThreads), 0,
-                    static_cast<cudaStream_t>(stream), *a);
+  const dim3 grid((a->rows + kWarps - 1) / kWarps), block(kRouteThreads);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (a->experts <= 32) return launch_pdl(route_softmax_kernel<1>, grid, block, 0, st, *a);
+  if (a->experts <= 128) return launch_pdl(route_softmax_kernel<4>, grid, block, 0, st, *a);
+  return launch_pdl(route_softmax_kernel<kRouteMax / 32>, grid, block, 0, st, *a);
 }
 
 extern "C" int ds41_gated_act(const float* x, int ld_x, int up_col, const float* row_w, int row_w_ld, const int* n_active,

@@ -517,6 +517,12 @@ def test_router_choices_weights_and_plan(rows, experts, top):
         assert all(used[s] == i for s, i in zip(slot_of.cpu()[live].tolist(), want_ids[live].tolist()))
 
 
+@pytest.mark.parametrize("rows,experts,top", [(8, 32, 4), (8, 32, 32), (9, 32, 4), (8, 128, 5), (7, 129, 31), (8, 512, 32)])
+def test_router_by_logits_a_lane(rows, experts, top):
+    """One, four or sixteen logits a lane, in a block that has all rows and in several."""
+    test_router_choices_weights_and_plan(rows, experts, top)
+
+
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 @pytest.mark.parametrize("rows", [1, 3, 32, 33, 150])
 def test_experts_planned_and_sorted(rows, dtype):
