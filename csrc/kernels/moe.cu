@@ -427,24 +427,45 @@ __device__ __forceinline__ void publish_all(unsigned int* counter, uint32_t* epo
   }
 }
 
+// Few rows: a chain of round trips to L2, so the shared expert's planes, the slots and then the routes' rows are each asked for together
+// (eight at a time) and added in their order.  What the launch adds to a step of one row, 6 routes of 5120 columns, in a graph: 7.9 us
+// route by route and plane by plane, 6.5 so.
 __global__ void __launch_bounds__(256) moe_combine_kernel(CombineParams p) {
+  constexpr int kUnder = 8;
   const int r = blockIdx.y;
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   pdl_launch_dependents();
   pdl_wait();
   if (c < p.H) {
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = 0; k < p.topk; ++k) {
-      const int s = p.slot_of[r * p.topk + k];
-      if (s >= 0) {
-        const float4 v = *reinterpret_cast<const float4*>(p.fc2 + (1ll * s * p.rows + r) * p.H + c);
-        // per-route bf16 boundary, then fp32 accumulation in route order
-        acc.x += bf16_round(v.x); acc.y += bf16_round(v.y); acc.z += bf16_round(v.z); acc.w += bf16_round(v.w);
-      }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), sh[kUnder];
+    auto ask_shared = [&](int s0) {
+#pragma unroll
+      for (int u = 0; u < kUnder; ++u)
+        if (s0 + u < p.shared_splits) sh[u] = *reinterpret_cast<const float4*>(p.shared + (1ll * (s0 + u) * p.rows + r) * p.H + c);
+    };
+    ask_shared(0);
+    for (int k0 = 0; k0 < p.topk; k0 += kUnder) {
+      int slot[kUnder];
+      float4 v[kUnder];
+#pragma unroll
+      for (int u = 0; u < kUnder; ++u) slot[u] = k0 + u < p.topk ? p.slot_of[r * p.topk + k0 + u] : -1;
+#pragma unroll
+      for (int u = 0; u < kUnder; ++u)
+        if (slot[u] >= 0) v[u] = *reinterpret_cast<const float4*>(p.fc2 + (1ll * slot[u] * p.rows + r) * p.H + c);
+#pragma unroll
+      for (int u = 0; u < kUnder; ++u)
+        if (slot[u] >= 0) {
+          // per-route bf16 boundary, then fp32 accumulation in route order
+          acc.x += bf16_round(v[u].x); acc.y += bf16_round(v[u].y); acc.z += bf16_round(v[u].z); acc.w += bf16_round(v[u].w);
+        }
     }
-    for (int s = 0; s < p.shared_splits; ++s) {
-      const float4 v = *reinterpret_cast<const float4*>(p.shared + (1ll * s * p.rows + r) * p.H + c);
-      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    for (int s0 = 0; s0 < p.shared_splits; s0 += kUnder) {
+      if (s0 > 0) ask_shared(s0);
+#pragma unroll
+      for (int u = 0; u < kUnder; ++u)
+        if (s0 + u < p.shared_splits) {
+          acc.x += sh[u].x; acc.y += sh[u].y; acc.z += sh[u].z; acc.w += sh[u].w;
+        }
     }
     *reinterpret_cast<float4*>(p.out + 1ll * r * p.H + c) = acc;
   }

@@ -972,3 +972,25 @@ def test_qkv_post_sums_planes_in_their_order(rows, Q, extra):
     ref = q * torch.rsqrt((q * q).mean(-1, keepdim=True) + 1e-6) * qn.double()
     assert float((ql.double() - ref).abs().max()) < 2.0 ** -7 * float(ref.abs().max())
     assert bool(win[0, 7:7 + rows].any(-1).all()) and not bool(win[0, :7].any())
+
+
+@pytest.mark.parametrize("rows,topk,splits", [(1, 6, 0), (1, 6, 8), (3, 8, 9), (2, 9, 1), (5, 17, 20)])
+def test_combine_of_routes_and_shared_planes(rows, topk, splits):
+    """Around the number of routes and planes that are under way together, absent routes among them; same order, same bits."""
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    torch.manual_seed(topk)
+    H, active = 1028, 11
+    fc2, shared = torch.randn(active, rows, H, device="cuda"), torch.randn(max(splits, 1), rows, H, device="cuda")
+    slot = torch.randint(-1, active, (rows, topk), device="cuda", dtype=torch.int32)
+    out = torch.full((rows, H), float("nan"), device="cuda")
+    lib.check(k.ds41_moe_combine(lib.ptr(fc2), lib.ptr(slot), lib.ptr(shared), splits, rows, topk, H, lib.ptr(out), lib.stream()),
+              "combine")
+    want = torch.zeros(rows, H, device="cuda")
+    for r in range(rows):
+        for s in slot[r].tolist():
+            if s >= 0:
+                want[r] += fc2[s, r].bfloat16().float()
+        for s in range(splits):
+            want[r] += shared[s, r]
+    assert torch.equal(out, want)
