@@ -90,18 +90,16 @@ class RowsEngine:
     @contextlib.contextmanager
     def rehearsal(self):
         """Around the eager pass and the capture that precede a graph's first replay: the pass inputs come back
-        unchanged, and nothing the pass does may count as a step of a request."""
+        unchanged, and nothing the pass does may count as a step of a request: no row owns a slot, so that caches and states
+        keep what they hold, whatever rows the last pass left behind."""
         keep = (self.in_tokens.clone(), self.row_pos.clone(), self.row_slot.clone())
-        self._enter_rehearsal()
+        self.row_slot.fill_(-1)
         try:
             yield
         finally:
             self.in_tokens.copy_(keep[0])
             self.row_pos.copy_(keep[1])
             self.row_slot.copy_(keep[2])
-
-    def _enter_rehearsal(self):
-        pass
 
     def capture(self, enqueue) -> torch.cuda.CUDAGraph:
         """Graph of the launches that `enqueue` makes; one eager pass first sets function attributes and warms every

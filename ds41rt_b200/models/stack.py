@@ -705,9 +705,6 @@ class StackEngine(RowsEngine):
                 self._keys[i] = torch.zeros(ceil_to(n, 1024) * w, dtype=BF16, device=self.device)
         return self._keys
 
-    def _enter_rehearsal(self):
-        self.row_slot.fill_(-1)       # no row owns a slot: caches and states keep what they hold
-
     def set_rows(self, tokens, positions, slots, row_hi=None, row_lo=None):
         """Host -> device copy of one pass's inputs.  Rows of one slot are adjacent, at consecutive positions."""
         assert row_lo is None and row_hi is None, "a layer stack has no window floor"

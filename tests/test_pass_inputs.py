@@ -65,3 +65,55 @@ def test_step_is_the_pass(graphs, n):
         got.append(out)
     for (a, x), (b, y) in zip(*got):
         assert a == b and torch.equal(x, y)
+
+
+def test_rehearsal_has_no_slots():
+    """The eager pass before a graph's capture may see rows that an earlier pass left: none of them may own a slot."""
+    from ds41rt_b200.models.base import RowsEngine
+    e = RowsEngine()
+    e.in_tokens, e.row_pos, e.row_slot = torch.tensor([3, 4]), torch.tensor([7, 8]), torch.tensor([0, 1])
+    with e.rehearsal():
+        assert e.row_slot.tolist() == [-1, -1]
+        e.in_tokens += 1
+        e.row_pos += 1
+    assert (e.in_tokens.tolist(), e.row_pos.tolist(), e.row_slot.tolist()) == ([3, 4], [7, 8], [0, 1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts,kv", [("bf16", "bf16"), ("mxfp8", "fp8")])
+@pytest.mark.parametrize("length", [9, 17])
+def test_first_steps_leave_other_rows_alone(length, experts, kv):
+    """A session's first step of a row count makes its graph: the rows of earlier passes, in the step's places, are neither
+    stepped again nor written anywhere.  One request alone beyond its ring, then both for the first time."""
+    from ds41rt_b200.config import ModelConfig
+    from ds41rt_b200.models.ds41 import DS41Engine, EngineWeights
+    from ds41rt_b200.runtime.session import DecodeSession
+    cfg, dev = ModelConfig.tiny(), torch.device("cuda", 0)
+    w = EngineWeights.random(cfg, 0, 1, dev, seed=3, expert_dtype=experts)
+    prompts = torch.randint(3, cfg.vocab, (2, 2 * length), generator=torch.Generator().manual_seed(length))
+    alone, both = cfg.window + 24, 5
+    got = []
+    for graphs in (True, False):
+        e = DS41Engine(cfg, w, max_rows=24, slots=2, max_ctx=256, kv_dtype=kv)
+        session = DecodeSession(e, use_graphs=graphs)
+        last, out = [], []
+        for slot in (0, 1):
+            assert e.cache.ensure(slot, 200)
+            last.append(e.prefill(slot, prompts[slot, :length].tolist()))
+        at = [length, length]
+        for step in range(alone + both):
+            slots = [1] if step < alone else [0, 1]
+            tokens = session.step([last[s] for s in slots], [at[s] for s in slots], slots)
+            for s, t in zip(slots, tokens):
+                last[s] = t
+                at[s] += 1
+            out.append(e.logits_rows(len(slots)).clone())
+        e.check_status()
+        got.append((out, e.cache.win, [e.cache.comp[s] for s in e.cache.comp], [e.cache.idx[s] for s in e.cache.idx],
+                    [e.cache.pending[s] for s in e.cache.pending]))
+    (out, *caches), (want, *there) = got
+    for i, (a, b) in enumerate(zip(out, want)):
+        assert torch.equal(a, b), f"step {i}"
+    flat = lambda c: [c[0], *c[1], *c[2], *c[3]]
+    for a, b in zip(flat(caches), flat(there)):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
