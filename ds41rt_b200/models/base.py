@@ -15,24 +15,36 @@ import torch
 from ..ops import lib
 
 
-def row_values(values, rows: int, fill: int) -> torch.Tensor:
-    """One number per row of a pass as a CPU tensor of `rows` numbers, filled up with `fill`.  Lists of thousands are what a
-    prompt pass waits for before its first launch: through `array` (8192 numbers 0.1 ms) rather than torch.tensor (0.4)."""
-    out = torch.full((rows,), fill, dtype=torch.int32)
-    n = len(values)
-    if n == 0:
-        return out
-    if isinstance(values, range):
-        t = torch.arange(values.start, values.stop, values.step, dtype=torch.int32)
-    elif isinstance(values, torch.Tensor):
-        t = values
-    else:
+def whole_numbers(values) -> torch.Tensor:
+    """A sequence's numbers as a CPU tensor of int32 by torch's rules: fractions are dropped, what does not fit is refused.  Lists of
+    thousands are what a prompt pass waits for before its first launch: through `array` (8192 numbers 0.1 ms) rather than
+    torch.tensor (0.4)."""
+    if isinstance(values, range) and (not values or -2 ** 31 <= min(values[0], values[-1]) <= max(values[0], values[-1]) < 2 ** 31 - 1):
+        return torch.arange(values.start, values.stop, values.step, dtype=torch.int32)
+    if isinstance(values, torch.Tensor):
+        if values.dtype == torch.int32:
+            return values.cpu()
+        if not values.is_floating_point():
+            values = values.tolist()
+    if isinstance(values, (list, tuple)) and values:
         try:
-            t = torch.frombuffer(array.array("i", values), dtype=torch.int32)
-        except (TypeError, OverflowError):            # other numbers, or none that fit: torch's rules
-            t = torch.tensor(list(values), dtype=torch.int32)
-    out[:n] = t
+            return torch.frombuffer(array.array("i", values), dtype=torch.int32)
+        except (TypeError, OverflowError):            # other numbers, or none that fit
+            pass
+    return torch.tensor(list(values), dtype=torch.int32)
+
+
+def row_values(values, rows: int, fill: int) -> torch.Tensor:
+    """One number per row of a pass as a CPU tensor of `rows` numbers, filled up with `fill`."""
+    out = torch.full((rows,), fill, dtype=torch.int32)
+    if len(values):
+        out[:len(values)] = whole_numbers(values)
     return out
+
+
+def sized(values):
+    """`values`, or what an iterator yields as a list."""
+    return values if values is None or hasattr(values, "__len__") else list(values)
 
 
 class RowsEngine:

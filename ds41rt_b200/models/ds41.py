@@ -30,7 +30,7 @@ from ..ops import attention as A
 from ..ops import gemm as G
 from ..ops import lib
 from ..parallel.fabric import Fabric, SymBuffer
-from .base import RowsEngine, row_values
+from .base import RowsEngine, row_values, sized
 from .paged import PagedSlots
 
 BF16 = torch.bfloat16
@@ -806,6 +806,7 @@ class DS41Engine(RowsEngine):
         floor under the attention windows of the pass: positions below it are not attended."""
         n = len(positions)
         self._floor_on = row_lo is not None
+        slots, row_lo, row_hi = sized(slots), sized(row_lo), sized(row_hi)
         assert all(x is None or len(x) == n for x in (row_lo, row_hi))
         if row_lo is not None:
             self.row_lo.copy_(row_values(row_lo, self.max_rows, 0), non_blocking=True)

@@ -22,7 +22,7 @@ from ..ops import lib
 from ..ops import stack as S
 from ..ops.stack import Matrix, Proj, ceil_to
 from ..stack_config import GroupedAttentionSpec, LatentAttentionSpec, MLSTMSpec, MoESpec, StackConfig
-from .base import RowsEngine, row_values
+from .base import RowsEngine, row_values, sized
 from .paged import PagedSlots
 
 BF16, F32, I32 = torch.bfloat16, torch.float32, torch.int32
@@ -709,8 +709,8 @@ class StackEngine(RowsEngine):
         """Host -> device copy of one pass's inputs.  Rows of one slot are adjacent, at consecutive positions."""
         assert row_lo is None and row_hi is None, "a layer stack has no window floor"
         n = len(positions)
-        assert n <= self.max_rows
-        assert n == len(slots)
+        slots = sized(slots)
+        assert n <= self.max_rows and n == len(slots)
         pos, slot = row_values(positions, self.max_rows, 0), row_values(slots, self.max_rows, -1)
         p, s = pos[:n], slot[:n]
         follows = (s[1:] == s[:-1]) & (s[1:] >= 0)            # a row of the same request as the row before it

@@ -17,7 +17,7 @@ from typing import Dict, List, Optional
 
 import torch
 
-from ..models.base import RowsEngine
+from ..models.base import RowsEngine, whole_numbers
 from ..ops import lib
 
 
@@ -60,7 +60,7 @@ class DecodeSession:
         if not 0 < n <= e.max_rows:
             raise ValueError(f"a step has 1 to {e.max_rows} rows, not {n}")
         for i, values in enumerate((tokens, positions, slots)):
-            self._in[i * n:(i + 1) * n] = values
+            self._in[i * n:(i + 1) * n] = whole_numbers(values)
         self.h2d_bytes += 3 * 4 * n
         g = self.graph(n)
         src, dst, s = lib.ptr(self.h_in), lib.ptr(self.h_chosen), lib.stream()

@@ -1,4 +1,7 @@
 """Inputs of a pass: numbers from the host's lists, and a session's steps against passes described by set_rows()."""
+import collections
+
+import numpy as np
 import pytest
 import torch
 
@@ -6,7 +9,9 @@ from ds41rt_b200.models.base import row_values
 
 
 @pytest.mark.parametrize("values", [[], [7], list(range(5, 69)), range(3, 67), range(10, 0, -3), (1, 2, 3), [True, False],
-                                    [2 ** 31 - 1, -2 ** 31], [1.9, -1.9], torch.arange(9), list(torch.arange(4))])
+                                    [2 ** 31 - 1, -2 ** 31], [1.9, -1.9], torch.arange(9), list(torch.arange(4)),
+                                    bytes(range(97, 105)), bytearray(4), range(7, 7), range(2 ** 31 - 3, 2 ** 31 - 1),
+                                    torch.tensor([3, 4], dtype=torch.int32), np.arange(5)])
 def test_row_values(values):
     want = torch.tensor(list(values) + [-1] * (64 - len(values)), dtype=torch.int32)
     assert torch.equal(row_values(values, 64, -1), want)
@@ -17,6 +22,33 @@ def test_row_values_refused():
         row_values([2 ** 31], 4, 0)
     with pytest.raises(RuntimeError):
         row_values([1, 2, 3], 2, 0)
+
+
+@pytest.mark.parametrize("values", [torch.tensor([2 ** 31]), range(2 ** 31 - 1, 2 ** 31 + 1), range(-2 ** 31 - 1, -2 ** 31),
+                                    [float("nan")], (0, -2 ** 31 - 1)])
+def test_numbers_that_do_not_fit(values):
+    with pytest.raises(RuntimeError):
+        row_values(values, 2, 0)
+
+
+def _host_rows(kind, rows):
+    """An engine that has nothing but the inputs of a pass, on the CPU."""
+    from ds41rt_b200.models.ds41 import DS41Engine
+    from ds41rt_b200.models.stack import StackEngine
+    e = object.__new__(StackEngine if kind == "stack" else DS41Engine)
+    e.max_rows, e.long_rows, e.f32, e.moe_rows, e.max_keys, e.idx_q = rows, 4, 0, 4, 64, None
+    e.in_tokens, e.row_pos, e.row_slot, e.row_lo, e.row_hi = torch.zeros(5, rows, dtype=torch.int32).unbind()
+    return e
+
+
+@pytest.mark.parametrize("kind", ["stack", "flash"])
+@pytest.mark.parametrize("rows", [8, 600])
+def test_set_rows_takes_what_yields_numbers(kind, rows):
+    e = _host_rows(kind, rows)
+    e.set_rows(b"abc", collections.deque([4, 5, 9]), iter([0, 0, 1]))
+    pad = [0] * (rows - 3)
+    assert e.in_tokens.tolist() == [97, 98, 99] + pad and e.row_pos.tolist() == [4, 5, 9] + pad
+    assert e.row_slot.tolist() == [0, 0, 1] + [-1] * (rows - 3)
 
 
 def _stack(rows):
