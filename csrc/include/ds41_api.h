@@ -491,6 +491,7 @@ typedef struct ds41_resid_args {
   int y_top, y_rows;
   int raw_h;            // next_w == NULL: h = the stream itself
   int post_rms;         // the norm of the result is an RMS norm whatever norm_kind says
+  int* status;          // or NULL
 } ds41_resid_args;
 int ds41_resid_step(const ds41_resid_args* args, void* stream);
 
@@ -543,6 +544,7 @@ typedef struct ds41_latent_attend_args {
   long long ld_q_abs, ld_q_rot;
   float scale;
   int rows, heads, kv_pad, row_len, q_rot_stride, n_splits, max_pages, page_tokens, f32;
+  int* status;                    // or NULL
 } ds41_latent_attend_args;
 int ds41_latent_attend(const ds41_latent_attend_args* args, void* stream);
 int ds41_latent_merge(const float* part_o, const float* part_ml, const float* sink, int n_splits, int rows, int heads,

@@ -376,12 +376,12 @@ __global__ void __launch_bounds__(MT * PW * 32) latent_attend_mma_kernel(ds41_la
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   const float scale2 = p.scale * 1.4426950408889634f;
   const int n_pairs = p.kv_pad / 16;
-  bool ok = mbar_wait(&full[2], 0, nullptr, 0);
+  bool ok = mbar_wait(&full[2], 0, p.status, 450);
   int tile = 0;
   for (int t0 = k0; t0 < k1; t0 += kKeyTile, ++tile) {
     const int buf = tile & 1;
     const __nv_bfloat16* later = tid < kKeyTile ? locate(t0 + 2 * kKeyTile + tid) : nullptr;      // looked up ahead of its copy
-    ok &= mbar_wait(&full[buf], (tile >> 1) & 1, nullptr, 0);
+    ok &= mbar_wait(&full[buf], (tile >> 1) & 1, p.status, 451);
     const __nv_bfloat16* kt = sk + buf * kKeyTile * RS;
     float s[2][4] = {}, s_odd[2][4] = {};       // two chains: consecutive products into one accumulator wait for each other
     if (w < 4) {

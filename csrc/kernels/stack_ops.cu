@@ -138,6 +138,7 @@ struct RowShare {
 struct ClusterExchange {
   RowShare* sh;
   int rank, warps;
+  int* status;
   __device__ __forceinline__ Moments operator()(Moments t) const {
     const int lane = threadIdx.x & 31, at = rank * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (lane < kShare) {
@@ -147,7 +148,9 @@ struct ClusterExchange {
                    : "memory");
     }
     __syncwarp();
-    mbar_wait(&sh->bar, 0, nullptr, 0);
+    if (!mbar_wait(&sh->bar, 0, status, 460))          // reported; what is on its way still lands before the memory changes hands
+      for (int i = 0; i < (1 << 20) && !mbar_test_wait(&sh->bar, 0); ++i) {
+      }
     const float4 m = sh->moments[lane < warps ? lane : lane & (warps - 1)];
     return {m.x, m.y, m.z};
   }
@@ -510,7 +513,7 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
       }
     float2 s = make_float2(0.f, 1.f);
     if (p.post_w != nullptr)
-      s = row_norm<NI, FULL>(y, n, p.W, p.post_rms ? 1 : p.norm_kind, p.eps, ClusterExchange{&share[0], part, warps});
+      s = row_norm<NI, FULL>(y, n, p.W, p.post_rms ? 1 : p.norm_kind, p.eps, ClusterExchange{&share[0], part, warps, p.status});
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (live[i] > 0) {
@@ -535,7 +538,7 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
     }
   }
   float2 s = make_float2(0.f, 1.f);
-  if (p.next_w != nullptr) s = row_norm<NI, FULL>(avg, n, p.W, p.norm_kind, p.eps, ClusterExchange{&share[1], part, warps});
+  if (p.next_w != nullptr) s = row_norm<NI, FULL>(avg, n, p.W, p.norm_kind, p.eps, ClusterExchange{&share[1], part, warps, p.status});
   cg::cluster_group::barrier_arrive();
 #pragma unroll
   for (int i = 0; i < NI; ++i) {

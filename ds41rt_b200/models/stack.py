@@ -238,7 +238,7 @@ class LatentAttention:
             a.row_pos, a.row_slot = e.row_pos[r0:].data_ptr(), e.row_slot[r0:].data_ptr()
             a.part_o, a.part_ml = e.part_o.data_ptr(), e.part_ml.data_ptr()
             a.scale, a.rows, a.heads, a.kv_pad, a.row_len, a.n_splits = sp.scale, n, H, self.kvp, self.row_len, splits
-            a.max_pages, a.page_tokens, a.f32 = e.cache.max_pages, e.cache.page_tokens, e.f32
+            a.max_pages, a.page_tokens, a.f32, a.status = e.cache.max_pages, e.cache.page_tokens, e.f32, lib.ptr(e.status)
             e._run("latent_attend", k.ds41_latent_attend, C.byref(a), lib.stream())
             e._run("latent_merge", k.ds41_latent_merge, lib.ptr(e.part_o), lib.ptr(e.part_ml), lib.ptr(self.sink), splits, n,
                    H, self.kvp, lib.ptr(e.o_lat), H * self.kvp, e.f32, lib.stream())
@@ -743,7 +743,7 @@ class StackEngine(RowsEngine):
             a.n_mix, a.x_avg = layer + 2, lib.ptr(self.x_avg)
         a.h, a.ldh, a.ldx, a.vocab, a.rows, a.W = lib.ptr(self.h), self.ldh, self.ldx, cfg.vocab, R, cfg.hidden
         a.norm_kind, a.eps, a.f32 = cfg.norm_kind, cfg.norm_eps, self.f32
-        a.raw_h, a.post_rms = int(next_w is None), int(post_rms)
+        a.raw_h, a.post_rms, a.status = int(next_w is None), int(post_rms), lib.ptr(self.status)
         if isinstance(y, S.RoutedProj):
             a.y_route, a.y_top, a.y_rows = lib.ptr(y.route), y.top, y.rows
         self._run("resid_step", self.k.ds41_resid_step, C.byref(a), lib.stream())

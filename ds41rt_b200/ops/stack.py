@@ -31,7 +31,7 @@ class ResidArgs(C.Structure):
                 ("x_avg", C.c_void_p), ("next_w", C.c_void_p), ("h", C.c_void_p), ("ldx", C.c_longlong),
                 ("ldh", C.c_int), ("n_mix", C.c_int), ("vocab", C.c_int), ("rows", C.c_int), ("W", C.c_int),
                 ("norm_kind", C.c_int), ("eps", C.c_float), ("f32", C.c_int), ("y_route", C.c_void_p), ("y_top", C.c_int),
-                ("y_rows", C.c_int), ("raw_h", C.c_int), ("post_rms", C.c_int)]
+                ("y_rows", C.c_int), ("raw_h", C.c_int), ("post_rms", C.c_int), ("status", C.c_void_p)]
 
 
 class LatentPostArgs(C.Structure):
@@ -48,7 +48,8 @@ class LatentAttendArgs(C.Structure):
                 ("row_pos", C.c_void_p), ("row_slot", C.c_void_p), ("part_o", C.c_void_p), ("part_ml", C.c_void_p),
                 ("ld_q_abs", C.c_longlong), ("ld_q_rot", C.c_longlong), ("scale", C.c_float), ("rows", C.c_int),
                 ("heads", C.c_int), ("kv_pad", C.c_int), ("row_len", C.c_int), ("q_rot_stride", C.c_int),
-                ("n_splits", C.c_int), ("max_pages", C.c_int), ("page_tokens", C.c_int), ("f32", C.c_int)]
+                ("n_splits", C.c_int), ("max_pages", C.c_int), ("page_tokens", C.c_int), ("f32", C.c_int),
+                ("status", C.c_void_p)]
 
 
 class LatentPrefillArgs(C.Structure):

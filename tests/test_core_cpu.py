@@ -450,3 +450,29 @@ def test_no_barrier_behind_a_condition_that_threads_read_for_themselves():
             if "status" in m.group(1) and "__syncthreads_or" not in m.group(1):
                 body = text[m.end() - 1:_end_of_block(text, m.end() - 1)]
                 assert "__syncthreads" not in body and "named_barrier" not in body, (name, m.group(0))
+
+
+def _arguments(text, at):
+    """The arguments of the call whose parenthesis opens at `at`."""
+    depth, start, out = 0, at + 1, []
+    for i in range(at, len(text)):
+        depth += {"(": 1, "[": 1, "{": 1, ")": -1, "]": -1, "}": -1}.get(text[i], 0)
+        if (text[i] == "," and depth == 1) or depth == 0:
+            out.append(text[start:i].strip())
+            start = i + 1
+        if depth == 0:
+            return out
+    raise AssertionError("unbalanced parentheses")
+
+
+def test_every_wait_that_can_give_up_has_a_status_word():
+    """mbar_wait(barrier, parity, status, site) and flag_wait_ge(flag, value, status, site) return after a limit; what follows is
+    only as good as the report."""
+    headers = {src.name: re.sub(r"//[^\n]*", "", src.read_text()) for src in sorted((ROOT / "csrc" / "include").glob("*.cuh"))}
+    calls = 0
+    for name, text in {**_sources(), **headers}.items():
+        for m in re.finditer(r"(?<!bool )\b(mbar_wait|flag_wait_ge)\(", text):
+            args = _arguments(text, m.end() - 1)
+            assert len(args) == 4 and "status" in args[2] and args[3] != "0", (name, args)
+            calls += 1
+    assert calls > 25, calls

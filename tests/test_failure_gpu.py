@@ -35,3 +35,25 @@ def test_flag_wait_runs_out_and_reports():
     lib.raise_on_status(st2, "gemm after timeout")
     ref = x.float() @ w.float().t()
     assert float((y.float() - ref).abs().max() / ref.abs().max()) < 1e-2
+
+
+@pytest.mark.parametrize("model", ["genesun-tiny", "belasun-tiny"])
+def test_layer_stacks_hand_their_status_word_to_every_step(model):
+    """The waits inside the residual step of few rows and inside the latent attention report where the engine looks."""
+    from ds41rt_b200.models import registry
+    from ds41rt_b200.ops import lib
+    fam, cfg = registry.preset(model)
+    dev = torch.device("cuda", 0)
+    e = fam.engine(cfg, fam.random_weights(cfg, dev), max_rows=8, slots=1, max_ctx=128)
+    seen, run = [], e._run
+
+    def watch(tag, fn, *args, **kw):
+        if tag in ("resid_step", "latent_attend"):
+            seen.append(tag)
+            assert args[0]._obj.status == lib.ptr(e.status).value
+        return run(tag, fn, *args, **kw)
+
+    e._run = watch
+    e.prefill(0, list(range(3, 9)))
+    e.check_status()
+    assert "resid_step" in seen and ("latent_attend" in seen) == (model == "genesun-tiny")
