@@ -822,10 +822,11 @@ class DS41Engine(RowsEngine):
         # A decode-sized pass over one request (a speculative verification, a lone request's step) scores on the tensor
         # cores too; its launches may be replayed from a graph while the context grows, so the key count is the static
         # bound (-1) and the visible count per row is worked out on the device.
-        one = n > 0 and int(s[0]) >= 0 and bool((s[:n] == s[0]).all())
+        slot = s.numpy()[:n]
+        one = n > 0 and 0 <= slot[0] == slot[-1] and (n < 3 or bool((slot == slot[0]).all()))
         self._pass_hint = None
         if one and n > self.moe_rows:
-            self._pass_hint = (n, int(p[:n].max()))
+            self._pass_hint = (n, int(p.numpy()[:n].max()))
         elif one and getattr(self, "idx_q", None) is not None and self.max_keys <= 32768:
             self._pass_hint = (n, -1)
         if self.row_hi is not None:

@@ -15,6 +15,7 @@ import ctypes as C
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from ..config import rope_inv_freq
@@ -557,6 +558,36 @@ class StackWeights:
 
 
 # ---------------------------------------------------------------------------------------------------- engine
+LOOP_ROWS = 64        # up to here a loop is faster than a dozen array operations: 8 rows 1.1 and 7.9 us, 64 rows 5.4 and 9.0, 128 rows 10.9 and 10.2
+
+
+def row_requests(pos: np.ndarray, slot: np.ndarray) -> int:
+    """How many requests the rows of a pass belong to; rows of one slot must be adjacent and at consecutive positions."""
+    if len(slot) <= LOOP_ROWS:
+        follow = adjacent = True
+        seen, last_p, last_s = set(), 0, -1
+        for p, s in zip(pos.tolist(), slot.tolist()):
+            if s >= 0:
+                if s == last_s:
+                    follow = follow and p == last_p + 1
+                else:
+                    adjacent = adjacent and s not in seen
+                    seen.add(s)
+            last_p, last_s = p, s
+        n = len(seen)
+    else:
+        follows = (slot[1:] == slot[:-1]) & (slot[1:] >= 0)            # a row of the same request as the row before it
+        follow = bool(((pos[1:] == pos[:-1] + 1) | ~follows).all())
+        first = slot >= 0
+        first[1:] &= ~follows
+        seen = slot[first].tolist()
+        n = len(set(seen))
+        adjacent = n == len(seen)
+    assert follow, "rows of a request must follow one another"
+    assert adjacent, "rows of a request must be adjacent"
+    return n
+
+
 class StackEngine(RowsEngine):
     partial_prefix = False        # recurrent states belong to a snapshot's whole length
     replay_window = 1 << 30       # the prefix banks then never prefer a truncated snapshot
@@ -712,15 +743,10 @@ class StackEngine(RowsEngine):
         slots = sized(slots)
         assert n <= self.max_rows and n == len(slots)
         pos, slot = row_values(positions, self.max_rows, 0), row_values(slots, self.max_rows, -1)
-        p, s = pos[:n], slot[:n]
-        follows = (s[1:] == s[:-1]) & (s[1:] >= 0)            # a row of the same request as the row before it
-        assert bool((p[1:] == p[:-1] + 1)[follows].all()), "rows of a request must follow one another"
-        first = s >= 0
-        first[1:] &= ~follows
-        seen = s[first].tolist()
-        assert len(set(seen)) == len(seen), "rows of a request must be adjacent"
+        p, s = pos.numpy()[:n], slot.numpy()[:n]
+        requests = row_requests(p, s)
         # what the host knows about the pass it just described: a long pass of one request
-        one = n >= self.long_rows and len(seen) == 1 and int(s.min()) >= 0 and not self.f32
+        one = n >= self.long_rows and requests == 1 and int(s.min()) >= 0 and not self.f32
         self._hint = (n, int(p[-1]) + 1) if one else None
         if tokens is not None:
             assert len(tokens) == n

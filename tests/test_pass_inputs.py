@@ -51,6 +51,39 @@ def test_set_rows_takes_what_yields_numbers(kind, rows):
     assert e.row_slot.tolist() == [0, 0, 1] + [-1] * (rows - 3)
 
 
+def test_requests_of_a_pass(monkeypatch):
+    """The loop over few rows and the array operations over many, against the rule stated plainly."""
+    from ds41rt_b200.models import stack
+
+    def plain(pos, slot):
+        for s in set(slot) - {-1}:
+            at = [i for i, x in enumerate(slot) if x == s]
+            if at != list(range(at[0], at[-1] + 1)) or [pos[i] for i in at] != list(range(pos[at[0]], pos[at[0]] + len(at))):
+                return None
+        return len(set(slot) - {-1})
+
+    g, kinds = torch.Generator().manual_seed(5), set()
+    for _ in range(600):
+        n = int(torch.randint(0, 9, (1,), generator=g))
+        slot = torch.randint(-1, 3, (n,), generator=g).sort(descending=bool(torch.randint(0, 2, (1,), generator=g))).values
+        if torch.rand(1, generator=g) < 0.2:
+            slot = slot[torch.randperm(n, generator=g)]
+        pos = torch.arange(n) + 7
+        if torch.rand(1, generator=g) < 0.3 and n:
+            pos[int(torch.randint(0, n, (1,), generator=g))] += 1
+        want = plain(pos.tolist(), slot.tolist())
+        kinds.add(want)
+        for line in (1000, -1):
+            monkeypatch.setattr(stack, "LOOP_ROWS", line)
+            rows = (pos.int().numpy(), slot.int().numpy())
+            if want is None:
+                with pytest.raises(AssertionError):
+                    stack.row_requests(*rows)
+            else:
+                assert stack.row_requests(*rows) == want
+    assert kinds == {None, 0, 1, 2, 3}
+
+
 def _stack(rows):
     from ds41rt_b200.models import registry
     fam, cfg = registry.preset("genesun-tiny")
