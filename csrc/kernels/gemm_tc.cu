@@ -1024,9 +1024,11 @@ extern "C" int ds41_gemm_tc(const ds41_gemm_args* a, void* stream) {
   if (1ll * (k_splits - 1) * ((kb_total + k_splits - 1) / k_splits) >= kb_total) return cudaErrorInvalidValue;   // no empty split
   if (kind == 2 && (K % 128 != 0 || a->sfa == nullptr || a->sfb == nullptr)) return cudaErrorInvalidValue;
   if (kind == 3 && (K % 256 != 0 || a->sfa == nullptr || a->sfb == nullptr || a->ag_world > 0 || a->rs_world > 0 ||
-                    out_mode == 6 || out_mode == 8 || (bn < 32 && N > bn)))
+                    out_mode == 6 || out_mode == 8))
     return cudaErrorInvalidValue;
-  if (kind == 2 && bn < 32 && N > bn) return cudaErrorInvalidValue;      // 16-row scale tiles cannot be lane-shifted
+  // A tile's column scales begin (first column % 128) / 32 TMEM columns into their atom.  16 columns begin between two of those, and
+  // 32 on an odd one, which the tensor cores do not take (a misaligned address): narrow tiles stand alone.
+  if (kind >= 2 && bn < 64 && N > bn) return cudaErrorInvalidValue;
   if (k_splits > 1 && out_mode != 1 && out_mode != 3) return cudaErrorInvalidValue;   // partials are fp32
   if (a->softcap < 0.f || (a->softcap > 0.f && (kind != 0 || k_splits > 1 || (out_mode != 1 && out_mode != 3)))) return cudaErrorInvalidValue;
   if ((out_mode == 4 || out_mode == 5 || out_mode == 8) && a->row_w == nullptr) return cudaErrorInvalidValue;

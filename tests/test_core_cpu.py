@@ -476,3 +476,34 @@ def test_every_wait_that_can_give_up_has_a_status_word():
             assert len(args) == 4 and "status" in args[2] and args[3] != "0", (name, args)
             calls += 1
     assert calls > 25, calls
+
+
+def test_block_scaled_products_of_several_narrow_tiles_are_refused():
+    """Tiles of 16 or 32 columns whose scales begin between the column pairs of tensor memory: on the host, before anything runs."""
+    import ctypes as C
+    import torch
+    from ds41rt_b200.ops import lib
+    if torch.cuda.is_available():
+        pytest.skip("the addresses below are made up: only where nothing can be launched")
+    k = lib.kernels()
+
+    def call(kind, bn, n, mode=1, table=False):
+        a = lib.GemmArgs()
+        a.A = a.B = a.out = a.sfa = a.sfb = a.row_w = a.scatter_meta = 1 << 20
+        a.M, a.N, a.K, a.batch, a.lda, a.ldb, a.ldo = 128, n, 256, 1, 256, 256, 1024
+        a.kind, a.bn, a.k_splits, a.out_mode = kind, bn, 1, mode
+        if table:
+            a.tile_group = a.tile_row0 = a.tile_end = a.n_tiles_dev = 1 << 20
+            a.max_tiles = 4
+        return k.ds41_gemm_tc(C.byref(a), None)
+
+    refused = 1                                            # cudaErrorInvalidValue
+    for kind in (2, 3):
+        for bn in (16, 32):
+            for mode in (1, 3, 4, 5):
+                assert call(kind, bn, bn + 1, mode) == refused
+                assert call(kind, bn, 4 * bn, mode, table=True) == refused
+    # what stays open ends here without a GPU, with another error
+    open_to = {call(2, 64, 65), call(2, 32, 32), call(3, 64, 200), call(3, 32, 17), call(2, 128, 1024, 3, table=True), call(0, 32, 300),
+               call(1, 16, 300)}
+    assert refused not in open_to
