@@ -77,6 +77,10 @@ struct SamplePart {                        // what one CTA found in its slice
 };
 
 constexpr int kSampleList = 512;           // candidates that are gathered and compared one by one instead of histogrammed
+// Lists that solve_short() takes.  A shared search has three more barriers and a pass of one warp, 1.5 to 2 us: 16 rows of 129280 with a
+// single filter of 40 tokens 45.1 us by it alone, 41.3 so; with nucleus as well 55.4 and 49.8.  Long lists are another matter: 64 rows of
+// 4096, nucleus, 49 us without it, 33 so.  Lines from 48 to 192 measure the same.
+constexpr int kSampleShort = 96;
 
 struct SampleMember {
   uint32_t key, count;
@@ -220,10 +224,47 @@ __device__ void gather_members(SampleShared<PER>& sh, SamplePeers<CL> cl, const 
 }
 
 // The highest key whose members and the ones above weigh at least the target (`frac` >= 0: that share of the list's weight).
-// Several lanes share a member and sum what is not below it, each over a part of the list.
+// A short list: every thread sums what lies above its own member.
+template <int PER>
+__device__ uint32_t solve_short(SampleShared<PER>& sh, int total, double target, double frac) {
+  const int tid = threadIdx.x;
+  uint32_t key = 0, equal = 0, higher = 0, low = 0xFFFFFFFFu;
+  unsigned long long above = 0, same = 0, all = 0;
+  if (tid == 0) sh.best_key = 0;
+  __syncthreads();
+  if (tid < total) {
+    key = sh.list[tid].key;
+#pragma unroll 4
+    for (int j = 0; j < total; ++j) {
+      const SampleMember m = sh.list[j];
+      all += m.mass;
+      above += m.key > key ? m.mass : 0ull;
+      same += m.key == key ? m.mass : 0ull;
+      higher += m.key > key ? m.count : 0u;
+      equal += m.key == key ? m.count : 0u;
+      low = min(low, m.key);
+    }
+    if (frac >= 0.0) target = frac * static_cast<double>(all);
+    // rounding can leave the target just above the total: then the lowest key present is the one
+    if (static_cast<double>(above + same) >= target || key == low) atomicMax(&sh.best_key, key);
+  }
+  __syncthreads();
+  const uint32_t best = sh.best_key;
+  if (tid < total && key == best) {              // members of one key write the same
+    sh.remaining = target - static_cast<double>(above);
+    sh.tie_count = equal;
+    sh.n_above = higher;
+    if (frac >= 0.0) sh.total = all;
+  }
+  __syncthreads();
+  return best;
+}
+
+// The same of any list: several lanes share a member and sum what is not below it, each over a part of the list.
 template <int PER>
 __device__ uint32_t solve_list(SampleShared<PER>& sh, bool tie, double target, double frac) {
   const int tid = threadIdx.x, total = sh.n_list + (tie ? 1 : 0);
+  if (total <= kSampleShort) return solve_short(sh, total, target, frac);
   int per = 32;                                  // lanes per member
   while (per > 1 && total * per > kSampleThreads) per >>= 1;
   const int member = tid / per, part = tid % per;

@@ -230,3 +230,25 @@ def test_a_row_gets_its_token_whatever_is_sampled_beside_it(vocab, counts):
     for m in counts:
         t, s = sample_rows(logits[:m], pack_params(rows[:m], dev), masks)
         assert torch.equal(t, tok[:m]) and not bool(s.any())
+
+
+@pytest.mark.parametrize("ties", [False, True])
+@pytest.mark.parametrize("members", [1, 2, 31, 94, 95, 96, 97, 98, 200, 510, 511, 600])
+def test_gathered_lists_of_any_length(members, ties):
+    """All that a selection has to tell apart in one bin of its histogram, around the length where a list is searched by lanes together."""
+    from ds41rt_b200.ops.sampling import RowParams, pack_params, sample_rows
+    rng = np.random.default_rng(members)
+    vocab, dev = 6000, torch.device("cuda")
+    row = rng.normal(-12, 1, size=vocab).astype(np.float32)
+    at = rng.choice(vocab, members, replace=False)
+    row[at] = 2.0 - (rng.integers(0, 7, members) / 256 if ties else rng.permutation(members) / (members * 40.0))
+    asked = [dict(top_k=max(1, members // 2)), dict(top_p=0.5), dict(top_p=0.97), dict(top_k=members, top_p=0.3), dict(min_p=0.5, top_p=0.8),
+             dict(top_k=members + 3), dict()]
+    rows = [RowParams(temperature=1.0, seed=s, position=s, **asked[s % len(asked)]) for s in range(4 * len(asked))]
+    logits = torch.from_numpy(row).to(dev).expand(len(rows), vocab).contiguous()
+    tok, st = sample_rows(logits, pack_params(rows, dev))
+    assert not bool(st.any())
+    for r, p in enumerate(rows):
+        want, _ = _oracle(row, None, p)
+        if int(tok[r]) != want:
+            assert {int(tok[r]), want} <= _tokens_at_the_draw(row, None, p), (r, int(tok[r]), want)
