@@ -98,12 +98,14 @@ def wide(rows: int, n: int, batch: int = 1) -> bool:
 
 
 def score_bn(m: int, n_keys: int) -> int:
-    """Keys per tile of the indexer's product: as many as still give every SM a tile.  One row over 2112 keys is nine tiles of 256
-    and waits for eight chunks of one tile's epilogue (16 us); sixty-six of 32 take 8."""
-    for bn in (256, 128, 64):
-        if n_keys >= bn and -(-m // 128) * -(-n_keys // bn) >= SMS:
+    """Keys per tile of the indexer's product: the narrowest tile that gives no SM a second one, else the widest, since a launch lasts as
+    long as its busiest SM.  32 heads a row, us with 32 / 64 / 128 / 256 keys a tile, the chosen one first: 1 row over 2048 keys 3.9
+    / 3.9 / 4.2 / 5.1; 5 over 4096 (64) 4.4, 5.3 / 4.3 / 5.3; 5 over 16384 (256) 5.9, 11.5 / 8.1 / 6.3; 16 over 4096 (128) 4.7,
+    7.5 / 5.6 / 5.4; 64 over 512 (64) 4.3, 5.3 / 4.3 / 5.3; 64 over 4096 (256) 8.2, 19.9 / 13.1 / 9.9."""
+    for bn in (32, 64, 128):
+        if n_keys <= bn or -(-m // 128) * -(-n_keys // bn) <= SMS:
             return bn
-    return 32
+    return 256
 
 
 def linear_planes(x: torch.Tensor, w: torch.Tensor, planes: torch.Tensor, splits: int, *, status=None, signal=None):

@@ -507,3 +507,13 @@ def test_block_scaled_products_of_several_narrow_tiles_are_refused():
     open_to = {call(2, 64, 65), call(2, 32, 32), call(3, 64, 200), call(3, 32, 17), call(2, 128, 1024, 3, table=True), call(0, 32, 300),
                call(1, 16, 300)}
     assert refused not in open_to
+
+
+def test_tiles_of_index_scores_give_no_multiprocessor_a_second_one_if_they_can():
+    from ds41rt_b200.ops.gemm import SMS, score_bn
+    for rows in (1, 2, 5, 16, 33, 64, 148, 149, 333, 2048):
+        for n_keys in (64, 65, 100, 128, 512, 1000, 2048, 4096, 16384, 32768):
+            tiles = {bn: -(-rows * 32 // 128) * -(-n_keys // bn) for bn in (32, 64, 128, 256)}
+            bn = score_bn(rows * 32, n_keys)
+            fits = [b for b in tiles if tiles[b] <= SMS or n_keys <= b]
+            assert bn == (min(fits) if fits else 256), (rows, n_keys, bn)
