@@ -402,9 +402,15 @@ __device__ void select_topk_row_stream(Key key, int n, int k, int* out, int* n_o
 }
 
 // Threads per row.  Many rows are bound by the barriers of their passes, so that what counts is the rows an SM has at a time: two of
-// 1024 threads, five of 256.  Few rows are better off with more threads each.  8192 rows of up to 4096 keys, 512 chosen: 307 us
-// with 1024, 153 with 256.
+// 1024 threads, five of 256.  Few rows are better off with more threads each.  512 chosen, all rows as long as the context, us with
+// 1024 and with 256 threads: two rows an SM (296) of 1024 / 4096 keys 11.5 / 12.3 with 1024; 297 rows 15.9 and 6.9 / 17.1 and 12.6; 1200
+// rows 47.8 and 18.4 / 50.9 and 33.7.  Rows of more than 16 keys a thread pay for more registers: 8192 keys, 297 rows 25.3 and 27.7,
+// 400 rows 26.1 and 27.8, 1200 rows 75.5 and 75.9; but only those at the end of a context are as long as it, and 8192 rows of
+// up to 4096 keys take 153 us with 256, 307 with 1024.
 constexpr int kRowThreads = 256, kRowKeys = 32 * kRowThreads;        // the most keys that those hold
+static bool topk_by_few_threads(int rows, int keys) {
+  return rows > 2 * sm_count() && keys <= (rows > 4 * sm_count() ? kRowKeys : 20 * kRowThreads);
+}
 template <int T, class Key>
 __device__ void select_topk_row(Key key, int n, int k, int* out, int* n_out) {
   if constexpr (T == 1024) {
@@ -1243,7 +1249,7 @@ extern "C" int ds41_topk_select_cand(const float* scores, int max_keys, const in
   TopkParams p{scores, max_keys, row_pos, row_slot, ratio, k, sel, n_sel,
                static_cast<const uint32_t*>(cand_mask), cand_words, cand_block};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (rows > 2 * sm_count() && ratio > 0 && max_keys / ratio <= kRowKeys)
+  if (ratio > 0 && topk_by_few_threads(rows, max_keys / ratio))
     return launch_pdl(topk_select_kernel<kRowThreads>, dim3(rows), dim3(kRowThreads), 0, st, p);
   return launch_pdl(topk_select_kernel<1024>, dim3(rows), dim3(1024), 0, st, p);
 }

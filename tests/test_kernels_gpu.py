@@ -68,6 +68,29 @@ def test_topk_of_many_rows(max_keys, ratio, masked):
     assert masked or int(got[0][1].max()) == topk          # a mask of random bits leaves half of the keys
 
 
+@pytest.mark.parametrize("rows", [296, 297, 592, 593])
+@pytest.mark.parametrize("keys", [4096, 5120, 5121, 8192, 8193])
+def test_topk_around_the_lines_of_its_forms(rows, keys):
+    """The rows of a long pass choose what each of them chooses in a pass of few."""
+    from ds41rt_b200.ops import lib
+    k, topk = lib.kernels(), 512
+    torch.manual_seed(keys + rows)
+    scores = torch.randn(rows, keys, device="cuda")
+    scores[::2] = (scores[::2] * 4).round()
+    pos = torch.randint(0, keys, (rows,), device="cuda", dtype=torch.int32)
+    pos[::3] = keys - 1
+    slot = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    got = []
+    for step in (rows, 74):
+        sel, n = torch.zeros(rows, topk, dtype=torch.int32, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda")
+        for r in range(0, rows, step):
+            lib.check(k.ds41_topk_select(lib.ptr(scores[r:]), keys, lib.ptr(pos[r:]), lib.ptr(slot[r:]), 1, topk, lib.ptr(sel[r:]),
+                                         lib.ptr(n[r:]), min(step, rows - r), lib.stream()), "topk")
+        torch.cuda.synchronize()
+        got.append((sel, n))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def _attend_ref(q, keys, sink, scale):
     # q [H, D], keys [n, D]
     logits = (q @ keys.t()) * scale
