@@ -481,11 +481,9 @@ __global__ void __launch_bounds__(128) group_attend_plain_kernel(ds41_group_atte
 // the warps in shared memory, over the CTAs of the cluster through distributed shared memory.
 // KD: 16-column pieces of the key width, NP: of the value width.  A warp's walk is a chain of latencies, so a CTA has eight
 // of them; four, and two CTAs share an SM, where there are more CTAs than SMs (or the value width takes the registers).
+// Asking L2 for the first tiles' rows before the wait for the previous kernel was slower, with rows in L2 and from memory: 4 rows of 32 heads
+// (8 kv) over 4097 keys, 4 splits 14.2 and 15.6 us, 17.1 and 18.3 with it; 32 rows of 8 heads, 8 splits 136 and 146, 157 and 164.
 constexpr int kMaxStages = 4;
-// Tiles of keys that a CTA asks for, on their way to L2, before the wait for the previous kernel.  With the gap between that wait and
-// the first copy (the producer waited for the queries, too), a step of belasun-1b with 8 rows over about 2200 keys and eight of these
-// launches: 1142 us, 1137 so.
-constexpr int kAheadTiles = 8;
 
 struct AttendPlan {
   int warps, kc, vc, stages, box;                     // 64-column chunks, ring length, rows per TMA box
@@ -542,31 +540,12 @@ group_attend_mma_kernel(const __grid_constant__ CUtensorMap pool, const ds41_gro
     tma_prefetch_desc(&pool);
   }
   pdl_launch_dependents();
-  int slot, pos, first, base, t0, t1;
-  auto find = [&]() {                    // this CTA's tiles of keys
-    slot = __ldcg(p.row_slot + r);       // again behind the wait: past L1, which may hold what stood there before
-    pos = __ldcg(p.row_pos + r);
-    first = chunk_start(pos, p.chunk);
-    base = first - first % plan.box;
-    const int tiles = (pos - base) / kTileKeys + 1, per = (tiles + p.n_splits - 1) / p.n_splits;
-    t0 = min(tiles, split * per);
-    t1 = min(tiles, t0 + per);
-  };
-  find();
-  if (slot >= 0) {                       // the cache's rows have left L2 since the last pass
-    const int k0 = base + t0 * kTileKeys, k1 = min(pos + 1, base + min(t1, t0 + kAheadTiles) * kTileKeys);
-    const int k_lines = (dp + 63) / 64, lines = k_lines + (vp + 63) / 64, row_len = p.kv_heads * (dp + vp);
-#pragma unroll 4
-    for (int i = tid; i < (k1 - k0) * lines; i += blockDim.x) {
-      const int key = i / lines, c = i - key * lines;
-      const __nv_bfloat16* kv = cache_row(static_cast<const __nv_bfloat16*>(p.pool), p.page_table, p.max_pages, p.page_tokens,
-                                          row_len, slot, k0 + key);
-      if (kv != nullptr) prefetch_l2(kv + (c < k_lines ? g * dp + 64 * c : p.kv_heads * dp + g * vp + 64 * (c - k_lines)));
-    }
-  }
   __syncthreads();                       // the barriers are ready
   pdl_wait();
-  find();
+  const int slot = p.row_slot[r], pos = p.row_pos[r];
+  const int first = chunk_start(pos, p.chunk), base = first - first % plan.box;      // this CTA's tiles of keys
+  const int tiles = (pos - base) / kTileKeys + 1, per = (tiles + p.n_splits - 1) / p.n_splits;
+  const int t0 = min(tiles, split * per), t1 = min(tiles, t0 + per);
   __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out) + 1ll * r * p.ld_out;
   if (slot < 0) {                        // the same in every CTA of the cluster
     if (split == 0)
