@@ -11,6 +11,7 @@
 #include "ds41_api.h"
 #include "ds41_launch.cuh"
 #include "ds41_ptx.cuh"
+#include "ds41_tma.h"
 
 namespace ds41 {
 
@@ -89,10 +90,14 @@ struct QkvPostParams {
   float eps;
 };
 
-// vals[n] += the planes of column c + n step, in their order, for the columns below `end`.  Four planes of all columns are under way
-// at once: with few rows the launch is a chain of round trips to L2.  One row of ten planes, 1280 + 512 columns, in a graph: 11 us
-// with a column after the other, 3.5 so (weights read before the wait).
-template <typename V, int N>
+// vals[n] += the planes of column c + n step, in their order, for the columns below `end`.
+// kFew: four planes of all columns are under way at once: with few rows the launch is a chain of round trips to L2.  One row of ten planes,
+// 1280 + 512 columns, in a graph: 11 us with a column after the other, 3.5 so (weights read before the wait).
+// Many rows want blocks on an SM instead: kOne, a single plane, and kMany, planes outside and columns inside, do with 46 registers where
+// kFew has 73.  2048 rows of 1280 + 512 columns, one plane 9.3 us (12.4 with kFew), two 12.2 (14.9); 333 rows of 192 + 512, two 3.3 (3.7).
+// 200 rows of 1280 + 512, two planes 3.2 with kMany, 2.3 with kFew.
+enum Planes { kOne, kFew, kMany };
+template <int PLANES, typename V, int N>
 __device__ __forceinline__ void add_columns(V (&vals)[N], const float* row, long long plane, int splits, int c, int step, int end) {
   constexpr int kUnder = 4;
   constexpr int kEach = sizeof(V) / sizeof(float);
@@ -105,31 +110,38 @@ __device__ __forceinline__ void add_columns(V (&vals)[N], const float* row, long
       a.y += b.y;
     }
   };
-  if (splits == 1) {
+  if constexpr (PLANES == kOne) {
 #pragma unroll
     for (int n = 0; n < N; ++n)
       if (c + n * step < end) add(vals[n], at(0, n));
-    return;
-  }
-  for (int s0 = 0; s0 < splits; s0 += kUnder) {
-    V t[kUnder][N];
-#pragma unroll
-    for (int u = 0; u < kUnder; ++u)
+  } else if constexpr (PLANES == kMany) {
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s)
 #pragma unroll
       for (int n = 0; n < N; ++n)
-        if (s0 + u < splits && c + n * step < end) t[u][n] = at(s0 + u, n);
+        if (c + n * step < end) add(vals[n], at(s, n));
+  } else {
+    for (int s0 = 0; s0 < splits; s0 += kUnder) {
+      V t[kUnder][N];
 #pragma unroll
-    for (int u = 0; u < kUnder; ++u)
+      for (int u = 0; u < kUnder; ++u)
 #pragma unroll
-      for (int n = 0; n < N; ++n)
-        if (s0 + u < splits && c + n * step < end) add(vals[n], t[u][n]);
+        for (int n = 0; n < N; ++n)
+          if (s0 + u < splits && c + n * step < end) t[u][n] = at(s0 + u, n);
+#pragma unroll
+      for (int u = 0; u < kUnder; ++u)
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+          if (s0 + u < splits && c + n * step < end) add(vals[n], t[u][n]);
+    }
   }
 }
 
 constexpr int kOwnExtras = 256;       // up to one column a thread (200 rows, 8 columns of 10 planes: 7.0 us by the kv block, 7.5)
 // grid (rows, 2 or 3): block y == 0 normalises the q latent, y == 1 handles kv (norm + RoPE + ring write), and the extras unless
 // there are enough for a block y == 2.
-__global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
+template <int PLANES>
+__global__ void __launch_bounds__(256, PLANES == kFew ? 3 : 5) qkv_post_kernel(QkvPostParams p) {
   __shared__ float scratch[8];
   const int r = blockIdx.x, tid = threadIdx.x;
   const long long plane = 1ll * p.rows * p.ntot;
@@ -145,7 +157,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
       w[n] = tid + 256 * n < p.Q ? p.q_norm_w[tid + 256 * n] : 0.f;      // weights: read before the wait
     }
     pdl_wait();
-    add_columns(vals, row0, plane, p.splits, tid, 256, p.Q);
+    add_columns<PLANES>(vals, row0, plane, p.splits, tid, 256, p.Q);
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       vals[n] = bf16_round(vals[n]);
@@ -164,7 +176,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
   auto extras = [&]() {
     for (int c0 = tid; c0 < p.extra_f32; c0 += 256 * 4) {
       float a[4] = {0.f, 0.f, 0.f, 0.f};
-      add_columns(a, row0 + p.Q + p.D, plane, p.splits, c0, 256, p.extra_f32);
+      add_columns<PLANES>(a, row0 + p.Q + p.D, plane, p.splits, c0, 256, p.extra_f32);
 #pragma unroll
       for (int n = 0; n < 4; ++n) {
         const int c = c0 + 256 * n;
@@ -191,7 +203,7 @@ __global__ void __launch_bounds__(256) qkv_post_kernel(QkvPostParams p) {
   }
   pdl_wait();
   const int pos = p.row_pos[r], slot = p.row_slot[r];
-  add_columns(kvv, row0 + p.Q, plane, p.splits, tid, 256, p.D / 2);
+  add_columns<PLANES>(kvv, row0 + p.Q, plane, p.splits, tid, 256, p.D / 2);
 #pragma unroll
   for (int n = 0; n < 4; ++n) {
     kvv[n] = make_float2(bf16_round(kvv[n].x), bf16_round(kvv[n].y));
@@ -385,8 +397,8 @@ extern "C" int ds41_qkv_post(const float* planes, int splits, int rows, int ntot
   // kv columns are read as aligned float2
   if (((Q + D) & 1) || ((ntot & 1) && (rows > 1 || splits > 1)) || (reinterpret_cast<uintptr_t>(planes) & 7))
     return cudaErrorInvalidValue;
-  return launch_pdl(qkv_post_kernel, dim3(rows, extra_f32 > kOwnExtras ? 3 : 2), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                    p);
+  const auto kernel = splits == 1 ? qkv_post_kernel<kOne> : 2 * rows > 3 * sm_count() ? qkv_post_kernel<kMany> : qkv_post_kernel<kFew>;
+  return launch_pdl(kernel, dim3(rows, extra_f32 > kOwnExtras ? 3 : 2), dim3(256), 0, static_cast<cudaStream_t>(stream), p);
 }
 
 extern "C" int ds41_compress(const float* extras, int extra_stride, int rows, int D, int ID, int rope_dim, int ratio,

@@ -997,6 +997,35 @@ def test_qkv_post_sums_planes_in_their_order(rows, Q, extra):
     assert bool(win[0, 7:7 + rows].any(-1).all()) and not bool(win[0, :7].any())
 
 
+@pytest.mark.parametrize("splits", [1, 2, 3, 5, 9])
+@pytest.mark.parametrize("rows", [222, 223, 600])
+@pytest.mark.parametrize("Q,extra", [(1280, 0), (192, 258), (2048, 32)])
+def test_qkv_post_of_many_rows(rows, splits, Q, extra):
+    """The rows of a long pass hold the bits that each of them gets in a pass of few."""
+    from ds41rt_b200.ops import lib
+    k = lib.kernels()
+    torch.manual_seed(rows + splits)
+    D, rope, ring = 512, 64, 640
+    ntot = Q + D + extra
+    planes = torch.randn(splits, rows, ntot, device="cuda")
+    qn, kn, inv = torch.rand(Q, device="cuda") + 0.5, torch.rand(D, device="cuda") + 0.5, torch.rand(rope // 2, device="cuda")
+    pos, slot = torch.arange(rows, dtype=torch.int32, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda")
+    got = []
+    for step in (rows, 75):
+        ql, win = torch.zeros(rows, Q, device="cuda", dtype=torch.bfloat16), torch.zeros(1, ring, D, device="cuda", dtype=torch.bfloat16)
+        ex = torch.zeros(rows, max(extra, 1), device="cuda")
+        for r in range(0, rows, step):
+            n = min(step, rows - r)
+            part = planes[:, r:r + n].contiguous()
+            lib.check(k.ds41_qkv_post(lib.ptr(part), splits, n, ntot, Q, D, rope, extra, min(extra, 4), C.c_float(0.25), lib.ptr(qn),
+                                      lib.ptr(kn), lib.ptr(inv), lib.ptr(pos[r:]), lib.ptr(slot[r:]), lib.ptr(ql[r:]), lib.ptr(win),
+                                      ring, lib.ptr(ex[r:]), C.c_float(1e-6), 0, lib.stream()), "qkv_post")
+        torch.cuda.synchronize()
+        got.append((ql, win, ex))
+    assert bool(got[0][0].any(1).all()) and bool(got[0][1][0, :rows].any(1).all())
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 @pytest.mark.parametrize("rows,topk,splits", [(1, 6, 0), (1, 6, 8), (3, 8, 9), (2, 9, 1), (5, 17, 20)])
 def test_combine_of_routes_and_shared_planes(rows, topk, splits):
     """Around the number of routes and planes that are under way together, absent routes among them; same order, same bits."""
