@@ -131,6 +131,9 @@ struct BlockExchange {
 // The CTAs of a cluster: every warp sends its moments to all of them, 16 bytes each, and counts on a barrier there; a warp waits for
 // its own CTA's copy alone.  (A barrier of the cluster and loads from the peers afterwards: 2000 cycles a norm instead of 1000.)
 constexpr int kShare = 8;              // CTAs that share a row
+// Rows of more than 16384 columns: beyond this many, a fourth block an SM counts for more than its registers.  20000 columns, three and four
+// blocks: 1 row of eight planes 13.7 and 15.5 us, with gate and kept streams 25 and 31; 200 rows 39 and 34, 133 and 118.
+constexpr int kLeanRows = 64;
 struct RowShare {
   float4 moments[32];
   uint64_t bar;
@@ -191,12 +194,9 @@ __device__ __forceinline__ void proj_pieces(const ds41_proj& a, long long row, c
     for (int i = 0; i < NI; ++i)
       v[i] = make_float4(__uint_as_float(raw[i].x << 16), __uint_as_float(raw[i].x & 0xffff0000u), __uint_as_float(raw[i].y << 16),
                          __uint_as_float(raw[i].y & 0xffff0000u));
-  } else if (a.splits == 1) {
+  } else {                                // one fp32 plane
 #pragma unroll
     for (int i = 0; i < NI; ++i) v[i] = *reinterpret_cast<const float4*>(static_cast<const float*>(a.data) + i0 + at[i]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < NI; ++i) v[i] = proj_at4(a, row, at[i]);
   }
 }
 // The same of the sum of a row's routed results (bf16 rows, one per route, at most four routes), in route order.
@@ -226,13 +226,15 @@ __device__ __forceinline__ void routed_pieces(const ds41_resid_args& p, int r, c
 }
 
 // Many rows: bound by latency, a block's loads and its two chains of merges one after the other.  Rows that fill the threads'
-// pieces (FULL) shorten the chain by every test of a column against the row's end, and ask for stream, result and gate at once.
-// Piece by piece, with a test of the projection's form between two loads, 2048 rows x 4096 columns took 28 us (plain result), 49
-// (gated, two norms), 73 (the same with four kept streams) and 54 (four routes); together 26, 44, 70 and 26; 953 rows with routes
-// 30 and 16.  Kept streams stay behind the first norm: asked for with the rest they cost the registers of a third block an SM
-// (kept streams 82 us).
-template <typename T, int NI, bool FULL>
-__global__ void __launch_bounds__(NI <= 4 ? 256 : 512) resid_step_kernel(ds41_resid_args p) {
+// pieces (FULL) shorten the chain by every test of a column against the row's end, and where their form allows it (TOGETHER, see
+// pieces_together) ask for stream, result and gate at once.  Piece by piece, with a test of the projection's form between two loads,
+// 2048 rows x 4096 columns took 28 us (plain result), 49 (gated, two norms), 73 (the same with four kept streams) and 54 (four
+// routes); together 26, 44, 70 and 26; 953 rows with routes 30 and 16.  Kept streams stay behind the first norm: asked for with the
+// rest they cost the registers of a third block an SM (kept streams 82 us).  The forms are kernels of their own: in one they
+// spilled, 2048 rows x 1024 columns 9.5 us (7.8 so).  Results of several planes come in passes of few rows, whose blocks need no
+// neighbours: those of two pieces take what registers they like (33 rows x 2048, gate and kept streams 8.2 and 7.2 us).
+template <typename T, int NI, bool FULL, bool TOGETHER>
+__global__ void __launch_bounds__(NI <= 4 ? 256 : 512, NI == 2 && FULL && !TOGETHER ? 1 : 0) resid_step_kernel(ds41_resid_args p) {
   __shared__ float slots[2][96];
   const int r = blockIdx.x, n_warps = blockDim.x >> 5;
   pdl_launch_dependents();
@@ -272,21 +274,15 @@ __global__ void __launch_bounds__(NI <= 4 ? 256 : 512) resid_step_kernel(ds41_re
       v.z *= sigmoid_f32(g.z + b.z);
       v.w *= sigmoid_f32(g.w + b.w);
     };
-    bool whole = false;
-    if constexpr (FULL) {
-      const bool routed = p.y_route != nullptr;
-      whole = !routed || (p.y.bf16 && p.y_rows == 0 && p.y_top <= kRoutes);
-      if (whole) {
-        if (routed) routed_pieces(p, r, at, y);
-        else proj_pieces(p.y, r, at, y);
-        float4 g[NI];
-        if (p.gate.data != nullptr) proj_pieces(p.gate, r, at, g);
-        if (p.gate.data != nullptr)
+    if constexpr (TOGETHER) {
+      if (p.y_route != nullptr) routed_pieces(p, r, at, y);
+      else proj_pieces(p.y, r, at, y);
+      float4 g[NI];
+      if (p.gate.data != nullptr) proj_pieces(p.gate, r, at, g);
+      if (p.gate.data != nullptr)
 #pragma unroll
-          for (int i = 0; i < NI; ++i) gated(y[i], g[i], load4(p.gate_bias + at[i], 4));
-      }
-    }
-    if (!whole) {
+        for (int i = 0; i < NI; ++i) gated(y[i], g[i], load4(p.gate_bias + at[i], 4));
+    } else {
 #pragma unroll
       for (int i = 0; i < NI; ++i) {
         y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -407,8 +403,8 @@ __device__ __forceinline__ float4 routed_few4(const ds41_resid_args& p, int r, i
 // columns, a piece of four a thread), and each norm costs one way to the peers.  Inside a graph, one row of 2048 columns with
 // kept streams and eight planes of result and gate: 10.3 us with loads plane by plane, divisions in every merge of moments and a
 // cluster barrier with loads from the peers behind it, 6.5 so; eight rows without kept streams 5.0 and 4.2.
-template <typename T, int NI, bool FULL>
-__global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
+template <typename T, int NI, bool FULL, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) resid_few_kernel(ds41_resid_args p) {
   __shared__ RowShare share[2];
   const int per = ((p.W + kShare - 1) / kShare + 3) / 4 * 4;
   const int part = blockIdx.x % kShare, r = blockIdx.x / kShare, lane = threadIdx.x & 31;
@@ -420,17 +416,26 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
   cg::cluster_group::barrier_arrive();
   pdl_launch_dependents();
   const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
-  float4 x[NI], y[NI], older[NI], w_next[NI], w_post[NI], bias[NI];
+  // More pieces than the registers hold beside their weights: those are read, and the stream stored, where they are needed.  With
+  // everything held, 200 rows of 20000 columns took 69 us (plain bf16 result), 95 (gated) and 190 (with kept streams).
+  constexpr bool kLean = NI > 2;
+  constexpr int kHeld = kLean ? 1 : NI;
+  float4 x[NI], y[NI], older[NI], w_next[kHeld], w_post[kHeld], bias[kHeld], stream[kHeld];
   int at[NI], live[NI];
+  auto next_at = [&](int i) { return p.next_w != nullptr && live[i] > 0 ? load4(p.next_w + at[i], live[i]) : zero; };
+  auto post_at = [&](int i) { return p.post_w != nullptr && live[i] > 0 ? load4(p.post_w + at[i], live[i]) : one; };
+  auto bias_at = [&](int i) { return p.gate.data != nullptr && live[i] > 0 ? load4(p.gate_bias + at[i], live[i]) : zero; };
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
     const int c = 4 * (threadIdx.x + i * blockDim.x);
     live[i] = FULL ? 4 : n - c;
     at[i] = c0 + c;
     x[i] = y[i] = older[i] = zero;
-    w_next[i] = p.next_w != nullptr && live[i] > 0 ? load4(p.next_w + at[i], live[i]) : zero;
-    w_post[i] = p.post_w != nullptr && live[i] > 0 ? load4(p.post_w + at[i], live[i]) : one;
-    bias[i] = p.gate.data != nullptr && live[i] > 0 ? load4(p.gate_bias + at[i], live[i]) : zero;
+    if constexpr (!kLean) {
+      w_next[i] = next_at(i);
+      w_post[i] = post_at(i);
+      bias[i] = bias_at(i);
+    }
   }
   const int n_old = p.mix != nullptr ? p.n_mix - 1 : 0;
   const float mix_lane = lane <= n_old && p.mix != nullptr ? p.mix[lane] : 0.f;
@@ -463,7 +468,7 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
   if (p.y.data != nullptr && p.y_route != nullptr)
 #pragma unroll
     for (int i = 0; i < NI; ++i)
-      if (live[i] > 0) y[i] = routed_few4(p, r, at[i]);
+      if (live[i] > 0) y[i] = kLean ? routed_at4(p, r, at[i]) : routed_few4(p, r, at[i]);
   // ---- the weighted sum of the older kept streams
   auto add_old = [&](int i, float c, float4 k) {
     older[i].x += c * k.x;
@@ -501,13 +506,14 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (live[i] > 0) {
-        if (plain) y[i] = kAhead ? ya.get(p.y, r, at[i]) : few_at4(p.y, r, at[i]);
+        if (plain) y[i] = kAhead ? ya.get(p.y, r, at[i]) : kLean ? proj_at4(p.y, r, at[i]) : few_at4(p.y, r, at[i]);
         if (p.gate.data != nullptr) {
-          const float4 g = kAhead ? ga.get(p.gate, r, at[i]) : few_at4(p.gate, r, at[i]);
-          y[i].x *= sigmoid_f32(g.x + bias[i].x);
-          y[i].y *= sigmoid_f32(g.y + bias[i].y);
-          y[i].z *= sigmoid_f32(g.z + bias[i].z);
-          y[i].w *= sigmoid_f32(g.w + bias[i].w);
+          const float4 g = kAhead ? ga.get(p.gate, r, at[i]) : kLean ? proj_at4(p.gate, r, at[i]) : few_at4(p.gate, r, at[i]);
+          const float4 b = kLean ? bias_at(i) : bias[i % kHeld];
+          y[i].x *= sigmoid_f32(g.x + b.x);
+          y[i].y *= sigmoid_f32(g.y + b.y);
+          y[i].z *= sigmoid_f32(g.z + b.z);
+          y[i].w *= sigmoid_f32(g.w + b.w);
         }
         clip(y[i], i);
       }
@@ -517,40 +523,41 @@ __global__ void __launch_bounds__(128) resid_few_kernel(ds41_resid_args p) {
 #pragma unroll
     for (int i = 0; i < NI; ++i)
       if (live[i] > 0) {
-        x[i].x += (y[i].x - s.x) * s.y * w_post[i].x;
-        x[i].y += (y[i].y - s.x) * s.y * w_post[i].y;
-        x[i].z += (y[i].z - s.x) * s.y * w_post[i].z;
-        x[i].w += (y[i].w - s.x) * s.y * w_post[i].w;
+        const float4 w = kLean ? post_at(i) : w_post[i % kHeld];
+        x[i].x += (y[i].x - s.x) * s.y * w.x;
+        x[i].y += (y[i].y - s.x) * s.y * w.y;
+        x[i].z += (y[i].z - s.x) * s.y * w.z;
+        x[i].w += (y[i].w - s.x) * s.y * w.w;
       }
   }
-#pragma unroll
-  for (int i = 0; i < NI; ++i) clip(x[i], i);
-  const float4(&stream)[NI] = x;
-  float4 avg[NI];
   const float last = p.mix != nullptr ? weight(n_old) : 0.f;      // the newest kept stream is the row this block holds
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
-    avg[i] = x[i];
-    if (p.mix != nullptr) {
-      avg[i] = make_float4(older[i].x + last * x[i].x, older[i].y + last * x[i].y, older[i].z + last * x[i].z,
-                           older[i].w + last * x[i].w);
-      clip(avg[i], i);
+    clip(x[i], i);
+    if constexpr (!kLean) stream[i] = x[i];
+    else if (p.x_out != nullptr && live[i] > 0) store4(p.x_out + r * p.ldx + at[i], x[i]);
+    if (p.mix != nullptr) {                  // from here on x is what the next sublayer sees
+      x[i] = make_float4(older[i].x + last * x[i].x, older[i].y + last * x[i].y, older[i].z + last * x[i].z,
+                         older[i].w + last * x[i].w);
+      clip(x[i], i);
     }
   }
   float2 s = make_float2(0.f, 1.f);
-  if (p.next_w != nullptr) s = row_norm<NI, FULL>(avg, n, p.W, p.norm_kind, p.eps, ClusterExchange{&share[1], part, warps, p.status});
+  if (p.next_w != nullptr) s = row_norm<NI, FULL>(x, n, p.W, p.norm_kind, p.eps, ClusterExchange{&share[1], part, warps, p.status});
   cg::cluster_group::barrier_arrive();
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
     if (live[i] <= 0) continue;
-    if (p.x_out != nullptr) store4(p.x_out + r * p.ldx + at[i], stream[i]);
-    if (p.mix != nullptr && p.x_avg != nullptr) store4(p.x_avg + r * p.ldx + at[i], avg[i]);
+    if (!kLean && p.x_out != nullptr) store4(p.x_out + r * p.ldx + at[i], stream[i % kHeld]);
+    if (p.mix != nullptr && p.x_avg != nullptr) store4(p.x_avg + r * p.ldx + at[i], x[i]);
     T* h = static_cast<T*>(p.h) + 1ll * r * p.ldh + at[i];
-    if (p.next_w != nullptr)
-      store4(h, make_float4((avg[i].x - s.x) * s.y * w_next[i].x, (avg[i].y - s.x) * s.y * w_next[i].y,
-                            (avg[i].z - s.x) * s.y * w_next[i].z, (avg[i].w - s.x) * s.y * w_next[i].w));
-    else if (p.raw_h)
-      store4(h, avg[i]);
+    if (p.next_w != nullptr) {
+      const float4 w = kLean ? next_at(i) : w_next[i % kHeld];
+      store4(h, make_float4((x[i].x - s.x) * s.y * w.x, (x[i].y - s.x) * s.y * w.y, (x[i].z - s.x) * s.y * w.z,
+                            (x[i].w - s.x) * s.y * w.w));
+    } else if (p.raw_h) {
+      store4(h, x[i]);
+    }
   }
   cg::cluster_group::barrier_wait();           // no CTA leaves while a peer may still send to it
 }
@@ -729,18 +736,35 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const T* src, int ld, 
   dst[1ll * r * ld + i] = s >= 0 && s < n_src ? src[1ll * s * ld + i] : from_f32<T>(0.f);
 }
 
+// Can result and gate be asked for in whole pieces: bf16 or one plane, or up to four routes of bf16 rows?  (Not for one piece a thread,
+// which has nothing to ask for together.)
+static bool pieces_together(const ds41_resid_args& a) {
+  auto one = [](const ds41_proj& p) { return p.bf16 || p.splits == 1; };
+  const bool y = a.y_route != nullptr ? a.y.bf16 && a.y_rows == 0 && a.y_top <= kRoutes : one(a.y);
+  return a.y.data != nullptr && y && (a.gate.data == nullptr || one(a.gate));
+}
+
 // FULL: a row fills the pieces of the threads that share it, whose warps' number is a power of two
 template <typename T, bool FEW, int NI>
 static cudaError_t launch_resid_ni(const ds41_resid_args& a, int threads, cudaStream_t st) {
   const bool even = (threads & (threads - 1)) == 0;
   if constexpr (!FEW) {
-    if (even && a.W == 4 * NI * threads)
-      return launch_pdl(resid_step_kernel<T, NI, true>, dim3(a.rows), dim3(threads), 0, st, a);
-    return launch_pdl(resid_step_kernel<T, NI, false>, dim3(a.rows), dim3(threads), 0, st, a);
+    if (even && a.W == 4 * NI * threads) {
+      if constexpr (NI > 1)
+        if (pieces_together(a)) return launch_pdl(resid_step_kernel<T, NI, true, true>, dim3(a.rows), dim3(threads), 0, st, a);
+      return launch_pdl(resid_step_kernel<T, NI, true, false>, dim3(a.rows), dim3(threads), 0, st, a);
+    }
+    return launch_pdl(resid_step_kernel<T, NI, false, false>, dim3(a.rows), dim3(threads), 0, st, a);
   } else {
-    if (even && a.W == kShare * 4 * NI * threads)
-      return launch_pdl_cluster(resid_few_kernel<T, NI, true>, dim3(a.rows * kShare), dim3(threads), kShare, 0, st, a);
-    return launch_pdl_cluster(resid_few_kernel<T, NI, false>, dim3(a.rows * kShare), dim3(threads), kShare, 0, st, a);
+    auto launch = [&](auto full, auto blocks) {
+      return launch_pdl_cluster(resid_few_kernel<T, NI, decltype(full)::value, decltype(blocks)::value>, dim3(a.rows * kShare), dim3(threads),
+                                kShare, 0, st, a);
+    };
+    auto pick = [&](auto full) {
+      if constexpr (NI < 8) return launch(full, std::integral_constant<int, 0>{});
+      else return a.rows > kLeanRows ? launch(full, std::integral_constant<int, 4>{}) : launch(full, std::integral_constant<int, 3>{});
+    };
+    return even && a.W == kShare * 4 * NI * threads ? pick(std::true_type{}) : pick(std::false_type{});
   }
 }
 
