@@ -10,6 +10,7 @@
 //  latent_merge  : sums the splits; the softmax denominator also contains exp(sink) per head
 #include "ds41_mma.cuh"
 #include "ds41_stack.cuh"
+#include "ds41_tma.h"
 
 namespace ds41 {
 
@@ -542,10 +543,11 @@ static int attend_mma_heads(const ds41_latent_attend_args& a) {
 }
 
 // One block per (head, row): the splits' weights first, a thread each, then every thread sums four columns over the splits in
-// their order.  A chain of latencies: in a graph one row of 32 splits 5.8 us with the splits one by one, 4.9 with sixteen under way.
+// their order, eight of them under way together (UNDER), which makes one row of 18 splits 3.3 us instead of 3.7, 5 splits 2.2 instead of
+// 2.8.  Sixteen took 127 registers: 32 rows of 64 heads 7.8 us for one split and 8.3 for four, 4.0 and 4.5 with a split at a time,
+// which is the form of many blocks and of single splits (44 registers).
 constexpr int kMaxSplits = 256;
-constexpr int kUnder = 16;             // splits whose loads are under way together
-template <typename T>
+template <typename T, int UNDER>        // UNDER: splits whose loads are under way together
 __global__ void __launch_bounds__(128) latent_merge_kernel(const float* part_o, const float* part_ml, const float* sink,
                                                            int n_splits, int heads, int kv_pad, T* out, int ld_out) {
   __shared__ float wt[kMaxSplits];
@@ -583,19 +585,33 @@ __global__ void __launch_bounds__(128) latent_merge_kernel(const float* part_o, 
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     const float* part = part_o + cell0 * kv_pad + i;
     const long long step = 1ll * heads * kv_pad;
-    for (int s0 = 0; s0 < n_splits; s0 += kUnder) {
-      float4 o[kUnder];
-#pragma unroll
-      for (int u = 0; u < kUnder; ++u)
-        if (s0 + u < n_splits && wt[s0 + u] > 0.f) o[u] = *reinterpret_cast<const float4*>(part + (s0 + u) * step);
-#pragma unroll
-      for (int u = 0; u < kUnder; ++u) {
-        const float e = s0 + u < n_splits ? wt[s0 + u] : 0.f;
+    if constexpr (UNDER == 1) {
+#pragma unroll 8
+      for (int s = 0; s < n_splits; ++s) {
+        const float e = wt[s];
         if (e > 0.f) {
-          a.x += e * o[u].x;
-          a.y += e * o[u].y;
-          a.z += e * o[u].z;
-          a.w += e * o[u].w;
+          const float4 o = *reinterpret_cast<const float4*>(part + s * step);
+          a.x += e * o.x;
+          a.y += e * o.y;
+          a.z += e * o.z;
+          a.w += e * o.w;
+        }
+      }
+    } else {
+      for (int s0 = 0; s0 < n_splits; s0 += UNDER) {
+        float4 o[UNDER];
+#pragma unroll
+        for (int u = 0; u < UNDER; ++u)
+          if (s0 + u < n_splits && wt[s0 + u] > 0.f) o[u] = *reinterpret_cast<const float4*>(part + (s0 + u) * step);
+#pragma unroll
+        for (int u = 0; u < UNDER; ++u) {
+          const float e = s0 + u < n_splits ? wt[s0 + u] : 0.f;
+          if (e > 0.f) {
+            a.x += e * o[u].x;
+            a.y += e * o[u].y;
+            a.z += e * o[u].z;
+            a.w += e * o[u].w;
+          }
         }
       }
     }
@@ -695,9 +711,11 @@ extern "C" int ds41_latent_merge(const float* part_o, const float* part_ml, cons
     return cudaErrorInvalidValue;
   const dim3 grid(heads, rows);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (f32)
-    return launch_pdl(latent_merge_kernel<float>, grid, dim3(128), 0, st, part_o, part_ml, sink, n_splits, heads, kv_pad,
-                      static_cast<float*>(out), ld_out);
-  return launch_pdl(latent_merge_kernel<__nv_bfloat16>, grid, dim3(128), 0, st, part_o, part_ml, sink, n_splits, heads,
-                    kv_pad, static_cast<__nv_bfloat16*>(out), ld_out);
+  auto launch = [&](auto kernel, auto* o) {
+    return launch_pdl(kernel, grid, dim3(128), 0, st, part_o, part_ml, sink, n_splits, heads, kv_pad, o, ld_out);
+  };
+  const bool under = n_splits > 1 && 1ll * heads * rows <= 4 * sm_count();      // 512 blocks of nine splits: 3.6 and 3.8 us
+  if (f32) return launch(under ? latent_merge_kernel<float, 8> : latent_merge_kernel<float, 1>, static_cast<float*>(out));
+  return launch(under ? latent_merge_kernel<__nv_bfloat16, 8> : latent_merge_kernel<__nv_bfloat16, 1>,
+                static_cast<__nv_bfloat16*>(out));
 }

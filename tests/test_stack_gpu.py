@@ -641,6 +641,25 @@ def test_absorbed_attention_over_many_splits(splits, dtype):
     test_absorbed_attention_over_pages(1, splits, dtype)
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("splits", [1, 2, 7, 8, 9, 33])
+def test_merge_of_many_blocks(splits, dtype):
+    """Rows of a large pass get the bits that each of them gets in a small one."""
+    lib, S, k = _stack()
+    rows, H, kvp, g = 150, 5, 144, gen(splits)
+    part, ml = torch.randn(rows, splits, H, kvp, generator=g).cuda(), torch.rand(rows, splits, H, 2, generator=g).cuda()
+    ml[::4, ::2] = torch.tensor([float("-inf"), 0.0], device="cuda")      # splits without a key
+    got = []
+    for step in (rows, 50):
+        out = torch.full((rows, H * kvp), float("nan"), dtype=dtype, device="cuda")
+        for r in range(0, rows, step):
+            _ok(k.ds41_latent_merge(lib.ptr(part[r:]), lib.ptr(ml[r:]), None, splits, step, H, kvp, lib.ptr(out[r:]), H * kvp,
+                                    int(dtype == F32), lib.stream()))
+        torch.cuda.synchronize()
+        got.append(out)
+    assert not got[0].isnan().any() and torch.equal(*got)
+
+
 @pytest.mark.parametrize("sink", [False, True])
 @pytest.mark.parametrize("splits,kvp", [(9, 144), (17, 512), (32, 512), (66, 576), (128, 16), (130, 144), (256, 48)])
 def test_merge_adds_the_splits_in_their_order(splits, kvp, sink):
