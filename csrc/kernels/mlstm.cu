@@ -15,6 +15,7 @@
 //               fp32 factors of a product (state, decayed scores, decayed values) enter as bf16 high and low parts.
 #include "ds41_mma.cuh"
 #include "ds41_stack.cuh"
+#include "ds41_tma.h"
 
 namespace ds41 {
 
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(256) mlstm_step_kernel(ds41_mlstm_args p) {
 // The same walk with the state in registers: thread (warp, lane) holds rows d = 32 i + 4 warp + lane / 8 and the four columns
 // 4 (lane % 8), i < NR.
 template <int NR>
-__global__ void __launch_bounds__(256) mlstm_walk_kernel(ds41_mlstm_args p) {
+__global__ void __launch_bounds__(256) mlstm_walk_kernel(ds41_mlstm_args p, int ask_early) {
   constexpr int D = NR * 32;
   __shared__ float qs[D], ks[D];
   __shared__ float n[D];
@@ -120,10 +121,9 @@ __global__ void __launch_bounds__(256) mlstm_walk_kernel(ds41_mlstm_args p) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   pdl_launch_dependents();
   int r = blockIdx.z;
-  // the state has left L2 since the last pass: its lines are asked for while the previous kernel ends (one row, 4 heads of 256 x 512:
-  // 8.8 and 8.1 us; 32 rows, 8 heads 55 and 53)
-  // (__ldcg: past L1, which would answer the reads behind the wait)
-  const int early = __ldcg(p.row_slot + r);
+  // The state has left L2 since the last pass: its lines are asked for while the previous kernel ends.  (__ldcg: past L1, which would
+  // answer the reads behind the wait.)
+  const int early = ask_early ? __ldcg(p.row_slot + r) : -1;
   if (early >= 0 && (r == 0 || __ldcg(p.row_slot + r - 1) != early) && early < p.slots && __ldcg(p.row_pos + r) != 0) {
     const long long head = 1ll * early * p.heads + h;
     for (int d = tid; d < p.dim_pad; d += 256)
@@ -789,11 +789,15 @@ extern "C" int ds41_mlstm_step(const ds41_mlstm_args* a, void* stream) {
   if (!(a->vdim_pad & 3) && a->dim_pad <= 512 && !(reinterpret_cast<uintptr_t>(a->state_s) & 15)) {
     const dim3 grid((a->vdim_pad + kStateCols - 1) / kStateCols, a->heads, a->rows);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (a->dim_pad <= 32) return launch_pdl(mlstm_walk_kernel<1>, grid, dim3(256), 0, st, *a);
-    if (a->dim_pad <= 64) return launch_pdl(mlstm_walk_kernel<2>, grid, dim3(256), 0, st, *a);
-    if (a->dim_pad <= 128) return launch_pdl(mlstm_walk_kernel<4>, grid, dim3(256), 0, st, *a);
-    if (a->dim_pad <= 256) return launch_pdl(mlstm_walk_kernel<8>, grid, dim3(256), 0, st, *a);
-    return launch_pdl(mlstm_walk_kernel<16>, grid, dim3(256), 0, st, *a);
+    // States of 256 x 512, us with and without early lines, from memory / from L2: 1 row of 4 heads (64 blocks) 4.9 and 5.7 / 4.5 and 4.8,
+    // 4 rows (256) 6.8 and 7.6 / 7.0 and 7.0; 4 rows of 8 heads (512) 10.1 and 10.4 / 8.5 and 7.5, 32 rows (4096) 63.0 and 62.1 /
+    // 62.3 and 61.9.
+    const int ask_early = 1ll * grid.x * grid.y * grid.z <= 2 * sm_count();
+    if (a->dim_pad <= 32) return launch_pdl(mlstm_walk_kernel<1>, grid, dim3(256), 0, st, *a, ask_early);
+    if (a->dim_pad <= 64) return launch_pdl(mlstm_walk_kernel<2>, grid, dim3(256), 0, st, *a, ask_early);
+    if (a->dim_pad <= 128) return launch_pdl(mlstm_walk_kernel<4>, grid, dim3(256), 0, st, *a, ask_early);
+    if (a->dim_pad <= 256) return launch_pdl(mlstm_walk_kernel<8>, grid, dim3(256), 0, st, *a, ask_early);
+    return launch_pdl(mlstm_walk_kernel<16>, grid, dim3(256), 0, st, *a, ask_early);
   }
   const size_t smem = (1ull * a->dim_pad * (kStateCols + 3) + kStateCols * 9) * sizeof(float);
   static size_t allowed = 48 * 1024 - 512;
