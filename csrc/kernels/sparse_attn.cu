@@ -544,6 +544,7 @@ struct AttendParams {
   const int* row_lo;           // optional [rows]: lowest visible window position (a window rebuilt from there on)
   int comp_row_bytes;          // > 0: comp_pool rows are FP4 (D/2 e2m1 bytes + D/16 E4M3 scales) of this many bytes;
                                // the window rows must then be FP8 rows (kv_row_bytes > 0)
+  int early;                   // attend_kernel: prepare before the wait for the previous kernel
 };
 
 // Eight values of an FP4 cache row -> bf16 (exact: a 2-bit-mantissa value times a 4-bit-mantissa scale).
@@ -588,13 +589,15 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
   pdl_launch_dependents();
   // While the previous kernel ends: the rotation's table and, on their way to L2, this CTA's rows of the window.  Both follow from the
   // pass's inputs; the table is made again should the position turn out to be another one.  (One row in a graph: 12.5 us with
-  // both behind the wait and the queries loaded before the keys were asked for, 9.2 so.)
+  // both behind the wait and the queries loaded before the keys were asked for, 9.2 so.)  Grids of more than a block an SM, most
+  // of whose blocks have nothing to do in a layer without a selection, are better off without: see launch_attend.
   auto turns = [&](int at) {
     if (tid < p.rope_dim / 2) rope_cs2(at, p.inv_freq[tid], &sCos[tid], &sSin[tid]);
   };
-  const int early_pos = __ldcg(p.row_pos + r);      // past L1, which would answer the read behind the wait
-  turns(early_pos);
-  {
+  int early_pos = -1;
+  if (p.early) {
+    early_pos = __ldcg(p.row_pos + r);              // past L1, which would answer the read behind the wait
+    turns(early_pos);
     const int lo = max(0, early_pos - p.window + 1), kp = lo + split * kKeysPerCta + (tid & 63), lane_slot = __ldcg(p.row_slot + r);
     const int row_bytes = p.kv_row_bytes > 0 ? p.kv_row_bytes : 2 * D;
     if (lane_slot >= 0 && kp <= early_pos) {
@@ -625,7 +628,7 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
     }
     return;
   }
-  if (pos != early_pos) turns(pos);
+  if (!p.early || pos != early_pos) turns(pos);
   if (tid < kHeadsPerCta) {
     sM[tid] = -INFINITY;
     sL[tid] = 0.f;
@@ -1195,7 +1198,11 @@ static cudaError_t launch_attend(const AttendParams& p, cudaStream_t stream) {
     return launch_pdl(attend_wide_kernel<D>, wgrid, dim3(512), wide, stream, p);
   }
   dim3 grid(p.n_splits, p.rows, (p.heads + kHeadsPerCta - 1) / kHeadsPerCta);
-  return launch_pdl(attend_kernel<D>, grid, dim3(128), smem, stream, p);
+  // Up to a block an SM prepares early.  64 heads of 512, FP8 rows, us with it everywhere, without, and before there was such a thing: layers
+  // without a selection 16 rows 25.3 / 20.6 / 20.3, 60 rows 68 / 60 / 58; with one, 16 rows 60.4 / 59.3 / 59.7; one row 15.8 (17.8).
+  AttendParams a = p;
+  a.early = 1ll * grid.x * grid.y * grid.z <= sm_count();
+  return launch_pdl(attend_kernel<D>, grid, dim3(128), smem, stream, a);
 }
 
 }  // namespace ds41
