@@ -112,6 +112,25 @@ __device__ __forceinline__ float4 few_at4(const ds41_proj& a, long long row, int
   if (a.bf16) return proj_at4(a, row, col);
   return sum_planes<float4>(static_cast<const float*>(a.data) + i, a.plane, a.splits);
 }
+// The one way or the other, by what the host knows of the pass.  Eight planes under way take 64 registers where a step has 32, so
+// they are for grids whose blocks all run at once (see planes_together), and pay from three planes on.
+template <bool FEW>
+__device__ __forceinline__ float at1(const ds41_proj& a, long long row, int col) {
+  if constexpr (FEW) return few_at(a, row, col);
+  else return proj_at(a, row, col);
+}
+template <bool FEW>
+__device__ __forceinline__ float2 at2(const ds41_proj& a, long long row, int col) {
+  if constexpr (FEW) return few_at2(a, row, col);
+  else return proj_at2(a, row, col);
+}
+template <bool FEW>
+__device__ __forceinline__ float4 at4(const ds41_proj& a, long long row, int col) {
+  if constexpr (FEW) return few_at4(a, row, col);
+  else return proj_at4(a, row, col);
+}
+inline bool planes_together(const ds41_proj& a, long long blocks, long long most) { return !a.bf16 && a.splits > 2 && blocks <= most; }
+
 __device__ __forceinline__ void store2(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
 __device__ __forceinline__ void store2(__nv_bfloat16* p, float x, float y) {
   *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y);

@@ -13,6 +13,7 @@
 #include <cooperative_groups.h>
 
 #include "ds41_stack.cuh"
+#include "ds41_tma.h"
 
 namespace ds41 {
 
@@ -613,19 +614,19 @@ __global__ void __launch_bounds__(512) polynorm_kernel(ds41_proj z, const float*
   }
 }
 
-template <typename T>
+template <typename T, bool FEW>
 __global__ void __launch_bounds__(256) gate_mul_kernel(ds41_proj y, ds41_proj gate, int n, T* out, int ld_out) {
   const int r = blockIdx.y, i = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   pdl_launch_dependents();
   pdl_wait();
   if (i >= n) return;
-  const float4 v = few_at4(y, r, i), g = few_at4(gate, r, i);
+  const float4 v = at4<FEW>(y, r, i), g = at4<FEW>(gate, r, i);
   store4(out + 1ll * r * ld_out + i, make_float4(v.x * sigmoid_f32(g.x), v.y * sigmoid_f32(g.y), v.z * sigmoid_f32(g.z),
                                                  v.w * sigmoid_f32(g.w)));
 }
 
 // one block per (row, head); columns [width, stride) of a head are padding and are written as zeros
-template <typename T>
+template <typename T, bool FEW>
 __global__ void __launch_bounds__(128) head_norm_gate_kernel(const float* o, int ld_o, ds41_proj gate, const float* w,
                                                              int width, int stride, float eps, T* out, int ld_out) {
   __shared__ float red[4];
@@ -640,7 +641,7 @@ __global__ void __launch_bounds__(128) head_norm_gate_kernel(const float* o, int
     const float4 v = load4(src + i, width - i);
     if (i < 4 * static_cast<int>(blockDim.x)) {
       v0 = v;
-      g0 = few_at4(gate, r, h * stride + i);
+      g0 = at4<FEW>(gate, r, h * stride + i);
       w0 = load4(w + h * stride + i, width - i);
     }
     q += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(256) head_norm_gate_warp_kernel(const float* o
 }
 
 // one block per row; columns [n, ld_out) are written as zeros
-template <typename T>
+template <typename T, bool FEW>
 __global__ void __launch_bounds__(128) side_act_kernel(ds41_proj z, const int* tokens, const __nv_bfloat16* embed,
                                                        long long embed_ld, int col, int vocab, int n, T* out, int ld_out) {
   const int r = blockIdx.x;
@@ -711,7 +712,7 @@ __global__ void __launch_bounds__(128) side_act_kernel(ds41_proj z, const int* t
   for (int j = threadIdx.x; j < ld_out; j += blockDim.x) {
     float v = 0.f;
     if (j < n) {
-      const float a = few_at(z, r, j);
+      const float a = at1<FEW>(z, r, j);
       const float e = known ? __bfloat162float(embed[tok * embed_ld + col + j]) : 0.f;
       v = 0.5f * a * (1.0f + tanhf(0.7978845608028654f * (a + 0.044715f * a * a * a))) * e;
     }
@@ -837,9 +838,13 @@ extern "C" int ds41_gate_mul(const ds41_proj* y, const ds41_proj* gate, int rows
     return cudaErrorInvalidValue;
   const dim3 grid((n + 1023) / 1024, rows);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (f32) return launch_pdl(gate_mul_kernel<float>, grid, dim3(256), 0, st, *y, *gate, n, static_cast<float*>(out), ld_out);
-  return launch_pdl(gate_mul_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, *y, *gate, n,
-                    static_cast<__nv_bfloat16*>(out), ld_out);
+  // 4096 columns, us with planes together / one after the other: 64 rows (256 blocks) of four 2.7 / 3.1, 200 rows (800) 4.0 / 3.6; 2048 rows
+  // of one 16.6 / 12.8
+  const long long blocks = 1ll * grid.x * rows;
+  const bool few = planes_together(*y, blocks, 4 * sm_count()) || planes_together(*gate, blocks, 4 * sm_count());
+  auto launch = [&](auto kernel, auto* o) { return launch_pdl(kernel, grid, dim3(256), 0, st, *y, *gate, n, o, ld_out); };
+  if (f32) return launch(few ? gate_mul_kernel<float, true> : gate_mul_kernel<float, false>, static_cast<float*>(out));
+  return launch(few ? gate_mul_kernel<__nv_bfloat16, true> : gate_mul_kernel<__nv_bfloat16, false>, static_cast<__nv_bfloat16*>(out));
 }
 
 extern "C" int ds41_head_norm_gate(const float* o, int ld_o, const ds41_proj* gate, const float* w, int rows, int heads,
@@ -858,11 +863,13 @@ extern "C" int ds41_head_norm_gate(const float* o, int ld_o, const ds41_proj* ga
     return launch_pdl(head_norm_gate_warp_kernel<__nv_bfloat16>, warps, dim3(256), 0, st, o, ld_o, *gate, w, rows * heads,
                       heads, width, stride, eps, static_cast<__nv_bfloat16*>(out), ld_out);
   }
-  if (f32)
-    return launch_pdl(head_norm_gate_kernel<float>, grid, block, 0, st, o, ld_o, *gate, w, width, stride, eps,
-                      static_cast<float*>(out), ld_out);
-  return launch_pdl(head_norm_gate_kernel<__nv_bfloat16>, grid, block, 0, st, o, ld_o, *gate, w, width, stride, eps,
-                    static_cast<__nv_bfloat16*>(out), ld_out);
+  // heads of 256, us with planes together / one after the other: 8 rows of 4096 (128 blocks) of four 2.3 / 2.4, of eight 2.4 / 2.7; 32 rows
+  // (512) of four 2.8 / 2.6, of one 2.4 / 2.2
+  const bool few = planes_together(*gate, 1ll * rows * heads, 2 * sm_count());
+  auto launch = [&](auto kernel, auto* x) { return launch_pdl(kernel, grid, block, 0, st, o, ld_o, *gate, w, width, stride, eps, x, ld_out); };
+  if (f32) return launch(few ? head_norm_gate_kernel<float, true> : head_norm_gate_kernel<float, false>, static_cast<float*>(out));
+  return launch(few ? head_norm_gate_kernel<__nv_bfloat16, true> : head_norm_gate_kernel<__nv_bfloat16, false>,
+                static_cast<__nv_bfloat16*>(out));
 }
 
 extern "C" int ds41_side_act(const ds41_proj* z, const int* tokens, const void* embed, long long embed_ld, int col, int vocab,
@@ -872,11 +879,11 @@ extern "C" int ds41_side_act(const ds41_proj* z, const int* tokens, const void* 
     return cudaErrorInvalidValue;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16* e = static_cast<const __nv_bfloat16*>(embed);
-  if (f32)
-    return launch_pdl(side_act_kernel<float>, dim3(rows), dim3(128), 0, st, *z, tokens, e, embed_ld, col, vocab, n,
-                      static_cast<float*>(out), ld_out);
-  return launch_pdl(side_act_kernel<__nv_bfloat16>, dim3(rows), dim3(128), 0, st, *z, tokens, e, embed_ld, col, vocab, n,
-                    static_cast<__nv_bfloat16*>(out), ld_out);
+  // 256 columns, us with planes together / one after the other: 200 rows of four 2.0 / 2.5, 2048 rows of two 4.1 / 3.7
+  const bool few = planes_together(*z, rows, 4 * sm_count());
+  auto launch = [&](auto kernel, auto* o) { return launch_pdl(kernel, dim3(rows), dim3(128), 0, st, *z, tokens, e, embed_ld, col, vocab, n, o, ld_out); };
+  if (f32) return launch(few ? side_act_kernel<float, true> : side_act_kernel<float, false>, static_cast<float*>(out));
+  return launch(few ? side_act_kernel<__nv_bfloat16, true> : side_act_kernel<__nv_bfloat16, false>, static_cast<__nv_bfloat16*>(out));
 }
 
 extern "C" int ds41_softcap_rows(float* x, long long n, float cap, void* stream) {
