@@ -12,6 +12,7 @@ Reference behaviour being replaced: lazily captured per-shape CUDA graphs keyed 
 """
 from __future__ import annotations
 
+import array
 import ctypes as C
 from typing import Dict, List, Optional
 
@@ -32,6 +33,7 @@ class DecodeSession:
         self.h_in = torch.zeros(3 * R, dtype=torch.int32).pin_memory()
         self.h_chosen = torch.zeros(R, dtype=torch.int32).pin_memory()
         self._in, self._chosen = self.h_in.numpy(), self.h_chosen.numpy()
+        self._view = memoryview(self._in)             # takes a list's numbers in a fifth of the array's time
         self.h2d_bytes = 0
         self.d2h_bytes = 0
 
@@ -60,7 +62,10 @@ class DecodeSession:
         if not 0 < n <= e.max_rows:
             raise ValueError(f"a step has 1 to {e.max_rows} rows, not {n}")
         for i, values in enumerate((tokens, positions, slots)):
-            self._in[i * n:(i + 1) * n] = whole_numbers(values)
+            try:
+                self._view[i * n:(i + 1) * n] = array.array("i", values if type(values) is list else whole_numbers(values))
+            except (TypeError, ValueError, OverflowError):       # other numbers, or one for all rows
+                self._in[i * n:(i + 1) * n] = whole_numbers(values)
         self.h2d_bytes += 3 * 4 * n
         g = self.graph(n)
         src, dst, s = lib.ptr(self.h_in), lib.ptr(self.h_chosen), lib.stream()
