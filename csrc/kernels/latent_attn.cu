@@ -8,6 +8,8 @@
 //  latent_attend : causal attention over the cache with absorbed queries (q W_uk, so that the latent row itself is key and
 //                  value), partial results per key split
 //  latent_merge  : sums the splits; the softmax denominator also contains exp(sink) per head
+#include <type_traits>
+
 #include "ds41_mma.cuh"
 #include "ds41_stack.cuh"
 #include "ds41_tma.h"
@@ -721,8 +723,15 @@ extern "C" int ds41_latent_merge(const float* part_o, const float* part_ml, cons
   auto launch = [&](auto kernel, auto* o) {
     return launch_pdl(kernel, grid, dim3(128), 0, st, part_o, part_ml, sink, n_splits, heads, kv_pad, o, ld_out);
   };
-  const bool under = n_splits > 1 && 1ll * heads * rows <= 4 * sm_count();      // 512 blocks of nine splits: 3.6 and 3.8 us
-  if (f32) return launch(under ? latent_merge_kernel<float, 8> : latent_merge_kernel<float, 1>, static_cast<float*>(out));
-  return launch(under ? latent_merge_kernel<__nv_bfloat16, 8> : latent_merge_kernel<__nv_bfloat16, 1>,
-                static_cast<__nv_bfloat16*>(out));
+  // 512 blocks of nine splits: eight under way 3.6 us, one 3.8.  One row of 16 heads, attention and merge: 18 splits 9.2 us with eight under
+  // way, 9.3 with sixteen; 32 splits 15.3 and 15.1.
+  auto by_type = [&](auto under) {
+    constexpr int U = decltype(under)::value;
+    if (f32) return launch(latent_merge_kernel<float, U>, static_cast<float*>(out));
+    return launch(latent_merge_kernel<__nv_bfloat16, U>, static_cast<__nv_bfloat16*>(out));
+  };
+  const long long blocks = 1ll * heads * rows;
+  if (n_splits == 1 || blocks > 4 * sm_count()) return by_type(std::integral_constant<int, 1>{});
+  if (n_splits > 24 && blocks <= sm_count()) return by_type(std::integral_constant<int, 16>{});
+  return by_type(std::integral_constant<int, 8>{});
 }
