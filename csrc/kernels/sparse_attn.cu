@@ -544,7 +544,6 @@ struct AttendParams {
   const int* row_lo;           // optional [rows]: lowest visible window position (a window rebuilt from there on)
   int comp_row_bytes;          // > 0: comp_pool rows are FP4 (D/2 e2m1 bytes + D/16 E4M3 scales) of this many bytes;
                                // the window rows must then be FP8 rows (kv_row_bytes > 0)
-  int early;                   // attend_kernel: prepare before the wait for the previous kernel
 };
 
 // Eight values of an FP4 cache row -> bf16 (exact: a 2-bit-mantissa value times a 4-bit-mantissa scale).
@@ -566,7 +565,9 @@ constexpr int kHeadsPerCta = 16;
 // grid (n_splits, rows, ceil(heads/16)), 128 threads: one CTA = 16 heads x the 64-key tiles split, split + n_splits, ...
 // of one row, folded with a running softmax; n_splits = number of tiles gives one tile per CTA (decode), a small
 // n_splits keeps the partial outputs of long passes small (prefill).
-template <int D>
+// EARLY: what follows from the pass's inputs is done before the wait for the previous kernel, and the queries are loaded while the first
+// keys are on their way.
+template <int D, bool EARLY>
 __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
   constexpr int LD = D + 8;                                // padded row (bf16 elements)
   extern __shared__ __align__(16) uint8_t smem_attn[];
@@ -589,13 +590,13 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
   pdl_launch_dependents();
   // While the previous kernel ends: the rotation's table and, on their way to L2, this CTA's rows of the window.  Both follow from the
   // pass's inputs; the table is made again should the position turn out to be another one.  (One row in a graph: 12.5 us with
-  // both behind the wait and the queries loaded before the keys were asked for, 9.2 so.)  Grids of more than a block an SM, most
-  // of whose blocks have nothing to do in a layer without a selection, are better off without: see launch_attend.
+  // both behind the wait and the queries loaded before the keys were asked for, 9.2 so.)  In larger grids most blocks have no previous
+  // kernel to wait for, or in a layer without a selection nothing to do at all: see launch_attend.
   auto turns = [&](int at) {
     if (tid < p.rope_dim / 2) rope_cs2(at, p.inv_freq[tid], &sCos[tid], &sSin[tid]);
   };
   int early_pos = -1;
-  if (p.early) {
+  if constexpr (EARLY) {
     early_pos = __ldcg(p.row_pos + r);              // past L1, which would answer the read behind the wait
     turns(early_pos);
     const int lo = max(0, early_pos - p.window + 1), kp = lo + split * kKeysPerCta + (tid & 63), lane_slot = __ldcg(p.row_slot + r);
@@ -628,7 +629,7 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
     }
     return;
   }
-  if (!p.early || pos != early_pos) turns(pos);
+  if (!EARLY || pos != early_pos) turns(pos);
   if (tid < kHeadsPerCta) {
     sM[tid] = -INFINITY;
     sL[tid] = 0.f;
@@ -655,6 +656,10 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
       *reinterpret_cast<uint4*>(sQ + h * LD + ch * 8) = raw;
     }
   };
+  if constexpr (!EARLY) {
+    __syncthreads();
+    load_q();
+  }
   constexpr int NT = D / 32;
   float acc[NT][4];
 #pragma unroll
@@ -697,7 +702,7 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
         if (src != nullptr) cp_async_16(dst, src + ch * 8);
         else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
       }
-      if (tile == split) load_q();
+      if (EARLY && tile == split) load_q();
       cp_async_wait_all();
       __syncthreads();
     } else {
@@ -712,7 +717,7 @@ __global__ void __launch_bounds__(128) attend_kernel(AttendParams p) {
         if (src == nullptr) *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
         else if (ch < (k0 + key >= n_w ? comp_chunks : chunks)) cp_async_16(dst, src + ch * 16);   // FP4 rows are shorter
       }
-      if (tile == split) load_q();
+      if (EARLY && tile == split) load_q();
       cp_async_wait_all();
       __syncthreads();
 #pragma unroll 4
@@ -1176,7 +1181,9 @@ static cudaError_t launch_attend(const AttendParams& p, cudaStream_t stream) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(attend_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max));
+    cudaError_t e = cudaFuncSetAttribute(attend_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(attend_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_max));
     if (e != cudaSuccess) return e;
     configured[dev] = true;
   }
@@ -1198,11 +1205,11 @@ static cudaError_t launch_attend(const AttendParams& p, cudaStream_t stream) {
     return launch_pdl(attend_wide_kernel<D>, wgrid, dim3(512), wide, stream, p);
   }
   dim3 grid(p.n_splits, p.rows, (p.heads + kHeadsPerCta - 1) / kHeadsPerCta);
-  // Up to a block an SM prepares early.  64 heads of 512, FP8 rows, us with it everywhere, without, and before there was such a thing: layers
-  // without a selection 16 rows 25.3 / 20.6 / 20.3, 60 rows 68 / 60 / 58; with one, 16 rows 60.4 / 59.3 / 59.7; one row 15.8 (17.8).
-  AttendParams a = p;
-  a.early = 1ll * grid.x * grid.y * grid.z <= sm_count();
-  return launch_pdl(attend_kernel<D>, grid, dim3(128), smem, stream, a);
+  // Up to a block an SM prepares early.  64 heads of 512, with the merge, us with that order everywhere / its opposite: FP8 rows without a
+  // selection, 16 rows 25.3 / 20.2, 60 rows 68 / 58; with one 60 / 57 and 218 / 205; bf16 rows with one, 60 rows 108 / 99; one row with a
+  // selection 13.7 / 15.6.
+  const bool early = 1ll * grid.x * grid.y * grid.z <= sm_count();
+  return launch_pdl(early ? attend_kernel<D, true> : attend_kernel<D, false>, grid, dim3(128), smem, stream, p);
 }
 
 }  // namespace ds41
