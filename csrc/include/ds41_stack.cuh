@@ -113,7 +113,7 @@ __device__ __forceinline__ float4 few_at4(const ds41_proj& a, long long row, int
   return sum_planes<float4>(static_cast<const float*>(a.data) + i, a.plane, a.splits);
 }
 // The one way or the other, by what the host knows of the pass.  Eight planes under way take 64 registers where a step has 32, so
-// they are for grids whose blocks all run at once (see planes_together), and pay from three planes on.
+// they are for grids whose blocks all run at once (see planes_together), and pay from two or three planes on.
 template <bool FEW>
 __device__ __forceinline__ float at1(const ds41_proj& a, long long row, int col) {
   if constexpr (FEW) return few_at(a, row, col);
@@ -129,7 +129,9 @@ __device__ __forceinline__ float4 at4(const ds41_proj& a, long long row, int col
   if constexpr (FEW) return few_at4(a, row, col);
   else return proj_at4(a, row, col);
 }
-inline bool planes_together(const ds41_proj& a, long long blocks, long long most) { return !a.bf16 && a.splits > 2 && blocks <= most; }
+inline bool planes_together(const ds41_proj& a, long long blocks, long long most, int least = 3) {
+  return !a.bf16 && a.splits >= least && blocks <= most;
+}
 
 __device__ __forceinline__ void store2(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
 __device__ __forceinline__ void store2(__nv_bfloat16* p, float x, float y) {

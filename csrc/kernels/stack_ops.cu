@@ -879,8 +879,8 @@ extern "C" int ds41_side_act(const ds41_proj* z, const int* tokens, const void* 
     return cudaErrorInvalidValue;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const __nv_bfloat16* e = static_cast<const __nv_bfloat16*>(embed);
-  // 256 columns, us with planes together / one after the other: 200 rows of four 2.0 / 2.5, 2048 rows of two 4.1 / 3.7
-  const bool few = planes_together(*z, rows, 4 * sm_count());
+  // 256 columns, us with planes together / one after the other: 1 row of two 1.5 / 1.7, 200 rows of four 2.0 / 2.5, 2048 rows of two 4.1 / 3.7
+  const bool few = planes_together(*z, rows, 4 * sm_count(), 2);
   auto launch = [&](auto kernel, auto* o) { return launch_pdl(kernel, dim3(rows), dim3(128), 0, st, *z, tokens, e, embed_ld, col, vocab, n, o, ld_out); };
   if (f32) return launch(few ? side_act_kernel<float, true> : side_act_kernel<float, false>, static_cast<float*>(out));
   return launch(few ? side_act_kernel<__nv_bfloat16, true> : side_act_kernel<__nv_bfloat16, false>, static_cast<__nv_bfloat16*>(out));
