@@ -113,6 +113,8 @@ int ds41_hc_finish(const float* partial, int n_slices, const float* scale, const
                    const void* streams, const float* norm_w, float* next_pre, float* post, float* comb, void* xn,
                    float* tap_mean, void* xq, void* xq_sf, int rows, int H, int iters, float hc_eps, float norm_eps,
                    const float* mix_planes, int mix_splits, long long mix_split_stride, int mix_ld, void* stream);
+// q[i] = v[i] / s[i] by the division of the mixes (ds41_hc.cuh), for comparison with the operator.
+int ds41_quotient(const float* v, const float* s, float* q, long long n, void* stream);
 // hc_post_mix with fn == NULL only expands, stores and leaves row r's sum of squares in partial[r * 25 + 24] (a
 // single slice: hc_finish is then called with n_slices = 1); the 24 mixes
 // projections then come from a GEMM of the stored streams [rows, 4H] with the matrix as bf16 high and low parts

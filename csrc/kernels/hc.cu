@@ -716,6 +716,10 @@ hc_mixes_kernel(const float* __restrict__ partial, const float* __restrict__ sca
   if (lane < 16) comb[r * 16 + lane] = v;
 }
 
+__global__ void __launch_bounds__(256) quotient_kernel(const float* v, const float* s, float* q, long long n) {
+  for (long long i = blockIdx.x * 256ll + threadIdx.x; i < n; i += 256ll * gridDim.x) q[i] = quotient(v[i], s[i]);
+}
+
 }  // namespace ds41
 
 using namespace ds41;
@@ -790,6 +794,13 @@ extern "C" int ds41_hc_post_mix(const void* streams_in, void* streams_out, const
   return launch_pdl(hc_post_mix_kernel, grid, dim3(256), kSmem, static_cast<cudaStream_t>(stream),
                     static_cast<const __nv_bfloat16*>(streams_in), static_cast<__nv_bfloat16*>(streams_out), parts,
                     post, comb, fn, partial, rows, H, wait_flags, wait_epoch, status, rpb);
+}
+
+extern "C" int ds41_quotient(const float* v, const float* s, float* q, long long n, void* stream) {
+  if (v == nullptr || s == nullptr || q == nullptr || n <= 0) return cudaErrorInvalidValue;
+  const long long blocks = (n + 255) / 256;
+  quotient_kernel<<<static_cast<unsigned>(blocks < 1024 ? blocks : 1024), 256, 0, static_cast<cudaStream_t>(stream)>>>(v, s, q, n);
+  return cudaGetLastError();
 }
 
 extern "C" int ds41_hc_finish(const float* partial, int n_slices, const float* scale, const float* base,

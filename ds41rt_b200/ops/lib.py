@@ -129,7 +129,7 @@ def dir_functions():
         "ds41_gemm_tc", "ds41_embed_streams", "ds41_hc_post_mix", "ds41_hc_finish", "ds41_qkv_post",
         "ds41_compress", "ds41_index_score", "ds41_topk_select", "ds41_attend", "ds41_router_select",
         "ds41_moe_plan", "ds41_moe_combine", "ds41_signal", "ds41_signal_all", "ds41_moe_combine_signal", "ds41_reduce_planes", "ds41_reduce_groups", "ds41_argmax_rows",
-        "ds41_argmax_merge", "ds41_spec_accept", "ds41_act_quant_mx", "ds41_decode_feedback", "ds41_step_inputs", "ds41_step_result", "ds41_graph_step", "ds41_hc_step", "ds41_taps_pack", "ds41_norm_rows", "ds41_markov_step", "ds41_dspark_confidence", "ds41_spec_feedback",
+        "ds41_argmax_merge", "ds41_spec_accept", "ds41_act_quant_mx", "ds41_decode_feedback", "ds41_step_inputs", "ds41_step_result", "ds41_graph_step", "ds41_hc_step", "ds41_quotient", "ds41_taps_pack", "ds41_norm_rows", "ds41_markov_step", "ds41_dspark_confidence", "ds41_spec_feedback",
         "ds41_copy_ints", "ds41_rs_reduce", "ds41_ep_count", "ds41_ep_plan", "ds41_ep_dispatch", "ds41_ep_mark",
         "ds41_ep_wait", "ds41_ep_combine", "ds41_act_quant_mx_rows", "ds41_act_quant_mx_tiles", "ds41_act_quant_nvfp4_tiles", "ds41_sample_rows", "ds41_engram_dequant", "ds41_engram_gate", "ds41_vis_rmsnorm", "ds41_vis_bias_act", "ds41_vis_silu_mul",
         "ds41_index_prepare", "ds41_candidate_select", "ds41_pp_signal", "ds41_pp_wait", "ds41_pp_pull", "ds41_attend_floor", "ds41_attend_kv", "ds41_index_score_cand", "ds41_topk_select_cand", "ds41_act_quant_nvfp4_rows", "ds41_vis_rope2d", "ds41_vis_softmax", "ds41_vis_merge", "ds41_vis_scatter",

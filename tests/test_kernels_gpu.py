@@ -441,6 +441,29 @@ def test_index_scores_by_tiles(rows, n_keys, static, bn):
         assert ((got[:, :n_keys].double() - want).abs() <= bound)[sees].all()
 
 
+@pytest.mark.parametrize("bn", [32, 64, 128, 256])
+def test_index_scores_of_eight_bit_operands(bn):
+    """E4M3 queries and keys: products are exact, sums as in the bf16 form."""
+    from ds41rt_b200.ops import gemm as G, lib
+    IH, ID, rows, n_keys, ld = 32, 128, 37, 300, 512
+    torch.manual_seed(bn)
+    q = (torch.randn(rows * IH, ID, device="cuda") * 4).to(torch.float8_e4m3fn)
+    keys = (torch.randn(n_keys, ID, device="cuda") * 4).to(torch.float8_e4m3fn)
+    w, limit = torch.randn(rows, IH, device="cuda"), torch.randint(0, n_keys + 20, (rows,), device="cuda", dtype=torch.int32)
+    limit[8:20] = 0
+    got, st = torch.full((rows, ld), float("nan"), device="cuda"), lib.new_status("cuda")
+    G.gemm_raw(q, keys, got, rows * IH, n_keys, ID, lda=ID, ldb=ID, ldo=ld, kind=1, out_mode=8, bn=bn, row_w=w, row_w_ld=IH,
+               col_limit=limit, status=st)
+    torch.cuda.synchronize()
+    lib.raise_on_status(st, "index gemm")
+    qh = q.double().view(rows, IH, ID)
+    want = torch.einsum("rh,rhk->rk", w.double(), (qh @ keys.double().T).relu())
+    bound = torch.einsum("rh,rhk->rk", w.double().abs(), qh.abs() @ keys.double().abs().T) * (ID + IH + 2) * 2.0 ** -23
+    sees = torch.arange(n_keys, device="cuda")[None] < limit[:, None]
+    assert torch.isneginf(got[:, :n_keys][~sees]).all() and got[:, n_keys:].isnan().all()
+    assert ((got[:, :n_keys].double() - want).abs() <= bound)[sees].all()
+
+
 def test_fp4_index_keys_and_queries_follow_the_quantisation_oracle():
     """Index keys stored as FP4 rows (E2M1 pairs + UE8M0 per 32 values, 68 bytes for 128 values): the per-key kernel and
     the tensor-core path both score the dequantised keys against queries quantised the same way; the per-key kernel
@@ -1046,3 +1069,63 @@ def test_combine_of_routes_and_shared_planes(rows, topk, splits):
         for s in range(splits):
             want[r] += shared[s, r]
     assert torch.equal(out, want)
+
+
+def test_quotient_against_the_division_operator():
+    """v / s of the hyper-connection mixes over the pairs that they can meet and far beyond: the bits of the operator, which rounds
+    correctly.  Zeros, powers of two and significands next to the end among them."""
+    from ds41rt_b200.ops import lib
+    n = 1 << 24
+    g = torch.Generator(device="cuda").manual_seed(1)
+    bits = lambda lo, hi: ((torch.randint(lo + 127, hi + 127, (n,), generator=g, device="cuda") << 23) |
+                           torch.randint(0, 1 << 23, (n,), generator=g, device="cuda")).int()
+    for v_range, s_range in (((-30, 1), (-20, 3)), ((0, 1), (0, 1)), ((-60, 60), (-60, 60))):
+        v, s = bits(*v_range), bits(*s_range)
+        v[::7] |= (1 << 23) - 1
+        s[::11] |= (1 << 23) - 1
+        s[5::11] &= ~((1 << 23) - 1)
+        v, s = v.view(torch.float32), s.view(torch.float32)
+        v[:8] = 0.0
+        q = torch.full((n,), float("nan"), device="cuda")
+        lib.check(lib.kernels().ds41_quotient(lib.ptr(v), lib.ptr(s), lib.ptr(q), C.c_longlong(n), lib.stream()), "quotient")
+        assert torch.equal(q, v / s)
+        assert float((q.double() * s.double() / v.double() - 1)[8:].abs().max()) <= 2.0 ** -24 * (1 + 2.0 ** -20)
+
+
+@pytest.mark.parametrize("form", ["finish", "mixes"])
+@pytest.mark.parametrize("spread", [0.5, 4.0, 12.0])
+@pytest.mark.parametrize("iters", [1, 2, 20])
+def test_mixes_against_64_bits(iters, spread, form):
+    """The 4 x 4 matrix of every row.  A step divides a positive matrix by its row or column sums: in the logarithm of the ratios of
+    its entries no step carries an error further than it found it, and each adds its own roundings (three additions, the
+    divisor's, the quotient's and those of eps: 6 x 2^-24).  The exponentials are off by 2 units, and by their argument's
+    rounding, |x| x 2^-23.  An entry is off by at most twice the largest of all that."""
+    from ds41rt_b200.ops import lib
+    k, rows, H, eps = lib.kernels(), 1000, 1024, 1e-6
+    g = torch.Generator().manual_seed(iters)
+    z = torch.randn(rows, 24, generator=g) * spread
+    part = torch.zeros(1, rows, 25)
+    part[0, :, :24], part[0, :, 24] = z, 4.0 * H                        # a row of unit size: its projections stand as they are
+    part, planes = part.cuda(), torch.cat([z, torch.zeros(rows, 24)], 1).contiguous().cuda()
+    scale, base = torch.ones(3).cuda(), torch.zeros(24).cuda()
+    streams, pre_in = torch.randn(rows, 4, H, device="cuda").bfloat16(), torch.rand(rows, 4, device="cuda")
+    pre, post, comb = torch.zeros(rows, 4).cuda(), torch.zeros(rows, 4).cuda(), torch.zeros(rows, 16).cuda()
+    xn = torch.zeros(rows, H, device="cuda").bfloat16()
+    finish = form == "finish"
+    lib.check(k.ds41_hc_finish(lib.ptr(part), 1, lib.ptr(scale), lib.ptr(base), lib.ptr(pre_in), lib.ptr(streams), lib.ptr(None),
+                               lib.ptr(pre), lib.ptr(post), lib.ptr(comb), lib.ptr(xn if finish else None), lib.ptr(None),
+                               lib.ptr(None), lib.ptr(None), rows, H, iters, C.c_float(eps), C.c_float(0.0),
+                               lib.ptr(None if finish else planes), 0 if finish else 1, C.c_longlong(rows * 48), 48, lib.stream()),
+              "mixes")
+    x = z[:, 8:].double().view(rows, 4, 4)
+    want = torch.softmax(x, 2) + eps
+    want = want / (want.sum(1, keepdim=True) + eps)
+    for _ in range(iters - 1):
+        want = want / (want.sum(2, keepdim=True) + eps)
+        want = want / (want.sum(1, keepdim=True) + eps)
+    reach = float((x.amax(2, keepdim=True) - x).max())
+    bound = 2 * ((2 + 2 * reach) * 2.0 ** -23 + 2 * iters * 6 * 2.0 ** -24)
+    off = float((comb.cpu().double().view(rows, 4, 4) / want - 1).abs().max())
+    assert off <= bound
+    assert float((pre.cpu().double() - (torch.sigmoid(z[:, :4].double()) + eps)).abs().max()) < 1e-5
+    assert float((post.cpu().double() - 2 * torch.sigmoid(z[:, 4:8].double())).abs().max()) < 1e-5

@@ -182,3 +182,40 @@ def test_first_steps_leave_other_rows_alone(length, experts, kv):
     flat = lambda c: [c[0], *c[1], *c[2], *c[3]]
     for a, b in zip(flat(caches), flat(there)):
         assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("model", ["genesun-tiny", "belasun-tiny", "flash"])
+def test_device_loop_without_graphs(model):
+    """Steps whose tokens and positions are fed on the device, launched one by one far ahead of the GPU, against captured ones."""
+    from ds41rt_b200.runtime.session import DecodeSession
+    dev, n, steps = torch.device("cuda", 0), 3, 20
+    if model == "flash":
+        from ds41rt_b200.config import ModelConfig
+        from ds41rt_b200.models.ds41 import DS41Engine, EngineWeights
+        cfg = ModelConfig.tiny()
+        w = EngineWeights.random(cfg, 0, 1, dev, seed=3)
+        make = lambda: DS41Engine(cfg, w, max_rows=24, slots=n, max_ctx=256)
+    else:
+        from ds41rt_b200.models import registry
+        fam, cfg = registry.preset(model)
+        torch.manual_seed(2)
+        w = fam.random_weights(cfg, dev)
+        make = lambda: fam.engine(cfg, w, max_rows=24, slots=n, max_ctx=256)
+    prompts = torch.randint(3, cfg.vocab, (n, 60), generator=torch.Generator().manual_seed(4))
+    got = []
+    for graphs in (True, False):
+        e = make()
+        session, last = DecodeSession(e, use_graphs=graphs), []
+        for s in range(n):
+            assert e.cache.ensure(s, 120)
+            last.append(e.prefill(s, prompts[s, :40 + 10 * s].tolist(), chunk=20))
+        e.set_rows(last, [40 + 10 * s for s in range(n)], list(range(n)))
+        torch.cuda.synchronize()
+        torch.cuda._sleep(20_000_000)                  # the launches are queued before the first one runs
+        session.run_device_loop(n, steps)
+        torch.cuda.synchronize()
+        e.check_status()
+        assert e.row_pos[:n].tolist() == [40 + 10 * s + steps for s in range(n)]
+        got.append((e.in_tokens[:n].clone(), e.logits_rows(n).clone()))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
