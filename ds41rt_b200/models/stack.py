@@ -710,9 +710,9 @@ class StackEngine(RowsEngine):
     # ------------------------------------------------------------------ helpers
     def attn_splits(self, rows: int, heads: int) -> int:
         """Key splits per row of the absorbed attention: enough blocks to fill the GPU about twice, static per batch
-        size (a captured pass replays while the context grows).  At most 32: the splits are the order in which a row's
-        keys are summed, and 66 of them (one tile of 64 keys each, 4097 keys of 16 heads in 9.7 us rather than 18.0) gave other
-        results than the model had before."""
+        size (a captured pass replays while the context grows).  At most 32: one row of 16 heads over 4097 keys takes 10.8 us and
+        4.1 for the merge with those, together 15.0; 66 of one tile of 64 keys each would take 5.4 and 7.2, together 13.4, and
+        change the order in which a row's keys are summed."""
         want = 2 * 148 // (rows * -(-heads // 32))
         return max(1, min(want, 32, -(-self.cache.max_ctx // 64)))
 
