@@ -483,6 +483,8 @@ __global__ void __launch_bounds__(128) group_attend_plain_kernel(ds41_group_atte
 // of them; four, and two CTAs share an SM, where there are more CTAs than SMs (or the value width takes the registers).
 // Asking L2 for the first tiles' rows before the wait for the previous kernel was slower, with rows in L2 and from memory: 4 rows of 32 heads
 // (8 kv) over 4097 keys, 4 splits 14.2 and 15.6 us, 17.1 and 18.3 with it; 32 rows of 8 heads, 8 splits 136 and 146, 157 and 164.
+// One tile, in grids that run at once, is within what the buffers' places do to a step of belasun-1b: 8 rows 1100 and 1103 us with eight
+// tiles, 1088 and 1094 with one, 1095 with none; 3 rows 849 and 834 us, 831 and 846, 839.
 constexpr int kMaxStages = 4;
 
 struct AttendPlan {
